@@ -18,6 +18,7 @@
 
 #include "kernels.h"
 #include "reg_fft.cuh"
+#include "tf_fft.cuh"
 
 namespace simrecon {
 
@@ -335,6 +336,56 @@ bool get_fft_plan(int n, FFTPlan* plan)
   p.tw = d;
   p.twr = P ? d + n : nullptr;
   g_plans[{dev, n}] = p;
+  *plan = p;
+  return true;
+}
+
+namespace {
+std::map<std::pair<int, int>, TfPlan> g_tf_plans;
+}  // namespace
+
+bool tf_factor(int n, int* r1, int* r2)
+{
+  for (int a : kTfSizes)
+    if (n % a == 0 && n / a <= a)
+      for (int b : kTfSizes)
+        if (b == n / a) {
+          *r1 = a;
+          *r2 = b;
+          return true;
+        }
+  return false;
+}
+
+bool get_tf_plan(int n, TfPlan* plan)
+{
+  TfPlan p{};
+  p.n = n;
+  if (!tf_factor(n, &p.r1, &p.r2)) return false;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(g_mu);
+  auto it = g_tf_plans.find({dev, n});
+  if (it != g_tf_plans.end()) {
+    *plan = it->second;
+    return true;
+  }
+  std::vector<float2> tw(2 * (size_t)n);
+  for (int k1 = 0; k1 < p.r1; ++k1)
+    for (int j = 0; j < p.r2; ++j)
+      for (int h = 0; h < 2; ++h) {
+        const double a = -M_PI * (double)(2 * j * k1 + h * j) / (double)n;
+        tw[(size_t)h * n + (size_t)k1 * p.r2 + j] = make_float2((float)cos(a), (float)sin(a));
+      }
+  float2* d = nullptr;
+  if (cudaMalloc(&d, sizeof(float2) * tw.size()) != cudaSuccess) return false;
+  if (cudaMemcpy(d, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaFree(d);
+    return false;
+  }
+  p.tw = d;
+  p.twh = d + n;
+  g_tf_plans[{dev, n}] = p;
   *plan = p;
   return true;
 }

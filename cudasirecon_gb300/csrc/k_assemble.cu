@@ -22,10 +22,11 @@
 #include <cmath>
 #include <vector>
 
+#include "assemble.h"
 #include "col_fft.cuh"
+#include "filter.cuh"
 #include "kernels.h"
 #include "reg_fft.cuh"
-#include "thresholds.h"
 
 namespace simrecon {
 
@@ -33,143 +34,6 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kMaxElems = kFftElems;
-
-__device__ __forceinline__ float dev_suppress(float x)
-{
-  float x6 = x * x * x;
-  x6 *= x6;
-  return 1.f / (1 + 20000 / (x6 + 20));  // float division: correctly rounded, like the double one rounded
-}
-
-// Per-launch constants derived on the host from FilterArgs (reciprocals and
-// products the per-term arithmetic would otherwise recompute per element).
-struct FilterK {
-  float rnv[kMaxDirs * kMaxOrders];    // 1 / noisevar
-  float kxo[kMaxDirs * kMaxOrders];    // order * k0x of each direction
-  float kyo[kMaxDirs * kMaxOrders];
-  float rdkrotf;                       // 1 / dkrotf
-  float min_dkr, rmin_dkr, supp_r;     // suppression radius (1/um) and its unit
-  float rrcut;                         // 1 / rdistcutoff
-  // exact squared-radius forms of the reference's float-radius decisions
-  // (sqrtf is correctly rounded and monotonic): sqrtf(r2) < rdistcutoff
-  // <=> r2 < r2_in, sqrtf(r2) <= suppRadius <=> r2 <= r2_supp
-  float r2_in, r2_supp;
-  float rapo, rzapo;                   // 1 / apocutoff, 1 / zapocutoff
-  // every direction's order-0 noise factor is the same (the reference's are
-  // all 1): the order-0 Wiener denominator is then one sum for all directions
-  int order0_shared;
-};
-
-
-// Wiener scale of pixel (x1f, y1f, z0) of band (dir, order): the body of
-// filterbands_kernel1 (gpuFunctionsImpl.cu:1504-1592) without the final
-// conjamp factor.  ND/NO: compile-time direction and order counts (0: use
-// the runtime values).
-// OTF value of order o at radial index krindex in the plane's kz: from the
-// plane's radial table (TAB; its entries are the kz interpolation of the
-// bilinear lookup, so the result is the same interpolation), else the
-// bilinear lookup itself
-template <bool CLAMP, bool TAB>
-__device__ __forceinline__ float2 filter_otf(const FilterArgs& a, const float2* tabz, int o, float krindex,
-                                             const OtfKz& kzi)
-{
-  if (TAB) {
-    const float2* T = tabz + o * a.otf.nxotf;
-    const int ir = (int)floorf(krindex);
-    const float ar = krindex - ir;
-    const float2 t0 = T[ir], t1 = T[ir + 1];
-    return make_float2((1 - ar) * t0.x + ar * t1.x, (1 - ar) * t0.y + ar * t1.y);
-  }
-  return otf_lookup_rr<CLAMP>(a.otf.otf[o], a.otf, krindex, kzi);
-}
-
-// FL >= 0: the suppress (bit 0), dampen-order-0 (bit 1) and filter-overlaps
-// (bit 2) switches fixed at compile time; FL < 0: read from the arguments.
-// termw: |amp|^2 / noisevar of every (direction, order) (FitDev::termw, in
-// registers on the compile-time paths); ampmag2: |amp|^2 of this band.
-template <int ND, int NO, bool CLAMP, bool TAB, int FL>
-__device__ __forceinline__ float2 filter_scale(const FilterArgs& a, const FilterK& k, const float* termw,
-                                               float ampmag2, int dir, int order, int z0, float rdist1, float x1f,
-                                               float y1f, const float2* tabz)
-{
-  const bool suppress = FL >= 0 ? (FL & 1) != 0 : a.suppress != 0;
-  const bool dampen0 = FL >= 0 ? (FL & 2) != 0 : a.dampen0 != 0;
-  const bool filteroverlaps = FL >= 0 ? (FL & 4) != 0 : a.filteroverlaps != 0;
-  const int nd = ND ? ND : a.ndirs, no = NO ? NO : a.norders;
-  const float xabs = x1f + k.kxo[dir * no + order], yabs = y1f + k.kyo[dir * no + order];
-  const OtfKz kzi = otf_kz(a.otf, z0);
-  // order-0 damping's axial part |z0 / zdc0|^3, the same for every term
-  const float zf = fabsf(z0 / (float)a.zdc[0]);
-  const float zf3 = zf * zf * zf;
-  float2 otf1 = filter_otf<CLAMP, TAB>(a, tabz, order, rdist1 * k.rdkrotf, kzi);
-  float weight = otf1.x * otf1.x + otf1.y * otf1.y;
-  if (order != 0) weight *= ampmag2;
-  float dampfact = k.rnv[dir * no + order];
-  if (suppress && order != 0 && rdist1 <= k.supp_r)
-    dampfact *= dev_suppress(rdist1 * k.rmin_dkr);
-  else if (!dampen0 && suppress && order == 0 && rdist1 <= k.supp_r)
-    dampfact *= dev_suppress(rdist1 * k.rmin_dkr);
-  else if (dampen0 && order == 0) {
-    const float rf = rdist1 * k.rrcut;
-    dampfact *= rf * rf + zf3;
-  }
-  if (order == 0 && z0 == 0 && a.nokz0) dampfact = 0;
-  weight *= dampfact;
-  float sumweight = weight;
-#pragma unroll
-  for (int dir2 = 0; dir2 < nd; dir2++) {
-#pragma unroll
-    for (int order2 = -(no - 1); order2 < no; order2++) {
-      if (dir2 == dir && order2 == order) continue;
-      if (!filteroverlaps && !(order2 == 0 && order == 0)) continue;
-      const int ao2 = order2 < 0 ? -order2 : order2;
-      const float sx = order2 < 0 ? -k.kxo[dir2 * no + ao2] : k.kxo[dir2 * no + ao2];
-      const float sy = order2 < 0 ? -k.kyo[dir2 * no + ao2] : k.kyo[dir2 * no + ao2];
-      const float x2 = xabs - sx, y2 = yabs - sy;
-      const float r2 = x2 * x2 + y2 * y2;
-      if (r2 < k.r2_in) {  // rdist2 < rdistcutoff
-        const float rdist2 = sqrt_approx(r2);
-        const float2 otf2 = filter_otf<CLAMP, TAB>(a, tabz, ao2, rdist2 * k.rdkrotf, kzi);
-        float w = (otf2.x * otf2.x + otf2.y * otf2.y) * termw[dir2 * no + ao2];
-        if (suppress && order2 != 0 && r2 <= k.r2_supp)
-          w *= dev_suppress(rdist2 * k.rmin_dkr);
-        else if (!dampen0 && suppress && order2 == 0 && r2 <= k.r2_supp)
-          w *= dev_suppress(rdist2 * k.rmin_dkr);
-        else if (dampen0 && order2 == 0) {
-          const float rf = rdist2 * k.rrcut;
-          w *= rf * rf + zf3;
-        }
-        if (a.nokz0 && order2 == 0 && z0 == 0) w = 0.0f;
-        sumweight += w;
-      }
-    }
-  }
-  sumweight += a.wiener2;
-  const float f = dampfact / sumweight;
-  float2 scale = make_float2(otf1.x * f, -otf1.y * f);
-  if (a.apodizeoutput) {
-    float rdistabs = sqrtf(xabs * xabs + yabs * yabs);
-    float rho;
-    float zdistabs = abs(z0);
-    const float ra = rdistabs * k.rapo;
-    if (a.zapocutoff > 0 && a.bessel) {  // gpuFunctionsImpl.cu:1572-1577
-      const float rhox = xabs * k.rrcut, rhoy = yabs * k.rapo, rhoz = zdistabs * k.rzapo;
-      rho = sqrtf(rhox * rhox + rhoy * rhoy + rhoz * rhoz);
-    } else if (a.zapocutoff > 0) {
-      const float rz = zdistabs * k.rzapo;
-      rho = sqrtf(ra * ra + rz * rz);
-    } else {
-      rho = ra;
-    }
-    if (rho > 1.f) rho = 1.0f;
-    float apofact = 1.f;
-    if (a.apodizeoutput == 1) apofact = cosf(1.57079632679f * rho);
-    else if (a.apodizeoutput == 2) apofact = 1.0f - rho;
-    scale.x *= apofact;
-    scale.y *= apofact;
-  }
-  return scale;
-}
 
 // split re/im into plus/minus, scale plus, recombine (gpuFunctionsImpl.cu:1617-1644)
 __device__ __forceinline__ void apply_side(float2& re, float2& im, float2 scale, bool conj)
@@ -189,13 +53,12 @@ __device__ __forceinline__ void apply_side(float2& re, float2& im, float2 scale,
   }
 }
 
-// TAB: the block (one kz plane) first builds, in shared memory, each order's
-// OTF interpolated to this plane's kz (+z0) and to the conjugate pass's kz
-// (-z0) along kr: [2][NO][nxotf]; only where no lookup can leave the table
+// TAB: the block (one kz plane) first builds its radial tables in shared
+// memory; only where no lookup can leave the table
 template <int ND, int NO, bool CLAMP, bool TAB, int FL = -1>
 __global__ void __launch_bounds__(kThreads) k_filter(const __grid_constant__ FilterArgs a, const __grid_constant__ FilterK k)
 {
-  extern __shared__ float2 tab[];
+  extern __shared__ float4 tab[];
   const int nx = a.nx, ny = a.ny, nz = a.nz, nxh = nx / 2 + 1;
   const int order = blockIdx.z, iz = blockIdx.y;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -203,17 +66,7 @@ __global__ void __launch_bounds__(kThreads) k_filter(const __grid_constant__ Fil
   const bool inband = (iz <= zdc) || (iz >= nz - zdc);
   if (TAB) {
     static_assert(!TAB || NO > 0, "the table needs the order count at compile time");
-    const int nxo = a.otf.nxotf, nzo = a.otf.nzotf;
-    if (inband) {
-      const int zp = iz <= zdc ? iz : iz - nz;
-      for (int t = threadIdx.x; t < 2 * NO * nxo; t += blockDim.x) {
-        const int pass = t / (NO * nxo), r = t - pass * NO * nxo, o = r / nxo, ir = r - o * nxo;
-        const OtfKz kz = otf_kz(a.otf, pass ? -zp : zp);
-        const float2 va = __ldg(a.otf.otf[o] + ir * nzo + kz.iz), vb = __ldg(a.otf.otf[o] + ir * nzo + kz.izp);
-        const float az = kz.az;
-        tab[t] = make_float2(va.x * (1 - az) + vb.x * az, va.y * (1 - az) + vb.y * az);
-      }
-    }
+    if (inband) build_filter_tab(a, NO, iz <= zdc ? iz : iz - nz, tab);
     __syncthreads();
   }
   if (e >= ny * nxh) return;
@@ -272,14 +125,6 @@ __global__ void __launch_bounds__(kThreads) k_filter(const __grid_constant__ Fil
     body(a.fit->termw);
   }
 }
-
-// One transformed plane: band (dir, order) at signed kz, summed into output
-// plane zout.  dir < 0 marks the order-0 slot of a plane: the order-0 bands
-// of all directions summed before the transforms (their phase ramps are all
-// 1, so the sum commutes with the inverse FFTs).
-struct Slot {
-  int dir, order, kz, zout;
-};
 
 // zero-padded inverse FFT along y of the in-band plane kz of band (d, o);
 // columns c = kx + nx/2 - 1, kx in [-nx/2+1, nx/2] (move_kernel ranges,
@@ -522,8 +367,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const S
   constexpr int R2 = CF::R2;
   static_assert(R2 * W <= kThreads, "one stage-1 item per thread");
   static_assert(Y * W <= CF::kSmemElems, "phase A fits the transform buffer");
-  extern __shared__ float2 sm[];
-  float2* tab = sm + CF::kSmemElems;  // [2][NO][nxotf]
+  extern __shared__ __align__(16) float2 sm[];
+  float4* tab = (float4*)(sm + CF::kSmemElems);  // [2][NO][nxotf]
   const Slot sl = slots[blockIdx.y];
   const int nx = a.nx, ny = a.ny, nz = a.nz, nxh = nx / 2 + 1;
   const int c0 = blockIdx.x * W;
@@ -534,15 +379,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const S
   const float2* bi = order == 0 ? nullptr : a.bands + ((size_t)d0 * a.nphases + 2 * order) * nz * plane;
   const size_t dstride = (size_t)a.nphases * nz * plane;  // next direction's band 0
   const int ylo = ny / 2 - 1;                              // ky in [-ylo, ny/2]
-  {  // OTF of every order interpolated to kz (pass 0) and -kz (pass 1) along kr
-    const int nxo = fa.otf.nxotf, nzo = fa.otf.nzotf;
-    for (int t = threadIdx.x; t < 2 * NO * nxo; t += blockDim.x) {
-      const int pass = t / (NO * nxo), r = t - pass * NO * nxo, o = r / nxo, ir = r - o * nxo;
-      const OtfKz kz = otf_kz(fa.otf, pass ? -sl.kz : sl.kz);
-      const float2 va = __ldg(fa.otf.otf[o] + ir * nzo + kz.iz), vb = __ldg(fa.otf.otf[o] + ir * nzo + kz.izp);
-      tab[t] = make_float2(va.x * (1 - kz.az) + vb.x * kz.az, va.y * (1 - kz.az) + vb.y * kz.az);
-    }
-  }
+  build_filter_tab(fa, NO, sl.kz, tab);
   float termw[ND * NO];
 #pragma unroll
   for (int i = 0; i < ND * NO; ++i) termw[i] = __ldg(fa.fit->termw + i);
@@ -583,7 +420,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const S
           const float xs = conj ? -x1f : x1f;
           const float ys = conj ? (float)(-ky) * fa.dky : y1f;
           const int zs = conj ? -sl.kz : sl.kz;
-          const float2* tz = tab + (conj ? NO * fa.otf.nxotf : 0);
+          const float4* tz = tab + (conj ? NO * fa.otf.nxotf : 0);
           if (fk.order0_shared) {
             // one denominator for every direction: direction d's own term and
             // the (d, 0) term its sum skips are the same OTF value
@@ -764,10 +601,14 @@ __global__ void __launch_bounds__(kXwWarps * 32, 2) k_asm_xw(AssembleArgs a, con
   }
 }
 
+// where output column x of a row of S is: the doubled-grid x pass stores the
+// even columns, then the odd ones
+__device__ __forceinline__ int s_column(int x, int X, int split) { return split ? (x & 1) * (X >> 1) + (x >> 1) : x; }
+
 // inverse FFT along z of S, real part -> out
 template <int NF>
 __global__ void __launch_bounds__(kThreads) k_asm_z(AssembleArgs a, const unsigned char* __restrict__ zactive,
-                                                    FFTPlan plan, int W)
+                                                    FFTPlan plan, int W, int split)
 {
   extern __shared__ float2 sm[];
   const int X = a.X, Y = a.Y, Z = a.Z;
@@ -775,7 +616,8 @@ __global__ void __launch_bounds__(kThreads) k_asm_z(AssembleArgs a, const unsign
   const int ld = W + 1;
   for (int t = threadIdx.x; t < Z * W; t += blockDim.x) {
     int z = t / W, w = t - z * W;
-    sm[z * ld + w] = (zactive[z] && c0 + w < X) ? a.S[((size_t)z * Y + yr) * X + c0 + w] : make_float2(0.f, 0.f);
+    sm[z * ld + w] = (zactive[z] && c0 + w < X) ? a.S[((size_t)z * Y + yr) * X + s_column(c0 + w, X, split)]
+                                                : make_float2(0.f, 0.f);
   }
   __syncthreads();
   const float2* res = fft_dispatch<NF, +1>(sm, sm + Z * ld, plan, W, 1, ld);
@@ -805,7 +647,7 @@ __global__ void __launch_bounds__(kThreads) k_asm_z1(const float4* __restrict__ 
 // k1 + R1 k2.
 template <int R1>
 __global__ void __launch_bounds__(kThreads) k_asm_z4(AssembleArgs a, const unsigned char* __restrict__ zactive,
-                                                    const float2* __restrict__ tw)
+                                                    const float2* __restrict__ tw, int split)
 {
   constexpr int R2 = 16, W = 64;
   constexpr int LD = R2 * W + 8;
@@ -814,14 +656,14 @@ __global__ void __launch_bounds__(kThreads) k_asm_z4(AssembleArgs a, const unsig
   const int yr = blockIdx.y, c0 = blockIdx.x * W;
   const int nc = min(W, X - c0);
   const size_t zstride = (size_t)Y * X;
-  const float2* src = a.S + (size_t)yr * X + c0;
+  const float2* src = a.S + (size_t)yr * X;
   for (int it = threadIdx.x; it < R2 * W; it += blockDim.x) {
-    const int c = it % W, j = it / W;
+    const int c = it % W, j = it / W, cs = s_column(c0 + c, X, split);
     float2 v[R1];
 #pragma unroll
     for (int e = 0; e < R1; ++e) {
       const int z = j + R2 * e;
-      v[e] = (c < nc && zactive[z]) ? src[z * zstride + c] : make_float2(0.f, 0.f);
+      v[e] = (c < nc && zactive[z]) ? src[z * zstride + cs] : make_float2(0.f, 0.f);
     }
     reg_dft<R1, +1>(v);
 #pragma unroll
@@ -848,7 +690,7 @@ __global__ void __launch_bounds__(kThreads) k_asm_z4(AssembleArgs a, const unsig
 }
 
 __global__ void k_ramp(const __grid_constant__ K0List k0, int ndirs, int norders, int X, int Y, float dxyz, float fact,
-                       float2* ex, float2* ey)
+                       float2* ex, float2* ey, int split)
 {
   int n = ndirs * norders * (X + Y);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
@@ -861,7 +703,7 @@ __global__ void k_ramp(const __grid_constant__ K0List k0, int ndirs, int norders
     double s, c;
     sincos(ang, &s, &c);
     float2 v = make_float2((float)c, (float)s);
-    if (r < X) ex[(size_t)ro * X + r] = v;
+    if (r < X) ex[(size_t)ro * X + s_column(r, X, split)] = v;
     else ey[(size_t)ro * Y + (r - X)] = v;
   }
 }
@@ -934,51 +776,6 @@ DevTables dev_tables(const AssembleArgs& a, const HostTables& t)
 
 }  // namespace
 
-namespace {
-FilterK make_filter_k(const FilterArgs& a)
-{
-  FilterK k{};
-  const int no = a.norders;
-  for (int d = 0; d < a.ndirs; ++d)
-    for (int o = 0; o < no; ++o) {
-      const int i = d * no + o;
-      k.rnv[i] = 1.f / a.noisevar[i];
-      k.kxo[i] = o * a.k0[d].x;
-      k.kyo[i] = o * a.k0[d].y;
-    }
-  k.rdkrotf = 1.f / a.otf.dkrotf;
-  k.min_dkr = a.dkx < a.dky ? a.dkx : a.dky;
-  k.rmin_dkr = 1.f / k.min_dkr;
-  k.supp_r = a.supp_radius * k.min_dkr;
-  k.rrcut = 1.f / a.rdistcutoff;
-  k.r2_in = r2_below(a.rdistcutoff);
-  k.r2_supp = r2_atmost(k.supp_r);
-  k.rapo = 1.f / a.apocutoff;
-  k.rzapo = a.zapocutoff > 0 ? 1.f / a.zapocutoff : 0.f;
-  k.order0_shared = 1;
-  for (int d = 1; d < a.ndirs; ++d)
-    if (a.noisevar[d * no] != a.noisevar[0]) k.order0_shared = 0;
-  return k;
-}
-
-// Every looked-up radius is <= rdistcutoff, so the table is never left when
-// floor(rdistcutoff / dkrotf) + 3 <= nxotf (+ 3: a cross term's interpolation
-// radius comes from an approximate square root and may pass rdistcutoff by
-// an ulp) and no kz index, |kz| <= nz/2, leaves it along kz; otherwise the
-// lookups clamp
-bool filter_needs_clamp(const FilterArgs& a, const FilterK& k)
-{
-  return !(std::floor(a.rdistcutoff * k.rdkrotf) + 3 <= a.otf.nxotf) ||
-         !(a.nz == 1 || (a.nz / 2) * (double)a.otf.kzscale + 1.0 < a.otf.nzotf);
-}
-
-// the switches fixed at compile time on the table path
-int filter_flags(const FilterArgs& a)
-{
-  return (a.suppress ? 1 : 0) | (a.dampen0 ? 2 : 0) | (a.filteroverlaps ? 4 : 0);
-}
-}  // namespace
-
 int launch_filter(const FilterArgs& a, cudaStream_t s, long long* launches)
 {
   const int nxh = a.nx / 2 + 1;
@@ -989,13 +786,16 @@ int launch_filter(const FilterArgs& a, cudaStream_t s, long long* launches)
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
   // per-plane radial tables when the lookups stay inside the table and the
-  // tables fit in 48 KB of shared memory
-  const size_t tabb = 2 * (size_t)no * a.otf.nxotf * sizeof(float2);
-  const bool tab = !clamp && tabb <= 48 * 1024;
+  // tables fit in 96 KB of shared memory
+  const size_t tabb = 2 * (size_t)no * a.otf.nxotf * sizeof(float4);
+  const bool tab = !clamp && tabb <= 96 * 1024;
   // the table path with the three switches fixed at compile time
   const int fl = filter_flags(a);
   auto tab_path = [&]<int NO>() {
-    auto go = [&]<int FL>() { k_filter<3, NO, false, true, FL><<<g, kThreads, tabb, s>>>(a, k); };
+    auto go = [&]<int FL>() {
+      allow_dynamic_smem((const void*)k_filter<3, NO, false, true, FL>, tabb);
+      k_filter<3, NO, false, true, FL><<<g, kThreads, tabb, s>>>(a, k);
+    };
     switch (fl) {
       case 0: go.template operator()<0>(); break;
       case 1: go.template operator()<1>(); break;
@@ -1028,12 +828,26 @@ int launch_filter(const FilterArgs& a, cudaStream_t s, long long* launches)
   return (int)cudaGetLastError();
 }
 
-int launch_ramp_tables(const K0List& k0, int ndirs, int norders, int X, int Y, float dxyz, float fact, float2* ex,
-                       float2* ey, cudaStream_t s, long long* launches)
+namespace {
+// Doubled grids take the half-length transforms of k_assemble2.cu, except
+// where a compiled doubled-length kernel is the faster one: per 512^2 x 48
+// volume the y pass takes 1.31 ms (k_asm_y4f) against 1.45, the x pass
+// 0.56 ms (k_asm_xw) against 0.87; per 256^2 x 32 volume 0.254 / 0.256 and
+// 0.096 / 0.102 ms
+bool use_y2(const AssembleArgs& a) { return !colfft_r1(a.Y) && asm_y2_supported(a); }
+bool use_x2(const AssembleArgs& a)
 {
+  return !(a.X == 2 * a.nx && (a.X == 1024 || a.X == 512 || a.X == 256)) && asm_x2_supported(a);
+}
+}  // namespace
+
+int launch_ramp_tables(const K0List& k0, const AssembleArgs& a, float dxyz, float fact, float2* ex, float2* ey,
+                       cudaStream_t s, long long* launches)
+{
+  const int ndirs = a.ndirs, norders = a.norders, X = a.X, Y = a.Y;
   if (ndirs < 1 || ndirs > kMaxDirs) return -1;
   int n = ndirs * norders * (X + Y);
-  k_ramp<<<std::min(1024, (n + 255) / 256), 256, 0, s>>>(k0, ndirs, norders, X, Y, dxyz, fact, ex, ey);
+  k_ramp<<<std::min(1024, (n + 255) / 256), 256, 0, s>>>(k0, ndirs, norders, X, Y, dxyz, fact, ex, ey, use_x2(a));
   if (launches) *launches += 1;
   return (int)cudaGetLastError();
 }
@@ -1083,9 +897,11 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
 
 bool assemble_filter_fusable(const AssembleArgs& a, const FilterArgs& f, bool one_otf)
 {
-  if (!one_otf || f.bessel || a.ndirs != 3 || f.ndirs != 3 || a.norders != f.norders) return false;
-  if (f.norders != 2 && f.norders != 3) return false;
-  if (!(a.Y == 1024 || a.Y == 512 || a.Y == 256) || a.nx != f.nx || a.ny != f.ny || a.nz != f.nz) return false;
+  if (!one_otf || f.bessel || a.ndirs != f.ndirs || a.norders != f.norders) return false;
+  if (a.nx != f.nx || a.ny != f.ny || a.nz != f.nz) return false;
+  // the compiled doubled-length kernels filter 3 directions with 2 or 3 orders
+  const bool y4f = colfft_r1(a.Y) && a.ndirs == 3 && (f.norders == 2 || f.norders == 3);
+  if (!y4f && !use_y2(a)) return false;
   const FilterK k = make_filter_k(f);
   if (filter_needs_clamp(f, k)) return false;
   return 2 * (size_t)f.norders * f.otf.nxotf * sizeof(float2) <= kFusedTabMax;
@@ -1116,6 +932,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
   const std::vector<Slot>& slots = tabs.slots;
   const std::vector<int>& p0 = tabs.p0;
   const std::vector<int>& pn = tabs.pn;
+  const size_t np_out = p0.size();
   const DevTables dt = dev_tables(a, tabs);
   Slot* d_slots = dt.slots;
   int* d_p0 = dt.p0;
@@ -1133,7 +950,9 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
   xlines = std::min(xlines, 16);
   size_t smx = fft_stage_smem(a.X, xlines, xlines * (a.X + 1), kThreads);
 
-  if (a.X > kAccPerThread * kThreads) return -3;
+  // one output plane and the x pass writes real parts: no z pass
+  const bool x2_real = a.Z == 1 && np_out == 1 && use_x2(a);
+  if (a.X > kAccPerThread * kThreads && !use_x2(a)) return -3;
   // process whole planes in groups whose slots fit in T
   size_t np = p0.size();
   size_t pi = 0;
@@ -1149,10 +968,13 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
     AssembleArgs ay = a;
     KernelTimer* kt = kernel_timer();
     if (kt) kt->begin(s);
-    if (filt) {
+    if (use_y2(a)) {
+      const int rc = launch_asm_y2(ay, d_slots + first, nsl, filt, s);
+      if (rc != 0) return rc;
+    } else if (filt) {
       const FilterK fk = make_filter_k(*filt);
       const int fl = filter_flags(*filt);
-      const size_t tabb = 2 * (size_t)filt->norders * filt->otf.nxotf * sizeof(float2);
+      const size_t tabb = 2 * (size_t)filt->norders * filt->otf.nxotf * sizeof(float4);
       auto go = [&]<int YN, int NO, int FL>() {
         const size_t bytes = ColFft<YN, colfft_r1(YN), 8>::kSmemElems * sizeof(float2) + tabb;
         allow_dynamic_smem((const void*)k_asm_y4f<YN, NO, FL>, bytes);
@@ -1211,7 +1033,10 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
                      s>>>(ax, d_p0 + pi, d_pn + pi, d_slots, d_pz + pi, px.twr);
     };
     // the warp kernel's prefetch ring holds X/2 = nx columns (zoom factor 2)
-    if (a.X == 1024 && a.nx == 512) launch_xw.template operator()<1024>();
+    if (use_x2(a)) {
+      const int rc = launch_asm_x2(ax, d_slots, d_p0 + pi, d_pn + pi, d_pz + pi, (int)(pj - pi), x2_real, s);
+      if (rc != 0) return rc;
+    } else if (a.X == 1024 && a.nx == 512) launch_xw.template operator()<1024>();
     else if (a.X == 512 && a.nx == 256) launch_xw.template operator()<512>();
     else if (a.X == 256 && a.nx == 128) launch_xw.template operator()<256>();
     else
@@ -1226,10 +1051,15 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
   }
   int Wz = std::max(1, std::min(32, kMaxElems / a.Z));
   size_t smz = fft_stage_smem(a.Z, Wz, a.Z * (Wz + 1), kThreads);
+  if (x2_real) {
+    if (launches) *launches += nl;
+    return (int)cudaGetLastError();
+  }
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
+  const int split = use_x2(a);
   const int zr1 = a.Z % 16 == 0 ? a.Z / 16 : 0;
-  if (a.Z == 1 && ((size_t)a.X * a.Y) % 2 == 0) {
+  if (a.Z == 1 && !split && ((size_t)a.X * a.Y) % 2 == 0) {
     const size_t npairs = (size_t)a.X * a.Y / 2;
     const unsigned nb = (unsigned)std::min<size_t>((npairs + kThreads - 1) / kThreads, 152 * 16);
     k_asm_z1<<<nb, kThreads, 0, s>>>((const float4*)a.S, (float2*)a.out, npairs, d_zact);
@@ -1237,7 +1067,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
     auto go = [&]<int R1>() {
       const size_t bytes = (size_t)R1 * (16 * 64 + 8) * sizeof(float2);
       allow_dynamic_smem((const void*)k_asm_z4<R1>, bytes);
-      k_asm_z4<R1><<<dim3((a.X + 63) / 64, a.Y), kThreads, bytes, s>>>(a, d_zact, pz.tw);
+      k_asm_z4<R1><<<dim3((a.X + 63) / 64, a.Y), kThreads, bytes, s>>>(a, d_zact, pz.tw, split);
     };
     switch (zr1) {
       case 2: go.template operator()<2>(); break;
@@ -1250,7 +1080,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
   } else {
     dispatch_fft_len(kSiteAsmZ, a.Z, [&]<int NF>() {
       allow_dynamic_smem((const void*)k_asm_z<NF>, smz);
-      k_asm_z<NF><<<dim3((a.X + Wz - 1) / Wz, a.Y), kThreads, smz, s>>>(a, d_zact, pz, Wz);
+      k_asm_z<NF><<<dim3((a.X + Wz - 1) / Wz, a.Y), kThreads, smz, s>>>(a, d_zact, pz, Wz, split);
     });
   }
   if (kt) kt->end("k_asm_z", s, (double)np * a.X * a.Y * 8 + (double)a.X * a.Y * a.Z * 4);

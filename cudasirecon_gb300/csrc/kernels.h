@@ -271,8 +271,9 @@ int launch_assemble_filtered(const AssembleArgs& a, const FilterArgs& f, bool on
 
 // Phase-ramp tables for assembly: ex[d*no+o][j] = exp(i fact pi (j - X/2) o k0x_d dxyz),
 // ey likewise along y (computed in double precision).
-int launch_ramp_tables(const K0List& k0, int ndirs, int norders, int X, int Y, float dxyz, float fact, float2* ex,
-                       float2* ey, cudaStream_t s, long long* launches);
+// The columns of ex are in the order of the geometry's x pass.
+int launch_ramp_tables(const K0List& k0, const AssembleArgs& a, float dxyz, float fact, float2* ex, float2* ey,
+                       cudaStream_t s, long long* launches);
 
 // FFT-engine self test on `nlines` lines of length n (in place, device memory)
 int launch_fft_selftest(float2* data, int n, int nlines, int inverse, int columns, cudaStream_t s);

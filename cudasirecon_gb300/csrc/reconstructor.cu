@@ -1567,9 +1567,7 @@ void SIM_Reconstructor::filter_and_assemble()
   K0List k0l{};
   for (int d = 0; d < ndirs_; ++d) k0l.k[d] = make_float2(k0_[d].x, k0_[d].y);
   float fact = p.explodefact / 0.5;
-  check_launch(launch_ramp_tables(k0l, ndirs_, norders_, X_, Y_, dxy / p.zoomfact, fact, d_ex_, d_ey_, stream_,
-                                  &launches_),
-               "ramp");
+  check_launch(launch_ramp_tables(k0l, aa, dxy / p.zoomfact, fact, d_ex_, d_ey_, stream_, &launches_), "ramp");
   if (fused) check_launch(launch_assemble_filtered(aa, fa, one_otf, stream_, &launches_), "filter + assemble");
   else check_launch(launch_assemble(aa, stream_, &launches_), "assemble");
   stage_end("assemble", ev, l0);

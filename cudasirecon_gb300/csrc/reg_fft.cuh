@@ -10,8 +10,8 @@
 //
 // The compile-time DFTs split composite lengths recursively (N = A*B,
 // inner DFT_B over x[i + A*j], twiddle W_N^(i*k1), outer DFT_A), with the
-// twiddles taken from a table of W_480 (every supported length divides 480
-// or is handled by the radix-16/32 butterflies).
+// twiddles taken from a table of W_480, or for lengths that do not divide 480
+// from a table formed at compile time.
 #pragma once
 #include "fft.cuh"
 
@@ -202,6 +202,56 @@ __device__ __forceinline__ float2 w480c(int m, int dir)
   return make_float2(c[m], dir < 0 ? -s[m] : s[m]);
 }
 
+// cos / sin of 2 pi m / N, formed by the compiler in double: the angle within
+// an eighth of a turn of a multiple of a quarter turn, then its Taylor series
+struct RootVal {
+  double c, s;
+};
+__host__ __device__ constexpr RootVal root_val(long long m, long long N)
+{
+  m = ((m % N) + N) % N;
+  const long long q = (4 * m + N / 2) / N;  // nearest quarter turn
+  const double x = 6.283185307179586476925286766559 * (double)(4 * m - q * N) / (double)(4 * N);
+  const double x2 = x * x;
+  double c = 1.0, s = x, tc = 1.0, ts = x;
+  for (int k = 1; k <= 10; ++k) {
+    tc *= -x2 / (double)((2 * k - 1) * (2 * k));
+    ts *= -x2 / (double)((2 * k) * (2 * k + 1));
+    c += tc;
+    s += ts;
+  }
+  switch (q & 3) {
+    case 0: return RootVal{c, s};
+    case 1: return RootVal{-s, c};
+    case 2: return RootVal{-c, -s};
+    default: return RootVal{s, -c};
+  }
+}
+template <int N>
+struct RootTable {
+  float c[N], s[N];
+  __host__ __device__ constexpr RootTable() : c{}, s{}
+  {
+    for (int m = 0; m < N; ++m) {
+      const RootVal r = root_val(m, N);
+      c[m] = (float)r.c;
+      s[m] = (float)r.s;
+    }
+  }
+};
+// exp(dir * 2 pi i m / N) for a compile-time m
+template <int N>
+__device__ __forceinline__ float2 w_root(int m, int dir)
+{
+  if constexpr (480 % N == 0) {
+    return w480c(m * (480 / N), dir);
+  } else {
+    constexpr RootTable<N> t;
+    m %= N;
+    return make_float2(t.c[m], dir < 0 ? -t.s[m] : t.s[m]);
+  }
+}
+
 template <int N, int DIR>
 __device__ __forceinline__ void reg_dft(float2* v)
 {
@@ -209,9 +259,8 @@ __device__ __forceinline__ void reg_dft(float2* v)
   } else if constexpr (N == 2 || N == 3 || N == 4 || N == 5 || N == 7 || N == 8 || N == 16 || N == 32) {
     dftR<N, DIR>(v);
   } else {
-    constexpr int A = (N % 4 == 0) ? 4 : ((N % 2 == 0) ? 2 : ((N % 3 == 0) ? 3 : 5));
+    constexpr int A = (N % 4 == 0) ? 4 : ((N % 2 == 0) ? 2 : ((N % 3 == 0) ? 3 : ((N % 5 == 0) ? 5 : 7)));
     constexpr int B = N / A;
-    static_assert(480 % N == 0, "in-register DFT length must divide 480");
     float2 a[N];
 #pragma unroll
     for (int i = 0; i < A; ++i) {
@@ -220,7 +269,7 @@ __device__ __forceinline__ void reg_dft(float2* v)
       for (int j = 0; j < B; ++j) t[j] = v[i + A * j];
       reg_dft<B, DIR>(t);
 #pragma unroll
-      for (int k1 = 0; k1 < B; ++k1) a[i * B + k1] = (i * k1 == 0) ? t[k1] : cmul(t[k1], w480c(i * k1 * (480 / N), DIR));
+      for (int k1 = 0; k1 < B; ++k1) a[i * B + k1] = (i * k1 == 0) ? t[k1] : cmul(t[k1], w_root<N>(i * k1, DIR));
     }
 #pragma unroll
     for (int k1 = 0; k1 < B; ++k1) {

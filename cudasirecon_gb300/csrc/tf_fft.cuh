@@ -1,0 +1,96 @@
+// Two-factor transforms of run-time length n = R1 * R2 for the lengths that
+// have no compiled transform of their own.
+//
+//   X[k1 + R1 k2] = sum_j W_n^(j k1) W_R2^(j k2) sum_e x[j + R2 e] W_R1^(e k1)
+//
+// Stage 1: the thread for (line, j < R2) takes x[j + R2 e] (e < R1), runs an
+// in-register DFT of R1 points, multiplies by W_n^(j k1) and leaves the R1
+// values in shared memory; stage 2: the thread for (line, k1 < R1) takes the
+// R2 values over j, runs an in-register DFT of R2 points and holds X[k1 + R1 k2].
+// One shared-memory round trip and two barriers per tile, where the Stockham
+// stages make one per radix and two more to fill and empty the tile.
+//
+// R1 and R2 are chosen at run time from a fixed set of compiled DFT sizes
+// (tf_switch: a branch that the whole CTA takes alike), so one kernel serves
+// every length; registers are those of the largest size it may take, hence
+// the two kernel classes MR = 16 and 32.
+//
+// Half-shifted form: the outputs of a transform zero-padded to twice its
+// length fall into two of length n, the even ones of x and the odd ones of
+// x[i] exp(DIR i pi k_i / n) with k_i the signed frequency i or i - n.  With
+// i = j + R2 e the factor is exp(DIR i pi e / R1) (a constant of the DFT)
+// times exp(DIR i pi j / n) (part of the stage twiddle), negated for k_i < 0.
+#pragma once
+#include "reg_fft.cuh"
+
+namespace simrecon {
+
+struct TfPlan {
+  int n, r1, r2;
+  const float2* tw;   // [r1][r2]: exp(-2 pi i j k1 / n) at k1 * r2 + j
+  const float2* twh;  // the same times exp(-i pi j / n)
+};
+// r1 >= r2 from the compiled sizes with r1 * r2 = n, the pair with the smallest r1
+bool tf_factor(int n, int* r1, int* r2);
+// plan with device twiddles, cached per (device, n); false where n has no pair
+bool get_tf_plan(int n, TfPlan* plan);
+
+constexpr int kTfSizes[] = {8, 9, 10, 12, 14, 15, 16, 18, 20, 21, 24, 25, 27, 28, 30, 32};
+constexpr int kTfMax = 32;
+// kernel class of a plan: the largest DFT it needs
+inline int tf_class(const TfPlan& p) { return p.r1 <= 16 ? 16 : 32; }
+
+#ifdef __CUDACC__
+
+// f.template operator()<R>() for the compiled size R == r, r <= MR
+template <int MR, typename F>
+__device__ __forceinline__ void tf_switch(int r, F&& f)
+{
+  switch (r) {
+#define SIMRECON_TF_CASE(R) \
+  case R:                   \
+    if constexpr (R <= MR) f.template operator()<R>(); \
+    break;
+    SIMRECON_TF_CASE(8)
+    SIMRECON_TF_CASE(9)
+    SIMRECON_TF_CASE(10)
+    SIMRECON_TF_CASE(12)
+    SIMRECON_TF_CASE(14)
+    SIMRECON_TF_CASE(15)
+    SIMRECON_TF_CASE(16)
+    SIMRECON_TF_CASE(18)
+    SIMRECON_TF_CASE(20)
+    SIMRECON_TF_CASE(21)
+    SIMRECON_TF_CASE(24)
+    SIMRECON_TF_CASE(25)
+    SIMRECON_TF_CASE(27)
+    SIMRECON_TF_CASE(28)
+    SIMRECON_TF_CASE(30)
+    SIMRECON_TF_CASE(32)
+#undef SIMRECON_TF_CASE
+  }
+}
+
+// v[e] *= exp(DIR i pi e / R): the half shift's constant part
+template <int R, int DIR>
+__device__ __forceinline__ void tf_half_shift(float2* v)
+{
+#pragma unroll
+  for (int e = 1; e < R; ++e) v[e] = cmul(v[e], w_root<2 * R>(e, DIR));
+}
+
+// v[k1] *= W_n^(j k1) from the plan's table (tw or twh), k1 * r2 + j
+template <int R, int DIR>
+__device__ __forceinline__ void tf_twiddle(float2* v, const float2* __restrict__ tw, int r2, int j)
+{
+#pragma unroll
+  for (int k1 = 0; k1 < R; ++k1) {
+    float2 w = __ldg(tw + k1 * r2 + j);
+    if (DIR > 0) w.y = -w.y;
+    v[k1] = cmul(v[k1], w);
+  }
+}
+
+#endif  // __CUDACC__
+
+}  // namespace simrecon
