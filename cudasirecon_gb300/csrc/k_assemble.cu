@@ -834,7 +834,12 @@ namespace {
 // volume the y pass takes 1.31 ms (k_asm_y4f) against 1.45, the x pass
 // 0.56 ms (k_asm_xw) against 0.87; per 256^2 x 32 volume 0.254 / 0.256 and
 // 0.096 / 0.102 ms
-bool use_y2(const AssembleArgs& a) { return !colfft_r1(a.Y) && asm_y2_supported(a); }
+// (k_asm_y4f filters 3 directions with 2 or 3 orders only)
+bool use_y2(const AssembleArgs& a)
+{
+  const bool y4f = colfft_r1(a.Y) && a.ndirs == 3 && (a.norders == 2 || a.norders == 3);
+  return !y4f && asm_y2_supported(a);
+}
 bool use_x2(const AssembleArgs& a)
 {
   return !(a.X == 2 * a.nx && (a.X == 1024 || a.X == 512 || a.X == 256)) && asm_x2_supported(a);
@@ -899,9 +904,7 @@ bool assemble_filter_fusable(const AssembleArgs& a, const FilterArgs& f, bool on
 {
   if (!one_otf || f.bessel || a.ndirs != f.ndirs || a.norders != f.norders) return false;
   if (a.nx != f.nx || a.ny != f.ny || a.nz != f.nz) return false;
-  // the compiled doubled-length kernels filter 3 directions with 2 or 3 orders
-  const bool y4f = colfft_r1(a.Y) && a.ndirs == 3 && (f.norders == 2 || f.norders == 3);
-  if (!y4f && !use_y2(a)) return false;
+  if (!use_y2(a) && !(colfft_r1(a.Y) && a.ndirs == 3 && (f.norders == 2 || f.norders == 3))) return false;
   const FilterK k = make_filter_k(f);
   if (filter_needs_clamp(f, k)) return false;
   return 2 * (size_t)f.norders * f.otf.nxotf * sizeof(float2) <= kFusedTabMax;

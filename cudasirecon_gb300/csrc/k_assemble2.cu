@@ -10,8 +10,8 @@
 // by parity, S[zout][yr][x & 1][x >> 1], so that the x pass stores runs
 #include <algorithm>
 
-#include "asm_x2.cuh"
 #include "assemble.h"
+#include "tf_kernels.h"
 
 namespace simrecon {
 
@@ -249,10 +249,9 @@ int launch_asm_x2(const AssembleArgs& a, const void* d_slots, const int* d_p0, c
                   int nplanes, bool real, cudaStream_t s)
 {
   TfPlan pl;
-  if (!get_tf_plan(a.nx, &pl)) return -1;
-  AsmX2Launch l{&a, (const Slot*)d_slots, d_p0, d_pn, d_pz, nplanes, real, pl, s};
-  if (!asm_x2_part0(l) && !asm_x2_part1(l) && !asm_x2_part2(l) && !asm_x2_part3(l)) return -1;
-  return (int)cudaGetLastError();
+  const TfKernels* k = tf_kernels(a.nx, &pl);
+  if (!k || !k->asm_x) return -1;
+  return k->asm_x(AsmX2Launch{&a, (const Slot*)d_slots, d_p0, d_pn, d_pz, nplanes, real}, pl, s);
 }
 
 }  // namespace simrecon

@@ -25,6 +25,7 @@
 #include "col_fft.cuh"
 #include "kernels.h"
 #include "reg_fft.cuh"
+#include "tf_kernels.h"
 #include "thresholds.h"
 
 namespace simrecon {
@@ -612,6 +613,11 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   FFTPlan px, py;
   if (!get_fft_plan(a.nx, &px) || !get_fft_plan(a.ny, &py)) return -1;
   const int nzb = 2 * a.zdc + 1;
+  // lengths without a compiled transform take the two-factor kernels; 1024
+  // rows too (1.25 ms a 1024^2 x 64 pair with the Stockham stages, 0.26 here)
+  TfPlan tx, ty;
+  const TfKernels* kx = reg_fft_lanes(a.nx) || a.otf.nxotf > kOvlTabMax ? nullptr : tf_kernels(a.nx, &tx);
+  const TfKernels* ky = reg_fft_lanes(a.ny) && a.ny != 1024 ? nullptr : tf_kernels(a.ny, &ty);
   // 1) build + x inverse FFT
   const int ldl = a.nx + 1;
   int rows = std::max(1, kMaxElems / (2 * a.nx));
@@ -632,7 +638,10 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   if (a.nx == 512) launch_w.template operator()<512>();
   else if (a.nx == 1024) launch_w.template operator()<1024>();
   else if (a.nx == 256) launch_w.template operator()<256>();
-  else
+  else if (kx) {
+    const int rc = kx->ovl_x(a, tx, s);
+    if (rc != 0) return rc;
+  } else
     dispatch_fft_len(kSiteOvlX, a.nx, [&]<int NF>() {
       allow_dynamic_smem((const void*)k_ovl_build_x<NF>, sm1);
       k_ovl_build_x<NF><<<nb1, kThreads, sm1, s>>>(a, px, rows, ldl);
@@ -655,6 +664,11 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
     groups = std::max(1, std::min(nzb, (4 * 152 + tiles - 1) / tiles));
     ppg = (nzb + groups - 1) / groups;
     groups = (nzb + ppg - 1) / ppg;
+  } else if (ky) {
+    tiles = (a.nx + ky->ovl_y_columns - 1) / ky->ovl_y_columns;
+    groups = std::max(1, std::min(nzb, (4 * 152 + tiles - 1) / tiles));
+    ppg = (nzb + groups - 1) / groups;
+    groups = (nzb + ppg - 1) / ppg;
   }
   if (kt) kt->begin(s);
   auto go4 = [&]<int N, int R1>() {
@@ -664,7 +678,10 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   };
   if (a.ny == 512) go4.template operator()<512, 32>();
   else if (a.ny == 256) go4.template operator()<256, 16>();
-  else
+  else if (ky) {
+    const int rc = ky->ovl_y(a, ty, ppg, groups, s);
+    if (rc != 0) return rc;
+  } else
     dispatch_fft_len(kSiteOvlY, a.ny, [&]<int NF>() {
       allow_dynamic_smem((const void*)k_ovl_y_accum<NF>, sm2);
       k_ovl_y_accum<NF><<<dim3(tiles, groups), threads, sm2, s>>>(a, py, W, ppg, xoff);
@@ -685,13 +702,22 @@ int launch_crosscorr_peak(const float2* pmap, float2* cc, int nx, int ny, float*
   size_t sm1 = fft_stage_smem(nx, nl, nl * (nx + 1), kThreads);
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
-  dispatch_fft_len(kSiteCorrRows, nx, [&]<int NF>() {
+  TfPlan tx, ty;
+  const TfKernels* kx = reg_fft_lanes(nx) ? nullptr : tf_kernels(nx, &tx);
+  const TfKernels* ky = reg_fft_lanes(ny) ? nullptr : tf_kernels(ny, &ty);
+  if (kx) {
+    const int rc = kx->fft_rows_conj(pmap, cc, ny, tx, s);
+    if (rc != 0) return rc;
+  } else dispatch_fft_len(kSiteCorrRows, nx, [&]<int NF>() {
     allow_dynamic_smem((const void*)k_fft_rows<-1, true, NF>, sm1);
     k_fft_rows<-1, true, NF><<<(ny + nl - 1) / nl, kThreads, sm1, s>>>(pmap, cc, nx, ny, px, nl);
   });
   int W = std::max(1, std::min(32, kMaxElems / ny));
   size_t sm2 = fft_stage_smem(ny, W, (W + 1) * ny, kThreads);
-  dispatch_fft_len(kSiteCorrCols, ny, [&]<int NF>() {
+  if (ky) {
+    const int rc = ky->fft_cols(cc, nx, 1, ty, s);
+    if (rc != 0) return rc;
+  } else dispatch_fft_len(kSiteCorrCols, ny, [&]<int NF>() {
     allow_dynamic_smem((const void*)k_fft_cols2<-1, NF>, sm2);
     k_fft_cols2<-1, NF><<<(nx + W - 1) / W, kThreads, sm2, s>>>(cc, ny, nx, py, W);
   });

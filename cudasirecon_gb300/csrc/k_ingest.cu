@@ -14,8 +14,10 @@
 #include <algorithm>
 
 #include "col_fft.cuh"
+#include "ingest_dev.cuh"
 #include "kernels.h"
 #include "reg_fft.cuh"
+#include "tf_kernels.h"
 
 namespace simrecon {
 
@@ -23,29 +25,6 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kMaxElems = kFftElems;  // complex elements per CTA and buffer
-
-__device__ __forceinline__ int raw_section(int d, int p, int z, int nz, int ndirs, int nph, int fastSI)
-{
-  // loadImageData section order, cudaSirecon.cpp:1374-1382
-  return fastSI ? (z * ndirs * nph + d * nph + p) : (d * nz * nph + z * nph + p);
-}
-
-template <typename T>
-__device__ __forceinline__ float flat(const T* __restrict__ plane, const IngestArgs& a, int y, int x)
-{
-  float v = (float)plane[(size_t)y * a.nx + x];
-  float bg = a.bg ? __ldg(a.bg + (size_t)y * a.nx + x) : a.bgconst;
-  float sl = a.slope ? __ldg(a.slope + (size_t)y * a.nx + x) : 1.0f;
-  return (v - bg - a.bgextra) * sl * a.inscale;
-}
-
-// flat() for a raw value already loaded
-__device__ __forceinline__ float flat_v(float v, const IngestArgs& a, int y, int x)
-{
-  float bg = a.bg ? __ldg(a.bg + (size_t)y * a.nx + x) : a.bgconst;
-  float sl = a.slope ? __ldg(a.slope + (size_t)y * a.nx + x) : 1.0f;
-  return (v - bg - a.bgextra) * sl * a.inscale;
-}
 
 // VEC consecutive raw pixels of row y starting at x (x % VEC == 0), as floats
 template <typename T, int VEC>
@@ -471,10 +450,17 @@ int launch_ingest(const IngestArgs& a, cudaStream_t s, long long* launches)
       k_ingest_xw<float, N><<<gw, kIngestWarps * 32, bytes, s>>>(a, px.twr);
     }
   };
+  // lengths without a compiled transform take the two-factor kernels
+  TfPlan tx, ty;
+  const TfKernels* kx = reg_fft_lanes(a.nx) ? nullptr : tf_kernels(a.nx, &tx);
+  const TfKernels* ky = reg_fft_lanes(a.ny) ? nullptr : tf_kernels(a.ny, &ty);
   if (a.nx == 512) go_w.template operator()<512>();
   else if (a.nx == 1024) go_w.template operator()<1024>();
   else if (a.nx == 256) go_w.template operator()<256>();
-  else
+  else if (kx && kx->ingest_x) {
+    const int rc = kx->ingest_x(a, tx, s);
+    if (rc != 0) return rc;
+  } else
   dispatch_fft_len(kSiteIngestX, a.nx, [&]<int NF>() {
     if (a.raw_is_u16) {
       if (a.nx % 8 == 0) {
@@ -509,6 +495,9 @@ int launch_ingest(const IngestArgs& a, cudaStream_t s, long long* launches)
     if (a.ny == 512) go.template operator()<512>();
     else if (a.ny == 1024) go.template operator()<1024>();
     else go.template operator()<256>();
+  } else if (ky) {
+    const int rc = ky->fft_cols(a.spec, nxh, nplanes, ty, s);
+    if (rc != 0) return rc;
   } else {
     dispatch_fft_len(kSiteIngestY, a.ny, [&]<int NF>() {
       allow_dynamic_smem((const void*)k_fft_cols<-1, NF>, smy);
