@@ -21,7 +21,7 @@ LIB = os.path.join(HERE, "libcudasirecon.so")
 CLI = os.path.join(HERE, "bin", "cudasirecon")
 MAKEOTF = os.path.join(HERE, "bin", "makeotf")
 SOURCES = ["fft_plan.cu", "k_selftest.cu", "k_ingest.cu", "k_fit.cu", "k_search.cu", "k_assemble.cu", "k_assemble2.cu",
-           *(f"k_tf_{i}.cu" for i in range(8)), "tf_table.cpp", "reconstructor.cu", "makeotf.cu", "params.cpp",
+           *(f"k_tf_{i}.cu" for i in range(8)), "tf_table.cpp", "k_sep_z.cu", "k_asm_zn.cu", "reconstructor.cu", "makeotf.cu", "params.cpp",
            "image_io.cpp", "makeotf_io.cpp", "server.cpp", "capi.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

@@ -27,6 +27,7 @@
 #include "filter.cuh"
 #include "kernels.h"
 #include "reg_fft.cuh"
+#include "z_fft.cuh"
 
 namespace simrecon {
 
@@ -1080,6 +1081,12 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
       case 6: go.template operator()<6>(); break;
       default: go.template operator()<8>(); break;
     }
+  } else if (z_length_ok(a.Z) && !reg_fft_lanes(a.Z)) {
+    unsigned long long active = 0;
+    for (int z = 0; z < a.Z; ++z)
+      if (tabs.zact[z]) active |= 1ull << z;
+    const int rc = launch_asm_zn(a.S, a.out, a.X, a.Y, a.Z, active, pz.tw, split, s);
+    if (rc != 0) return rc;
   } else {
     dispatch_fft_len(kSiteAsmZ, a.Z, [&]<int NF>() {
       allow_dynamic_smem((const void*)k_asm_z<NF>, smz);

@@ -18,6 +18,7 @@
 #include "kernels.h"
 #include "reg_fft.cuh"
 #include "tf_kernels.h"
+#include "z_fft.cuh"
 
 namespace simrecon {
 
@@ -676,6 +677,9 @@ int launch_separate(float2* spec, const float* scale, const float* sepmat, int n
       case 6: go.template operator()<6>(); break;
       default: go.template operator()<8>(); break;
     }
+  } else if (z_length_ok(nz) && !reg_fft_lanes(nz) && (nphases == 3 || nphases == 5)) {
+    const int rc = launch_separate_z(spec, scale, sepmat, (size_t)ny * nxh, nz, ndirs, nphases, pz.tw, s);
+    if (rc != 0) return rc;
   } else {
     dispatch_fft_len(kSiteSeparateZ, nz, [&]<int NF>() {
       allow_dynamic_smem((const void*)k_separate<NF>, sm);
