@@ -7,7 +7,7 @@
 // k_k0_search       one thread-block cluster per direction (all directions in
 //                   one launch, side by side on the GPU): the angle and
 //                   magnitude line searches with their parabola fits and the
-//                   final modulation amplitude.  The cluster's eight CTAs
+//                   final modulation amplitude.  The cluster's CTAs
 //                   evaluate batches of candidate k0s over the overlap map P
 //                   (each CTA one tile of P, its partial sums written into
 //                   the leader CTA's shared memory); one thread of the
@@ -82,13 +82,16 @@ __global__ void k_findk0_finish(const float* __restrict__ pk, float2 guess, int 
   *k1out = polar_rn(mag, atan2f(k0.y, k0.x));
 }
 
-constexpr int kSC = 8;        // CTAs per cluster: one direction's search
+constexpr int kSCmax = 16;    // CTAs per cluster at most: one direction's search
 constexpr int kST = 512;      // threads per CTA
 constexpr int kSW = kST / 32;
 constexpr int kSB = 32;       // candidates per batch at most
+constexpr long long kSearchWide = 256 * 256;
 constexpr int kSL = 1024;     // line cache: steps -kSL..kSL from the start value
-constexpr int kSLine0 = 12;   // first batch of a line: the start and 12 steps each way
-constexpr int kSLineK = 16;   // later batches: 16 steps further along the climb
+// first batch of a line: the start and 3 to 12 steps each way (line_start),
+// later batches 8 steps further along the climb
+constexpr int kSLine0Min = 3, kSLine0Max = 12;
+constexpr int kSLineK = 8;
 // every batch but the two line starts and the final evaluation extends a
 // climb by kSLineK steps, so this bounds the batches of a search
 constexpr int kSMaxBatches = 2 * (2 * kSL / kSLineK + 2) + 4;
@@ -109,7 +112,7 @@ struct __align__(16) SearchCtl {
   float pos[kSB];            // the batch's positions along its line
   int j[kSB];                // their line steps
   float2 kc[kSB];            // candidate vectors k1 * fitorder2
-  double red[kSC][kSB][2];   // every CTA's partial XStarY (leader only)
+  double red[kSCmax][kSB][2];  // every CTA's partial XStarY (leader only)
   double res[kSB][2];        // the batch's XStarY (leader only)
 };
 
@@ -181,7 +184,19 @@ struct Controller {
   float afit, mfit;    // fitted angle, magnitude
   float x1, amp1;      // carried between the lines
   float sx;            // sum |X|^2 as float
+  float angle_px;      // pixels of the overlaps' spectrum per step of angle, of magnitude
+  float mag_px;
 };
+
+// Steps each way that a line's first batch evaluates: the cross-correlation's
+// parabola leaves the start within about 0.4 pixel of the peak, and the climb
+// looks one or two steps past it.  Every step costs a pass of FMAs over P, a
+// missing one a further batch.
+__device__ __forceinline__ int line_start(float px_per_step)
+{
+  const int n = (int)ceilf(0.4f / px_per_step) + 2;
+  return min(max(n, kSLine0Min), kSLine0Max);
+}
 
 // position of step j from its neighbour towards the start (float-accumulated
 // like the reference's angle += deltaangle)
@@ -208,9 +223,10 @@ __device__ void request_line(const Controller& c, SearchLine& L, SearchCtl& ctl,
     ++n;
   };
   if (j == 0 || j == 1) {
+    const int n0 = line_start(ang ? c.angle_px : c.mag_px);
     add(0);
-    for (int i = 1; i <= kSLine0; ++i) add(i);
-    for (int i = 1; i <= kSLine0; ++i) add(-i);
+    for (int i = 1; i <= n0; ++i) add(i);
+    for (int i = 1; i <= n0; ++i) add(-i);
   } else {
     const int s = j > 0 ? 1 : -1;
     for (int i = 0; i < kSLineK; ++i) add(j + s * i);
@@ -334,66 +350,83 @@ __device__ __forceinline__ void tile_sums(const float2* __restrict__ pmap, int n
   }
 }
 
-// the CTA's sums of CC candidates in double (warps by shuffles, then the
-// warps in order) into the leader's partial-sum table at candidate c0
+// The CTA's sums of CC candidates into the leader's partial-sum table at
+// candidate c0: the threads' float sums transposed through shared memory, each
+// thread adding 2 CC values' share of kSeg neighbours as a float pair (the
+// rounding error of every addition kept, 48 bits; the FP64 adder runs at a
+// sixtyfourth of the FP32 rate here, and shuffling doubles through the warps
+// took 20 us a batch), the segments' totals in double.
 template <int CC>
-__device__ __forceinline__ void tile_reduce(const float2 (&acc)[CC], double (*wsum)[2 * 16], SearchCtl* lead,
-                                            int rank, int c0, int tid, int warp, int lane)
+__device__ __forceinline__ void tile_reduce(const float2 (&acc)[CC], float* sacc, double* sseg, SearchCtl* lead,
+                                            int rank, int c0, int tid)
 {
+  constexpr int V = 2 * CC, kPitch = V + 1;
+  constexpr int kSegs = kST / (V <= 8 ? 8 : V <= 16 ? 16 : 32), kSeg = kST / kSegs;  // V segment threads or more
 #pragma unroll
   for (int k = 0; k < CC; ++k) {
-    double sr = acc[k].x, si = acc[k].y;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sr += __shfl_xor_sync(0xffffffffu, sr, o);
-      si += __shfl_xor_sync(0xffffffffu, si, o);
-    }
-    if (lane == 0) {
-      wsum[warp][2 * k] = sr;
-      wsum[warp][2 * k + 1] = si;
-    }
+    sacc[tid * kPitch + 2 * k] = acc[k].x;
+    sacc[tid * kPitch + 2 * k + 1] = acc[k].y;
   }
   __syncthreads();
-  if (tid < 2 * CC) {
-    double s = 0.0;
-    for (int w = 0; w < kSW; ++w) s += wsum[w][tid];
-    lead->red[rank][c0 + (tid >> 1)][tid & 1] = s;
+  const int v = tid % (kST / kSegs), seg = tid / (kST / kSegs);
+  if (v < V) {
+    float s = 0.f, e = 0.f;
+    for (int i = 0; i < kSeg; ++i) {
+      const float x = sacc[(seg * kSeg + i) * kPitch + v];
+      const float t = __fadd_rn(s, x), bb = __fsub_rn(t, s);
+      e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(x, bb)));
+      s = t;
+    }
+    sseg[seg * V + v] = (double)s + (double)e;
+  }
+  __syncthreads();
+  if (tid < V) {
+    double t = 0.0;
+    for (int g = 0; g < kSegs; ++g) t += sseg[g * V + tid];
+    lead->red[rank][c0 + (tid >> 1)][tid & 1] = t;
   }
 }
 
 template <int CC>
 __device__ void chunk(const float2* __restrict__ pmap, int nx, const float2* ex, const float2* ey, int tw, int th,
-                      int x0, int y0, double (*wsum)[2 * 16], SearchCtl* lead, int rank, int c0)
+                      int x0, int y0, float* sacc, double* sseg, SearchCtl* lead, int rank, int c0)
 {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float2 acc[CC];
   tile_sums<CC>(pmap, nx, ex, ey, tw, th, x0, y0, warp, lane, acc);
-  tile_reduce<CC>(acc, wsum, lead, rank, c0, tid, warp, lane);
+  tile_reduce<CC>(acc, sacc, sseg, lead, rank, c0, tid);
 }
 
-// C: the most candidates one pass holds (phase tables in shared memory)
-template <int C>
-__global__ void __cluster_dims__(kSC, 1, 1) __launch_bounds__(kST, 1) k_k0_search(const __grid_constant__ K0SearchArgs a)
+// C: the most candidates one pass holds (phase tables in shared memory);
+// SC: CTAs per cluster.
+// Bound by latency: per batch two cluster barriers, the phase tables, one pass
+// of FMAs over P and the reduction.  Whole search of three directions, with 25
+// candidates a first batch, doubles shuffled through the warps and 8 CTAs,
+// and now: 128^2 131 -> 39 us, 512^2 215 -> 63, 1024 x 960 433 -> 132 us.
+template <int C, int SC>
+__global__ void __launch_bounds__(kST, 1) k_k0_search(const __grid_constant__ K0SearchArgs a)
 {
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned rank = cluster.block_rank();
-  const int dir = blockIdx.x / kSC;  // one cluster per direction
+  const int dir = blockIdx.x / SC;  // one cluster per direction
   const float2* __restrict__ pmap = a.pmap[dir];
   __shared__ SearchCtl ctl;
   __shared__ SearchLine lines[2];
-  __shared__ double wsum[kSW][2 * 16];
+  __shared__ double sseg[kST / 8 * 8];
   __shared__ float2 kloc[kSB];
   __shared__ float2 khl[kSB][2];  // k dxy of each candidate and axis as hi + lo floats
   __shared__ int nloc;
-  extern __shared__ float2 tab[];
+  extern __shared__ float2 tab[];  // phase tables, then the reduction's transposed sums
   SearchCtl* lead = cluster.map_shared_rank(&ctl, 0);
   const int tid = threadIdx.x;
   const int nx = a.nx, ny = a.ny;
-  // tile of P: 2 column halves x 4 row quarters
-  const int tx = rank & 1, ty = rank >> 1;
-  const int x0 = tx * nx / 2, x1 = (tx + 1) * nx / 2;
+  // tile of P: SC / 4 column parts x 4 row quarters
+  constexpr int TX = SC / 4;
+  const int tx = rank % TX, ty = rank / TX;
+  const int x0 = tx * nx / TX, x1 = (tx + 1) * nx / TX;
   const int y0 = ty * ny / 4, y1 = (ty + 1) * ny / 4;
   const int tw = x1 - x0, th = y1 - y0;
+  float* sacc = (float*)(tab + (size_t)C * ((nx + TX - 1) / TX + (ny + 3) / 4));
 
   Controller c{};
   if (rank == 0) {
@@ -406,6 +439,10 @@ __global__ void __cluster_dims__(kSC, 1, 1) __launch_bounds__(kST, 1) k_k0_searc
       c.delta_angle = a.delta_angle;
       c.delta_mag = a.delta_mag;
       c.sx = __double2float_rn(a.sumxy[dir][0]);
+      // the overlaps beat at k0 * fitorder2; one pixel is 1 / (n dxy)
+      const float ext = (float)max(nx, ny) * a.dxy * (float)a.fitorder2;
+      c.angle_px = c.k0mag * a.delta_angle * ext;
+      c.mag_px = a.delta_mag * ext;
       ctl.nbatch = 0;
     }
   }
@@ -431,6 +468,8 @@ __global__ void __cluster_dims__(kSC, 1, 1) __launch_bounds__(kST, 1) k_k0_searc
     __syncthreads();
     const int nb = nloc;
     if (nb == 0) break;
+    if (tid < 2 * kSB) khl[tid >> 1][tid & 1] = make_float2(0.f, 0.f);  // padding of the last pass
+    __syncthreads();
     if (tid < 2 * nb) {  // the double products once per candidate and axis (FP64 is slow on this GPU)
       const float2 kk = kloc[tid >> 1];
       const double kd = (double)((tid & 1) ? kk.y : kk.x) * (double)a.dxy;
@@ -439,8 +478,10 @@ __global__ void __cluster_dims__(kSC, 1, 1) __launch_bounds__(kST, 1) k_k0_searc
     }
     __syncthreads();
     for (int c0 = 0; c0 < nb;) {
+      // the smallest compiled pass that takes what is left (padded with zero
+      // vectors, whose sums nothing reads)
       const int rem = nb - c0;
-      const int cc = rem >= 16 && C >= 16 ? 16 : rem >= 8 && C >= 8 ? 8 : rem >= 4 ? 4 : rem >= 2 ? 2 : 1;
+      const int cc = rem == 1 ? 1 : rem <= 4 ? 4 : rem <= 8 || C < 12 ? (C < 8 ? 4 : 8) : rem <= 12 || C < 16 ? 12 : 16;
       float2* ex = tab;                    // [cc][tw]
       float2* ey = tab + (size_t)cc * tw;  // [cc][th]
       for (int e = tid; e < cc * (tw + th); e += kST) {
@@ -451,18 +492,18 @@ __global__ void __cluster_dims__(kSC, 1, 1) __launch_bounds__(kST, 1) k_k0_searc
         else ey[k * th + (r - tw)] = phase_factor(y0 + (r - tw), ny, hl.x, hl.y);
       }
       __syncthreads();
-      if (cc == 16) chunk<16>(pmap, nx, ex, ey, tw, th, x0, y0, wsum, lead, rank, c0);
-      else if (cc == 8) chunk<8>(pmap, nx, ex, ey, tw, th, x0, y0, wsum, lead, rank, c0);
-      else if (cc == 4) chunk<4>(pmap, nx, ex, ey, tw, th, x0, y0, wsum, lead, rank, c0);
-      else if (cc == 2) chunk<2>(pmap, nx, ex, ey, tw, th, x0, y0, wsum, lead, rank, c0);
-      else chunk<1>(pmap, nx, ex, ey, tw, th, x0, y0, wsum, lead, rank, c0);
-      __syncthreads();  // tables and wsum are reused by the next chunk
+      if (C >= 16 && cc == 16) chunk<C >= 16 ? 16 : 1>(pmap, nx, ex, ey, tw, th, x0, y0, sacc, sseg, lead, rank, c0);
+      else if (C >= 12 && cc == 12) chunk<C >= 12 ? 12 : 1>(pmap, nx, ex, ey, tw, th, x0, y0, sacc, sseg, lead, rank, c0);
+      else if (C >= 8 && cc == 8) chunk<C >= 8 ? 8 : 1>(pmap, nx, ex, ey, tw, th, x0, y0, sacc, sseg, lead, rank, c0);
+      else if (cc == 4) chunk<4>(pmap, nx, ex, ey, tw, th, x0, y0, sacc, sseg, lead, rank, c0);
+      else chunk<1>(pmap, nx, ex, ey, tw, th, x0, y0, sacc, sseg, lead, rank, c0);
+      __syncthreads();  // tables and sums are reused by the next pass
       c0 += cc;
     }
     cluster.sync();  // every CTA's partial sums are in the leader
     if (rank == 0 && tid < 2 * nb) {
       double s = 0.0;
-      for (int r = 0; r < kSC; ++r) s += ctl.red[r][tid >> 1][tid & 1];
+      for (int r = 0; r < SC; ++r) s += ctl.red[r][tid >> 1][tid & 1];
       ctl.res[tid >> 1][tid & 1] = s;
     }
   }
@@ -485,13 +526,24 @@ int launch_findk0_finish(const float* peak, float2 guess, int nx, int ny, float 
   return (int)cudaGetLastError();
 }
 
-// candidates per chunk: the phase tables of a tile (C x (tw + th) complex)
-// within 160 KB of shared memory
-static int search_chunk(int nx, int ny)
+// CTAs per cluster: sixteen where P gives each at least 4096 elements (smaller
+// maps are all barriers and control, which more CTAs lengthen); a non-portable
+// size, so only where the device can hold such a cluster
+static int search_ctas(int nx, int ny) { return (long long)nx * ny >= kSearchWide ? 16 : 8; }
+
+// dynamic shared memory of a search with C candidates per pass
+static size_t search_smem(int nx, int ny, int C, int sc)
 {
-  const size_t per = ((size_t)(nx + 1) / 2 + (size_t)(ny + 3) / 4) * sizeof(float2);
-  for (int c : {16, 8, 4})
-    if (c * per <= 160 * 1024) return c;
+  const size_t tw = ((size_t)nx + sc / 4 - 1) / (sc / 4), th = ((size_t)ny + 3) / 4;
+  return C * (tw + th) * sizeof(float2) + (size_t)kST * (2 * C + 1) * sizeof(float);
+}
+
+// candidates per pass: the phase tables of a tile and the transposed sums
+// within 160 KB of shared memory
+static int search_chunk(int nx, int ny, int sc)
+{
+  for (int c : {16, 12, 8, 4})
+    if (search_smem(nx, ny, c, sc) <= 160 * 1024) return c;
   return 0;
 }
 
@@ -501,25 +553,55 @@ static int search_chunk(int nx, int ny)
 // tile.
 bool k0_search_supported(int nx, int ny)
 {
-  return nx >= 64 && ny >= 8 && (long long)nx * ny <= 1024LL * 1024 && search_chunk(nx, ny) > 0;
+  return nx >= 64 && ny >= 8 && (long long)nx * ny <= 1024LL * 1024 && search_chunk(nx, ny, 8) > 0;
 }
 
 int launch_k0_search(const K0SearchArgs& a, cudaStream_t s, long long* launches)
 {
-  const int C = search_chunk(a.nx, a.ny);
-  if (C == 0 || a.nx < 64 || a.ny < 8 || a.ndirs < 1 || a.ndirs > kMaxDirs) return -1;
-  const size_t tw = (size_t)(a.nx + 1) / 2, th = (size_t)(a.ny + 3) / 4;
-  const size_t smem = (size_t)C * (tw + th) * sizeof(float2);
-  auto go = [&](auto kern) {
+  if (a.nx < 64 || a.ny < 8 || a.ndirs < 1 || a.ndirs > kMaxDirs) return -1;
+  auto go = [&](auto kern, int C, int sc) -> int {
+    const size_t smem = search_smem(a.nx, a.ny, C, sc);
     // raised only (under a lock): handles of other shapes launch concurrently
     allow_dynamic_smem((const void*)kern, smem);
-    kern<<<kSC * a.ndirs, kST, smem, s>>>(a);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = sc;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(sc * a.ndirs);
+    cfg.blockDim = dim3(kST);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (sc > 8) {
+      if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return -2;
+      }
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+        (void)cudaGetLastError();
+        return -2;
+      }
+    }
+    return (int)cudaLaunchKernelEx(&cfg, kern, a);
   };
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
-  if (C == 16) go(k_k0_search<16>);
-  else if (C == 8) go(k_k0_search<8>);
-  else go(k_k0_search<4>);
+  auto by_chunk = [&]<int SC>() {
+    switch (search_chunk(a.nx, a.ny, SC)) {
+      case 16: return go(k_k0_search<16, SC>, 16, SC);
+      case 12: return go(k_k0_search<12, SC>, 12, SC);
+      case 8: return go(k_k0_search<8, SC>, 8, SC);
+      case 4: return go(k_k0_search<4, SC>, 4, SC);
+      default: return -1;
+    }
+  };
+  int rc = -2;
+  if (search_ctas(a.nx, a.ny) == 16) rc = by_chunk.template operator()<16>();
+  if (rc == -2) rc = by_chunk.template operator()<8>();
+  if (rc != 0) return rc;
   if (kt) kt->end("k_k0_search", s, (double)a.ndirs * a.nx * a.ny * sizeof(float2));
   if (launches) *launches += 1;
   return (int)cudaGetLastError();

@@ -185,7 +185,7 @@ struct K0SearchArgs {
 };
 // whether the search's phase tables fit a CTA's shared memory at this size
 bool k0_search_supported(int nx, int ny);
-// one thread-block cluster (8 CTAs) per direction, all directions at once:
+// one thread-block cluster (8 or 16 CTAs) per direction, all directions at once:
 // both line searches, their parabola fits and the amplitude at the fitted k0
 // (fitk0andmodamps, gpuFunctionsImpl.cu:874-1020)
 int launch_k0_search(const K0SearchArgs& a, cudaStream_t s, long long* launches);
