@@ -66,35 +66,56 @@ __global__ void __launch_bounds__(kMoThreads) k_mo_section(float* psf, float* bg
   if (use_const) {
     if (threadIdx.x == 0) s_bg = bgconst;
   } else {
-    double s = 0.0;
-    for (int t = threadIdx.x; t < nx * ny; t += blockDim.x) {
-      int y = t / nx, x = t - y * nx;
-      if (y < kBorder || y > ny - kBorder || x < kBorder || x > nx - kBorder) s += (double)sec[t];
+    // a thread's sum as a float pair (the rounding error of every addition
+    // kept; the FP64 adder has a sixtyfourth of the FP32 rate here)
+    float hi = 0.f, lo = 0.f;
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int y = threadIdx.x >> 5; y < ny; y += nw) {
+      const bool full = y < kBorder || y > ny - kBorder;
+      const float* row = sec + (size_t)y * nx;
+      for (int x0 = lane; x0 < nx; x0 += 128) {
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int x = x0 + 32 * q;
+          v[q] = x < nx && (full || x < kBorder || x > nx - kBorder) ? row[x] : 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float h = __fadd_rn(hi, v[q]), w = __fsub_rn(h, hi);
+          lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(h, w)), __fsub_rn(v[q], w)));
+          hi = h;
+        }
+      }
     }
+    double s = (double)hi + (double)lo;
     s = block_sum_d(s, red);
     if (threadIdx.x == 0) s_bg = (float)(s / border_count);
   }
   __syncthreads();
   if (threadIdx.x == 0) bg[blockIdx.x] = s_bg;
-  // apodize: columns (top/bottom rows) first, then rows (left/right columns)
-  for (int k = threadIdx.x; k < nx; k += blockDim.x) {
-    float d = __fdiv_rn(__fsub_rn(sec[(size_t)(ny - 1) * nx + k], sec[k]), 2.f);
+  // apodize: columns (top/bottom rows) first, then rows (left/right columns);
+  // a line's 2 kNapodize values (sections are at least 2 kNapodize wide and
+  // high, so they are distinct) are loaded together
+  static_assert(kBorder >= 2 * kNapodize, "the two edges of a line must not overlap");
+  auto blend = [&](float* line, size_t step, int n) {
+    float lo[kNapodize], hi[kNapodize];
+#pragma unroll
     for (int l = 0; l < kNapodize; ++l) {
-      float df = __fmul_rn(d, fact.f[l]);
-      sec[(size_t)l * nx + k] = __fadd_rn(sec[(size_t)l * nx + k], df);
-      sec[(size_t)(ny - 1 - l) * nx + k] = __fsub_rn(sec[(size_t)(ny - 1 - l) * nx + k], df);
+      lo[l] = line[l * step];
+      hi[l] = line[(n - 1 - l) * step];
     }
-  }
+    const float d = __fdiv_rn(__fsub_rn(hi[0], lo[0]), 2.f);
+#pragma unroll
+    for (int l = 0; l < kNapodize; ++l) {
+      const float df = __fmul_rn(d, fact.f[l]);
+      line[l * step] = __fadd_rn(lo[l], df);
+      line[(n - 1 - l) * step] = __fsub_rn(hi[l], df);
+    }
+  };
+  for (int k = threadIdx.x; k < nx; k += blockDim.x) blend(sec + k, nx, ny);
   __syncthreads();
-  for (int l = threadIdx.x; l < ny; l += blockDim.x) {
-    float* row = sec + (size_t)l * nx;
-    float d = __fdiv_rn(__fsub_rn(row[nx - 1], row[0]), 2.f);
-    for (int k = 0; k < kNapodize; ++k) {
-      float df = __fmul_rn(d, fact.f[k]);
-      row[k] = __fadd_rn(row[k], df);
-      row[nx - 1 - k] = __fsub_rn(row[nx - 1 - k], df);
-    }
-  }
+  for (int l = threadIdx.x; l < ny; l += blockDim.x) blend(sec + (size_t)l * nx, 1, nx);
 }
 
 // ------------------------------------------------------------------- centre
@@ -270,15 +291,16 @@ __global__ void __launch_bounds__(kMoThreads) k_mo_fft_rows(float2* data, int n,
 }
 
 // forward transform of the columns c < ncols of length n at element stride
-// es; blockIdx.y selects the outer index (base offset blockIdx.y * ostride)
+// es; blockIdx.y selects the outer index (base offset blockIdx.y * ostride),
+// blockIdx.z the band (offset bstride)
 template <int NF>
 __global__ void __launch_bounds__(kMoThreads) k_mo_fft_cols(float2* data, int n, size_t es, int ncols,
-                                                            size_t ostride, FFTPlan plan, int W)
+                                                            size_t ostride, FFTPlan plan, int W, size_t bstride)
 {
   extern __shared__ float2 sm[];
   const int c0 = blockIdx.x * W;
   const int ld = W + 1;
-  float2* base = data + (size_t)blockIdx.y * ostride;
+  float2* base = data + (size_t)blockIdx.y * ostride + blockIdx.z * bstride;
   for (int t = threadIdx.x; t < n * W; t += blockDim.x) {
     int i = t / W, w = t - i * W;
     sm[i * ld + w] = (c0 + w < ncols) ? base[(size_t)i * es + c0 + w] : make_float2(0.f, 0.f);
@@ -298,20 +320,85 @@ struct ShiftCompArgs {
   float k0x[kMoMaxPhases];   // per order
   float k0y[kMoMaxPhases];
   float radius, limit;       // bead radius, sphere FT at the origin (float)
+  float c_hi, c_lo;          // 2 pi radius / 6 as a float pair
+  float g_hi, g_lo;          // (4 pi radius^3 / 3) / limit as a float pair
 };
 
+// sphereFT(rho) / limit of beadsize_compensate (radialft.cpp:784-841,
+// 1155-1167) by the power series of the sphere's form factor,
+//   3 (sin x - x cos x) / x^3 = sum_k a_k x^2k,  a_k = (-1)^k 6 (k + 1) / (2k + 3)!,
+// x = 2 pi radius rho, in powers of (x / 6)^2 and float pairs (48 bits; the FP64 unit has a
+// sixtyfourth of the FP32 rate here): 18 terms reach 1e-16 up to x = 6.
+// Larger x, and values near the form factor's zeros, take the closed form in
+// double.
+constexpr int kSphereTerms = 18;
+struct SphereCoef {
+  float hi[kSphereTerms], lo[kSphereTerms];
+  __host__ __device__ constexpr SphereCoef() : hi{}, lo{}
+  {
+    double a = 1.0;  // a_0
+    for (int k = 0; k < kSphereTerms; ++k) {
+      hi[k] = (float)a;
+      lo[k] = (float)(a - (double)hi[k]);
+      a = -a * 36.0 / ((2.0 * k + 2.0) * (2.0 * k + 5.0));
+    }
+  }
+};
+
+// (ah, al) * (bh, bl), the product's rounding error kept
+__device__ __forceinline__ float2 pair_mul(float2 a, float bh, float bl)
+{
+  const float h = __fmul_rn(a.x, bh);
+  float l = fmaf(a.x, bh, -h);
+  l = fmaf(a.x, bl, l);
+  l = fmaf(a.y, bh, l);
+  const float s = __fadd_rn(h, l);
+  return make_float2(s, __fsub_rn(l, __fsub_rn(s, h)));
+}
+
+__device__ __forceinline__ float sphere_ratio(const ShiftCompArgs& a, float rho)
+{
+  const float2 x = pair_mul(make_float2(rho, 0.f), a.c_hi, a.c_lo);
+  if (x.x <= 1.f) {
+    constexpr SphereCoef co;
+    const float2 u = pair_mul(x, x.x, x.y);
+    float2 s = make_float2(co.hi[kSphereTerms - 1], co.lo[kSphereTerms - 1]);
+#pragma unroll
+    for (int k = kSphereTerms - 2; k >= 0; --k) {
+      const float2 p = pair_mul(s, u.x, u.y);
+      const float h = __fadd_rn(co.hi[k], p.x), v = __fsub_rn(h, co.hi[k]);
+      const float l = __fadd_rn(__fadd_rn(__fsub_rn(co.hi[k], __fsub_rn(h, v)), __fsub_rn(p.x, v)),
+                                __fadd_rn(co.lo[k], p.y));
+      const float t = __fadd_rn(h, l);
+      s = make_float2(t, __fsub_rn(l, __fsub_rn(t, h)));
+    }
+    if (fabsf(s.x) > 1e-3f) return pair_mul(s, a.g_hi, a.g_lo).x;
+  }
+  double sph;
+  if (rho > 0.f || rho < 0.f) {
+    double xx = 2.0 * M_PI * (double)a.radius * (double)rho;
+    sph = (double)a.radius / (M_PI * (double)rho * (double)rho) * (sin(xx) / xx - cos(xx));
+  } else {
+    sph = 4.0 * M_PI * pow((double)a.radius, 3.0) / 3.0;
+  }
+  return (float)(sph / (double)a.limit);
+}
+
+// blockIdx.y: the order; its one or two bands share the shift's rotation and
+// the compensation.  Bound by HBM and the series' issue: 128^2 x 64 x 5 with
+// the closed form in double for every band 370 us, 73 us here (cold caches).
 __global__ void __launch_bounds__(kMoThreads) k_mo_shift_comp(float2* bands, const float* center, ShiftCompArgs a)
 {
   const int nxh = a.nx / 2 + 1;
-  const int b = blockIdx.y;
-  const int order = (b + 1) / 2;
+  const int order = blockIdx.y;
   const size_t nh = (size_t)a.nz * a.ny * nxh;
   const float xc = center[0], yc = center[1], zc = center[2];
   // radialft.cpp:853-855: 2*M_PI*c/n in double, stored as float
   const float dphiz = (float)(2.0 * M_PI * (double)zc / a.nz);
   const float dphiy = (float)(2.0 * M_PI * (double)yc / a.ny);
   const float dphix = (float)(2.0 * M_PI * (double)xc / a.nx);
-  float2* band = bands + (size_t)b * a.nz * a.ny * a.nx;
+  const size_t vol = (size_t)a.nz * a.ny * a.nx;
+  const int b0 = order == 0 ? 0 : 2 * order - 1, b1 = order == 0 ? 0 : min(2 * order, a.nph - 1);
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nh; t += (size_t)gridDim.x * blockDim.x) {
     int x = (int)(t % nxh);
     size_t r = t / nxh;
@@ -321,51 +408,68 @@ __global__ void __launch_bounds__(kMoThreads) k_mo_shift_comp(float2* bands, con
     float phi = __fadd_rn(__fadd_rn(__fmul_rn(dphiz, (float)kz), __fmul_rn(dphiy, (float)ky)),
                           __fmul_rn(dphix, (float)x));
     float c = cosf(phi), s = sinf(phi);
-    size_t idx = ((size_t)z * a.ny + y) * a.nx + x;
-    float2 v = band[idx];
-    float2 w = make_float2(__fsub_rn(__fmul_rn(v.x, c), __fmul_rn(v.y, s)),
-                           __fadd_rn(__fmul_rn(v.x, s), __fmul_rn(v.y, c)));
-    if (a.compensate && !(order == 0 && t == 0)) {
+    const bool comp = a.compensate && !(order == 0 && t == 0);
+    float ratio = 1.f;
+    if (comp) {
       float fkz = __fmul_rn((float)kz, a.dkz);
       float fky = __fadd_rn(__fmul_rn((float)ky, a.dky), a.k0y[order]);
       float fkx = __fadd_rn(__fmul_rn((float)x, a.dkx), a.k0x[order]);
       float rho = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(fkz, fkz), __fmul_rn(fky, fky)), __fmul_rn(fkx, fkx)));
-      double sph;
-      if (rho > 0.f || rho < 0.f) {
-        double xx = 2.0 * M_PI * (double)a.radius * (double)rho;
-        sph = (double)a.radius / (M_PI * (double)rho * (double)rho) * (sin(xx) / xx - cos(xx));
-      } else {
-        sph = 4.0 * M_PI * pow((double)a.radius, 3.0) / 3.0;
-      }
-      float ratio = (float)(sph / (double)a.limit);
-      w.x = __fdiv_rn(w.x, ratio);
-      w.y = __fdiv_rn(w.y, ratio);
+      ratio = sphere_ratio(a, rho);
     }
-    band[idx] = w;
+    for (int b = b0; b <= b1; ++b) {
+      float2* e = bands + b * vol + ((size_t)z * a.ny + y) * a.nx + x;
+      const float2 v = *e;
+      float2 w = make_float2(__fsub_rn(__fmul_rn(v.x, c), __fmul_rn(v.y, s)),
+                             __fadd_rn(__fmul_rn(v.x, s), __fmul_rn(v.y, c)));
+      if (comp) {
+        w.x = __fdiv_rn(w.x, ratio);
+        w.y = __fdiv_rn(w.y, ratio);
+      }
+      *e = w;
+    }
   }
 }
 
 // ------------------------------------------------------------ radial average
-// thread per (band, kz, bin): float sums over the bin's pixels in the
-// reference's order (ky rows, then kx), then / count (radialft.cpp:893-921)
+// warp per (band, kz, bin): float sums over the bin's pixels in the
+// reference's order (ky rows, then kx), then / count (radialft.cpp:893-921).
+// The lanes load 32 pixels at a time and every lane adds them in order: a
+// bin's additions are one chain, its loads are not (a thread per bin waited
+// for each: 66 us at 128^2 x 64 x 5, 26 us here).
 __global__ void __launch_bounds__(128) k_mo_radial(const float2* __restrict__ bands, const int* __restrict__ bin_start,
                                                    const int* __restrict__ bin_pix, int nbins, int nx, int ny, int nz,
                                                    float2* avg)
 {
-  const int bin = blockIdx.x * blockDim.x + threadIdx.x;
+  const int bin = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int kz = blockIdx.y, b = blockIdx.z;
   if (bin >= nbins) return;
   const int nxh = nx / 2 + 1;
   const float2* plane = bands + ((size_t)b * nz + kz) * ny * nx;
   const int s0 = bin_start[bin], s1 = bin_start[bin + 1];
   float re = 0.f, im = 0.f;
-  for (int i = s0; i < s1; ++i) {
-    int p = bin_pix[i];
-    int y = p / nxh, x = p - y * nxh;
-    float2 v = plane[(size_t)y * nx + x];
-    re = __fadd_rn(re, v.x);
-    im = __fadd_rn(im, v.y);
+  for (int i0 = s0; i0 < s1; i0 += 32) {
+    const int n = min(32, s1 - i0);
+    float2 v = make_float2(0.f, 0.f);
+    if (lane < n) {
+      const int p = bin_pix[i0 + lane];
+      const int y = p / nxh, x = p - y * nxh;
+      v = plane[(size_t)y * nx + x];
+    }
+    if (n == 32) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        re = __fadd_rn(re, __shfl_sync(0xffffffffu, v.x, i));
+        im = __fadd_rn(im, __shfl_sync(0xffffffffu, v.y, i));
+      }
+    } else {
+      for (int i = 0; i < n; ++i) {
+        re = __fadd_rn(re, __shfl_sync(0xffffffffu, v.x, i));
+        im = __fadd_rn(im, __shfl_sync(0xffffffffu, v.y, i));
+      }
+    }
   }
+  if (lane != 0) return;
   const int cnt = s1 - s0;
   float2 r = make_float2(re, im);
   if (cnt > 0) r = make_float2(__fdiv_rn(re, (float)cnt), __fdiv_rn(im, (float)cnt));
@@ -391,16 +495,19 @@ __global__ void __launch_bounds__(1024) k_mo_finish(float2* avg, FinishArgs a, f
   __shared__ float s_scale;
   __shared__ double s_sums[64];
   const int nz = a.nz, nb = a.nbins;
-  // Hermitian symmetry along kz per (band, bin)
-  for (int t = threadIdx.x; t < a.nph * nb; t += blockDim.x) {
-    float2* r = avg + (size_t)t * nz;
-    r[0].y = 0.f;
-    for (int kz = 1; kz <= nz / 2; ++kz) {
-      float2 u = r[kz], w = r[nz - kz];
-      float2 v = make_float2(__fdiv_rn(__fadd_rn(u.x, w.x), 2.f), __fdiv_rn(__fsub_rn(u.y, w.y), 2.f));
-      r[kz] = v;
-      r[nz - kz] = make_float2(v.x, -v.y);
+  // Hermitian symmetry along kz per (band, bin), a thread per (row, kz pair)
+  const int half = nz / 2;
+  for (int t = threadIdx.x; t < a.nph * nb * (half + 1); t += blockDim.x) {
+    const int row = t / (half + 1), kz = t - row * (half + 1);
+    float2* r = avg + (size_t)row * nz;
+    if (kz == 0) {
+      r[0].y = 0.f;
+      continue;
     }
+    float2 u = r[kz], w = r[nz - kz];
+    float2 v = make_float2(__fdiv_rn(__fadd_rn(u.x, w.x), 2.f), __fdiv_rn(__fsub_rn(u.y, w.y), 2.f));
+    r[kz] = v;
+    r[nz - kz] = make_float2(v.x, -v.y);
   }
   __syncthreads();
   if (threadIdx.x == 0) s_scale = 1.f;
@@ -457,12 +564,13 @@ __global__ void __launch_bounds__(1024) k_mo_finish(float2* avg, FinishArgs a, f
     __syncthreads();
     // fixorigin on band 0 (radialft.cpp:1188-1224)
     if (p == 0 && a.fix_kx1 > 0) {
-      for (int i = threadIdx.x; i <= a.fix_kx2; i += blockDim.x) {
+      // a warp per kr: the lanes' double sums, then across the warp
+      const int lane = threadIdx.x & 31;
+      for (int i = threadIdx.x >> 5; i <= a.fix_kx2; i += blockDim.x >> 5) {
         double s = 0.0;
-        if (i == 0) s = o[0].x;
-        else
-          for (int j = 0; j < nz; ++j) s += o[(size_t)i * nz + j].x;
-        s_sums[i] = s;
+        for (int j = lane; j < (i == 0 ? 1 : nz); j += 32) s += o[(size_t)i * nz + j].x;
+        for (int q = 16; q > 0; q >>= 1) s += __shfl_down_sync(0xffffffffu, s, q);
+        if (lane == 0) s_sums[i] = s;
       }
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -724,6 +832,10 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
     const float k0mag = 1 / o.ls;
     sc.radius = (float)(o.beaddiam * 0.5);
     sc.limit = (float)(4 * M_PI * sc.radius * sc.radius * sc.radius / 3);
+    const double c = 2.0 * M_PI * (double)sc.radius / 6.0;
+    const double g = 4.0 * M_PI * std::pow((double)sc.radius, 3.0) / 3.0 / (double)sc.limit;
+    sc.c_hi = (float)c, sc.c_lo = (float)(c - (double)sc.c_hi);
+    sc.g_hi = (float)g, sc.g_lo = (float)(g - (double)sc.g_hi);
     for (int ord = 0; ord < norders; ++ord) {
       volatile float frac = ((float)ord) / (norders - 1);  // 0/0 for one order, as the reference
       sc.k0x[ord] = frac * k0mag * std::cos(o.angle);
@@ -807,21 +919,20 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
     dispatch_fft_len(kSiteMakeOtf, ny, [&]<int NF>() {
       set_smem(k_mo_fft_cols<NF>, smy);
       k_mo_fft_cols<NF><<<dim3((nxh + Wy - 1) / Wy, nph * nz), kMoThreads, smy, s>>>(d_bands, ny, (size_t)nx, nxh,
-                                                                                     nxy, py, Wy);
+                                                                                     nxy, py, Wy, 0);
     });
     if (nz > 1) {
       int Wz = std::max(1, std::min(32, kFftElems / nz));
       size_t smz = fft_stage_smem(nz, Wz, nz * (Wz + 1), kMoThreads);
       dispatch_fft_len(kSiteMakeOtf, nz, [&]<int NF>() {
         set_smem(k_mo_fft_cols<NF>, smz);
-        for (int b = 0; b < nph; ++b)
-          k_mo_fft_cols<NF><<<dim3((nxh + Wz - 1) / Wz, ny), kMoThreads, smz, s>>>(d_bands + (size_t)b * nvox, nz,
-                                                                                   nxy, nxh, (size_t)nx, pz, Wz);
+        k_mo_fft_cols<NF><<<dim3((nxh + Wz - 1) / Wz, ny, nph), kMoThreads, smz, s>>>(d_bands, nz, nxy, nxh,
+                                                                                     (size_t)nx, pz, Wz, nvox);
       });
     }
   }
-  k_mo_shift_comp<<<dim3(2 * 152, nph), kMoThreads, 0, s>>>(d_bands, d_center, sc);
-  k_mo_radial<<<dim3((nbins + 127) / 128, nz, nph), 128, 0, s>>>(d_bands, d_bstart, d_bpix, nbins, nx, ny, nz,
+  k_mo_shift_comp<<<dim3(8 * 152, nph / 2 + 1), kMoThreads, 0, s>>>(d_bands, d_center, sc);
+  k_mo_radial<<<dim3((nbins + 3) / 4, nz, nph), 128, 0, s>>>(d_bands, d_bstart, d_bpix, nbins, nx, ny, nz,
                                                                  d_avg);
   k_mo_finish<<<1, 1024, 0, s>>>(d_avg, fa, d_out, d_scal);
   cudaEventRecord(ev1, s);
