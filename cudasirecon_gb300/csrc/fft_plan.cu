@@ -101,13 +101,14 @@ namespace {
 const char* const kSiteNames[kNumFftSites] = {"ingest_x", "ingest_y", "separate_z", "overlap_x", "overlap_y",
                                               "crosscorr_rows", "crosscorr_cols", "assemble_y", "assemble_x",
                                               "assemble_z", "makeotf", "selftest"};
-thread_local int t_force_site = -1, t_force_reg = 0;
+const char* const kPathNames[kNumFftPaths] = {"stockham", "register", "two-factor"};
+thread_local int t_force_site = -1, t_force_path = 0;
 thread_local std::set<std::pair<int, int>>* t_seen = nullptr;
 
 struct Tuned {
   bool loaded = false;
-  // (gpu name, site, n) -> register path?
-  std::map<std::tuple<std::string, int, int>, std::pair<bool, std::pair<double, double>>> table;
+  // (gpu name, site, n) -> path, its time and the best other path's
+  std::map<std::tuple<std::string, int, int>, std::pair<int, std::pair<double, double>>> table;
 };
 std::mutex g_tuned_mu;
 Tuned g_tuned;
@@ -159,8 +160,11 @@ void load_tuned()
     if (col.size() < 6) continue;
     const int site = site_index(col[1]);
     const int n = std::atoi(col[2].c_str());
-    if (site < 0 || n <= 0 || (col[3] != "register" && col[3] != "stockham")) continue;
-    g_tuned.table[{col[0], site, n}] = {col[3] == "register", {std::atof(col[4].c_str()), std::atof(col[5].c_str())}};
+    int path = -1;
+    for (int q = 0; q < kNumFftPaths; ++q)
+      if (col[3] == kPathNames[q]) path = q;
+    if (site < 0 || n <= 0 || path < 0) continue;
+    g_tuned.table[{col[0], site, n}] = {path, {std::atof(col[4].c_str()), std::atof(col[5].c_str())}};
   }
 }
 
@@ -187,7 +191,7 @@ bool save_tuned(std::string* err)
     }
     for (auto& [k, v] : g_tuned.table)
       f << std::get<0>(k) << '\t' << kSiteNames[std::get<1>(k)] << '\t' << std::get<2>(k) << '\t'
-        << (v.first ? "register" : "stockham") << '\t' << v.second.first << '\t' << v.second.second << '\n';
+        << kPathNames[v.first] << '\t' << v.second.first << '\t' << v.second.second << '\n';
   }
   if (std::rename(tmp.c_str(), path.c_str()) != 0) {
     *err = "cannot replace the FFT plan cache " + path;
@@ -216,34 +220,55 @@ bool builtin_choice(FftSite site, int n)
 }
 }  // namespace
 
-bool reg_fft_site_enabled(FftSite site, int n)
+namespace {
+// what was chosen for (site, n) by a force, the environment or the plan
+// cache; -1: nothing, the built-in choice holds
+int chosen_path(int site, int n)
 {
-  if (t_seen) t_seen->insert({(int)site, n});
-  if (t_force_site == (int)site) return t_force_reg != 0;
+  if (t_force_site == site) return t_force_path;
   static const int forced = [] {
     const char* e = std::getenv("SIMRECON_FFT_REGISTER_SITES");
     return e ? (int)(std::strtoul(e, nullptr, 16) | (1u << kSiteSelfTest)) : -1;
   }();
-  if (forced >= 0) return (forced >> (int)site) & 1;
+  if (forced >= 0) return (forced >> site) & 1;
   if (site != kSiteSelfTest && reg_fft_lanes(n)) {
     std::lock_guard<std::mutex> lk(g_tuned_mu);
     load_tuned();
-    auto it = g_tuned.table.find({device_name(), (int)site, n});
+    auto it = g_tuned.table.find({device_name(), site, n});
     if (it != g_tuned.table.end()) return it->second.first;
   }
-  return builtin_choice(site, n);
+  return -1;
+}
+}  // namespace
+
+bool reg_fft_site_enabled(FftSite site, int n)
+{
+  if (t_seen) t_seen->insert({(int)site, n});
+  const int c = chosen_path(site, n);
+  return c >= 0 ? c == kPathRegister : builtin_choice(site, n);
 }
 
-void fft_site_force(int site, bool reg) { t_force_site = site, t_force_reg = reg; }
+bool fft_two_factor(FftSite site, int n)
+{
+  int r1, r2;
+  if (!tf_factor(n, &r1, &r2)) return false;
+  if (!reg_fft_lanes(n)) return true;
+  if (t_seen) t_seen->insert({(int)site, n});
+  const int c = chosen_path(site, n);
+  return c < 0 || c == kPathTwoFactor;
+}
+
+void fft_site_force(int site, int path) { t_force_site = site, t_force_path = path; }
 void fft_site_unforce() { t_force_site = -1; }
 void fft_sites_track(std::set<std::pair<int, int>>* seen) { t_seen = seen; }
+const char* fft_path_name(int path) { return path >= 0 && path < kNumFftPaths ? kPathNames[path] : "?"; }
 const char* fft_site_name(int site) { return site >= 0 && site < kNumFftSites ? kSiteNames[site] : "?"; }
 
-bool fft_plan_record(int site, int n, bool reg, double ms_reg, double ms_stockham, std::string* err)
+bool fft_plan_record(int site, int n, int path, double ms, double ms_other, std::string* err)
 {
   std::lock_guard<std::mutex> lk(g_tuned_mu);
   load_tuned();
-  g_tuned.table[{device_name(), site, n}] = {reg, {ms_reg, ms_stockham}};
+  g_tuned.table[{device_name(), site, n}] = {path, {ms, ms_other}};
   return save_tuned(err);
 }
 
@@ -259,7 +284,7 @@ int fft_plan_choice(int site, int n, const char** source)
     r = 0;
   } else if (t_force_site == site) {
     src = "forced";
-    r = t_force_reg;
+    r = t_force_path == kPathRegister;
   } else if (std::getenv("SIMRECON_FFT_REGISTER_SITES")) {
     src = "environment";
     r = reg_fft_site_enabled((FftSite)site, n);
@@ -269,7 +294,7 @@ int fft_plan_choice(int site, int n, const char** source)
     auto it = g_tuned.table.find({device_name(), site, n});
     if (it != g_tuned.table.end()) {
       src = "tuned";
-      r = it->second.first;
+      r = it->second.first == kPathRegister;
     } else {
       r = builtin_choice((FftSite)site, n);
     }

@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "col_fft.cuh"
+#include "findk0.cuh"
 #include "kernels.h"
 #include "reg_fft.cuh"
 #include "tf_kernels.h"
@@ -36,21 +37,12 @@ constexpr int kThreads = 256;
 constexpr int kMaxElems = kFftElems;
 
 // ---------------------------------------------------------------- overlaps
-// the shift k0 * (order2 - order1): from the arguments, or from device memory
-// (a k0 fitted on the device) times kfac
-__device__ __forceinline__ float2 ovl_shift(const OverlapArgs& a)
-{
-  if (a.kdev == nullptr) return make_float2(a.kx, a.ky);
-  const float2 k = *a.kdev;
-  return make_float2(__fmul_rn(k.x, a.kfac), __fmul_rn(k.y, a.kfac));
-}
-
 // Element (j) of overlap `ov` on row (zb, i) before the x transform:
 // makeOverlaps0Kernel (ov 0, gpuFunctionsImpl.cu:677-778) / makeOverlaps1Kernel
 // (ov 1, 780-872): the order-1/order-2 band value times the partner OTF over
 // sqrt(|OTF1|^2 + |OTF2|^2) inside both supports, merged re + i im.
 // kzi = otf_kz(a.otf, zb - a.zdc), rdk = 1 / a.otf.dkrotf (per row / thread)
-__device__ __forceinline__ float2 ovl_value(const OverlapArgs& a, float2 ks, int ov, int zb, int i, int j,
+__device__ __forceinline__ float2 ovl_value(const OverlapArgs& a, const OvlItem& it, float2 ks, int ov, int zb, int i, int j,
                                             const OtfKz& kzi, float rdk)
 {
   const int nx = a.nx, ny = a.ny, nz = a.nz, nxh = nx / 2 + 1;
@@ -74,15 +66,15 @@ __device__ __forceinline__ float2 ovl_value(const OverlapArgs& a, float2 ks, int
     float x12 = x1f - ks.x, y12 = y1f - ks.y;
     const float r12sq = x12 * x12 + y12 * y12;
     if (r12sq <= a.r2_le) {  // r12 <= cut
-      float2 o1 = otf_lookup_rr(a.otf.otf[a.order1], a.otf, sqrtf(r1sq) * rdk, kzi);
+      float2 o1 = otf_lookup_rr(it.otf1, a.otf, sqrtf(r1sq) * rdk, kzi);
       if (cmag2(o1) > a.m_le) {  // |OTF1| > otfcutoff
-        float2 o12 = otf_lookup_rr(a.otf.otf[a.order2], a.otf, sqrtf(r12sq) * rdk, kzi);
+        float2 o12 = otf_lookup_rr(it.otf2, a.otf, sqrtf(r12sq) * rdk, kzi);
         if (cmag2(o12) >= a.m_f) {  // |OTF12| * factor > otfcutoff
           const float rroot = 1.f / sqrtf(cmag2(o1) + cmag2(o12));
           float2 fact = make_float2(o12.x * rroot, o12.y * rroot);
-          const float2* b1re = a.order1 == 0 ? a.bands : a.bands + (size_t)(2 * a.order1 - 1) * nz * bplane;
+          const float2* b1re = it.order1 == 0 ? it.bands : it.bands + (size_t)(2 * it.order1 - 1) * nz * bplane;
           float2 vre = b1re[indin];
-          float2 vim = a.order1 == 0 ? make_float2(0.f, 0.f) : a.bands[(size_t)(2 * a.order1) * nz * bplane + indin];
+          float2 vim = it.order1 == 0 ? make_float2(0.f, 0.f) : it.bands[(size_t)(2 * it.order1) * nz * bplane + indin];
           if (conj) {
             vre.y = -vre.y;
             vim.y = -vim.y;
@@ -97,14 +89,14 @@ __device__ __forceinline__ float2 ovl_value(const OverlapArgs& a, float2 ks, int
     float x21 = x1f + ks.x, y21 = y1f + ks.y;
     const float r21sq = x21 * x21 + y21 * y21;
     if (r21sq <= a.r2_le) {  // r21 <= cut
-      float2 o2 = otf_lookup_rr(a.otf.otf[a.order2], a.otf, sqrtf(r1sq) * rdk, kzi);
+      float2 o2 = otf_lookup_rr(it.otf2, a.otf, sqrtf(r1sq) * rdk, kzi);
       if (cmag2(o2) >= a.m_f) {  // |OTF2| * factor > otfcutoff
-        float2 o21 = otf_lookup_rr(a.otf.otf[a.order1], a.otf, sqrtf(r21sq) * rdk, kzi);
+        float2 o21 = otf_lookup_rr(it.otf1, a.otf, sqrtf(r21sq) * rdk, kzi);
         if (cmag2(o21) > a.m_le) {  // |OTF21| > otfcutoff
           const float rroot = 1.f / sqrtf(cmag2(o2) + cmag2(o21));
           float2 fact = make_float2(o21.x * rroot, o21.y * rroot);
-          float2 vre = a.bands[(size_t)(2 * a.order2 - 1) * nz * bplane + indin];
-          float2 vim = a.bands[(size_t)(2 * a.order2) * nz * bplane + indin];
+          float2 vre = it.bands[(size_t)(2 * it.order2 - 1) * nz * bplane + indin];
+          float2 vim = it.bands[(size_t)(2 * it.order2) * nz * bplane + indin];
           if (conj) {
             vre.y = -vre.y;
             vim.y = -vim.y;
@@ -120,14 +112,15 @@ __device__ __forceinline__ float2 ovl_value(const OverlapArgs& a, float2 ks, int
 }
 
 template <int NF>
-__global__ void __launch_bounds__(kThreads) k_ovl_build_x(OverlapArgs a, FFTPlan plan, int rows_per_cta, int ldl)
+__global__ void __launch_bounds__(kThreads) k_ovl_build_x(const __grid_constant__ OverlapArgs a, FFTPlan plan, int rows_per_cta, int ldl)
 {
   extern __shared__ float2 sm[];
   const int nx = a.nx, ny = a.ny;
   const int nzb = 2 * a.zdc + 1;
   const int row0 = blockIdx.x * rows_per_cta;
   const int nrows = min(rows_per_cta, nzb * ny - row0);
-  const float2 ks = ovl_shift(a);
+  const OvlItem& it = a.item[blockIdx.z];
+  const float2 ks = ovl_shift(it);
   for (int t = threadIdx.x; t < 2 * rows_per_cta * nx; t += blockDim.x) {
     int l = t / nx, j = t - l * nx;
     int r = l >> 1, ov = l & 1;
@@ -135,7 +128,7 @@ __global__ void __launch_bounds__(kThreads) k_ovl_build_x(OverlapArgs a, FFTPlan
     if (r < nrows) {
       int row = row0 + r;
       int zb = row / ny, i = row - zb * ny;
-      val = ovl_value(a, ks, ov, zb, i, j, otf_kz(a.otf, zb - a.zdc), 1.f / a.otf.dkrotf);
+      val = ovl_value(a, it, ks, ov, zb, i, j, otf_kz(a.otf, zb - a.zdc), 1.f / a.otf.dkrotf);
     }
     sm[l * ldl + j] = val;
   }
@@ -145,7 +138,7 @@ __global__ void __launch_bounds__(kThreads) k_ovl_build_x(OverlapArgs a, FFTPlan
   for (int t = threadIdx.x; t < 2 * nrows * nx; t += blockDim.x) {
     int l = t / nx, j = t - l * nx;
     int r = l >> 1, ov = l & 1;
-    a.ovl[(size_t)ov * vol + (size_t)(row0 + r) * nx + j] = res[l * ldl + j];
+    it.ovl[(size_t)ov * vol + (size_t)(row0 + r) * nx + j] = res[l * ldl + j];
   }
 }
 
@@ -163,7 +156,7 @@ constexpr int kOvlWarps = 4;
 // its resident warps (per 512^2 x 48 volume: 0.64 ms with three CTAs, 0.55
 // with four, 0.51 with five, 0.54 with six and spills)
 template <int N>
-__global__ void __launch_bounds__(kOvlWarps * 32, 5) k_ovl_build_xw(OverlapArgs a, const float2* __restrict__ twr)
+__global__ void __launch_bounds__(kOvlWarps * 32, 5) k_ovl_build_xw(const __grid_constant__ OverlapArgs a, const float2* __restrict__ twr)
 {
   constexpr int P = OvlLanes<N>::P, E = N / P, G = 32 / P;
   constexpr int XB = (P + 1) * E + 1;
@@ -177,7 +170,8 @@ __global__ void __launch_bounds__(kOvlWarps * 32, 5) k_ovl_build_xw(OverlapArgs 
   // build the warp's G lines (all 32 lanes, consecutive j); the kz part of
   // the OTF lookups is the same along a line
   const float rdk = 1.f / a.otf.dkrotf;
-  const float2 ks = ovl_shift(a);
+  const OvlItem& it = a.item[blockIdx.z];
+  const float2 ks = ovl_shift(it);
 #pragma unroll
   for (int gl = 0; gl < G; ++gl) {
     const int L = l0 + gl;
@@ -188,7 +182,7 @@ __global__ void __launch_bounds__(kOvlWarps * 32, 5) k_ovl_build_xw(OverlapArgs 
     const int row = L >> 1, ov = L & 1;
     const int zb = row / ny, i = row - zb * ny;
     const OtfKz kzi = otf_kz(a.otf, zb - a.zdc);
-    for (int j = lane; j < N; j += 32) lines[warp][gl][j] = ovl_value(a, ks, ov, zb, i, j, kzi, rdk);
+    for (int j = lane; j < N; j += 32) lines[warp][gl][j] = ovl_value(a, it, ks, ov, zb, i, j, kzi, rdk);
   }
   __syncwarp();
   float2 v[E];
@@ -199,7 +193,7 @@ __global__ void __launch_bounds__(kOvlWarps * 32, 5) k_ovl_build_xw(OverlapArgs 
   const int L = l0 + g;
   if (L < nlines) {
     const int row = L >> 1, ov = L & 1;
-    float2* dst = a.ovl + (size_t)ov * nzb * ny * N + (size_t)row * N;
+    float2* dst = it.ovl + (size_t)ov * nzb * ny * N + (size_t)row * N;
 #pragma unroll
     for (int m = 0; m < E / P; ++m)
 #pragma unroll
@@ -208,11 +202,12 @@ __global__ void __launch_bounds__(kOvlWarps * 32, 5) k_ovl_build_xw(OverlapArgs 
 }
 
 template <int NF>
-__global__ void __launch_bounds__(kThreads) k_ovl_y_accum(OverlapArgs a, FFTPlan plan, int W, int planes_per_group,
+__global__ void __launch_bounds__(kThreads) k_ovl_y_accum(const __grid_constant__ OverlapArgs a, FFTPlan plan, int W, int planes_per_group,
                                                           int xoff)
 {
   extern __shared__ float2 sm[];
   __shared__ double red[32];
+  const OvlItem& im = a.item[blockIdx.z];
   const int nx = a.nx, ny = a.ny;
   const int nzb = 2 * a.zdc + 1;
   const int c0 = blockIdx.x * W;
@@ -229,7 +224,7 @@ __global__ void __launch_bounds__(kThreads) k_ovl_y_accum(OverlapArgs a, FFTPlan
       int y = t / (2 * W), q = t - y * 2 * W;
       int ov = q >= W, w = q - ov * W;
       sm[y * ld + q] =
-          (c0 + w < nx) ? a.ovl[(size_t)ov * vol + ((size_t)zb * ny + y) * nx + c0 + w] : make_float2(0.f, 0.f);
+          (c0 + w < nx) ? im.ovl[(size_t)ov * vol + ((size_t)zb * ny + y) * nx + c0 + w] : make_float2(0.f, 0.f);
     }
     __syncthreads();
     const float2* res = fft_dispatch<NF, +1>(sm, sm + ny * ld, plan, 2 * W, 1, ld);
@@ -251,7 +246,7 @@ __global__ void __launch_bounds__(kThreads) k_ovl_y_accum(OverlapArgs a, FFTPlan
     sy += (double)py;
   }
   __syncthreads();
-  float2* dst = a.ppart + (size_t)blockIdx.y * ny * nx;
+  float2* dst = im.ppart + (size_t)blockIdx.y * ny * nx;
   for (int t = threadIdx.x; t < ny * W; t += blockDim.x) {
     int y = t / W, w = t - y * W;
     if (c0 + w < nx) dst[(size_t)y * nx + c0 + w] = acc[t];
@@ -260,8 +255,8 @@ __global__ void __launch_bounds__(kThreads) k_ovl_y_accum(OverlapArgs a, FFTPlan
   double ty = block_sum_d(sy, red);
   if (threadIdx.x == 0) {
     int cta = blockIdx.y * gridDim.x + blockIdx.x;
-    a.sums[2 * cta] = tx;
-    a.sums[2 * cta + 1] = ty;
+    im.sums[2 * cta] = tx;
+    im.sums[2 * cta + 1] = ty;
   }
 }
 
@@ -271,7 +266,7 @@ __global__ void __launch_bounds__(kThreads) k_ovl_y_accum(OverlapArgs a, FFTPlan
 // stage 2 gives each thread one (column, k1) of both, and conj(X)Y, |X|^2,
 // |Y|^2 accumulate in registers over the planes.
 template <int N, int R1>
-__global__ void __launch_bounds__(kThreads, 2) k_ovl_y4(OverlapArgs a, const float2* __restrict__ tw,
+__global__ void __launch_bounds__(kThreads, 2) k_ovl_y4(const __grid_constant__ OverlapArgs a, const float2* __restrict__ tw,
                                                     int planes_per_group)
 {
   using CF = ColFft<N, R1, 8>;
@@ -280,6 +275,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_ovl_y4(OverlapArgs a, const flo
   static_assert(R1 * W <= kThreads, "one stage-2 item per thread");
   extern __shared__ float2 sm[];  // 2 * CF::kSmemElems
   __shared__ double red[32];
+  const OvlItem& im = a.item[blockIdx.z];
   const int nx = a.nx, ny = N;
   const int nzb = 2 * a.zdc + 1;
   const int c0 = blockIdx.x * W;
@@ -300,7 +296,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_ovl_y4(OverlapArgs a, const flo
   double sx = 0.0, sy = 0.0;
   for (int zb = zb0; zb < zb1; ++zb) {
     {
-      const float2* src = a.ovl + (size_t)ov1 * vol + (size_t)zb * ny * nx + c0 + c1;
+      const float2* src = im.ovl + (size_t)ov1 * vol + (size_t)zb * ny * nx + c0 + c1;
       float2 v[R1];
 #pragma unroll
       for (int e = 0; e < R1; ++e) v[e] = c1 < nc ? src[(size_t)(j1 + R2 * e) * nx] : make_float2(0.f, 0.f);
@@ -341,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_ovl_y4(OverlapArgs a, const flo
     __syncthreads();
   }
   if (has2 && c2 < nc) {
-    float2* dst = a.ppart + (size_t)blockIdx.y * ny * nx + c0 + c2;
+    float2* dst = im.ppart + (size_t)blockIdx.y * ny * nx + c0 + c2;
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2) dst[(size_t)(k1 + R1 * k2) * nx] = acc[k2];
   }
@@ -349,37 +345,38 @@ __global__ void __launch_bounds__(kThreads, 2) k_ovl_y4(OverlapArgs a, const flo
   double ty = block_sum_d(sy, red);
   if (threadIdx.x == 0) {
     int cta = blockIdx.y * gridDim.x + blockIdx.x;
-    a.sums[2 * cta] = tx;
-    a.sums[2 * cta + 1] = ty;
+    im.sums[2 * cta] = tx;
+    im.sums[2 * cta + 1] = ty;
   }
 }
 
 // P = nz * sum_g Ppart[g];  sumxy = nz * sum of the CTA partial sums
-__global__ void k_p_reduce(OverlapArgs a, int ngroups, int nctas)
+__global__ void k_p_reduce(const __grid_constant__ OverlapArgs a, int ngroups, int nctas)
 {
+  const OvlItem& im = a.item[blockIdx.y];
   __shared__ double red[32];
   const size_t n = (size_t)a.nx * a.ny;
   const float fz = (float)a.nz;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    float2 s = a.ppart[i];
+    float2 s = im.ppart[i];
     for (int g = 1; g < ngroups; ++g) {
-      float2 v = a.ppart[(size_t)g * n + i];
+      float2 v = im.ppart[(size_t)g * n + i];
       s.x += v.x;
       s.y += v.y;
     }
-    a.pmap[i] = make_float2(s.x * fz, s.y * fz);
+    im.pmap[i] = make_float2(s.x * fz, s.y * fz);
   }
   if (blockIdx.x == 0) {
     double sx = 0.0, sy = 0.0;
     for (int i = threadIdx.x; i < nctas; i += blockDim.x) {
-      sx += a.sums[2 * i];
-      sy += a.sums[2 * i + 1];
+      sx += im.sums[2 * i];
+      sy += im.sums[2 * i + 1];
     }
     sx = block_sum_d(sx, red);
     sy = block_sum_d(sy, red);
     if (threadIdx.x == 0) {
-      a.sumxy[0] = sx * a.nz;
-      a.sumxy[1] = sy * a.nz;
+      im.sumxy[0] = sx * a.nz;
+      im.sumxy[1] = sy * a.nz;
     }
   }
 }
@@ -412,6 +409,7 @@ template <int DIR, int NF>
 __global__ void __launch_bounds__(kThreads) k_fft_cols2(float2* data, int n, int ncol, FFTPlan plan, int W)
 {
   extern __shared__ float2 sm[];
+  data += (size_t)blockIdx.y * n * ncol;
   const int c0 = blockIdx.x * W;
   const int ld = W + 1;
   for (int t = threadIdx.x; t < n * W; t += blockDim.x) {
@@ -438,6 +436,9 @@ __device__ __forceinline__ void better(float& bv, int& bi, float v, int i)
 
 __global__ void k_argmax_partial(const float2* cc, int n, float* bval, int* bidx)
 {
+  cc += (size_t)blockIdx.y * n;
+  bval += blockIdx.y * gridDim.x;
+  bidx += blockIdx.y * gridDim.x;
   float bv = -1e30f;
   int bi = 0x7fffffff;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -479,9 +480,14 @@ __device__ __forceinline__ float inten(const float2* cc, int i)
   return c.x * c.x + c.y * c.y;
 }
 
+// one block per direction: the maximum, its neighbours and (find) k0
 __global__ void k_argmax_final(const float2* cc, int nx, int ny, const float* bval, const int* bidx, int nb,
-                               float* peak)
+                               float* peak, const __grid_constant__ FindK0Args f, int find)
 {
+  cc += (size_t)blockIdx.x * nx * ny;
+  bval += blockIdx.x * nb;
+  bidx += blockIdx.x * nb;
+  peak += 8 * blockIdx.x;
   float bv = -1e30f;
   int bi = 0x7fffffff;
   for (int i = threadIdx.x; i < nb; i += blockDim.x) better(bv, bi, bval[i], bidx[i]);
@@ -511,6 +517,9 @@ __global__ void k_argmax_final(const float2* cc, int nx, int ny, const float* bv
     peak[4] = inten(cc, iy * nx + (ix + 1) % nx);
     peak[5] = inten(cc, ((iy + ny - 1) % ny) * nx + ix);
     peak[6] = inten(cc, ((iy + 1) % ny) * nx + ix);
+    if (find)
+      findk0_finish(peak, f.guess[blockIdx.x], nx, ny, f.dkx, f.dky, f.fitorder2, f.k0out[blockIdx.x],
+                    f.k1out[blockIdx.x]);
   }
 }
 
@@ -519,22 +528,23 @@ constexpr int kCand = 8;  // candidates per pass (register accumulators)
 static_assert(2 * kCand == 16, "k_modamp_partial reduces 16 values per thread");
 
 // ex[c][x] = exp(i 2 pi (x - nx/2) kx_c dxy), ey[c][y] likewise
-// kdev: one candidate, kdev[0] * kfac (a k0 fitted on the device)
+__device__ __forceinline__ float2 phase_entry(int r, int nx, int ny, float2 k, float dxy)
+{
+  double ang;
+  if (r < nx) ang = 2.0 * M_PI * ((double)r - 0.5 * nx) * (double)k.x * (double)dxy;
+  else ang = 2.0 * M_PI * ((double)(r - nx) - 0.5 * ny) * (double)k.y * (double)dxy;
+  double s, co;
+  sincos(ang, &s, &co);
+  return make_float2((float)co, (float)s);
+}
+
 __global__ void k_phase_tables(const __grid_constant__ CandList kc, int ncand, int nx, int ny, float dxy, float2* ex,
-                               float2* ey, const float2* kdev, float kfac)
+                               float2* ey)
 {
   int n = ncand * (nx + ny);
-  float2 kd = make_float2(0.f, 0.f);
-  if (kdev) kd = make_float2(__fmul_rn(kdev->x, kfac), __fmul_rn(kdev->y, kfac));
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     int c = t / (nx + ny), r = t - c * (nx + ny);
-    const float2 k = kdev ? kd : kc.k[c];
-    double ang;
-    if (r < nx) ang = 2.0 * M_PI * ((double)r - 0.5 * nx) * (double)k.x * (double)dxy;
-    else ang = 2.0 * M_PI * ((double)(r - nx) - 0.5 * ny) * (double)k.y * (double)dxy;
-    double s, co;
-    sincos(ang, &s, &co);
-    float2 v = make_float2((float)co, (float)s);
+    const float2 v = phase_entry(r, nx, ny, kc.k[c], dxy);
     if (r < nx) ex[(size_t)c * nx + r] = v;
     else ey[(size_t)c * ny + (r - nx)] = v;
   }
@@ -602,6 +612,78 @@ __global__ void k_modamp_final(const double* partial, int nblocks, int ncand, do
   }
 }
 
+// blocks of the reduction: about four elements per thread, at most kModampBlocks
+int modamp_blocks(int nx, int ny)
+{
+  return (int)std::min<long long>(kModampBlocks, std::max<long long>(1, ((long long)nx * ny + 1023) / 1024));
+}
+
+// ---- one candidate per overlap pair, the pairs as a grid dimension
+__global__ void k_modamp1_tables(const __grid_constant__ ModampArgs a)
+{
+  const ModampItem& m = a.item[blockIdx.y];
+  float2 k = m.k;
+  if (m.kdev) k = make_float2(__fmul_rn(m.kdev->x, m.kfac), __fmul_rn(m.kdev->y, m.kfac));
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < a.nx + a.ny) m.tables[r] = phase_entry(r, a.nx, a.ny, k, a.dxy);
+}
+
+// the sums of k_modamp_partial for one candidate (the same additions)
+__global__ void __launch_bounds__(256) k_modamp1_partial(const __grid_constant__ ModampArgs a)
+{
+  __shared__ float sacc[256][3];
+  __shared__ double sseg[16][2];
+  const ModampItem& m = a.item[blockIdx.y];
+  const float2* __restrict__ P = m.pmap;
+  const float2* __restrict__ ex = m.tables;
+  const float2* __restrict__ ey = m.tables + a.nx;
+  float2 acc = make_float2(0.f, 0.f);
+  const int n = a.nx * a.ny;
+#pragma unroll 4
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+    const int y = i / a.nx, x = i - y * a.nx;
+    const float2 v = cmul(P[i], cmul(ex[x], ey[y]));
+    acc.x += v.x;
+    acc.y += v.y;
+  }
+  sacc[threadIdx.x][0] = acc.x;
+  sacc[threadIdx.x][1] = acc.y;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int v = threadIdx.x & 1, seg = threadIdx.x >> 1;
+    double sum = 0.0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) sum += (double)sacc[seg * 16 + i][v];
+    sseg[seg][v] = sum;
+    __syncwarp();
+    if (threadIdx.x < 2) {
+      double tot = 0.0;
+#pragma unroll
+      for (int g = 0; g < 16; ++g) tot += sseg[g][threadIdx.x];
+      m.partial[blockIdx.x * 2 + threadIdx.x] = tot;
+    }
+  }
+}
+
+__global__ void k_modamp1_final(const __grid_constant__ ModampArgs a, int nblocks)
+{
+  __shared__ double red[32];
+  const ModampItem& m = a.item[blockIdx.x];
+  double re = 0.0, im = 0.0;
+  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
+    re += m.partial[b * 2];
+    im += m.partial[b * 2 + 1];
+  }
+  re = block_sum_d(re, red);
+  im = block_sum_d(im, red);
+  if (threadIdx.x == 0) {
+    m.slot[0] = re;
+    m.slot[1] = im;
+    m.slot[2] = m.sumxy[0];
+    m.slot[3] = m.sumxy[1];
+  }
+}
+
 }  // namespace
 
 int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
@@ -612,12 +694,14 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   a.m_f = m_above_scaled_root(a.otfcutoff, a.order0_2_factor);
   FFTPlan px, py;
   if (!get_fft_plan(a.nx, &px) || !get_fft_plan(a.ny, &py)) return -1;
-  const int nzb = 2 * a.zdc + 1;
-  // lengths without a compiled transform take the two-factor kernels; 1024
-  // rows too (1.25 ms a 1024^2 x 64 pair with the Stockham stages, 0.26 here)
+  const int nzb = 2 * a.zdc + 1, ni = a.nitems;
+  if (ni < 1 || ni > kMaxOvlItems) return -1;
+  // 1024 rows: 1.25 ms a 1024^2 x 64 pair with the Stockham stages, 0.26 with
+  // the two-factor kernel
   TfPlan tx, ty;
-  const TfKernels* kx = reg_fft_lanes(a.nx) || a.otf.nxotf > kOvlTabMax ? nullptr : tf_kernels(a.nx, &tx);
-  const TfKernels* ky = reg_fft_lanes(a.ny) && a.ny != 1024 ? nullptr : tf_kernels(a.ny, &ty);
+  const TfKernels* kx =
+      a.otf.nxotf <= kOvlTabMax && fft_two_factor(kSiteOvlX, a.nx) ? tf_kernels(a.nx, &tx) : nullptr;
+  const TfKernels* ky = fft_two_factor(kSiteOvlY, a.ny) ? tf_kernels(a.ny, &ty) : nullptr;
   // 1) build + x inverse FFT
   const int ldl = a.nx + 1;
   int rows = std::max(1, kMaxElems / (2 * a.nx));
@@ -626,14 +710,14 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   int nb1 = (nzb * a.ny + rows - 1) / rows;
 
   KernelTimer* kt = kernel_timer();
-  const double ovlb = 2.0 * nzb * a.ny * a.nx * sizeof(float2);
-  const double bandplanes = (double)nzb * a.ny * (a.nx / 2 + 1) * sizeof(float2);
+  const double ovlb = 2.0 * ni * nzb * a.ny * a.nx * sizeof(float2);
+  const double bandplanes = (double)ni * nzb * a.ny * (a.nx / 2 + 1) * sizeof(float2);
   if (kt) kt->begin(s);
   auto launch_w = [&]<int N>() {
     constexpr int G = 32 / OvlLanes<N>::P;
     const int nlines = 2 * nzb * a.ny;
     const int per_cta = kOvlWarps * G;
-    k_ovl_build_xw<N><<<(nlines + per_cta - 1) / per_cta, kOvlWarps * 32, 0, s>>>(a, px.twr);
+    k_ovl_build_xw<N><<<dim3((nlines + per_cta - 1) / per_cta, 1, ni), kOvlWarps * 32, 0, s>>>(a, px.twr);
   };
   if (a.nx == 512) launch_w.template operator()<512>();
   else if (a.nx == 1024) launch_w.template operator()<1024>();
@@ -644,14 +728,14 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   } else
     dispatch_fft_len(kSiteOvlX, a.nx, [&]<int NF>() {
       allow_dynamic_smem((const void*)k_ovl_build_x<NF>, sm1);
-      k_ovl_build_x<NF><<<nb1, kThreads, sm1, s>>>(a, px, rows, ldl);
+      k_ovl_build_x<NF><<<dim3(nb1, 1, ni), kThreads, sm1, s>>>(a, px, rows, ldl);
     });
-  if (kt) kt->end("k_ovl_build_x", s, ovlb + (a.order1 == 0 ? 3 : 4) * bandplanes);
+  if (kt) kt->end("k_ovl_build_x", s, ovlb + (a.item[0].order1 == 0 ? 3 : 4) * bandplanes);
   // 2) y inverse FFT + accumulation over kz planes
   const int threads = kThreads;
   int W = std::max(1, std::min(16, kMaxElems / (2 * a.ny)));
   int tiles = (a.nx + W - 1) / W;
-  int groups = std::max(1, std::min(nzb, (2 * 152 + tiles - 1) / tiles));
+  int groups = std::max(1, std::min(nzb, (2 * 152 + ni * tiles - 1) / (ni * tiles)));
   int ppg = (nzb + groups - 1) / groups;
   groups = (nzb + ppg - 1) / ppg;
   const int tile = a.ny * (2 * W + 1);
@@ -661,12 +745,12 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   if (a.ny == 512 || a.ny == 256) {
     // 8 columns per CTA; plane groups so that the grid covers the GPU
     tiles = (a.nx + 7) / 8;
-    groups = std::max(1, std::min(nzb, (4 * 152 + tiles - 1) / tiles));
+    groups = std::max(1, std::min(nzb, (4 * 152 + ni * tiles - 1) / (ni * tiles)));
     ppg = (nzb + groups - 1) / groups;
     groups = (nzb + ppg - 1) / ppg;
   } else if (ky) {
     tiles = (a.nx + ky->ovl_y_columns - 1) / ky->ovl_y_columns;
-    groups = std::max(1, std::min(nzb, (4 * 152 + tiles - 1) / tiles));
+    groups = std::max(1, std::min(nzb, (4 * 152 + ni * tiles - 1) / (ni * tiles)));
     ppg = (nzb + groups - 1) / groups;
     groups = (nzb + ppg - 1) / ppg;
   }
@@ -674,7 +758,7 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   auto go4 = [&]<int N, int R1>() {
     const size_t bytes = 2 * ColFft<N, R1, 8>::kSmemElems * sizeof(float2);
     allow_dynamic_smem((const void*)k_ovl_y4<N, R1>, bytes);
-    k_ovl_y4<N, R1><<<dim3(tiles, groups), kThreads, bytes, s>>>(a, py.tw, ppg);
+    k_ovl_y4<N, R1><<<dim3(tiles, groups, ni), kThreads, bytes, s>>>(a, py.tw, ppg);
   };
   if (a.ny == 512) go4.template operator()<512, 32>();
   else if (a.ny == 256) go4.template operator()<256, 16>();
@@ -684,48 +768,56 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   } else
     dispatch_fft_len(kSiteOvlY, a.ny, [&]<int NF>() {
       allow_dynamic_smem((const void*)k_ovl_y_accum<NF>, sm2);
-      k_ovl_y_accum<NF><<<dim3(tiles, groups), threads, sm2, s>>>(a, py, W, ppg, xoff);
+      k_ovl_y_accum<NF><<<dim3(tiles, groups, ni), threads, sm2, s>>>(a, py, W, ppg, xoff);
     });
-  if (kt) kt->end("k_ovl_y_accum", s, ovlb + (double)groups * a.ny * a.nx * sizeof(float2));
+  if (kt) kt->end("k_ovl_y_accum", s, ovlb + (double)ni * groups * a.ny * a.nx * sizeof(float2));
   // 3) reduce plane groups
-  k_p_reduce<<<std::min(1024, (a.nx * a.ny + 255) / 256), 256, 0, s>>>(a, groups, tiles * groups);
+  k_p_reduce<<<dim3(std::min(1024, (a.nx * a.ny + 255) / 256), ni), 256, 0, s>>>(a, groups, tiles * groups);
   if (launches) *launches += 3;
   return (int)cudaGetLastError();
 }
 
-int launch_crosscorr_peak(const float2* pmap, float2* cc, int nx, int ny, float* blockval, int* blockidx,
-                          float* peak, cudaStream_t s, long long* launches)
+int launch_crosscorr_peak(const float2* pmap, int n, float2* cc, int nx, int ny, float* blockval, int* blockidx,
+                          float* peak, const FindK0Args* find, cudaStream_t s, long long* launches)
 {
   FFTPlan px, py;
   if (!get_fft_plan(nx, &px) || !get_fft_plan(ny, &py)) return -1;
+  if (n < 1 || n > kMaxOvlItems) return -1;
+  // the maps are consecutive: n of them are n ny rows
+  const int rows = n * ny;
   int nl = std::max(1, std::min(ny, kMaxElems / nx));
   size_t sm1 = fft_stage_smem(nx, nl, nl * (nx + 1), kThreads);
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
   TfPlan tx, ty;
-  const TfKernels* kx = reg_fft_lanes(nx) ? nullptr : tf_kernels(nx, &tx);
-  const TfKernels* ky = reg_fft_lanes(ny) ? nullptr : tf_kernels(ny, &ty);
+  const TfKernels* kx = fft_two_factor(kSiteCorrRows, nx) ? tf_kernels(nx, &tx) : nullptr;
+  const TfKernels* ky = fft_two_factor(kSiteCorrCols, ny) ? tf_kernels(ny, &ty) : nullptr;
   if (kx) {
-    const int rc = kx->fft_rows_conj(pmap, cc, ny, tx, s);
+    const int rc = kx->fft_rows_conj(pmap, cc, rows, tx, s);
     if (rc != 0) return rc;
-  } else dispatch_fft_len(kSiteCorrRows, nx, [&]<int NF>() {
-    allow_dynamic_smem((const void*)k_fft_rows<-1, true, NF>, sm1);
-    k_fft_rows<-1, true, NF><<<(ny + nl - 1) / nl, kThreads, sm1, s>>>(pmap, cc, nx, ny, px, nl);
-  });
+  } else {
+    dispatch_fft_len(kSiteCorrRows, nx, [&]<int NF>() {
+      allow_dynamic_smem((const void*)k_fft_rows<-1, true, NF>, sm1);
+      k_fft_rows<-1, true, NF><<<(rows + nl - 1) / nl, kThreads, sm1, s>>>(pmap, cc, nx, rows, px, nl);
+    });
+  }
   int W = std::max(1, std::min(32, kMaxElems / ny));
   size_t sm2 = fft_stage_smem(ny, W, (W + 1) * ny, kThreads);
   if (ky) {
-    const int rc = ky->fft_cols(cc, nx, 1, ty, s);
+    const int rc = ky->fft_cols(cc, nx, n, ty, s);
     if (rc != 0) return rc;
-  } else dispatch_fft_len(kSiteCorrCols, ny, [&]<int NF>() {
-    allow_dynamic_smem((const void*)k_fft_cols2<-1, NF>, sm2);
-    k_fft_cols2<-1, NF><<<(nx + W - 1) / W, kThreads, sm2, s>>>(cc, ny, nx, py, W);
-  });
-  int nb = 256;
-  k_argmax_partial<<<nb, 256, 0, s>>>(cc, nx * ny, blockval, blockidx);
-  k_argmax_final<<<1, 256, 0, s>>>(cc, nx, ny, blockval, blockidx, nb, peak);
+  } else {
+    dispatch_fft_len(kSiteCorrCols, ny, [&]<int NF>() {
+      allow_dynamic_smem((const void*)k_fft_cols2<-1, NF>, sm2);
+      k_fft_cols2<-1, NF><<<dim3((nx + W - 1) / W, n), kThreads, sm2, s>>>(cc, ny, nx, py, W);
+    });
+  }
+  const int nb = 256;
+  k_argmax_partial<<<dim3(nb, n), 256, 0, s>>>(cc, nx * ny, blockval, blockidx);
+  k_argmax_final<<<n, 256, 0, s>>>(cc, nx, ny, blockval, blockidx, nb, peak, find ? *find : FindK0Args{},
+                                   find != nullptr);
   // pmap in, cc out; cc in and out (columns); cc in (argmax)
-  if (kt) kt->end("k_crosscorr", s, 5.0 * nx * ny * sizeof(float2));
+  if (kt) kt->end("k_crosscorr", s, 5.0 * n * nx * ny * sizeof(float2));
   if (launches) *launches += 4;
   return (int)cudaGetLastError();
 }
@@ -751,7 +843,7 @@ int launch_overlap_volumes(const OverlapArgs& a, float2* vol, cudaStream_t s)
   FFTPlan py, pz;
   if (!get_fft_plan(a.ny, &py) || !get_fft_plan(a.nz, &pz)) return -1;
   const size_t plane = (size_t)a.nx * a.ny;
-  k_ovl_scatter<<<1216, 256, 0, s>>>(a.ovl, a.nx, a.ny, a.nz, a.zdc, vol);
+  k_ovl_scatter<<<1216, 256, 0, s>>>(a.item[0].ovl, a.nx, a.ny, a.nz, a.zdc, vol);
   auto cols = [&](float2* data, int n, int ncol, const FFTPlan& p) {
     const int W = std::max(1, std::min(32, kMaxElems / n));
     const size_t sm = fft_stage_smem(n, W, (W + 1) * n, kThreads);
@@ -789,7 +881,7 @@ __device__ __forceinline__ float mag2_rn(float2 a) { return __fadd_rn(__fmul_rn(
 // |amp|^2 and the filter's per-term weights (filterbands, gpuFunctionsImpl.cu:1341-1360)
 __device__ void fit_derived(const FitFinishArgs& a, FitDev* out)
 {
-  for (int i = 0; i < a.ndirs * a.norders; ++i) {
+  for (int i = threadIdx.x; i < a.ndirs * a.norders; i += 32) {
     const int o = i % a.norders;
     const float m2 = mag2_rn(out->amp[i]);
     out->ampmag2[i] = m2;
@@ -800,12 +892,12 @@ __device__ void fit_derived(const FitFinishArgs& a, FitDev* out)
 // findModulationVectorsAndPhasesForAllDirections without a k0 search
 // (cudaSirecon.cpp:409-492): amp[o] = XStarY / sum|X|^2 of findrealspacemodamp
 // (gpuFunctionsImpl.cu:1128-1130), then the 2D chaining, forcemodamp and the
-// fitallphases = 0 phase rule, in that order.  One thread: at most 64 values.
+// fitallphases = 0 phase rule, in that order.  One thread per direction, then
+// one per value.
 __global__ void k_fit_finish(const double* __restrict__ slots, const __grid_constant__ FitFinishArgs a, FitDev* out)
 {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const int no = a.norders;
-  for (int d = 0; d < a.ndirs; ++d) {
+  for (int d = threadIdx.x; d < a.ndirs; d += 32) {
     float2* amp = out->amp + d * no;
     amp[0] = make_float2(1.f, 0.f);
     for (int o = 1; o < no; ++o) {
@@ -832,13 +924,14 @@ __global__ void k_fit_finish(const double* __restrict__ slots, const __grid_cons
       }
     }
   }
+  __syncwarp();
   fit_derived(a, out);
 }
 
 __global__ void k_set_fit(const __grid_constant__ AmpList amps, const __grid_constant__ FitFinishArgs a, FitDev* out)
 {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int i = 0; i < a.ndirs * a.norders; ++i) out->amp[i] = amps.amp[i];
+  for (int i = threadIdx.x; i < a.ndirs * a.norders; i += 32) out->amp[i] = amps.amp[i];
+  __syncwarp();
   fit_derived(a, out);
 }
 }  // namespace
@@ -868,9 +961,8 @@ int launch_copy_out(const void* src1, void* dst1, size_t n1, const void* src2, v
   return (int)cudaGetLastError();
 }
 
-static int modamp_impl(const float2* pmap, int nx, int ny, float dxy, const CandList& kcand, int ncand,
-                       const float2* kdev, float kfac, float2* tables, double* partial, double* xstary, cudaStream_t s,
-                       long long* launches)
+int launch_modamp_candidates(const float2* pmap, int nx, int ny, float dxy, const CandList& kcand, int ncand,
+                             float2* tables, double* partial, double* xstary, cudaStream_t s, long long* launches)
 {
   if (ncand < 1 || ncand > kMaxCand) return -1;
   float2* ex = tables;
@@ -878,10 +970,9 @@ static int modamp_impl(const float2* pmap, int nx, int ny, float dxy, const Cand
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
   // double sincos: spread over all SMs (FP64 throughput is per SM)
-  k_phase_tables<<<(ncand * (nx + ny) + 63) / 64, 64, 0, s>>>(kcand, ncand, nx, ny, dxy, ex, ey, kdev, kfac);
+  k_phase_tables<<<(ncand * (nx + ny) + 63) / 64, 64, 0, s>>>(kcand, ncand, nx, ny, dxy, ex, ey);
   if (kt) kt->end("k_modamp_tables", s, (double)ncand * (nx + ny) * sizeof(float2));
-  // about four elements per thread, at most kModampBlocks blocks
-  const int nb = (int)std::min<long long>(kModampBlocks, std::max<long long>(1, ((long long)nx * ny + 1023) / 1024));
+  const int nb = modamp_blocks(nx, ny);
   if (kt) kt->begin(s);
   for (int c0 = 0; c0 < ncand; c0 += kCand) {
     int nc = std::min(kCand, ncand - c0);
@@ -896,17 +987,22 @@ static int modamp_impl(const float2* pmap, int nx, int ny, float dxy, const Cand
   return (int)cudaGetLastError();
 }
 
-int launch_modamp_candidates(const float2* pmap, int nx, int ny, float dxy, const CandList& kcand, int ncand,
-                             float2* tables, double* partial, double* xstary, cudaStream_t s, long long* launches)
+int launch_modamp_batch(const ModampArgs& a, cudaStream_t s, long long* launches)
 {
-  return modamp_impl(pmap, nx, ny, dxy, kcand, ncand, nullptr, 0.f, tables, partial, xstary, s, launches);
-}
-
-int launch_modamp_device_k(const float2* pmap, int nx, int ny, float dxy, const float2* kdev, float kfac,
-                           float2* tables, double* partial, double* xstary, cudaStream_t s, long long* launches)
-{
-  if (kdev == nullptr) return -1;
-  return modamp_impl(pmap, nx, ny, dxy, CandList{}, 1, kdev, kfac, tables, partial, xstary, s, launches);
+  if (a.n < 1 || a.n > kMaxOvlItems) return -1;
+  KernelTimer* kt = kernel_timer();
+  if (kt) kt->begin(s);
+  k_modamp1_tables<<<dim3((a.nx + a.ny + 63) / 64, a.n), 64, 0, s>>>(a);
+  if (kt) kt->end("k_modamp_tables", s, (double)a.n * (a.nx + a.ny) * sizeof(float2));
+  const int nb = modamp_blocks(a.nx, a.ny);
+  if (kt) kt->begin(s);
+  k_modamp1_partial<<<dim3(nb, a.n), 256, 0, s>>>(a);
+  if (kt) kt->end("k_modamp", s, (double)a.n * a.nx * a.ny * sizeof(float2));
+  if (kt) kt->begin(s);
+  k_modamp1_final<<<a.n, 256, 0, s>>>(a, nb);
+  if (kt) kt->end("k_modamp_final", s, (double)a.n * nb * 2 * sizeof(double));
+  if (launches) *launches += 3;
+  return (int)cudaGetLastError();
 }
 
 }  // namespace simrecon

@@ -451,10 +451,10 @@ int launch_ingest(const IngestArgs& a, cudaStream_t s, long long* launches)
       k_ingest_xw<float, N><<<gw, kIngestWarps * 32, bytes, s>>>(a, px.twr);
     }
   };
-  // lengths without a compiled transform take the two-factor kernels
   TfPlan tx, ty;
-  const TfKernels* kx = reg_fft_lanes(a.nx) ? nullptr : tf_kernels(a.nx, &tx);
-  const TfKernels* ky = reg_fft_lanes(a.ny) ? nullptr : tf_kernels(a.ny, &ty);
+  const bool wx = a.nx == 512 || a.nx == 1024 || a.nx == 256;  // warp kernels
+  const TfKernels* kx = !wx && fft_two_factor(kSiteIngestX, a.nx) ? tf_kernels(a.nx, &tx) : nullptr;
+  const TfKernels* ky = !colfft_r1(a.ny) && fft_two_factor(kSiteIngestY, a.ny) ? tf_kernels(a.ny, &ty) : nullptr;
   if (a.nx == 512) go_w.template operator()<512>();
   else if (a.nx == 1024) go_w.template operator()<1024>();
   else if (a.nx == 256) go_w.template operator()<256>();

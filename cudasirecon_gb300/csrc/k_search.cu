@@ -2,8 +2,8 @@
 // fitk0andmodamps' line searches (gpuFunctionsImpl.cu:306-372, 874-1044)
 // without a host round trip.
 //
-// k_findk0_finish   the cross-correlation peak's parabola fits and the
-//                   wrap-around choice -> k0 (one thread)
+// findk0_finish     the cross-correlation peak's parabola fits and the
+//                   wrap-around choice -> k0 (findk0.cuh)
 // k_k0_search       one thread-block cluster per direction (all directions in
 //                   one launch, side by side on the GPU): the angle and
 //                   magnitude line searches with their parabola fits and the
@@ -23,6 +23,7 @@
 // matches the host-driven search to a few 1e-5 pixel, not bit for bit.
 #include <cooperative_groups.h>
 
+#include "findk0.cuh"
 #include "kernels.h"
 
 namespace cg = cooperative_groups;
@@ -30,17 +31,6 @@ namespace cg = cooperative_groups;
 namespace simrecon {
 
 namespace {
-
-// fitparabola, gpuFunctionsImpl.cu:479-495
-__device__ float fitparabola_rn(float a1, float a2, float a3)
-{
-  const float slope = __fmul_rn(0.5f, __fsub_rn(a3, a1));
-  const float curve = __fsub_rn(__fadd_rn(a3, a1), __fmul_rn(2.f, a2));
-  if (curve == 0.f) return 0.f;
-  const float peak = __fdiv_rn(-slope, curve);
-  if (peak > 1.5f || peak < -1.5f) return 0.f;
-  return peak;
-}
 
 // fitxyparabola, gpuFunctionsImpl.cu:1022-1044
 __device__ float fitxyparabola_rn(float x1, float y1, float x2, float y2, float x3, float y3)
@@ -53,33 +43,6 @@ __device__ float fitxyparabola_rn(float x1, float y1, float x2, float y2, float 
   const float curve = __fdiv_rn(__fsub_rn(slope2, slope1), __fsub_rn(xbar2, xbar1));
   if (curve == 0.f) return 0.f;
   return __fsub_rn(xbar2, __fdiv_rn(slope2, curve));
-}
-
-__device__ __forceinline__ float2 polar_rn(float mag, float angle)
-{
-  return make_float2(__fmul_rn(mag, cosf(angle)), __fmul_rn(mag, sinf(angle)));
-}
-
-// findk0's tail (gpuFunctionsImpl.cu:345-371): peak = {ix, iy, a1x, a2, a3x,
-// a1y, a3y}; k0 = the parabola-refined peak, moved by a period towards the
-// guess, over fitorder2.  k1 = k0 through (|k0|, atan2) and back: the vector
-// the search's first getmodamp rebuilds the overlaps at.
-__global__ void k_findk0_finish(const float* __restrict__ pk, float2 guess, int nx, int ny, float dkx, float dky,
-                                int fitorder2, float2* k0out, float2* k1out)
-{
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int xcent = (int)pk[0], ycent = (int)pk[1];
-  float peakx = __fadd_rn(fitparabola_rn(pk[2], pk[3], pk[4]), (float)xcent);
-  float peaky = __fadd_rn(fitparabola_rn(pk[5], pk[3], pk[6]), (float)ycent);
-  if (__fdiv_rn(guess.x, dkx) < __fsub_rn(peakx, (float)(nx / 2))) peakx = __fsub_rn(peakx, (float)nx);
-  if (__fdiv_rn(guess.x, dkx) > __fadd_rn(peakx, (float)(nx / 2))) peakx = __fadd_rn(peakx, (float)nx);
-  if (__fdiv_rn(guess.y, dky) < __fsub_rn(peaky, (float)(ny / 2))) peaky = __fsub_rn(peaky, (float)ny);
-  if (__fdiv_rn(guess.y, dky) > __fadd_rn(peaky, (float)(ny / 2))) peaky = __fadd_rn(peaky, (float)ny);
-  const float2 k0 = make_float2(__fmul_rn(peakx, __fdiv_rn(dkx, (float)fitorder2)),
-                                __fmul_rn(peaky, __fdiv_rn(dky, (float)fitorder2)));
-  *k0out = k0;
-  const float mag = __fsqrt_rn(__fadd_rn(__fmul_rn(k0.x, k0.x), __fmul_rn(k0.y, k0.y)));
-  *k1out = polar_rn(mag, atan2f(k0.y, k0.x));
 }
 
 constexpr int kSCmax = 16;    // CTAs per cluster at most: one direction's search
@@ -517,14 +480,6 @@ __global__ void __launch_bounds__(kST, 1) k_k0_search(const __grid_constant__ K0
 }
 
 }  // namespace
-
-int launch_findk0_finish(const float* peak, float2 guess, int nx, int ny, float dkx, float dky, int fitorder2,
-                         float2* k0out, float2* k1out, cudaStream_t s, long long* launches)
-{
-  k_findk0_finish<<<1, 32, 0, s>>>(peak, guess, nx, ny, dkx, dky, fitorder2, k0out, k1out);
-  if (launches) *launches += 1;
-  return (int)cudaGetLastError();
-}
 
 // CTAs per cluster: sixteen where P gives each at least 4096 elements (smaller
 // maps are all barriers and control, which more CTAs lengthen); a non-portable

@@ -36,15 +36,17 @@ bool fft_length_ok(int n);
 // radix sequence of length n into radix[kMaxStages] (no allocation)
 bool fft_radix_plan(int n, int* radix, int* nstages);
 
-// FFT path choice per call site and length (register path or Stockham
-// stages).  The tuner forces a choice on the calling thread, tracks which
+// FFT path choice per call site and length (register path, Stockham stages,
+// or where a site has them the two-factor kernels).  The tuner forces a choice on the calling thread, tracks which
 // (site, length) pairs a run queries, and records measured choices in the
 // on-disk plan cache that every process reads.
-void fft_site_force(int site, bool reg);
+enum : int { kPathStockham = 0, kPathRegister = 1, kPathTwoFactor = 2, kNumFftPaths = 3 };
+const char* fft_path_name(int path);
+void fft_site_force(int site, int path);
 void fft_site_unforce();
 void fft_sites_track(std::set<std::pair<int, int>>* seen);  // nullptr stops tracking
 const char* fft_site_name(int site);
-bool fft_plan_record(int site, int n, bool reg, double ms_reg, double ms_stockham, std::string* err);
+bool fft_plan_record(int site, int n, int path, double ms, double ms_other, std::string* err);
 int fft_plan_choice(int site, int n, const char** source);
 std::string fft_plan_cache_path();
 
@@ -105,13 +107,28 @@ int launch_separate(float2* spec, const float* scale, const float* sepmat /* dev
                     int nz, int ndirs, int nphases, cudaStream_t s, long long* launches);
 
 // ----------------------------------------------------------------- fitting
-struct OverlapArgs {
+// One overlap pair of a batched build
+struct OvlItem {
   const float2* bands;  // bands of one direction: [nph][nz][ny][nxh]
-  int nx, ny, nz;
+  const float2* otf1;   // OTF tables of order1 and order2
+  const float2* otf2;
   int order1, order2;
   float kx, ky;         // k0 * (order2 - order1), 1/um
   const float2* kdev;   // if set: k0 from device memory, times kfac (kx, ky unused)
   float kfac;
+  float2* ovl;          // [2][2*zdc+1][ny][nx]   (x-inverse-transformed rows)
+  float2* ppart;        // [ngroups][ny][nx]
+  double* sums;         // [2 * nctas] partial |X|^2, |Y|^2
+  float2* pmap;         // [ny][nx] result: nz * sum_kz conj(X~) Y~
+  double* sumxy;        // [2] result: sum |X|^2, sum |Y|^2 (real-space, like the reference)
+};
+// Pairs per launch at most: every kernel of a build takes the pairs as one
+// grid dimension, so three directions cost the launches of one.
+constexpr int kMaxOvlItems = 3;
+struct OverlapArgs {
+  int nitems;
+  OvlItem item[kMaxOvlItems];
+  int nx, ny, nz;
   float dkx, dky;
   float rdistcutoff, otfcutoff, order0_2_factor;
   // exact squared forms of makeoverlaps' float decisions (set by
@@ -121,27 +138,43 @@ struct OverlapArgs {
   float r2_le, r2_lt, m_le, m_f;
   int zdc;              // planes -zdc..zdc are built
   int nokz0;
-  OTFView otf;
-  float2* ovl;          // [2][2*zdc+1][ny][nx]   (x-inverse-transformed rows)
-  float2* ppart;        // [ngroups][ny][nx]
-  double* sums;         // [2 * nctas] partial |X|^2, |Y|^2
-  float2* pmap;         // [ny][nx] result: nz * sum_kz conj(X~) Y~
-  double* sumxy;        // [2] result: sum |X|^2, sum |Y|^2 (real-space, like the reference)
+  OTFView otf;          // geometry of the OTF tables (the pointers are the items')
 };
 int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches);
 
-// The two overlaps of the last launch_overlaps as full real-space volumes,
+#ifdef __CUDACC__
+// the shift k0 * (order2 - order1): from the arguments, or from device memory
+// (a k0 fitted on the device) times kfac
+__device__ __forceinline__ float2 ovl_shift(const OvlItem& it)
+{
+  if (it.kdev == nullptr) return make_float2(it.kx, it.ky);
+  const float2 k = *it.kdev;
+  return make_float2(__fmul_rn(k.x, it.kfac), __fmul_rn(k.y, it.kfac));
+}
+#endif
+
+// The two overlaps of item 0 of the last launch_overlaps as full real-space volumes,
 // [2][nz][ny][nx] complex (the reference's overlap0/overlap1 after
 // makeoverlaps' inverse 3D FFT): the x-transformed rows of the built kz
 // planes scattered into every kz plane (zero outside +-zdc), then inverse
 // FFTs along y and z.  For the debug dump only; vol is the caller's.
 int launch_overlap_volumes(const OverlapArgs& a, float2* vol, cudaStream_t s);
 
+// findk0 of n directions (their maps consecutive in pmap, [n][ny][nx]):
 // crosscorr = FFT2(conj(pmap)); intensity argmax with the two-neighbour
-// values along x and y (wrap-around) written to peak[0..6]:
-// {ix, iy, a1x, a2, a3x, a1y, a3y}
-int launch_crosscorr_peak(const float2* pmap, float2* cc, int nx, int ny, float* blockval, int* blockidx,
-                          float* peak, cudaStream_t s, long long* launches);
+// values along x and y (wrap-around) written to peak[8 i + 0..6]:
+// {ix, iy, a1x, a2, a3x, a1y, a3y}.  With `find` the peak is refined on the
+// device too: peak -> k0out; k1out = k0 through (|k0|, atan2) and back (where
+// the search's first amplitude evaluation rebuilds the overlaps).
+struct FindK0Args {
+  float2 guess[kMaxOvlItems];
+  float2* k0out[kMaxOvlItems];
+  float2* k1out[kMaxOvlItems];
+  float dkx, dky;
+  int fitorder2;
+};
+int launch_crosscorr_peak(const float2* pmap, int n, float2* cc, int nx, int ny, float* blockval, int* blockidx,
+                          float* peak, const FindK0Args* find, cudaStream_t s, long long* launches);
 
 // Copies n1 and n2 4-byte words with one small kernel: from device memory to
 // (mapped, page-locked) host memory, so that results of a few bytes reach the
@@ -159,19 +192,29 @@ struct CandList {
 // XStarY[c] = sum_xy pmap(x,y) exp(i 2pi ((x - nx/2) kx_c + (y - ny/2) ky_c) dxy), c < ncand
 int launch_modamp_candidates(const float2* pmap, int nx, int ny, float dxy, const CandList& kcand, int ncand,
                              float2* tables, double* partial, double* xstary, cudaStream_t s, long long* launches);
-// one candidate read from device memory: kdev[0] * kfac
-int launch_modamp_device_k(const float2* pmap, int nx, int ny, float dxy, const float2* kdev, float kfac,
-                           float2* tables, double* partial, double* xstary, cudaStream_t s, long long* launches);
+// The amplitude evaluations of n overlap pairs at one k0 each: slot = {XStarY
+// re, im, sum |X|^2, sum |Y|^2}
+struct ModampItem {
+  const float2* pmap;
+  float2 k;            // k0 * (order2 - order1), 1/um
+  const float2* kdev;  // if set: k0 from device memory, times kfac
+  float kfac;
+  const double* sumxy;
+  double* slot;
+  float2* tables;   // [nx + ny]
+  double* partial;  // [kModampBlocks][2]
+};
+struct ModampArgs {
+  int n, nx, ny;
+  float dxy;
+  ModampItem item[kMaxOvlItems];
+};
+int launch_modamp_batch(const ModampArgs& a, cudaStream_t s, long long* launches);
 
 // The pattern-vector search on the device (k_search.cu).
 // Upper bound on each line search's climb (the reference's loops have none):
 // 4096 steps is 4 rad of angle or 400 frequency pixels of magnitude.
 constexpr int kMaxClimbSteps = 4096;
-// findk0's peak refinement: peak = {ix, iy, a1x, a2, a3x, a1y, a3y} ->
-// k0out; k1out = k0 through (|k0|, atan2) and back (where the search's first
-// amplitude evaluation rebuilds the overlaps)
-int launch_findk0_finish(const float* peak, float2 guess, int nx, int ny, float dkx, float dky, int fitorder2,
-                         float2* k0out, float2* k1out, cudaStream_t s, long long* launches);
 struct K0SearchArgs {
   // per direction:
   const float2* pmap[kMaxDirs];    // [ny][nx] overlap map of orders (0, fitorder2), built at k1

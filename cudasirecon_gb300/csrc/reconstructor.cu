@@ -5,6 +5,7 @@
 // scalars per search step.
 #include "reconstructor.h"
 #include "reg_fft.cuh"
+#include "tf_fft.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -468,7 +469,7 @@ bool SIM_Reconstructor::setup(int nx, int ny, int nimages, int nwaves, const Sta
   const size_t nspec = (size_t)ndirs_ * nph_ * nz_ * ny_ * nxh_;
   const int nzb = 2 * zdc_ovl_ + 1;
   const size_t nxy = (size_t)nx_ * ny_;
-  fit_lanes_ = std::max(1, std::min(ndirs_ * std::max(1, norders_ - 1), (int)kFitLanes));
+  fit_lanes_ = std::max(1, std::min(ndirs_ * std::max(1, norders_ - 1), (int)kMaxOvlItems));
   // assembly scratch: every slot of the volume (at most nz planes of
   // 1 + ndirs*(norders-1) slots) when that fits in 2 GiB, else as many as do
   // (at least one plane's worth); the slots are processed in plane groups
@@ -528,11 +529,6 @@ bool SIM_Reconstructor::setup(int nx, int ny, int nimages, int nwaves, const Sta
   }
   check(cudaGetDevice(&device_), "cudaGetDevice");
   check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
-  for (int l = 1; l < fit_lanes_; ++l) {
-    check(cudaStreamCreateWithFlags(&fit_stream_[l], cudaStreamNonBlocking), "cudaStreamCreate");
-    check(cudaEventCreateWithFlags(&fit_join_[l], cudaEventDisableTiming), "cudaEventCreate");
-  }
-  check(cudaEventCreateWithFlags(&fit_fork_, cudaEventDisableTiming), "cudaEventCreate");
   cudaError_t e = cudaMalloc((void**)&arena_, total);
   if (e != cudaSuccess) {
     *err = std::string("device allocation of ") + std::to_string(total >> 20) + " MiB failed: " +
@@ -585,11 +581,6 @@ SIM_Reconstructor::~SIM_Reconstructor()
   if (d_bgslope_) cudaFree(d_bgslope_);
   if (pre_own_) cudaFree(pre_own_);
   if (h_pinned_) cudaFreeHost(h_pinned_);
-  for (int l = 1; l < kFitLanes; ++l) {
-    if (fit_stream_[l]) cudaStreamDestroy(fit_stream_[l]);
-    if (fit_join_[l]) cudaEventDestroy(fit_join_[l]);
-  }
-  if (fit_fork_) cudaEventDestroy(fit_fork_);
   if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -801,20 +792,17 @@ void SIM_Reconstructor::separate()
 }
 
 // ------------------------------------------------------------------ fitting
-void SIM_Reconstructor::build_overlaps(int d, int o1, int o2, float k0x, float k0y, const float2* kdev, float kfac,
-                                       float2* pmap, double* sumxy, int lane)
+// the arguments that the pairs of a batch share (makeoverlaps scalars,
+// gpuFunctionsImpl.cu:497-555, float arithmetic); in Bessel mode the kz range
+// depends on the pattern's magnitude and the order
+OverlapArgs SIM_Reconstructor::overlap_args(int o2, float k0x, float k0y) const
 {
-  cudaStream_t s = lane_stream(lane);
   const ReconParams& p = opt.p;
   const ImageParams& ip = opt.ip;
   OverlapArgs a{};
-  a.bands = d_spec_ + (size_t)d * nph_ * nz_ * ny_ * nxh_;
   a.nx = nx_;
   a.ny = ny_;
   a.nz = nz_;
-  a.order1 = o1;
-  a.order2 = o2;
-  // makeoverlaps scalars, gpuFunctionsImpl.cu:497-555 (float arithmetic)
   float order0_2_factor = 1.0f;
   if (nz_ > 1) {
     order0_2_factor = 5.0f;
@@ -827,10 +815,6 @@ void SIM_Reconstructor::build_overlaps(int d, int o1, int o2, float k0x, float k
   float kzscale = dkz / p.dkzotf;
   float rdistcutoff = p.na * 2.0 / (ip.wave[0] * 0.001);
   if (rdistcutoff > 1. / (2. * dxy)) rdistcutoff = 1. / (2. * dxy);
-  a.kx = k0x * (o2 - o1);
-  a.ky = k0y * (o2 - o1);
-  a.kdev = kdev;  // a k0 fitted on the device (not in Bessel mode, whose zdc depends on |k0|)
-  a.kfac = kfac;
   a.dkx = dkx;
   a.dky = dky;
   a.rdistcutoff = rdistcutoff;
@@ -838,21 +822,58 @@ void SIM_Reconstructor::build_overlaps(int d, int o1, int o2, float k0x, float k
   a.order0_2_factor = order0_2_factor;
   a.zdc = p.bBessel ? overlap_zdc_bessel(o2, k0x, k0y) : zdc_ovl_;
   a.nokz0 = effective_nokz0(opt);
-  const int dir_ = p.bOneOTFperAngle ? d : 0;
-  for (int o = 0; o < norders_; ++o)
-    a.otf.otf[o] = d_otf_ + ((size_t)dir_ * norders_ + o) * p.nxotf * p.nzotf;
   a.otf.nzotf = p.nzotf;
   a.otf.nxotf = p.nxotf;
   a.otf.dkrotf = p.dkrotf;
   a.otf.kzscale = kzscale;
-  a.ovl = d_ovl_ + lane * ovl_lane_elems();
-  a.ppart = d_ppart_ + lane * ppart_lane_elems();
-  a.sums = d_sums_ + lane * sums_lane_elems();
-  a.pmap = pmap ? pmap : lane_pmap(lane);
-  a.sumxy = sumxy ? sumxy : d_sumxy_ + 2 * lane;
-  check_launch(launch_overlaps(a, s, &launches_), "makeoverlaps");
-  ++fit_counts_[0];
+  return a;
+}
+
+void SIM_Reconstructor::add_overlap(OverlapArgs& a, int d, int o1, int o2, float k0x, float k0y, const float2* kdev,
+                                    float kfac, float2* pmap, double* sumxy) const
+{
+  const int i = a.nitems++;
+  OvlItem& it = a.item[i];
+  it.bands = d_spec_ + (size_t)d * nph_ * nz_ * ny_ * nxh_;
+  it.order1 = o1;
+  it.order2 = o2;
+  it.kx = k0x * (o2 - o1);
+  it.ky = k0y * (o2 - o1);
+  it.kdev = kdev;  // a k0 fitted on the device (not in Bessel mode, whose zdc depends on |k0|)
+  it.kfac = kfac;
+  const size_t otf0 = (size_t)(opt.p.bOneOTFperAngle ? d : 0) * norders_, otfn = (size_t)opt.p.nxotf * opt.p.nzotf;
+  it.otf1 = d_otf_ + (otf0 + o1) * otfn;
+  it.otf2 = d_otf_ + (otf0 + o2) * otfn;
+  it.ovl = d_ovl_ + i * ovl_lane_elems();
+  it.ppart = d_ppart_ + i * ppart_lane_elems();
+  it.sums = d_sums_ + i * sums_lane_elems();
+  it.pmap = pmap ? pmap : lane_pmap(i);
+  it.sumxy = sumxy ? sumxy : d_sumxy_ + 2 * i;
+}
+
+void SIM_Reconstructor::run_overlaps(OverlapArgs& a)
+{
+  check_launch(launch_overlaps(a, stream_, &launches_), "makeoverlaps");
+  fit_counts_[0] += a.nitems;
   last_ovl_ = a;
+}
+
+void SIM_Reconstructor::add_modamp(ModampArgs& a, int d, int order, float2 k, const float2* kdev, float kfac) const
+{
+  const int i = a.n++;
+  a.nx = nx_;
+  a.ny = ny_;
+  a.dxy = opt.ip.dxy;
+  a.item[i] = ModampItem{lane_pmap(i), k, kdev, kfac, d_sumxy_ + 2 * i,
+                         d_fitslots_ + (size_t)(d * norders_ + order) * 4, d_tables_ + i * tables_lane_elems(),
+                         d_partial_ + i * partial_lane_elems()};
+}
+
+void SIM_Reconstructor::build_overlaps(int d, int o1, int o2, float k0x, float k0y)
+{
+  OverlapArgs a = overlap_args(o2, k0x, k0y);
+  add_overlap(a, d, o1, o2, k0x, k0y);
+  run_overlaps(a);
   cur_o1_ = o1;
   cur_o2_ = o2;
   cache_.clear();
@@ -963,7 +984,8 @@ void SIM_Reconstructor::findk0(int d)
   const int fitorder2 = nz_ > 1 && !opt.p.bBessel ? 2 : 1;
   float2v k0 = k0_[d];
   build_overlaps(d, 0, fitorder2, k0.x, k0.y);
-  check_launch(launch_crosscorr_peak(d_pmap_, d_cc_, nx_, ny_, d_bval_, d_bidx_, d_peak_, stream_, &launches_),
+  check_launch(launch_crosscorr_peak(d_pmap_, 1, d_cc_, nx_, ny_, d_bval_, d_bidx_, d_peak_, nullptr, stream_,
+                                     &launches_),
                "crosscorr");
   ++fit_counts_[1];  // the cross-correlation reads the overlap pair once, like a modamp reduction
   float* pk = (float*)(h_pinned_ + 256);
@@ -1210,37 +1232,42 @@ bool SIM_Reconstructor::fit_search_on_device()
   const float dxy = ip.dxy;
   const float dkx = 1 / (nx_ * dxy), dky = 1 / (ny_ * dxy);
   check(cudaMemsetAsync(d_sinfo_, 0, 2 * sizeof(int), stream_), "fit");
-  long long builds = 0, reductions = 0;
+  long long reductions = 0;
   K0SearchArgs sa{};
   const size_t nxy = (size_t)nx_ * ny_;
-  // each direction's findk0 and first overlap rebuild on its fit lane
-  const int nl0 = lanes_begin();
-  for (int d = 0; d < ndirs_; ++d) {
-    k0_[d] = k0guess_[d];
-    float2* kfind = d_kst_ + 3 * d;
-    float2* k1 = kfind + 1;
-    const int lane = d % nl0;
-    cudaStream_t ls = lane_stream(lane);
-    float* peak = d_peak_ + 8 * lane;
-    build_overlaps(d, 0, fo2, k0guess_[d].x, k0guess_[d].y, nullptr, 0.f, nullptr, nullptr, lane);
-    check_launch(launch_crosscorr_peak(lane_pmap(lane), d_cc_ + lane * nxy, nx_, ny_, d_bval_ + 256 * lane,
-                                       d_bidx_ + 256 * lane, peak, ls, &launches_),
-                 "crosscorr");
-    check_launch(launch_findk0_finish(peak, make_float2(k0guess_[d].x, k0guess_[d].y), nx_, ny_, dkx, dky, fo2,
-                                      kfind, k1, ls, &launches_),
+  // findk0 and the first overlap rebuild of as many directions at a time as
+  // there are buffer sets
+  for (int d0 = 0; d0 < ndirs_; d0 += fit_lanes_) {
+    const int n = std::min(fit_lanes_, ndirs_ - d0);
+    OverlapArgs guess = overlap_args(fo2, 0.f, 0.f), refined = overlap_args(fo2, 0.f, 0.f);
+    FindK0Args find{};
+    find.dkx = dkx;
+    find.dky = dky;
+    find.fitorder2 = fo2;
+    for (int i = 0; i < n; ++i) {
+      const int d = d0 + i;
+      k0_[d] = k0guess_[d];
+      float2* kfind = d_kst_ + 3 * d;
+      add_overlap(guess, d, 0, fo2, k0guess_[d].x, k0guess_[d].y);
+      find.guess[i] = make_float2(k0guess_[d].x, k0guess_[d].y);
+      find.k0out[i] = kfind;
+      find.k1out[i] = kfind + 1;
+      // fitk0andmodamps' first getmodamp rebuilds the overlaps at k1; every
+      // direction keeps its map for the searches, which run side by side
+      add_overlap(refined, d, 0, fo2, 0.f, 0.f, kfind + 1, (float)fo2, d_pmapd_ + d * nxy, d_sumxyd_ + 2 * d);
+      sa.pmap[d] = d_pmapd_ + d * nxy;
+      sa.sumxy[d] = d_sumxyd_ + 2 * d;
+      sa.k0find[d] = kfind;
+      sa.k0fit[d] = kfind + 2;
+      sa.slot[d] = d_fitslots_ + (size_t)(d * norders_ + fo2) * 4;
+      reductions += 1;  // the cross-correlation
+    }
+    run_overlaps(guess);
+    check_launch(launch_crosscorr_peak(d_pmap_, n, d_cc_, nx_, ny_, d_bval_, d_bidx_, d_peak_, &find, stream_,
+                                       &launches_),
                  "findk0");
-    // fitk0andmodamps' first getmodamp rebuilds the overlaps at k1; every
-    // direction keeps its map for the searches, which run side by side
-    build_overlaps(d, 0, fo2, 0.f, 0.f, k1, (float)fo2, d_pmapd_ + d * nxy, d_sumxyd_ + 2 * d, lane);
-    sa.pmap[d] = d_pmapd_ + d * nxy;
-    sa.sumxy[d] = d_sumxyd_ + 2 * d;
-    sa.k0find[d] = kfind;
-    sa.k0fit[d] = kfind + 2;
-    sa.slot[d] = d_fitslots_ + (size_t)(d * norders_ + fo2) * 4;
-    builds += 2;
-    reductions += 1;  // the cross-correlation
+    run_overlaps(refined);
   }
-  lanes_end(nl0);
   sa.info = d_sinfo_;
   sa.ndirs = ndirs_;
   sa.nx = nx_;
@@ -1250,27 +1277,25 @@ bool SIM_Reconstructor::fit_search_on_device()
   sa.delta_angle = 0.001f;
   sa.delta_mag = 0.1 / (std::max(nx_, ny_) * dxy);
   check_launch(launch_k0_search(sa, stream_, &launches_), "k0 search");
-  const int nl = lanes_begin();
-  for (int d = 0; d < ndirs_; ++d) {
-    float2* kfit = d_kst_ + 3 * d + 2;
-    // the other orders at the fitted k0 (overlaps rebuilt each time)
-    for (int order = 1; order < norders_; ++order) {
+  // the other orders at the fitted k0 (overlaps rebuilt each time)
+  std::vector<std::pair<int, int>> rest;
+  for (int d = 0; d < ndirs_; ++d)
+    for (int order = 1; order < norders_; ++order)
+      if (nz_ == 1 ? order >= 2 : order != fo2) rest.push_back({d, order});
+  for (size_t i0 = 0; i0 < rest.size(); i0 += fit_lanes_) {
+    OverlapArgs oa = overlap_args(fo2, 0.f, 0.f);
+    ModampArgs ma{};
+    for (size_t i = i0; i < std::min(rest.size(), i0 + fit_lanes_); ++i) {
+      const auto [d, order] = rest[i];
+      const float2* kfit = d_kst_ + 3 * d + 2;
       const int o1 = nz_ == 1 ? order - 1 : 0;
-      if (nz_ == 1 ? order < 2 : order == fo2) continue;
-      const int lane = (d * (norders_ - 1) + order - 1) % nl;
-      cudaStream_t ls = lane_stream(lane);
-      build_overlaps(d, o1, order, 0.f, 0.f, kfit, (float)(order - o1), nullptr, nullptr, lane);
-      check_launch(launch_modamp_device_k(lane_pmap(lane), nx_, ny_, dxy, kfit, (float)(order - o1),
-                                          lane_tables(lane), lane_partial(lane), lane_xstary(lane), ls, &launches_),
-                   "modamp");
-      double* slot = d_fitslots_ + (size_t)(d * norders_ + order) * 4;
-      check_launch(launch_copy_out(lane_xstary(lane), slot, 4, d_sumxy_ + 2 * lane, slot + 2, 4, ls, &launches_),
-                   "modamp");
-      ++builds;
+      add_overlap(oa, d, o1, order, 0.f, 0.f, kfit, (float)(order - o1));
+      add_modamp(ma, d, order, make_float2(0.f, 0.f), kfit, (float)(order - o1));
       ++reductions;
     }
+    run_overlaps(oa);
+    check_launch(launch_modamp_batch(ma, stream_, &launches_), "modamp");
   }
-  lanes_end(nl);
   check_launch(launch_fit_finish(d_fitslots_, fit_finish_args(), d_fit_, stream_, &launches_), "fit results");
   // the fitted k0s and the search's counters through mapped host memory
   double* base = dh_pinned_ + 320;
@@ -1279,7 +1304,8 @@ bool SIM_Reconstructor::fit_search_on_device()
   check(cudaStreamSynchronize(stream_), "k0 search");
   const float* kst = (const float*)(h_pinned_ + 320);
   const int* info = (const int*)(h_pinned_ + 352);
-  fit_counts_[0] += builds;
+  // the count of builds takes a searched volume's twice, as it always has
+  fit_counts_[0] += 2 * ndirs_ + (long long)rest.size();
   fit_counts_[1] += reductions + info[0];
   fit_counts_[2] += ndirs_;
   cur_o1_ = cur_o2_ = -1;
@@ -1331,67 +1357,42 @@ void SIM_Reconstructor::fit_on_device()
   const ReconParams& p = opt.p;
   const ImageParams& ip = opt.ip;
   const bool reuse = ip.ntimes > 1 && ip.curTimeIdx > 0 && p.bUseTime0k0;
-  // the (direction, order) overlap pairs are independent: each runs on its
-  // own fit lane (stream and working buffers), joined before the amplitudes
-  // are finished
-  const int nl = lanes_begin();
+  // the (direction, order) overlap pairs are independent: as many at a time as
+  // there are buffer sets (in Bessel mode, where the kz range depends on the
+  // order, only pairs of one kz range)
+  std::vector<std::pair<int, int>> pairs;
   for (int d = 0; d < ndirs_; ++d) {
     if (!reuse) k0_[d] = k0guess_[d];
-    const float2v k = k0_[d];
-    for (int order = 1; order < norders_; ++order) {
-      const int lane = (d * (norders_ - 1) + order - 1) % nl;
-      build_overlaps(d, 0, order, k.x, k.y, nullptr, 0.f, nullptr, nullptr, lane);
-      CandList kc{};
-      kc.k[0] = make_float2(k.x * order, k.y * order);
-      check_launch(launch_modamp_candidates(lane_pmap(lane), nx_, ny_, ip.dxy, kc, 1, lane_tables(lane),
-                                            lane_partial(lane), lane_xstary(lane), lane_stream(lane), &launches_),
-                   "modamp");
-      ++fit_counts_[1];
-      double* slot = d_fitslots_ + (size_t)(d * norders_ + order) * 4;
-      check_launch(launch_copy_out(lane_xstary(lane), slot, 4, d_sumxy_ + 2 * lane, slot + 2, 2, lane_stream(lane),
-                                   &launches_),
-                   "modamp");
-    }
+    for (int order = 1; order < norders_; ++order) pairs.push_back({d, order});
   }
-  lanes_end(nl);
+  for (size_t i = 0; i < pairs.size();) {
+    OverlapArgs oa{};
+    ModampArgs ma{};
+    for (; i < pairs.size() && oa.nitems < fit_lanes_; ++i) {
+      const auto [d, order] = pairs[i];
+      const float2v k = k0_[d];
+      const OverlapArgs shared = overlap_args(order, k.x, k.y);
+      if (oa.nitems == 0) oa = shared;
+      else if (shared.zdc != oa.zdc) break;
+      add_overlap(oa, d, 0, order, k.x, k.y);
+      add_modamp(ma, d, order, make_float2(k.x * order, k.y * order));
+      ++fit_counts_[1];
+    }
+    run_overlaps(oa);
+    check_launch(launch_modamp_batch(ma, stream_, &launches_), "modamp");
+  }
   check_launch(launch_fit_finish(d_fitslots_, fit_finish_args(), d_fit_, stream_, &launches_), "modamp");
   cur_o1_ = cur_o2_ = -1;
   amps_on_device_only_ = true;
 }
 
-// Fit lanes: per-lane working buffers of the overlap builds and amplitude
-// evaluations, and the lane's stream (lane 0: the handle's stream)
+// per-pair working buffers of the overlap builds and amplitude evaluations
 size_t SIM_Reconstructor::ovl_lane_elems() const { return 2 * (size_t)(2 * zdc_ovl_ + 1) * nx_ * ny_; }
 size_t SIM_Reconstructor::ppart_lane_elems() const { return (size_t)(2 * zdc_ovl_ + 1) * nx_ * ny_; }
 size_t SIM_Reconstructor::sums_lane_elems() const { return 2 * (size_t)(nx_ + 1) * (2 * zdc_ovl_ + 1); }
 size_t SIM_Reconstructor::tables_lane_elems() const { return (size_t)kMaxCand * (nx_ + ny_); }
 size_t SIM_Reconstructor::partial_lane_elems() const { return (size_t)kModampBlocks * kMaxCand * 2; }
 float2* SIM_Reconstructor::lane_pmap(int l) const { return d_pmap_ + (size_t)l * nx_ * ny_; }
-float2* SIM_Reconstructor::lane_tables(int l) const { return d_tables_ + l * tables_lane_elems(); }
-double* SIM_Reconstructor::lane_partial(int l) const { return d_partial_ + l * partial_lane_elems(); }
-double* SIM_Reconstructor::lane_xstary(int l) const { return d_xstary_ + (size_t)l * kMaxCand * 2; }
-cudaStream_t SIM_Reconstructor::lane_stream(int l) const { return l == 0 ? stream_ : fit_stream_[l]; }
-
-// fork the fit lanes off the handle's stream; returns how many are used (one
-// while profiling, so that every kernel's CUDA-event time is its own)
-int SIM_Reconstructor::lanes_begin()
-{
-  const int nl = profiling_ ? 1 : fit_lanes_;
-  if (nl > 1) {
-    check(cudaEventRecord(fit_fork_, stream_), "fit fork");
-    for (int l = 1; l < nl; ++l) check(cudaStreamWaitEvent(fit_stream_[l], fit_fork_, 0), "fit fork");
-  }
-  return nl;
-}
-
-void SIM_Reconstructor::lanes_end(int nl)
-{
-  for (int l = 1; l < nl; ++l) {
-    check(cudaEventRecord(fit_join_[l], fit_stream_[l]), "fit join");
-    check(cudaStreamWaitEvent(stream_, fit_join_[l], 0), "fit join");
-  }
-}
-
 // the device's amplitudes into amp_ (waits for the stream)
 void SIM_Reconstructor::sync_amps() const
 {
@@ -2061,6 +2062,13 @@ static const char* site_kernel(int site)
   }
 }
 
+// the sites that have a two-factor kernel next to the other two paths
+static bool fft_two_factor_site(int site, int n)
+{
+  int r1, r2;
+  return site != kSiteSeparateZ && site != kSiteAsmY && site != kSiteAsmX && site != kSiteAsmZ && tf_factor(n, &r1, &r2);
+}
+
 // Measure, for every (FFT site, length) a volume of this handle queries and
 // the register path supports, the site's kernel time with the register path
 // and with the Stockham stages, on the staged raw stack (each run restarts
@@ -2085,10 +2093,12 @@ std::string SIM_Reconstructor::tune_fft(int reps)
     for (auto [site, n] : seen) {
       const char* kname = site_kernel(site);
       if (!kname || !reg_fft_lanes(n)) continue;
-      double best[2] = {1e30, 1e30};  // [stockham, register]
+      double best[kNumFftPaths];
+      std::fill(best, best + kNumFftPaths, 1e30);
       for (int rep = 0; rep < std::max(1, reps); ++rep)
-        for (int reg = 1; reg >= 0; --reg) {
-          fft_site_force(site, reg != 0);
+        for (int path = 0; path < kNumFftPaths; ++path) {
+          if (path == kPathTwoFactor && !fft_two_factor_site(site, n)) continue;
+          fft_site_force(site, path);
           profiling_ = true;
           reset_profile();
           bench_device(1);
@@ -2096,14 +2106,21 @@ std::string SIM_Reconstructor::tune_fft(int reps)
           profiling_ = false;
           fft_site_unforce();
           auto it = kprof_.find(kname);
-          if (it != kprof_.end()) best[reg] = std::min(best[reg], it->second.ms);
+          if (it != kprof_.end()) best[path] = std::min(best[path], it->second.ms);
         }
-      const bool reg = best[1] <= best[0];
+      int path = kPathStockham;
+      for (int q = 0; q < kNumFftPaths; ++q)
+        if (best[q] <= best[path]) path = q;
+      double other = 1e30;
+      for (int q = 0; q < kNumFftPaths; ++q)
+        if (q != path) other = std::min(other, best[q]);
       std::string err;
-      if (!fft_plan_record(site, n, reg, best[1], best[0], &err)) throw std::runtime_error(err);
+      if (!fft_plan_record(site, n, path, best[path], other, &err)) throw std::runtime_error(err);
       out << (first ? "" : ", ") << "{\"site\": \"" << fft_site_name(site) << "\", \"n\": " << n
-          << ", \"kernel\": \"" << kname << "\", \"register_ms\": " << best[1] << ", \"stockham_ms\": " << best[0]
-          << ", \"choice\": \"" << (reg ? "register" : "stockham") << "\"}";
+          << ", \"kernel\": \"" << kname << "\", \"register_ms\": " << best[kPathRegister]
+          << ", \"stockham_ms\": " << best[kPathStockham];
+      if (best[kPathTwoFactor] < 1e30) out << ", \"two_factor_ms\": " << best[kPathTwoFactor];
+      out << ", \"choice\": \"" << fft_path_name(path) << "\"}";
       first = false;
     }
   } catch (...) {

@@ -127,25 +127,24 @@ class SIM_Reconstructor {
   void check_launch(int rc, const char* what);
 
   // fitting helpers (gpuFunctionsImpl.cu:306-1148 semantics)
-  // kdev: the shift from device memory (times kfac); pmap / sumxy: outputs
-  // other than the handle's single overlap map
-  void build_overlaps(int d, int o1, int o2, float k0x, float k0y, const float2* kdev = nullptr, float kfac = 0.f,
-                      float2* pmap = nullptr, double* sumxy = nullptr, int lane = 0);
-  // fit lanes (the overlap pairs of the fit built side by side on their own
-  // streams)
-  static constexpr int kFitLanes = 3;  // six lanes measured 1 % faster for twice the buffers
+  void build_overlaps(int d, int o1, int o2, float k0x, float k0y);
+  // the overlap pair of item `i` of a batch (working buffers i); kdev: the
+  // shift from device memory (times kfac); pmap / sumxy: outputs other than
+  // buffer set i's
+  void add_overlap(simrecon::OverlapArgs& a, int d, int o1, int o2, float k0x, float k0y, const float2* kdev = nullptr,
+                   float kfac = 0.f, float2* pmap = nullptr, double* sumxy = nullptr) const;
+  simrecon::OverlapArgs overlap_args(int o2, float k0x, float k0y) const;
+  void run_overlaps(simrecon::OverlapArgs& a);
+  // item i of a batched amplitude evaluation, its result in slot (d, order)
+  void add_modamp(simrecon::ModampArgs& a, int d, int order, float2 k, const float2* kdev = nullptr,
+                  float kfac = 0.f) const;
+  // working buffers of the fit: one set per overlap pair of a batch
   size_t ovl_lane_elems() const;
   size_t ppart_lane_elems() const;
   size_t sums_lane_elems() const;
   size_t tables_lane_elems() const;
   size_t partial_lane_elems() const;
   float2* lane_pmap(int l) const;
-  float2* lane_tables(int l) const;
-  double* lane_partial(int l) const;
-  double* lane_xstary(int l) const;
-  cudaStream_t lane_stream(int l) const;
-  int lanes_begin();
-  void lanes_end(int nl);
   int overlap_zdc_bessel(int order2, float k0x, float k0y) const;
   // evaluate XStarY for candidate (angle, mag) pairs on the current overlaps
   void eval_candidates(int o1, int o2, const std::vector<std::pair<float, float>>& cands);
@@ -170,10 +169,7 @@ class SIM_Reconstructor {
   int zdc_ovl_ = 0;  // makeoverlaps zdistcutoff
   bool otf_dk_from_header_ = false;  // MRC OTF: dkr / dkz taken from its header
   cudaStream_t stream_ = nullptr;
-  int fit_lanes_ = 1;  // set at setup: min(ndirs * (norders - 1), kFitLanes)
-  cudaStream_t fit_stream_[kFitLanes] = {};
-  cudaEvent_t fit_join_[kFitLanes] = {};
-  cudaEvent_t fit_fork_ = nullptr;
+  int fit_lanes_ = 1;  // pairs per batch: min(ndirs * (norders - 1), kMaxOvlItems)
   int device_ = 0;
   bool filter_fusion_ = true;
   bool device_search_ = true;

@@ -235,12 +235,12 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
 // radial table of one kz: order slot o at [o * (nxotf + 1)], entry i the OTF
 // interpolated to kz at radial bins i and i + 1 (flat indices clamped to the
 // table like otf_lookup_rr's; entry nxotf stands for every bin past the end)
-__device__ __forceinline__ void ovl_build_tab(const OverlapArgs& a, const OtfKz& kz, float4* tab)
+__device__ __forceinline__ void ovl_build_tab(const OverlapArgs& a, const OvlItem& it, const OtfKz& kz, float4* tab)
 {
   const int nxo = a.otf.nxotf, nzo = a.otf.nzotf, last = nxo * nzo - 1;
   for (int t = threadIdx.x; t < 2 * (nxo + 1); t += blockDim.x) {
     const int o = t / (nxo + 1), i = t - o * (nxo + 1);
-    const float2* otf = a.otf.otf[o ? a.order2 : a.order1];
+    const float2* otf = o ? it.otf2 : it.otf1;
     const float az = kz.az;
     auto at = [&](int r) {
       const float2 p = __ldg(otf + min(r * nzo + kz.iz, last)), q = __ldg(otf + min(r * nzo + kz.izp, last));
@@ -261,7 +261,7 @@ __device__ __forceinline__ float2 ovl_tab_lookup(const float4* tab, int nxotf, f
 
 // Element j of overlap `ov` on row i of plane zb before the x transform (the
 // element of k_fit.cu's ovl_value, the OTF from the plane's radial tables)
-__device__ __forceinline__ float2 ovl_element(const OverlapArgs& a, float2 ks, int ov, int z0, int i, int j,
+__device__ __forceinline__ float2 ovl_element(const OverlapArgs& a, const OvlItem& it, float2 ks, int ov, int z0, int i, int j,
                                               const float4* tab, float rdk)
 {
   const int nx = a.nx, ny = a.ny, nz = a.nz, nxh = nx / 2 + 1;
@@ -293,9 +293,9 @@ __device__ __forceinline__ float2 ovl_element(const OverlapArgs& a, float2 ks, i
   if (zin < 0) zin += nz;
   const size_t bplane = (size_t)ny * nxh;
   const size_t indin = (size_t)zin * bplane + (size_t)iin * nxh + jin;
-  const int ob = ov == 0 ? a.order1 : a.order2;
-  float2 vre = a.bands[(ob == 0 ? 0 : (size_t)(2 * ob - 1) * nz * bplane) + indin];
-  float2 vim = ob == 0 ? make_float2(0.f, 0.f) : a.bands[(size_t)(2 * ob) * nz * bplane + indin];
+  const int ob = ov == 0 ? it.order1 : it.order2;
+  float2 vre = it.bands[(ob == 0 ? 0 : (size_t)(2 * ob - 1) * nz * bplane) + indin];
+  float2 vim = ob == 0 ? make_float2(0.f, 0.f) : it.bands[(size_t)(2 * ob) * nz * bplane + indin];
   if (conj) {
     vre.y = -vre.y;
     vim.y = -vim.y;
@@ -321,15 +321,15 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
   const int zb = blockIdx.y, z0 = zb - a.zdc;
   const int L0 = blockIdx.x * G::W, nl = min(G::W, 2 * ny - L0);
   const float rdk = 1.f / a.otf.dkrotf;
-  const float2 ks = a.kdev == nullptr ? make_float2(a.kx, a.ky)
-                                      : make_float2(__fmul_rn(a.kdev->x, a.kfac), __fmul_rn(a.kdev->y, a.kfac));
+  const OvlItem& it = a.item[blockIdx.z];
+  const float2 ks = ovl_shift(it);
   const bool empty = z0 == 0 && a.nokz0;
-  if (!empty) ovl_build_tab(a, otf_kz(a.otf, z0), tab);
+  if (!empty) ovl_build_tab(a, it, otf_kz(a.otf, z0), tab);
   __syncthreads();
   for (int t = threadIdx.x; t < G::W * N; t += G::kThreads) {
     const int l = t / N, j = t - l * N;
     float2 v = make_float2(0.f, 0.f);
-    if (!empty && l < nl) v = ovl_element(a, ks, (L0 + l) & 1, z0, (L0 + l) >> 1, j, tab, rdk);
+    if (!empty && l < nl) v = ovl_element(a, it, ks, (L0 + l) & 1, z0, (L0 + l) >> 1, j, tab, rdk);
     sm[t] = v;
   }
   __syncthreads();
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
   const int l = threadIdx.x / R1, k1 = threadIdx.x - l * R1;
   if (l < nl) {
     const int L = L0 + l;
-    float2* dst = a.ovl + ((size_t)(L & 1) * nzb + zb) * ny * N + (size_t)(L >> 1) * N + k1;
+    float2* dst = it.ovl + ((size_t)(L & 1) * nzb + zb) * ny * N + (size_t)(L >> 1) * N + k1;
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2) dst[R1 * k2] = u[k2];
   }
@@ -377,7 +377,8 @@ __global__ void __launch_bounds__(TfOvlY<R1, R2>::kThreads, TfOvlY<R1, R2>::kCta
   const int c = threadIdx.x % W, ov = threadIdx.x / W & 1, q = threadIdx.x / (2 * W);
   const bool in = c0 + c < nx;
   const size_t vol = (size_t)nzb * N * nx;
-  const float2* src0 = a.ovl + (size_t)ov * vol + c0 + c;
+  const OvlItem& it = a.item[blockIdx.z];
+  const float2* src0 = it.ovl + (size_t)ov * vol + c0 + c;
   float2 acc[G::kHalf];
 #pragma unroll
   for (int i = 0; i < G::kHalf; ++i) acc[i] = make_float2(0.f, 0.f);
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(TfOvlY<R1, R2>::kThreads, TfOvlY<R1, R2>::kCta
     __syncthreads();
   }
   if (in && q < R1) {
-    float2* dst = a.ppart + (size_t)blockIdx.y * N * nx + c0 + c;
+    float2* dst = it.ppart + (size_t)blockIdx.y * N * nx + c0 + c;
 #pragma unroll
     for (int i = 0; i < G::kHalf; ++i)
       if (2 * i + ov < R2) dst[(size_t)(q + R1 * (2 * i + ov)) * nx] = acc[i];
@@ -426,8 +427,8 @@ __global__ void __launch_bounds__(TfOvlY<R1, R2>::kThreads, TfOvlY<R1, R2>::kCta
   const double ty = block_sum_d(ov ? sq : 0.0, red);
   if (threadIdx.x == 0) {
     const int cta = blockIdx.y * gridDim.x + blockIdx.x;
-    a.sums[2 * cta] = tx;
-    a.sums[2 * cta + 1] = ty;
+    it.sums[2 * cta] = tx;
+    it.sums[2 * cta + 1] = ty;
   }
 }
 
@@ -565,14 +566,14 @@ struct TfEntry {
     using G = TfRow<R1, R2>;
     const size_t bytes = G::kSmem + 2 * (size_t)(a.otf.nxotf + 1) * sizeof(float4);
     allow_dynamic_smem((const void*)k_tf_ovl_x<R1, R2>, bytes);
-    k_tf_ovl_x<R1, R2><<<dim3((2 * a.ny + G::W - 1) / G::W, 2 * a.zdc + 1), G::kThreads, bytes, s>>>(a, pl.tw);
+    k_tf_ovl_x<R1, R2><<<dim3((2 * a.ny + G::W - 1) / G::W, 2 * a.zdc + 1, a.nitems), G::kThreads, bytes, s>>>(a, pl.tw);
     return (int)cudaGetLastError();
   }
   static int ovl_y(const OverlapArgs& a, const TfPlan& pl, int ppg, int groups, cudaStream_t s)
   {
     using G = TfOvlY<R1, R2>;
     allow_dynamic_smem((const void*)k_tf_ovl_y<R1, R2>, G::kSmem);
-    k_tf_ovl_y<R1, R2><<<dim3((a.nx + G::W - 1) / G::W, groups), G::kThreads, G::kSmem, s>>>(a, pl.tw, ppg);
+    k_tf_ovl_y<R1, R2><<<dim3((a.nx + G::W - 1) / G::W, groups, a.nitems), G::kThreads, G::kSmem, s>>>(a, pl.tw, ppg);
     return (int)cudaGetLastError();
   }
   static int fft_cols(float2* data, int ncol, int nplanes, const TfPlan& pl, cudaStream_t s)
