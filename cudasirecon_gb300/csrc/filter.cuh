@@ -203,6 +203,268 @@ __device__ __forceinline__ float2 filter_scale(const FilterArgs& a, const Filter
   return scale;
 }
 
+// ------------------------------------------------------ pairs of pixels
+// Two float operations in one instruction (each half rounded as the scalar one)
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
+{
+  float2 r;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
+{
+  float2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+  float2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(r))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
+        "l"(reinterpret_cast<unsigned long long&>(c)));
+  return r;
+}
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+
+// |OTF|^2 of order slot T at two radial indices (filter_otf's table lookup)
+__device__ __forceinline__ float2 otf_mag2_pair(const float4* T, float2 kri)
+{
+  const float2 m = add2(add2(kri, dup2(-0.5f)), dup2(12582912.f));
+  const float2 ar = add2(kri, mul2(add2(m, dup2(-12582912.f)), dup2(-1.f)));
+  const float4 t0 = T[__float_as_int(m.x) - 0x4B400000], t1 = T[__float_as_int(m.y) - 0x4B400000];
+  const float2 v0 = fma2(dup2(ar.x), make_float2(t0.z, t0.w), make_float2(t0.x, t0.y));
+  const float2 v1 = fma2(dup2(ar.y), make_float2(t1.z, t1.w), make_float2(t1.x, t1.y));
+  return make_float2(fmaf(v0.x, v0.x, v0.y * v0.y), fmaf(v1.x, v1.x, v1.y * v1.y));
+}
+
+// The terms of the Wiener denominator that a CTA's pixels can meet, in shared
+// memory: (shift x, shift y, |amp|^2 / noisevar, first entry of the order's
+// radial table).  The side orders' terms come first (nside), then the order-0
+// ones.  A term whose support no column of the CTA reaches is left out.
+struct FilterTerms {
+  float4 t[kMaxDirs * (2 * kMaxOrders - 1)];
+  int nside, n;
+};
+
+// built by the CTA's first warp; a barrier must follow.  kx0: the CTA's first
+// column, ncol of them.
+__device__ __forceinline__ void build_filter_terms(const FilterArgs& a, const FilterK& k, int dir, int order, int kz,
+                                                   int kx0, int ncol, FilterTerms& out)
+{
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x, no = a.norders, per = 2 * no - 1, all = a.ndirs * per;
+  int n = 0;
+  for (int zero = 0; zero < 2; ++zero) {  // side orders, then order 0
+    for (int i0 = 0; i0 < all; i0 += 32) {
+      const int i = i0 + lane, d2 = i / per, o2 = i - d2 * per - (no - 1), ao = abs(o2);
+      bool use = i < all && (o2 == 0) == (zero != 0) && !(d2 == dir && o2 == order);
+      if (!a.filteroverlaps && !(o2 == 0 && order == 0)) use = false;
+      if (o2 == 0 && a.nokz0 && kz == 0) use = false;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (use) {
+        const float sx = k.kxo[d2 * no + ao], sy = k.kyo[d2 * no + ao];
+        v = make_float4(o2 < 0 ? -sx : sx, o2 < 0 ? -sy : sy, __ldg(a.fit->termw + d2 * no + ao),
+                        __int_as_float(ao * a.otf.nxotf));
+        bool reach = false;
+        for (int c = 0; c < ncol; ++c) {
+          float x1f = (kx0 + c) * a.dkx;
+          if (order == 0) x1f = fabsf(x1f);  // order 0 is filtered at the stored element's own pixel
+          const float x2 = x1f + k.kxo[dir * no + order] - v.x;
+          reach = reach || x2 * x2 < k.r2_in;
+        }
+        use = reach;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, use);
+      if (use) out.t[n + __popc(m & ((1u << lane) - 1))] = v;
+      n += __popc(m);
+    }
+    if (lane == 0) (zero ? out.n : out.nside) = n;
+  }
+}
+
+// filter_scale's Wiener scale (table path) of two pixels of one column, (x1f,
+// y1f.x) and (x1f, y1f.y).  Two pixels of neighbouring rows take nearly always
+// the same side of a term's support test, share the x half of the distance,
+// and their additions and products pair up in one instruction each.  The terms
+// are a loop over the CTA's list: unrolled over directions and orders the code
+// did not fit the instruction cache, whose misses were the largest stall
+// (2.6 of 8 warps an issue), and a third of its tests were for terms out of
+// the columns' reach.
+__device__ __forceinline__ void filter_scale_pair(const FilterArgs& a, const FilterK& k, const FilterTerms& terms,
+                                                  float ampmag2, int dir, int order, int z0, float2 rdist1, float x1f,
+                                                  float2 y1f, const float4* tabz, float2& s0, float2& s1)
+{
+  const int no = a.norders;
+  const float xabs = x1f + k.kxo[dir * no + order];
+  const float2 yabs = add2(y1f, dup2(k.kyo[dir * no + order]));
+  const float zf = fabsf(z0 / (float)a.zdc[0]);
+  const float zf3 = zf * zf * zf;
+  float2 sum = make_float2(0.f, 0.f);
+  // squared OTF times weight at the radii rd, looked up at the edge (and
+  // dropped by the caller) for a pixel outside
+  const int nside = terms.nside, n = terms.n;
+  const float rsupp = a.suppress ? k.r2_supp : -1.f;
+#pragma unroll 2
+  for (int i = 0; i < nside; ++i) {
+    const float4 t = terms.t[i];
+    const float x2 = xabs - t.x;
+    const float2 y2 = add2(yabs, dup2(-t.y));
+    const float2 r2 = fma2(y2, y2, dup2(x2 * x2));
+    const bool in0 = r2.x < k.r2_in, in1 = r2.y < k.r2_in;  // rdist2 < rdistcutoff
+    if (in0 || in1) {
+      const float2 rd = make_float2(sqrt_approx(fminf(r2.x, k.r2_in)), sqrt_approx(fminf(r2.y, k.r2_in)));
+      float2 w = mul2(otf_mag2_pair(tabz + __float_as_int(t.w), mul2(rd, dup2(k.rdkrotf))), dup2(t.z));
+      if (fminf(r2.x, r2.y) <= rsupp) {
+        if (r2.x <= rsupp) w.x *= dev_suppress(rd.x * k.rmin_dkr);
+        if (r2.y <= rsupp) w.y *= dev_suppress(rd.y * k.rmin_dkr);
+      }
+      sum = add2(sum, make_float2(in0 ? w.x : 0.f, in1 ? w.y : 0.f));
+    }
+  }
+  const bool dampen0 = a.dampen0 != 0;
+#pragma unroll 1
+  for (int i = nside; i < n; ++i) {
+    const float4 t = terms.t[i];
+    const float x2 = xabs - t.x;
+    const float2 y2 = add2(yabs, dup2(-t.y));
+    const float2 r2 = fma2(y2, y2, dup2(x2 * x2));
+    const bool in0 = r2.x < k.r2_in, in1 = r2.y < k.r2_in;
+    if (in0 || in1) {
+      const float2 rd = make_float2(sqrt_approx(fminf(r2.x, k.r2_in)), sqrt_approx(fminf(r2.y, k.r2_in)));
+      float2 w = mul2(otf_mag2_pair(tabz, mul2(rd, dup2(k.rdkrotf))), dup2(t.z));
+      if (dampen0) {
+        const float2 rf = mul2(rd, dup2(k.rrcut));
+        w = mul2(w, fma2(rf, rf, dup2(zf3)));
+      } else {
+        if (r2.x <= rsupp) w.x *= dev_suppress(rd.x * k.rmin_dkr);
+        if (r2.y <= rsupp) w.y *= dev_suppress(rd.y * k.rmin_dkr);
+      }
+      sum = add2(sum, make_float2(in0 ? w.x : 0.f, in1 ? w.y : 0.f));
+    }
+  }
+  const bool drop0 = a.nokz0 && z0 == 0;
+  auto finish = [&](float r1, float yabs1, float others) {
+    const float2 otf1 = filter_otf<false, true>(a, tabz, order, r1 * k.rdkrotf, OtfKz{});
+    float weight = otf1.x * otf1.x + otf1.y * otf1.y;
+    if (order != 0) weight *= ampmag2;
+    float dampfact = k.rnv[dir * no + order];
+    if (dampen0 && order == 0) {
+      const float rf = r1 * k.rrcut;
+      dampfact *= rf * rf + zf3;
+    } else if (a.suppress && r1 <= k.supp_r) {
+      dampfact *= dev_suppress(r1 * k.rmin_dkr);
+    }
+    if (order == 0 && drop0) dampfact = 0;
+    const float f = dampfact / (weight * dampfact + others + a.wiener2);
+    float2 scale = make_float2(otf1.x * f, -otf1.y * f);
+    if (a.apodizeoutput) {
+      const float ra = sqrtf(xabs * xabs + yabs1 * yabs1) * k.rapo;
+      float rho = ra;
+      if (a.zapocutoff > 0) {
+        const float rz = abs(z0) * k.rzapo;
+        rho = sqrtf(ra * ra + rz * rz);
+      }
+      if (rho > 1.f) rho = 1.0f;
+      float apofact = 1.f;
+      if (a.apodizeoutput == 1) apofact = cosf(1.57079632679f * rho);
+      else if (a.apodizeoutput == 2) apofact = 1.0f - rho;
+      scale.x *= apofact;
+      scale.y *= apofact;
+    }
+    return scale;
+  };
+  s0 = finish(rdist1.x, yabs.x, sum.x);
+  s1 = finish(rdist1.y, yabs.y, sum.y);
+}
+
+// The slot whose plane a CTA of the fused assembly filters
+struct FilterSlot {
+  const float2 *br, *bi;  // order 0: band of direction 0 and null
+  size_t plane, dstride;
+  int nx, ny, nz, order, dir, kz;
+  float ampmag2;
+  float2 conjamp;
+};
+
+// Filtered values of column kx on the data rows r0 and r0 + 1 (r0 + 1 may be
+// past the end): rows in transform order, row r at ky = r or r - ny.  A row
+// ny/2 holds the pixel ky = -ny/2 for the filter (both passes of the reference
+// index rows as y in [-ny/2, ny/2 - 1]).
+__device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const FilterK& fk, const FilterSlot& f,
+                                              const FilterTerms& terms, const float4* tab, int kx, int r0, float2& v0,
+                                              float2& v1)
+{
+  v0 = v1 = make_float2(0.f, 0.f);
+  const int nd = fa.ndirs, no = fa.norders;
+  const int nxh = f.nx / 2 + 1;
+  int ky[2];
+  size_t ind[2];
+  float yf[2], rd[2];
+  bool in[2];
+  const float x1f = kx * fa.dkx;
+  const bool conj = kx < 0;
+  int z = conj ? -f.kz : f.kz;
+  if (z < 0) z += f.nz;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = r0 + i;
+    ky[i] = r <= f.ny / 2 ? r : r - f.ny;
+    const int kyf = ky[i] == f.ny / 2 ? -(f.ny / 2) : ky[i];
+    yf[i] = kyf * fa.dky;
+    rd[i] = sqrtf(x1f * x1f + yf[i] * yf[i]);
+    in[i] = r < f.ny && rd[i] <= fa.rdistcutoff;
+    int y = conj ? -ky[i] : ky[i];
+    if (y < 0) y += f.ny;
+    ind[i] = (size_t)z * f.plane + (size_t)y * nxh + (conj ? -kx : kx);
+  }
+  if (!in[0] && !in[1]) return;
+  if (f.order == 0) {
+    // each direction's order-0 band at the stored element's own pixel
+    const float xs = conj ? -x1f : x1f;
+    const float2 ys = make_float2(conj ? (float)(-ky[0]) * fa.dky : yf[0], conj ? (float)(-ky[1]) * fa.dky : yf[1]);
+    const int zs = conj ? -f.kz : f.kz;
+    const float4* tz = tab + (conj ? no * fa.otf.nxotf : 0);
+    // one denominator for every direction (fk.order0_shared): direction d's own
+    // term and the (d, 0) term its sum skips are the same OTF value
+    float2 b0 = in[0] ? f.br[ind[0]] : make_float2(0.f, 0.f), b1 = in[1] ? f.br[ind[1]] : make_float2(0.f, 0.f);
+    for (int d = 1; d < nd; ++d) {
+      if (in[0]) b0 = cadd(b0, f.br[d * f.dstride + ind[0]]);
+      if (in[1]) b1 = cadd(b1, f.br[d * f.dstride + ind[1]]);
+    }
+    float2 s0, s1;
+    filter_scale_pair(fa, fk, terms, 0.f, 0, 0, zs, make_float2(rd[0], rd[1]), xs, ys, tz, s0, s1);
+    v0 = cmul(b0, s0);
+    v1 = cmul(b1, s1);
+    if (conj) {
+      v0.y = -v0.y;
+      v1.y = -v1.y;
+    }
+  } else {
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 re0 = in[0] ? f.br[ind[0]] : zero, im0 = in[0] ? f.bi[ind[0]] : zero;
+    float2 re1 = in[1] ? f.br[ind[1]] : zero, im1 = in[1] ? f.bi[ind[1]] : zero;
+    float2 s0, s1;
+    filter_scale_pair(fa, fk, terms, f.ampmag2, f.dir, f.order, f.kz, make_float2(rd[0], rd[1]), x1f,
+                                  make_float2(yf[0], yf[1]), tab, s0, s1);
+    if (conj) {
+      re0.y = -re0.y;
+      im0.y = -im0.y;
+      re1.y = -re1.y;
+      im1.y = -im1.y;
+    }
+    v0 = cmul(make_float2(re0.x - im0.y, re0.y + im0.x), cmul(s0, f.conjamp));
+    v1 = cmul(make_float2(re1.x - im1.y, re1.y + im1.x), cmul(s1, f.conjamp));
+  }
+  if (!in[0]) v0 = make_float2(0.f, 0.f);
+  if (!in[1]) v1 = make_float2(0.f, 0.f);
+}
+
 // The radial tables of plane zp: each order's OTF interpolated to kz = zp
 // (pass 0) and to the conjugate pass's kz = -zp (pass 1) along kr, with the
 // step to the next bin: [2][no][nxotf]

@@ -356,20 +356,20 @@ __global__ void __launch_bounds__(kThreads, 2) k_asm_y4(AssembleArgs a, const Sl
 // Three CTAs per SM (at most 80 registers): the filter phase needs the warps
 // more than the transform stages need registers (1.61 -> 1.31 ms per
 // 512^2 x 48 volume against two CTAs per SM).
-template <int Y, int NO, int FL>
+template <int Y>
 __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const Slot* __restrict__ slots,
                                                      const float2* __restrict__ tw,
                                                      const __grid_constant__ FilterArgs fa,
                                                      const __grid_constant__ FilterK fk)
 {
-  constexpr int ND = 3;
   constexpr int R1 = colfft_r1(Y), W = 8;
   using CF = ColFft<Y, R1, W>;
   constexpr int R2 = CF::R2;
   static_assert(R2 * W <= kThreads, "one stage-1 item per thread");
   static_assert(Y * W <= CF::kSmemElems, "phase A fits the transform buffer");
   extern __shared__ __align__(16) float2 sm[];
-  float4* tab = (float4*)(sm + CF::kSmemElems);  // [2][NO][nxotf]
+  float4* tab = (float4*)(sm + CF::kSmemElems);  // [2][norders][nxotf]
+  __shared__ FilterTerms terms;
   const Slot sl = slots[blockIdx.y];
   const int nx = a.nx, ny = a.ny, nz = a.nz, nxh = nx / 2 + 1;
   const int c0 = blockIdx.x * W;
@@ -380,84 +380,27 @@ __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const S
   const float2* bi = order == 0 ? nullptr : a.bands + ((size_t)d0 * a.nphases + 2 * order) * nz * plane;
   const size_t dstride = (size_t)a.nphases * nz * plane;  // next direction's band 0
   const int ylo = ny / 2 - 1;                              // ky in [-ylo, ny/2]
-  build_filter_tab(fa, NO, sl.kz, tab);
-  float termw[ND * NO];
-#pragma unroll
-  for (int i = 0; i < ND * NO; ++i) termw[i] = __ldg(fa.fit->termw + i);
+  build_filter_tab(fa, fa.norders, sl.kz, tab);
+  build_filter_terms(fa, fk, d0, order, sl.kz, c0 - (nx / 2 - 1), min(W, nx - c0), terms);
   float ampmag2 = 0.f;
   float2 conjamp = make_float2(1.f, 0.f);
   if (order != 0) {
-    ampmag2 = __ldg(fa.fit->ampmag2 + d0 * NO + order);
-    const float2 am = __ldg(fa.fit->amp + d0 * NO + order);
+    ampmag2 = __ldg(fa.fit->ampmag2 + d0 * fa.norders + order);
+    const float2 am = __ldg(fa.fit->amp + d0 * fa.norders + order);
     conjamp = make_float2(am.x, -am.y);
   }
   __syncthreads();
-  // phase A over the ny data rows (ky in [-ylo, ny/2]); not unrolled (two
-  // copies of the filter code in flight measured 46 % slower)
-  for (int t = threadIdx.x; t < ny * W; t += blockDim.x) {
-    const int r = t / W, w = t - r * W;
-    const int yr = r <= ny / 2 ? r : r + (Y - ny);
-    const int ky = r <= ny / 2 ? r : r - ny;
-    const int c = c0 + w;
-    float2 v = make_float2(0.f, 0.f);
-    if (c < nx) {
-      const int kx = c - (nx / 2 - 1);
-      const int kyf = ky == ny / 2 ? -(ny / 2) : ky;
-      const float x1f = kx * fa.dkx, y1f = kyf * fa.dky;
-      const float rdist1 = sqrtf(x1f * x1f + y1f * y1f);
-      if (rdist1 <= fa.rdistcutoff) {
-        int x = kx, y = ky, z = sl.kz;
-        const bool conj = x < 0;
-        if (conj) {
-          x = -x;
-          y = -y;
-          z = -z;
-        }
-        if (y < 0) y += ny;
-        if (z < 0) z += nz;
-        const size_t indin = (size_t)z * plane + (size_t)y * nxh + x;
-        if (order == 0) {
-          // each direction's order-0 band at the stored element's own pixel
-          const float xs = conj ? -x1f : x1f;
-          const float ys = conj ? (float)(-ky) * fa.dky : y1f;
-          const int zs = conj ? -sl.kz : sl.kz;
-          const float4* tz = tab + (conj ? NO * fa.otf.nxotf : 0);
-          if (fk.order0_shared) {
-            // one denominator for every direction: direction d's own term and
-            // the (d, 0) term its sum skips are the same OTF value
-            const float2 sc = filter_scale<ND, NO, false, true, FL>(fa, fk, termw, 0.f, 0, 0, zs, rdist1, xs, ys, tz);
-            float2 b = br[indin];
-#pragma unroll
-            for (int d = 1; d < ND; ++d) {
-              const float2 u = br[d * dstride + indin];
-              b.x += u.x;
-              b.y += u.y;
-            }
-            v = cmul(b, sc);
-          } else {
+  // phase A over the ny data rows (ky in [-ylo, ny/2]), two rows per thread
+  const FilterSlot fsl{br, bi, plane, dstride, nx, ny, nz, order, d0, sl.kz, ampmag2, conjamp};
 #pragma unroll 1
-            for (int d = 0; d < ND; ++d) {
-              const float2 sc =
-                  filter_scale<ND, NO, false, true, FL>(fa, fk, termw, 0.f, d, 0, zs, rdist1, xs, ys, tz);
-              const float2 b = br[d * dstride + indin];
-              v.x += b.x * sc.x - b.y * sc.y;
-              v.y += b.x * sc.y + b.y * sc.x;
-            }
-          }
-          if (conj) v.y = -v.y;
-        } else {
-          const float2 sc = filter_scale<ND, NO, false, true, FL>(fa, fk, termw, ampmag2, d0, order, sl.kz, rdist1,
-                                                                   x1f, y1f, tab);
-          float2 re = br[indin], im = bi[indin];
-          if (conj) {
-            re.y = -re.y;
-            im.y = -im.y;
-          }
-          v = cmul(make_float2(re.x - im.y, re.y + im.x), cmul(sc, conjamp));
-        }
-      }
-    }
-    sm[yr * W + w] = v;
+  for (int t = threadIdx.x; t < (ny + 1) / 2 * W; t += blockDim.x) {
+    const int r = 2 * (t / W), w = t % W;
+    const int c = c0 + w;
+    float2 v0 = make_float2(0.f, 0.f), v1 = v0;
+    if (c < nx) filtered_rows(fa, fk, fsl, terms, tab, c - (nx / 2 - 1), r, v0, v1);
+    const int yr0 = r <= ny / 2 ? r : r + (Y - ny), yr1 = r + 1 <= ny / 2 ? r + 1 : r + 1 + (Y - ny);
+    sm[yr0 * W + w] = v0;
+    if (r + 1 < ny) sm[yr1 * W + w] = v1;
   }
   __syncthreads();
   // stage 1 from the row-major values (zero-padding rows read as zero)
@@ -516,7 +459,7 @@ __global__ void __launch_bounds__(kXwWarps * 32, 2) k_asm_xw(AssembleArgs a, con
                                                           const int* __restrict__ plane_nslot,
                                                           const Slot* __restrict__ slots,
                                                           const int* __restrict__ plane_zout,
-                                                          const float2* __restrict__ twr)
+                                                          const float2* __restrict__ twr, int real)
 {
   constexpr int P = XwLanes<X>::P, E = X / P, G = 32 / P;
   constexpr int XB = (P + 1) * E + 1;
@@ -593,7 +536,13 @@ __global__ void __launch_bounds__(kXwWarps * 32, 2) k_asm_xw(AssembleArgs a, con
         }
     }
   }
-  if (act) {
+  if (act && real) {  // Z = 1: the real part is the result itself
+    float* dst = a.out + ((size_t)zout * Y + yr) * X;
+#pragma unroll
+    for (int m = 0; m < E / P; ++m)
+#pragma unroll
+      for (int k2 = 0; k2 < P; ++k2) dst[p + P * m + E * k2] = acc[m * P + k2].x;
+  } else if (act) {
     float2* dst = a.S + ((size_t)zout * Y + yr) * X;
 #pragma unroll
     for (int m = 0; m < E / P; ++m)
@@ -835,12 +784,7 @@ namespace {
 // volume the y pass takes 1.31 ms (k_asm_y4f) against 1.45, the x pass
 // 0.56 ms (k_asm_xw) against 0.87; per 256^2 x 32 volume 0.254 / 0.256 and
 // 0.096 / 0.102 ms
-// (k_asm_y4f filters 3 directions with 2 or 3 orders only)
-bool use_y2(const AssembleArgs& a)
-{
-  const bool y4f = colfft_r1(a.Y) && a.ndirs == 3 && (a.norders == 2 || a.norders == 3);
-  return !y4f && asm_y2_supported(a);
-}
+bool use_y2(const AssembleArgs& a) { return !colfft_r1(a.Y) && asm_y2_supported(a); }
 bool use_x2(const AssembleArgs& a)
 {
   return !(a.X == 2 * a.nx && (a.X == 1024 || a.X == 512 || a.X == 256)) && asm_x2_supported(a);
@@ -905,8 +849,9 @@ bool assemble_filter_fusable(const AssembleArgs& a, const FilterArgs& f, bool on
 {
   if (!one_otf || f.bessel || a.ndirs != f.ndirs || a.norders != f.norders) return false;
   if (a.nx != f.nx || a.ny != f.ny || a.nz != f.nz) return false;
-  if (!use_y2(a) && !(colfft_r1(a.Y) && a.ndirs == 3 && (f.norders == 2 || f.norders == 3))) return false;
+  if (!use_y2(a) && !colfft_r1(a.Y)) return false;
   const FilterK k = make_filter_k(f);
+  if (!k.order0_shared) return false;
   if (filter_needs_clamp(f, k)) return false;
   return 2 * (size_t)f.norders * f.otf.nxotf * sizeof(float2) <= kFusedTabMax;
 }
@@ -954,8 +899,9 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
   xlines = std::min(xlines, 16);
   size_t smx = fft_stage_smem(a.X, xlines, xlines * (a.X + 1), kThreads);
 
-  // one output plane and the x pass writes real parts: no z pass
-  const bool x2_real = a.Z == 1 && np_out == 1 && use_x2(a);
+  // one output plane and an x pass that writes real parts: no z pass
+  const bool xw = a.X == 2 * a.nx && (a.X == 1024 || a.X == 512 || a.X == 256);
+  const bool x_real = a.Z == 1 && np_out == 1 && (xw || use_x2(a));
   if (a.X > kAccPerThread * kThreads && !use_x2(a)) return -3;
   // process whole planes in groups whose slots fit in T
   size_t np = p0.size();
@@ -977,32 +923,15 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
       if (rc != 0) return rc;
     } else if (filt) {
       const FilterK fk = make_filter_k(*filt);
-      const int fl = filter_flags(*filt);
       const size_t tabb = 2 * (size_t)filt->norders * filt->otf.nxotf * sizeof(float4);
-      auto go = [&]<int YN, int NO, int FL>() {
+      auto go = [&]<int YN>() {
         const size_t bytes = ColFft<YN, colfft_r1(YN), 8>::kSmemElems * sizeof(float2) + tabb;
-        allow_dynamic_smem((const void*)k_asm_y4f<YN, NO, FL>, bytes);
-        k_asm_y4f<YN, NO, FL><<<dim3((nx + 7) / 8, nsl), kThreads, bytes, s>>>(ay, d_slots + first, py.tw, *filt, fk);
+        allow_dynamic_smem((const void*)k_asm_y4f<YN>, bytes);
+        k_asm_y4f<YN><<<dim3((nx + 7) / 8, nsl), kThreads, bytes, s>>>(ay, d_slots + first, py.tw, *filt, fk);
       };
-      auto by_fl = [&]<int YN, int NO>() {
-        switch (fl) {
-          case 0: go.template operator()<YN, NO, 0>(); break;
-          case 1: go.template operator()<YN, NO, 1>(); break;
-          case 2: go.template operator()<YN, NO, 2>(); break;
-          case 3: go.template operator()<YN, NO, 3>(); break;
-          case 4: go.template operator()<YN, NO, 4>(); break;
-          case 5: go.template operator()<YN, NO, 5>(); break;
-          case 6: go.template operator()<YN, NO, 6>(); break;
-          default: go.template operator()<YN, NO, 7>(); break;
-        }
-      };
-      auto by_no = [&]<int YN>() {
-        if (filt->norders == 3) by_fl.template operator()<YN, 3>();
-        else by_fl.template operator()<YN, 2>();
-      };
-      if (a.Y == 1024) by_no.template operator()<1024>();
-      else if (a.Y == 512) by_no.template operator()<512>();
-      else by_no.template operator()<256>();
+      if (a.Y == 1024) go.template operator()<1024>();
+      else if (a.Y == 512) go.template operator()<512>();
+      else go.template operator()<256>();
     } else if (colfft_r1(a.Y)) {
       auto go = [&]<int YN>() {
         const size_t bytes = ColFft<YN, colfft_r1(YN), 8>::kSmemElems * sizeof(float2);
@@ -1034,11 +963,11 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
       constexpr size_t bytes = xw_smem_bytes<XN>();
       allow_dynamic_smem((const void*)k_asm_xw<XN>, bytes);
       k_asm_xw<XN><<<dim3((a.Y + rows_per_cta - 1) / rows_per_cta, (unsigned)(pj - pi)), kXwWarps * 32, bytes,
-                     s>>>(ax, d_p0 + pi, d_pn + pi, d_slots, d_pz + pi, px.twr);
+                     s>>>(ax, d_p0 + pi, d_pn + pi, d_slots, d_pz + pi, px.twr, x_real);
     };
     // the warp kernel's prefetch ring holds X/2 = nx columns (zoom factor 2)
     if (use_x2(a)) {
-      const int rc = launch_asm_x2(ax, d_slots, d_p0 + pi, d_pn + pi, d_pz + pi, (int)(pj - pi), x2_real, s);
+      const int rc = launch_asm_x2(ax, d_slots, d_p0 + pi, d_pn + pi, d_pz + pi, (int)(pj - pi), x_real, s);
       if (rc != 0) return rc;
     } else if (a.X == 1024 && a.nx == 512) launch_xw.template operator()<1024>();
     else if (a.X == 512 && a.nx == 256) launch_xw.template operator()<512>();
@@ -1055,7 +984,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
   }
   int Wz = std::max(1, std::min(32, kMaxElems / a.Z));
   size_t smz = fft_stage_smem(a.Z, Wz, a.Z * (Wz + 1), kThreads);
-  if (x2_real) {
+  if (x_real) {
     if (launches) *launches += nl;
     return (int)cudaGetLastError();
   }

@@ -33,7 +33,7 @@ constexpr int kThreads = 256;
 // 25.3 -> 7.5 ms, 640 x 384 x 30 2.87 -> 0.89 ms, 1024 x 960 0.293 -> 0.080 ms.
 // At 256/512/1024 output rows the compiled k_asm_y4f stays: 1.31 against
 // 1.45 ms per 512^2 x 48 volume.
-template <int ND, int NO, int FL, bool FILT, int MR>
+template <bool FILT, int MR>
 __global__ void __launch_bounds__(kThreads, MR <= 16 ? 4 : 3) k_asm_y2(AssembleArgs a, const Slot* __restrict__ slots,
                                                                     TfPlan pl, int lw,
                                                                     const __grid_constant__ FilterArgs fa,
@@ -51,107 +51,67 @@ __global__ void __launch_bounds__(kThreads, MR <= 16 ? 4 : 3) k_asm_y2(AssembleA
   const float2* br = a.bands + ((size_t)d0 * a.nphases + (order == 0 ? 0 : 2 * order - 1)) * nz * plane;
   const float2* bi = order == 0 ? nullptr : a.bands + ((size_t)d0 * a.nphases + 2 * order) * nz * plane;
   const size_t dstride = (size_t)a.nphases * nz * plane;  // next direction's band 0
-  const int nd = ND ? ND : a.ndirs, no = NO ? NO : a.norders;
+  const int no = a.norders;
   // the row-major values, then the exchange of both parities over them
   float4* tab = (float4*)(sm + ((2 * R1 * ld + 1) & ~1));  // [2][no][nxotf]
   if constexpr (FILT) {
+    __shared__ FilterTerms terms;
     build_filter_tab(fa, no, sl.kz, tab);
-    __syncthreads();
-  }
-  float termw[ND * NO ? ND * NO : 1];
-  float ampmag2 = 0.f;
-  float2 conjamp = make_float2(1.f, 0.f);
-  if constexpr (FILT) {
-    if constexpr (ND * NO > 0) {
-#pragma unroll
-      for (int i = 0; i < ND * NO; ++i) termw[i] = __ldg(fa.fit->termw + i);
-    }
+    build_filter_terms(fa, fk, d0, order, sl.kz, c0 - (nx / 2 - 1), min(W, nx - c0), terms);
+    float ampmag2 = 0.f;
+    float2 conjamp = make_float2(1.f, 0.f);
     if (order != 0) {
       ampmag2 = __ldg(fa.fit->ampmag2 + d0 * no + order);
       const float2 am = __ldg(fa.fit->amp + d0 * no + order);
       conjamp = make_float2(am.x, -am.y);
     }
-  }
-  const float* tw_p = ND * NO > 0 ? termw : fa.fit->termw;
-  for (int t = threadIdx.x; t < ny << lw; t += kThreads) {
-    const int r = t >> lw, w = t & (W - 1);
-    const int ky = r <= ny / 2 ? r : r - ny;
-    const int c = c0 + w;
-    float2 v = make_float2(0.f, 0.f);
-    if (c < nx) {
-      const int kx = c - (nx / 2 - 1);
-      int x = kx, y = ky, z = sl.kz;
-      const bool conj = x < 0;
-      if (conj) {
-        x = -x;
-        y = -y;
-        z = -z;
-      }
-      if (y < 0) y += ny;
-      if (z < 0) z += nz;
-      const size_t indin = (size_t)z * plane + (size_t)y * nxh + x;
-      if constexpr (FILT) {
-        const int kyf = ky == ny / 2 ? -(ny / 2) : ky;
-        const float x1f = kx * fa.dkx, y1f = kyf * fa.dky;
-        const float rdist1 = sqrtf(x1f * x1f + y1f * y1f);
-        if (rdist1 <= fa.rdistcutoff) {
-          if (order == 0) {
-            // each direction's order-0 band at the stored element's own pixel
-            const float xs = conj ? -x1f : x1f;
-            const float ys = conj ? (float)(-ky) * fa.dky : y1f;
-            const int zs = conj ? -sl.kz : sl.kz;
-            const float4* tz = tab + (conj ? no * fa.otf.nxotf : 0);
-            if (fk.order0_shared) {
-              const float2 sc =
-                  filter_scale<ND, NO, false, true, FL>(fa, fk, tw_p, 0.f, 0, 0, zs, rdist1, xs, ys, tz);
-              float2 b = br[indin];
-              for (int d = 1; d < nd; ++d) {
-                const float2 u = br[d * dstride + indin];
-                b.x += u.x;
-                b.y += u.y;
-              }
-              v = cmul(b, sc);
-            } else {
+    __syncthreads();
+    const FilterSlot fsl{br, bi, plane, dstride, nx, ny, nz, order, d0, sl.kz, ampmag2, conjamp};
 #pragma unroll 1
-              for (int d = 0; d < nd; ++d) {
-                const float2 sc =
-                    filter_scale<ND, NO, false, true, FL>(fa, fk, tw_p, 0.f, d, 0, zs, rdist1, xs, ys, tz);
-                const float2 b = br[d * dstride + indin];
-                v.x += b.x * sc.x - b.y * sc.y;
-                v.y += b.x * sc.y + b.y * sc.x;
-              }
-            }
-            if (conj) v.y = -v.y;
-          } else {
-            const float2 sc = filter_scale<ND, NO, false, true, FL>(fa, fk, tw_p, ampmag2, d0, order, sl.kz, rdist1,
-                                                                     x1f, y1f, tab);
-            float2 re = br[indin], im = bi[indin];
-            if (conj) {
-              re.y = -re.y;
-              im.y = -im.y;
-            }
-            v = cmul(make_float2(re.x - im.y, re.y + im.x), cmul(sc, conjamp));
-          }
-        }
-      } else if (order == 0) {
-        v = br[indin];
-        if (sl.dir < 0)
-          for (int d = 1; d < a.ndirs; ++d) {
-            const float2 u = br[d * dstride + indin];
-            v.x += u.x;
-            v.y += u.y;
-          }
-        if (conj) v.y = -v.y;
-      } else {
-        float2 re = br[indin], im = bi[indin];
-        if (conj) {
-          re.y = -re.y;
-          im.y = -im.y;
-        }
-        v = make_float2(re.x - im.y, re.y + im.x);
-      }
+    for (int t = threadIdx.x; t < (ny / 2) << lw; t += kThreads) {
+      const int r = 2 * (t >> lw), w = t & (W - 1);
+      const int c = c0 + w;
+      float2 v0 = make_float2(0.f, 0.f), v1 = v0;
+      if (c < nx) filtered_rows(fa, fk, fsl, terms, tab, c - (nx / 2 - 1), r, v0, v1);
+      sm[(r << lw) + w] = v0;
+      sm[((r + 1) << lw) + w] = v1;
     }
-    sm[t] = v;
+  } else {
+    for (int t = threadIdx.x; t < ny << lw; t += kThreads) {
+      const int r = t >> lw, w = t & (W - 1);
+      const int c = c0 + w;
+      float2 v = make_float2(0.f, 0.f);
+      if (c < nx) {
+        int x = c - (nx / 2 - 1), y = r <= ny / 2 ? r : r - ny, z = sl.kz;
+        const bool conj = x < 0;
+        if (conj) {
+          x = -x;
+          y = -y;
+          z = -z;
+        }
+        if (y < 0) y += ny;
+        if (z < 0) z += nz;
+        const size_t indin = (size_t)z * plane + (size_t)y * nxh + x;
+        if (order == 0) {
+          v = br[indin];
+          if (sl.dir < 0)
+            for (int d = 1; d < a.ndirs; ++d) {
+              const float2 u = br[d * dstride + indin];
+              v.x += u.x;
+              v.y += u.y;
+            }
+          if (conj) v.y = -v.y;
+        } else {
+          float2 re = br[indin], im = bi[indin];
+          if (conj) {
+            re.y = -re.y;
+            im.y = -im.y;
+          }
+          v = make_float2(re.x - im.y, re.y + im.x);
+        }
+      }
+      sm[t] = v;
+    }
   }
   __syncthreads();
   {  // stage 1: thread (parity b, j, column c)
@@ -223,25 +183,18 @@ int launch_asm_y2(const AssembleArgs& a, const void* d_slots, int nslots, const 
   const size_t bytes = elems * sizeof(float2) + tabb;
   const dim3 g((a.nx + (1 << lw) - 1) >> lw, nslots);
   const Slot* slots = (const Slot*)d_slots;
-  auto go = [&]<int ND, int NO, int FL, bool FILT>() {
+  auto go = [&]<bool FILT>() {
     const FilterArgs fa = filt ? *filt : FilterArgs{};
     const FilterK fk = filt ? make_filter_k(*filt) : FilterK{};
     auto run = [&]<int MR>() {
-      allow_dynamic_smem((const void*)k_asm_y2<ND, NO, FL, FILT, MR>, bytes);
-      k_asm_y2<ND, NO, FL, FILT, MR><<<g, kThreads, bytes, s>>>(a, slots, pl, lw, fa, fk);
+      allow_dynamic_smem((const void*)k_asm_y2<FILT, MR>, bytes);
+      k_asm_y2<FILT, MR><<<g, kThreads, bytes, s>>>(a, slots, pl, lw, fa, fk);
     };
     if (tf_class(pl) == 16) run.template operator()<16>();
     else run.template operator()<32>();
   };
-  // the switches that acquisitions use are compiled in (suppression and
-  // overlap filtering on, order 0 damped in 3D and not in 2D); any other set
-  // is read from the arguments
-  const int fl = filt ? filter_flags(*filt) : 0;
-  if (!filt) go.template operator()<0, 0, 0, false>();
-  else if (a.ndirs == 3 && a.norders == 3 && fl == 7) go.template operator()<3, 3, 7, true>();
-  else if (a.ndirs == 3 && a.norders == 3) go.template operator()<3, 3, -1, true>();
-  else if (a.ndirs == 3 && a.norders == 2 && fl == 5) go.template operator()<3, 2, 5, true>();
-  else go.template operator()<0, 0, -1, true>();
+  if (filt) go.template operator()<true>();
+  else go.template operator()<false>();
   return (int)cudaGetLastError();
 }
 
