@@ -236,20 +236,32 @@ __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 otf_mag2_pair(const float4* T, float2 kri)
 {
   const float2 m = add2(add2(kri, dup2(-0.5f)), dup2(12582912.f));
-  const float2 ar = add2(kri, mul2(add2(m, dup2(-12582912.f)), dup2(-1.f)));
+  const float2 ar = fma2(add2(m, dup2(-12582912.f)), dup2(-1.f), kri);
   const float4 t0 = T[__float_as_int(m.x) - 0x4B400000], t1 = T[__float_as_int(m.y) - 0x4B400000];
   const float2 v0 = fma2(dup2(ar.x), make_float2(t0.z, t0.w), make_float2(t0.x, t0.y));
   const float2 v1 = fma2(dup2(ar.y), make_float2(t1.z, t1.w), make_float2(t1.x, t1.y));
   return make_float2(fmaf(v0.x, v0.x, v0.y * v0.y), fmaf(v1.x, v1.x, v1.y * v1.y));
 }
 
+// square root for the interpolation radius of a pair (subnormal squares flushed)
+__device__ __forceinline__ float2 sqrt_pair(float2 x)
+{
+  float2 r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
+  return r;
+}
+
 // The terms of the Wiener denominator that a CTA's pixels can meet, in shared
-// memory: (shift x, shift y, |amp|^2 / noisevar, first entry of the order's
-// radial table).  The side orders' terms come first (nside), then the order-0
-// ones.  A term whose support no column of the CTA reaches is left out.
+// memory: p = (-shift y twice, |amp|^2 / noisevar twice), aligned pairs for the
+// paired instructions; q = (shift x, first entry of the order's radial table).
+// Three runs: side orders whose suppressed centre no column of the CTA reaches
+// (up to nplain), the other side orders (up to nside), order 0 (up to n).  A
+// term whose support no column reaches is left out.
 struct FilterTerms {
-  float4 t[kMaxDirs * (2 * kMaxOrders - 1)];
-  int nside, n;
+  float4 p[kMaxDirs * (2 * kMaxOrders - 1)];
+  float2 q[kMaxDirs * (2 * kMaxOrders - 1)];
+  int nplain, nside, n;
 };
 
 // built by the CTA's first warp; a barrier must follow.  kx0: the CTA's first
@@ -260,32 +272,68 @@ __device__ __forceinline__ void build_filter_terms(const FilterArgs& a, const Fi
   if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x, no = a.norders, per = 2 * no - 1, all = a.ndirs * per;
   int n = 0;
-  for (int zero = 0; zero < 2; ++zero) {  // side orders, then order 0
+  for (int run = 0; run < 3; ++run) {  // plain side orders, suppressed ones, order 0
     for (int i0 = 0; i0 < all; i0 += 32) {
       const int i = i0 + lane, d2 = i / per, o2 = i - d2 * per - (no - 1), ao = abs(o2);
-      bool use = i < all && (o2 == 0) == (zero != 0) && !(d2 == dir && o2 == order);
+      bool use = i < all && (o2 == 0) == (run == 2) && !(d2 == dir && o2 == order);
       if (!a.filteroverlaps && !(o2 == 0 && order == 0)) use = false;
       if (o2 == 0 && a.nokz0 && kz == 0) use = false;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      float sx = 0.f, sy = 0.f, w = 0.f;
       if (use) {
-        const float sx = k.kxo[d2 * no + ao], sy = k.kyo[d2 * no + ao];
-        v = make_float4(o2 < 0 ? -sx : sx, o2 < 0 ? -sy : sy, __ldg(a.fit->termw + d2 * no + ao),
-                        __int_as_float(ao * a.otf.nxotf));
-        bool reach = false;
+        sx = o2 < 0 ? -k.kxo[d2 * no + ao] : k.kxo[d2 * no + ao];
+        sy = o2 < 0 ? -k.kyo[d2 * no + ao] : k.kyo[d2 * no + ao];
+        w = __ldg(a.fit->termw + d2 * no + ao);
+        bool reach = false, supp = false;
         for (int c = 0; c < ncol; ++c) {
           float x1f = (kx0 + c) * a.dkx;
           if (order == 0) x1f = fabsf(x1f);  // order 0 is filtered at the stored element's own pixel
-          const float x2 = x1f + k.kxo[dir * no + order] - v.x;
+          const float x2 = x1f + k.kxo[dir * no + order] - sx;
           reach = reach || x2 * x2 < k.r2_in;
+          supp = supp || (a.suppress && x2 * x2 <= k.r2_supp);
         }
-        use = reach;
+        use = reach && (run == 2 || supp == (run == 1));
       }
       const unsigned m = __ballot_sync(0xffffffffu, use);
-      if (use) out.t[n + __popc(m & ((1u << lane) - 1))] = v;
+      if (use) {
+        const int at = n + __popc(m & ((1u << lane) - 1));
+        out.p[at] = make_float4(-sy, -sy, w, w);
+        out.q[at] = make_float2(sx, __int_as_float(ao * a.otf.nxotf));
+      }
       n += __popc(m);
     }
-    if (lane == 0) (zero ? out.n : out.nside) = n;
+    if (lane == 0) (run == 0 ? out.nplain : run == 1 ? out.nside : out.n) = n;
   }
+}
+
+// One run of the term list: the sum of the terms' weights at two pixels
+enum : int { kTermPlain = 0, kTermSuppressed = 1, kTermOrder0 = 2 };
+template <int KIND>
+__device__ __forceinline__ float2 sum_terms(const FilterArgs& a, const FilterK& k, const FilterTerms& terms, int i0,
+                                            int i1, float xabs, float2 yabs, float zf3, const float4* tabz, float2 sum)
+{
+#pragma unroll 1
+  for (int i = i0; i < i1; ++i) {
+    const float4 p = terms.p[i];
+    const float2 q = terms.q[i];
+    const float x2 = xabs - q.x;
+    const float2 y2 = add2(yabs, make_float2(p.x, p.y));
+    const float2 r2 = fma2(y2, y2, dup2(x2 * x2));
+    const bool in0 = r2.x < k.r2_in, in1 = r2.y < k.r2_in;  // rdist2 < rdistcutoff
+    if (in0 || in1) {
+      // the one outside (if any) is looked up at the edge and dropped
+      const float2 rd = sqrt_pair(make_float2(fminf(r2.x, k.r2_in), fminf(r2.y, k.r2_in)));
+      float2 w = mul2(otf_mag2_pair(tabz + __float_as_int(q.y), mul2(rd, dup2(k.rdkrotf))), make_float2(p.z, p.w));
+      if (KIND == kTermOrder0 && a.dampen0) {
+        const float2 rf = mul2(rd, dup2(k.rrcut));
+        w = mul2(w, fma2(rf, rf, dup2(zf3)));
+      } else if (KIND == kTermSuppressed || (KIND == kTermOrder0 && a.suppress)) {
+        if (r2.x <= k.r2_supp) w.x *= dev_suppress(rd.x * k.rmin_dkr);
+        if (r2.y <= k.r2_supp) w.y *= dev_suppress(rd.y * k.rmin_dkr);
+      }
+      sum = add2(sum, make_float2(in0 ? w.x : 0.f, in1 ? w.y : 0.f));
+    }
+  }
+  return sum;
 }
 
 // filter_scale's Wiener scale (table path) of two pixels of one column, (x1f,
@@ -306,48 +354,10 @@ __device__ __forceinline__ void filter_scale_pair(const FilterArgs& a, const Fil
   const float zf = fabsf(z0 / (float)a.zdc[0]);
   const float zf3 = zf * zf * zf;
   float2 sum = make_float2(0.f, 0.f);
-  // squared OTF times weight at the radii rd, looked up at the edge (and
-  // dropped by the caller) for a pixel outside
-  const int nside = terms.nside, n = terms.n;
-  const float rsupp = a.suppress ? k.r2_supp : -1.f;
-#pragma unroll 2
-  for (int i = 0; i < nside; ++i) {
-    const float4 t = terms.t[i];
-    const float x2 = xabs - t.x;
-    const float2 y2 = add2(yabs, dup2(-t.y));
-    const float2 r2 = fma2(y2, y2, dup2(x2 * x2));
-    const bool in0 = r2.x < k.r2_in, in1 = r2.y < k.r2_in;  // rdist2 < rdistcutoff
-    if (in0 || in1) {
-      const float2 rd = make_float2(sqrt_approx(fminf(r2.x, k.r2_in)), sqrt_approx(fminf(r2.y, k.r2_in)));
-      float2 w = mul2(otf_mag2_pair(tabz + __float_as_int(t.w), mul2(rd, dup2(k.rdkrotf))), dup2(t.z));
-      if (fminf(r2.x, r2.y) <= rsupp) {
-        if (r2.x <= rsupp) w.x *= dev_suppress(rd.x * k.rmin_dkr);
-        if (r2.y <= rsupp) w.y *= dev_suppress(rd.y * k.rmin_dkr);
-      }
-      sum = add2(sum, make_float2(in0 ? w.x : 0.f, in1 ? w.y : 0.f));
-    }
-  }
+  sum = sum_terms<kTermPlain>(a, k, terms, 0, terms.nplain, xabs, yabs, zf3, tabz, sum);
+  sum = sum_terms<kTermSuppressed>(a, k, terms, terms.nplain, terms.nside, xabs, yabs, zf3, tabz, sum);
+  sum = sum_terms<kTermOrder0>(a, k, terms, terms.nside, terms.n, xabs, yabs, zf3, tabz, sum);
   const bool dampen0 = a.dampen0 != 0;
-#pragma unroll 1
-  for (int i = nside; i < n; ++i) {
-    const float4 t = terms.t[i];
-    const float x2 = xabs - t.x;
-    const float2 y2 = add2(yabs, dup2(-t.y));
-    const float2 r2 = fma2(y2, y2, dup2(x2 * x2));
-    const bool in0 = r2.x < k.r2_in, in1 = r2.y < k.r2_in;
-    if (in0 || in1) {
-      const float2 rd = make_float2(sqrt_approx(fminf(r2.x, k.r2_in)), sqrt_approx(fminf(r2.y, k.r2_in)));
-      float2 w = mul2(otf_mag2_pair(tabz, mul2(rd, dup2(k.rdkrotf))), dup2(t.z));
-      if (dampen0) {
-        const float2 rf = mul2(rd, dup2(k.rrcut));
-        w = mul2(w, fma2(rf, rf, dup2(zf3)));
-      } else {
-        if (r2.x <= rsupp) w.x *= dev_suppress(rd.x * k.rmin_dkr);
-        if (r2.y <= rsupp) w.y *= dev_suppress(rd.y * k.rmin_dkr);
-      }
-      sum = add2(sum, make_float2(in0 ? w.x : 0.f, in1 ? w.y : 0.f));
-    }
-  }
   const bool drop0 = a.nokz0 && z0 == 0;
   auto finish = [&](float r1, float yabs1, float others) {
     const float2 otf1 = filter_otf<false, true>(a, tabz, order, r1 * k.rdkrotf, OtfKz{});
