@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(kThreads) k_asm_z1(const float4* __restrict__ 
   }
 }
 
-// Four-step variant of k_asm_z for Z = 16 * R1: 64 columns of one output row
+// Four-step variant of k_asm_z for Z = 16 * R1 above 64 (80, 96, 128): 64 columns of one output row
 // per CTA.  Stage 1: the thread for (column c, j < 16) loads the R1 planes
 // z = j + 16 e of S (only the in-band ones; the rest are zero) and runs the
 // inverse R1-point DFT times conj(W_Z^(j k1)); stage 2: the thread for
@@ -996,26 +996,25 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
     const size_t npairs = (size_t)a.X * a.Y / 2;
     const unsigned nb = (unsigned)std::min<size_t>((npairs + kThreads - 1) / kThreads, 152 * 16);
     k_asm_z1<<<nb, kThreads, 0, s>>>((const float4*)a.S, (float2*)a.out, npairs, d_zact);
-  } else if (zr1 == 2 || zr1 == 3 || zr1 == 4 || zr1 == 5 || zr1 == 6 || zr1 == 8) {
+  } else if (z_length_ok(a.Z)) {
+    // (for Z = 32, 48, 64 against k_asm_z4's 64-column tiles: 28.6 -> 16.3 us
+    // per 256^2 x 32 volume, 0.129 -> 0.117 ms per 512^2 x 48)
+    unsigned long long active = 0;
+    for (int z = 0; z < a.Z; ++z)
+      if (tabs.zact[z]) active |= 1ull << z;
+    const int rc = launch_asm_zn(a.S, a.out, a.X, a.Y, a.Z, active, pz.tw, split, s);
+    if (rc != 0) return rc;
+  } else if (zr1 == 5 || zr1 == 6 || zr1 == 8) {
     auto go = [&]<int R1>() {
       const size_t bytes = (size_t)R1 * (16 * 64 + 8) * sizeof(float2);
       allow_dynamic_smem((const void*)k_asm_z4<R1>, bytes);
       k_asm_z4<R1><<<dim3((a.X + 63) / 64, a.Y), kThreads, bytes, s>>>(a, d_zact, pz.tw, split);
     };
     switch (zr1) {
-      case 2: go.template operator()<2>(); break;
-      case 3: go.template operator()<3>(); break;
-      case 4: go.template operator()<4>(); break;
       case 5: go.template operator()<5>(); break;
       case 6: go.template operator()<6>(); break;
       default: go.template operator()<8>(); break;
     }
-  } else if (z_length_ok(a.Z) && !reg_fft_lanes(a.Z)) {
-    unsigned long long active = 0;
-    for (int z = 0; z < a.Z; ++z)
-      if (tabs.zact[z]) active |= 1ull << z;
-    const int rc = launch_asm_zn(a.S, a.out, a.X, a.Y, a.Z, active, pz.tw, split, s);
-    if (rc != 0) return rc;
   } else {
     dispatch_fft_len(kSiteAsmZ, a.Z, [&]<int NF>() {
       allow_dynamic_smem((const void*)k_asm_z<NF>, smz);

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kThreads, MR <= 16 ? 4 : 3) k_asm_y2(AssembleA
       if (act) {
         if (b) tf_half_shift<R, +1>(v);
         reg_dft<R, +1>(v);
-        tf_twiddle<R, +1>(v, b ? pl.twh : pl.tw, R2, j);
+        tf_twiddle_half<R, +1>(v, b ? pl.twh : pl.tw, R2, j);
         float2* ex = sm + b * R1 * ld;
 #pragma unroll
         for (int k1 = 0; k1 < R; ++k1) ex[k1 * ld + (j << lw) + c] = v[k1];

@@ -302,8 +302,10 @@ __global__ void __launch_bounds__(kIngestWarps * 32, 3) k_ingest_xw(IngestArgs a
 
 // Four-step variant (col_fft.cuh) for the lengths with a column
 // configuration: 8 columns of one plane per CTA, loaded straight from HBM.
+// Held to half of the registers (left alone the 1024-point kernel takes more:
+// 2.39 instead of 1.72 ms per 1024^2 x 64 volume).
 template <int N>
-__global__ void __launch_bounds__(kThreads) k_fft_cols_4s(float2* data, int ncol, const float2* __restrict__ tw)
+__global__ void __launch_bounds__(kThreads, 2) k_fft_cols_4s(float2* data, int ncol, const float2* __restrict__ tw)
 {
   constexpr int R1 = colfft_r1(N), W = 8;
   extern __shared__ float2 sm[];  // ColFft<N, R1, W>::kSmemElems
@@ -454,7 +456,11 @@ int launch_ingest(const IngestArgs& a, cudaStream_t s, long long* launches)
   TfPlan tx, ty;
   const bool wx = a.nx == 512 || a.nx == 1024 || a.nx == 256;  // warp kernels
   const TfKernels* kx = !wx && fft_two_factor(kSiteIngestX, a.nx) ? tf_kernels(a.nx, &tx) : nullptr;
-  const TfKernels* ky = !colfft_r1(a.ny) && fft_two_factor(kSiteIngestY, a.ny) ? tf_kernels(a.ny, &ty) : nullptr;
+  // 1024 rows keep their compiled kernel: 1.72 against 1.93 ms per 1024^2 x 64
+  // volume (256 rows: 0.046 two-factor against 0.057 ms per 256^2 x 32)
+  const TfKernels* ky = a.ny == 512 || a.ny == 256 || (a.ny != 1024 && fft_two_factor(kSiteIngestY, a.ny))
+                            ? tf_kernels(a.ny, &ty)
+                            : nullptr;
   if (a.nx == 512) go_w.template operator()<512>();
   else if (a.nx == 1024) go_w.template operator()<1024>();
   else if (a.nx == 256) go_w.template operator()<256>();
@@ -486,16 +492,10 @@ int launch_ingest(const IngestArgs& a, cudaStream_t s, long long* launches)
   size_t smy = fft_smem(a.ny, W, a.ny * (W + 1));
   dim3 gy((nxh + W - 1) / W, nplanes);
   if (kt) kt->begin(s);
-  if (colfft_r1(a.ny)) {
-    dim3 g4((nxh + 7) / 8, nplanes);
-    auto go = [&]<int N>() {
-      const size_t bytes = ColFft<N, colfft_r1(N), 8>::kSmemElems * sizeof(float2);
-      allow_dynamic_smem((const void*)k_fft_cols_4s<N>, bytes);
-      k_fft_cols_4s<N><<<g4, kThreads, bytes, s>>>(a.spec, nxh, py.tw);
-    };
-    if (a.ny == 512) go.template operator()<512>();
-    else if (a.ny == 1024) go.template operator()<1024>();
-    else go.template operator()<256>();
+  if (a.ny == 1024) {
+    const size_t bytes = ColFft<1024, colfft_r1(1024), 8>::kSmemElems * sizeof(float2);
+    allow_dynamic_smem((const void*)k_fft_cols_4s<1024>, bytes);
+    k_fft_cols_4s<1024><<<dim3((nxh + 7) / 8, nplanes), kThreads, bytes, s>>>(a.spec, nxh, py.tw);
   } else if (ky) {
     const int rc = ky->fft_cols(a.spec, nxh, nplanes, ty, s);
     if (rc != 0) return rc;

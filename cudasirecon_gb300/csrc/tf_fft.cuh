@@ -83,9 +83,21 @@ __device__ __forceinline__ void tf_half_shift(float2* v)
   for (int e = 1; e < R; ++e) v[e] = cmul(v[e], w_root<2 * R>(e, DIR));
 }
 
-// v[k1] *= W_n^(j k1) from the plan's table (tw or twh), k1 * r2 + j
+// v[k1] *= W_n^(j k1) from the plan's table tw, k1 * r2 + j (k1 = 0: 1)
 template <int R, int DIR>
 __device__ __forceinline__ void tf_twiddle(float2* v, const float2* __restrict__ tw, int r2, int j)
+{
+#pragma unroll
+  for (int k1 = 1; k1 < R; ++k1) {
+    float2 w = __ldg(tw + k1 * r2 + j);
+    if (DIR > 0) w.y = -w.y;
+    v[k1] = cmul(v[k1], w);
+  }
+}
+
+// the same from tw or, half shifted, twh (whose k1 = 0 is not 1)
+template <int R, int DIR>
+__device__ __forceinline__ void tf_twiddle_half(float2* v, const float2* __restrict__ tw, int r2, int j)
 {
 #pragma unroll
   for (int k1 = 0; k1 < R; ++k1) {
