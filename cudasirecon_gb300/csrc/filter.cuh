@@ -271,6 +271,7 @@ __device__ __forceinline__ void build_filter_terms(const FilterArgs& a, const Fi
 {
   if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x, no = a.norders, per = 2 * no - 1, all = a.ndirs * per;
+  const float kxo = __ldg(a.fit->kxo + dir * no + order);
   int n = 0;
   for (int run = 0; run < 3; ++run) {  // plain side orders, suppressed ones, order 0
     for (int i0 = 0; i0 < all; i0 += 32) {
@@ -280,14 +281,18 @@ __device__ __forceinline__ void build_filter_terms(const FilterArgs& a, const Fi
       if (o2 == 0 && a.nokz0 && kz == 0) use = false;
       float sx = 0.f, sy = 0.f, w = 0.f;
       if (use) {
-        sx = o2 < 0 ? -k.kxo[d2 * no + ao] : k.kxo[d2 * no + ao];
-        sy = o2 < 0 ? -k.kyo[d2 * no + ao] : k.kyo[d2 * no + ao];
+        sx = __ldg(a.fit->kxo + d2 * no + ao);
+        sy = __ldg(a.fit->kyo + d2 * no + ao);
+        if (o2 < 0) {
+          sx = -sx;
+          sy = -sy;
+        }
         w = __ldg(a.fit->termw + d2 * no + ao);
         bool reach = false, supp = false;
         for (int c = 0; c < ncol; ++c) {
           float x1f = (kx0 + c) * a.dkx;
           if (order == 0) x1f = fabsf(x1f);  // order 0 is filtered at the stored element's own pixel
-          const float x2 = x1f + k.kxo[dir * no + order] - sx;
+          const float x2 = x1f + kxo - sx;
           reach = reach || x2 * x2 < k.r2_in;
           supp = supp || (a.suppress && x2 * x2 <= k.r2_supp);
         }
@@ -336,6 +341,31 @@ __device__ __forceinline__ float2 sum_terms(const FilterArgs& a, const FilterK& 
   return sum;
 }
 
+// The slot whose plane a CTA of the fused assembly filters
+struct FilterSlot {
+  const float2 *br, *bi;  // order 0: band of direction 0 and null
+  size_t plane, dstride;
+  int nx, ny, nz, order, dir, kz;
+  float ampmag2;
+  float2 conjamp;
+  float kxo, kyo, rapo;  // the fit's values for (dir, order): FitDev
+};
+// the fit's part of the slot (dir = 0 for the summed order 0)
+__device__ __forceinline__ void load_fit(const FilterArgs& a, FilterSlot& f)
+{
+  const int i = f.dir * a.norders + f.order;
+  f.ampmag2 = 0.f;
+  f.conjamp = make_float2(1.f, 0.f);
+  if (f.order != 0) {
+    f.ampmag2 = __ldg(a.fit->ampmag2 + i);
+    const float2 am = __ldg(a.fit->amp + i);
+    f.conjamp = make_float2(am.x, -am.y);
+  }
+  f.kxo = __ldg(a.fit->kxo + i);
+  f.kyo = __ldg(a.fit->kyo + i);
+  f.rapo = __ldg(&a.fit->rapo);
+}
+
 // filter_scale's Wiener scale (table path) of two pixels of one column, (x1f,
 // y1f.x) and (x1f, y1f.y).  Two pixels of neighbouring rows take nearly always
 // the same side of a term's support test, share the x half of the distance,
@@ -345,12 +375,13 @@ __device__ __forceinline__ float2 sum_terms(const FilterArgs& a, const FilterK& 
 // (2.6 of 8 warps an issue), and a third of its tests were for terms out of
 // the columns' reach.
 __device__ __forceinline__ void filter_scale_pair(const FilterArgs& a, const FilterK& k, const FilterTerms& terms,
-                                                  float ampmag2, int dir, int order, int z0, float2 rdist1, float x1f,
-                                                  float2 y1f, const float4* tabz, float2& s0, float2& s1)
+                                                  const FilterSlot& f, int z0, float2 rdist1, float x1f, float2 y1f,
+                                                  const float4* tabz, float2& s0, float2& s1)
 {
-  const int no = a.norders;
-  const float xabs = x1f + k.kxo[dir * no + order];
-  const float2 yabs = add2(y1f, dup2(k.kyo[dir * no + order]));
+  const int order = f.order, i1 = f.dir * a.norders + order;
+  const float ampmag2 = f.ampmag2;
+  const float xabs = x1f + f.kxo;
+  const float2 yabs = add2(y1f, dup2(f.kyo));
   const float zf = fabsf(z0 / (float)a.zdc[0]);
   const float zf3 = zf * zf * zf;
   float2 sum = make_float2(0.f, 0.f);
@@ -363,7 +394,7 @@ __device__ __forceinline__ void filter_scale_pair(const FilterArgs& a, const Fil
     const float2 otf1 = filter_otf<false, true>(a, tabz, order, r1 * k.rdkrotf, OtfKz{});
     float weight = otf1.x * otf1.x + otf1.y * otf1.y;
     if (order != 0) weight *= ampmag2;
-    float dampfact = k.rnv[dir * no + order];
+    float dampfact = k.rnv[i1];
     if (dampen0 && order == 0) {
       const float rf = r1 * k.rrcut;
       dampfact *= rf * rf + zf3;
@@ -371,10 +402,10 @@ __device__ __forceinline__ void filter_scale_pair(const FilterArgs& a, const Fil
       dampfact *= dev_suppress(r1 * k.rmin_dkr);
     }
     if (order == 0 && drop0) dampfact = 0;
-    const float f = dampfact / (weight * dampfact + others + a.wiener2);
-    float2 scale = make_float2(otf1.x * f, -otf1.y * f);
+    const float q = dampfact / (weight * dampfact + others + a.wiener2);
+    float2 scale = make_float2(otf1.x * q, -otf1.y * q);
     if (a.apodizeoutput) {
-      const float ra = sqrtf(xabs * xabs + yabs1 * yabs1) * k.rapo;
+      const float ra = sqrtf(xabs * xabs + yabs1 * yabs1) * f.rapo;
       float rho = ra;
       if (a.zapocutoff > 0) {
         const float rz = abs(z0) * k.rzapo;
@@ -392,15 +423,6 @@ __device__ __forceinline__ void filter_scale_pair(const FilterArgs& a, const Fil
   s0 = finish(rdist1.x, yabs.x, sum.x);
   s1 = finish(rdist1.y, yabs.y, sum.y);
 }
-
-// The slot whose plane a CTA of the fused assembly filters
-struct FilterSlot {
-  const float2 *br, *bi;  // order 0: band of direction 0 and null
-  size_t plane, dstride;
-  int nx, ny, nz, order, dir, kz;
-  float ampmag2;
-  float2 conjamp;
-};
 
 // Filtered values of column kx on the data rows r0 and r0 + 1 (r0 + 1 may be
 // past the end): rows in transform order, row r at ky = r or r - ny.  A row
@@ -448,7 +470,7 @@ __device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const Filter
       if (in[1]) b1 = cadd(b1, f.br[d * f.dstride + ind[1]]);
     }
     float2 s0, s1;
-    filter_scale_pair(fa, fk, terms, 0.f, 0, 0, zs, make_float2(rd[0], rd[1]), xs, ys, tz, s0, s1);
+    filter_scale_pair(fa, fk, terms, f, zs, make_float2(rd[0], rd[1]), xs, ys, tz, s0, s1);
     v0 = cmul(b0, s0);
     v1 = cmul(b1, s1);
     if (conj) {
@@ -460,8 +482,7 @@ __device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const Filter
     float2 re0 = in[0] ? f.br[ind[0]] : zero, im0 = in[0] ? f.bi[ind[0]] : zero;
     float2 re1 = in[1] ? f.br[ind[1]] : zero, im1 = in[1] ? f.bi[ind[1]] : zero;
     float2 s0, s1;
-    filter_scale_pair(fa, fk, terms, f.ampmag2, f.dir, f.order, f.kz, make_float2(rd[0], rd[1]), x1f,
-                                  make_float2(yf[0], yf[1]), tab, s0, s1);
+    filter_scale_pair(fa, fk, terms, f, f.kz, make_float2(rd[0], rd[1]), x1f, make_float2(yf[0], yf[1]), tab, s0, s1);
     if (conj) {
       re0.y = -re0.y;
       im0.y = -im0.y;

@@ -382,16 +382,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const S
   const int ylo = ny / 2 - 1;                              // ky in [-ylo, ny/2]
   build_filter_tab(fa, fa.norders, sl.kz, tab);
   build_filter_terms(fa, fk, d0, order, sl.kz, c0 - (nx / 2 - 1), min(W, nx - c0), terms);
-  float ampmag2 = 0.f;
-  float2 conjamp = make_float2(1.f, 0.f);
-  if (order != 0) {
-    ampmag2 = __ldg(fa.fit->ampmag2 + d0 * fa.norders + order);
-    const float2 am = __ldg(fa.fit->amp + d0 * fa.norders + order);
-    conjamp = make_float2(am.x, -am.y);
-  }
+  FilterSlot fsl{br, bi, plane, dstride, nx, ny, nz, order, d0, sl.kz};
+  load_fit(fa, fsl);
   __syncthreads();
   // phase A over the ny data rows (ky in [-ylo, ny/2]), two rows per thread
-  const FilterSlot fsl{br, bi, plane, dstride, nx, ny, nz, order, d0, sl.kz, ampmag2, conjamp};
 #pragma unroll 1
   for (int t = threadIdx.x; t < (ny + 1) / 2 * W; t += blockDim.x) {
     const int r = 2 * (t / W), w = t % W;
@@ -639,14 +633,14 @@ __global__ void __launch_bounds__(kThreads) k_asm_z4(AssembleArgs a, const unsig
   }
 }
 
-__global__ void k_ramp(const __grid_constant__ K0List k0, int ndirs, int norders, int X, int Y, float dxyz, float fact,
+__global__ void k_ramp(const FitDev* __restrict__ fit, int ndirs, int norders, int X, int Y, float dxyz, float fact,
                        float2* ex, float2* ey, int split)
 {
   int n = ndirs * norders * (X + Y);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     int ro = t / (X + Y), r = t - ro * (X + Y);
     int d = ro / norders, o = ro - d * norders;
-    float kx = k0.k[d].x * (float)o, ky = k0.k[d].y * (float)o;
+    float kx = fit->k0[d].x * (float)o, ky = fit->k0[d].y * (float)o;
     double ang;
     if (r < X) ang = (double)fact * M_PI * (double)(r - X / 2) * (double)kx * (double)dxyz;
     else ang = (double)fact * M_PI * (double)((r - X) - Y / 2) * (double)ky * (double)dxyz;
@@ -791,13 +785,13 @@ bool use_x2(const AssembleArgs& a)
 }
 }  // namespace
 
-int launch_ramp_tables(const K0List& k0, const AssembleArgs& a, float dxyz, float fact, float2* ex, float2* ey,
+int launch_ramp_tables(const FitDev* fit, const AssembleArgs& a, float dxyz, float fact, float2* ex, float2* ey,
                        cudaStream_t s, long long* launches)
 {
   const int ndirs = a.ndirs, norders = a.norders, X = a.X, Y = a.Y;
   if (ndirs < 1 || ndirs > kMaxDirs) return -1;
   int n = ndirs * norders * (X + Y);
-  k_ramp<<<std::min(1024, (n + 255) / 256), 256, 0, s>>>(k0, ndirs, norders, X, Y, dxyz, fact, ex, ey, use_x2(a));
+  k_ramp<<<std::min(1024, (n + 255) / 256), 256, 0, s>>>(fit, ndirs, norders, X, Y, dxyz, fact, ex, ey, use_x2(a));
   if (launches) *launches += 1;
   return (int)cudaGetLastError();
 }

@@ -58,15 +58,9 @@ __global__ void __launch_bounds__(kThreads, MR <= 16 ? 4 : 3) k_asm_y2(AssembleA
     __shared__ FilterTerms terms;
     build_filter_tab(fa, no, sl.kz, tab);
     build_filter_terms(fa, fk, d0, order, sl.kz, c0 - (nx / 2 - 1), min(W, nx - c0), terms);
-    float ampmag2 = 0.f;
-    float2 conjamp = make_float2(1.f, 0.f);
-    if (order != 0) {
-      ampmag2 = __ldg(fa.fit->ampmag2 + d0 * no + order);
-      const float2 am = __ldg(fa.fit->amp + d0 * no + order);
-      conjamp = make_float2(am.x, -am.y);
-    }
+    FilterSlot fsl{br, bi, plane, dstride, nx, ny, nz, order, d0, sl.kz};
+    load_fit(fa, fsl);
     __syncthreads();
-    const FilterSlot fsl{br, bi, plane, dstride, nx, ny, nz, order, d0, sl.kz, ampmag2, conjamp};
 #pragma unroll 1
     for (int t = threadIdx.x; t < (ny / 2) << lw; t += kThreads) {
       const int r = 2 * (t >> lw), w = t & (W - 1);

@@ -878,7 +878,8 @@ __device__ __forceinline__ float2 cmul_rn(float2 a, float2 b)
 }
 __device__ __forceinline__ float mag2_rn(float2 a) { return __fadd_rn(__fmul_rn(a.x, a.x), __fmul_rn(a.y, a.y)); }
 
-// |amp|^2 and the filter's per-term weights (filterbands, gpuFunctionsImpl.cu:1341-1360)
+// |amp|^2, the filter's per-term weights (filterbands, gpuFunctionsImpl.cu:1341-1360)
+// and shifts, and the copy for the host
 __device__ void fit_derived(const FitFinishArgs& a, FitDev* out)
 {
   for (int i = threadIdx.x; i < a.ndirs * a.norders; i += 32) {
@@ -886,7 +887,21 @@ __device__ void fit_derived(const FitFinishArgs& a, FitDev* out)
     const float m2 = mag2_rn(out->amp[i]);
     out->ampmag2[i] = m2;
     out->termw[i] = o == 0 ? a.rnv[i] : __fdiv_rn(m2, a.noisevar[i]);
+    const int d = i / a.norders;
+    const float2 k = a.kdev ? a.kdev[3 * d] : a.k0[d];
+    out->kxo[i] = __fmul_rn((float)o, k.x);
+    out->kyo[i] = __fmul_rn((float)o, k.y);
+    if (o == 0) out->k0[d] = k;
+    if (i == 0) {  // filterbands' apocutoff (gpuFunctionsImpl.cu:1241-1298), float arithmetic
+      const float mag = __fsqrt_rn(mag2_rn(k));
+      out->rapo = __fdiv_rn(1.f, __fadd_rn(a.rdistcutoff, __fmul_rn(mag, (float)(a.norders - 1))));
+    }
+    if (a.host) {
+      a.host->amp[i] = out->amp[i];
+      if (o == 0) a.host->k0[d] = k;
+    }
   }
+  if (a.host && threadIdx.x < 2) a.host->info[threadIdx.x] = a.info[threadIdx.x];
 }
 
 // findModulationVectorsAndPhasesForAllDirections without a k0 search

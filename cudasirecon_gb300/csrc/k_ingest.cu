@@ -355,14 +355,14 @@ __global__ void __launch_bounds__(kThreads) k_separate(float2* spec, const float
   __syncthreads();
   const size_t plane = (size_t)ny * nxh;
   float2* dbase = spec + (size_t)d * nph * nz * plane + (size_t)ky * nxh + c0;
-  const float* dscale = scale + d * nph * nz;
+  const float* dscale = scale ? scale + d * nph * nz : nullptr;
   const int ld = nph * W + 1;  // odd pitch
   for (int t = threadIdx.x; t < nz * W; t += blockDim.x) {
     int z = t / W, w = t - z * W;
     float2 in[kMaxPhases];
     bool ok = c0 + w < nxh;
     for (int p = 0; p < nph; ++p) {
-      float s = dscale[p * nz + z];
+      float s = dscale ? dscale[p * nz + z] : 1.f;
       float2 v = ok ? dbase[((size_t)p * nz + z) * plane + w] : make_float2(0.f, 0.f);
       in[p] = make_float2(v.x * s, v.y * s);
     }
@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(kThreads) k_separate_z1(float2* spec, const fl
   float2 in[NPH];
 #pragma unroll
   for (int p = 0; p < NPH; ++p) {
-    const float s = scale[d * NPH + p];
+    const float s = scale ? scale[d * NPH + p] : 1.f;
     const float2 v = base[(size_t)p * plane];
     in[p] = make_float2(v.x * s, v.y * s);
   }
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(kThreads) k_separate4(float2* spec, const floa
   __syncthreads();
   const size_t plane = (size_t)ny * nxh;
   float2* dbase = spec + (size_t)d * nph * NZ * plane + (size_t)ky * nxh + c0;
-  const float* dscale = scale + d * nph * NZ;
+  const float* dscale = scale ? scale + d * nph * NZ : nullptr;
   const int nc = min(W, nxh - c0);
   {
     const int c = threadIdx.x % W, j = threadIdx.x / W;  // R2 * W == blockDim
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(kThreads) k_separate4(float2* spec, const floa
       const int z = j + R2 * e;
 #pragma unroll
       for (int p = 0; p < nph; ++p) {
-        float sc = dscale[p * NZ + z];
+        float sc = dscale ? dscale[p * NZ + z] : 1.f;
         float2 v = c < nc ? dbase[((size_t)p * NZ + z) * plane + c] : make_float2(0.f, 0.f);
         in[p][e] = make_float2(v.x * sc, v.y * sc);
       }

@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(kThreads) k_separate_zn(float2* spec, const fl
   __shared__ float sc[NPH * N];
   const int d = blockIdx.y;
   for (int i = threadIdx.x; i < NPH * NPH; i += kThreads) M[i] = sepmat[i];
-  for (int i = threadIdx.x; i < NPH * N; i += kThreads) sc[i] = scale[d * NPH * N + i];
+  for (int i = threadIdx.x; i < NPH * N; i += kThreads) sc[i] = scale ? scale[d * NPH * N + i] : 1.f;
   __syncthreads();
   const size_t e0 = (size_t)blockIdx.x * kW;
   const int nc = (int)(plane - e0 < kW ? plane - e0 : kW);

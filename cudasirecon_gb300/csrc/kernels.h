@@ -102,7 +102,7 @@ int launch_rescale(const float2* spec, int nx, int ny, int nz, int ndirs, int np
                    int equalizet, double* sdp0, float* scale, cudaStream_t s, long long* launches);
 
 // Separation (band_i = sum_j M[i][j] * scale[p][z] * spec_j) + forward z FFT,
-// in place, all directions.
+// in place, all directions; scale null: unit ratios.
 int launch_separate(float2* spec, const float* scale, const float* sepmat /* device [nb][nph] */, int nx, int ny,
                     int nz, int ndirs, int nphases, cudaStream_t s, long long* launches);
 
@@ -241,6 +241,18 @@ struct FitDev {
   float2 amp[kMaxDirs * kMaxOrders];
   float ampmag2[kMaxDirs * kMaxOrders];  // |amp|^2
   float termw[kMaxDirs * kMaxOrders];    // |amp|^2 / noisevar; order 0: 1 / noisevar
+  // the pattern vectors of the fit and what the filter derives from them
+  float2 k0[kMaxDirs];
+  float kxo[kMaxDirs * kMaxOrders];      // order * k0
+  float kyo[kMaxDirs * kMaxOrders];
+  float rapo;                            // 1 / (rdistcutoff + |k0 of direction 0| (norders - 1))
+};
+// What a searched volume's fit tells the host, written by its last kernel into
+// mapped page-locked memory
+struct FitHost {
+  float2 k0[kMaxDirs];
+  float2 amp[kMaxDirs * kMaxOrders];
+  int info[2];  // K0SearchArgs::info
 };
 struct FitFinishArgs {
   int ndirs, norders;
@@ -250,6 +262,11 @@ struct FitFinishArgs {
   int fitallphases;  // 0: orders >= 2 take order * phase of order 1 (cudaSirecon.cpp:465-482)
   float noisevar[kMaxDirs * kMaxOrders];
   float rnv[kMaxDirs * kMaxOrders];  // 1 / noisevar
+  float2 k0[kMaxDirs];               // the pattern vectors ...
+  const float2* kdev;                // ... or, if set, direction d's in kdev[3 d]
+  float rdistcutoff;
+  FitHost* host;                     // mapped host memory, or null
+  const int* info;                   // the search's counters (with host)
 };
 // The no-search branch of the modamp fit (findrealspacemodamp at the known k0
 // for every direction and order, cudaSirecon.cpp:409-492) finished on the
@@ -276,11 +293,6 @@ struct FilterArgs {
   OTFView otf;
 };
 int launch_filter(const FilterArgs& a, cudaStream_t s, long long* launches);
-
-// Pattern vectors of every direction, by value (1/um)
-struct K0List {
-  float2 k[kMaxDirs];
-};
 
 struct AssembleArgs {
   const float2* bands;  // all directions [ndirs][nph][nz][ny][nxh]
@@ -313,9 +325,9 @@ int launch_assemble_filtered(const AssembleArgs& a, const FilterArgs& f, bool on
                              long long* launches);
 
 // Phase-ramp tables for assembly: ex[d*no+o][j] = exp(i fact pi (j - X/2) o k0x_d dxyz),
-// ey likewise along y (computed in double precision).
+// ey likewise along y (computed in double precision), k0 the fit's.
 // The columns of ex are in the order of the geometry's x pass.
-int launch_ramp_tables(const K0List& k0, const AssembleArgs& a, float dxyz, float fact, float2* ex, float2* ey,
+int launch_ramp_tables(const FitDev* fit, const AssembleArgs& a, float dxyz, float fact, float2* ex, float2* ey,
                        cudaStream_t s, long long* launches);
 
 // FFT-engine self test on `nlines` lines of length n (in place, device memory)

@@ -742,8 +742,6 @@ void SIM_Reconstructor::ingest()
     ia.inscale = 1.f;
   }
   check_launch(launch_ingest(ia, stream_, &launches_), "ingest");
-  // processOneVolume without loadAndRescaleImage uses unit ratios
-  check_launch(launch_fill(d_scale_, (size_t)ndirs_ * nph_ * nz_, 1.0f, stream_, &launches_), "scale init");
   stage_end("ingest", a, l0);
   rescaled_ = false;
 }
@@ -786,7 +784,9 @@ void SIM_Reconstructor::separate()
   cudaEvent_t a;
   long long l0;
   stage_begin("separate", &a, &l0);
-  check_launch(launch_separate(d_spec_, d_scale_, d_sepmat_, nx_, ny_, nz_, ndirs_, nph_, stream_, &launches_),
+  // processOneVolume without loadAndRescaleImage uses unit ratios
+  check_launch(launch_separate(d_spec_, rescaled_ ? d_scale_ : nullptr, d_sepmat_, nx_, ny_, nz_, ndirs_, nph_,
+                               stream_, &launches_),
                "separate");
   stage_end("separate", a, l0);
 }
@@ -1188,7 +1188,9 @@ bool SIM_Reconstructor::fit_without_search() const
   return reuse || !p.bSearchforvector;
 }
 
-void SIM_Reconstructor::fit_all()
+// defer: a device search may leave its results on the device (search_pending_;
+// finish_search after the next synchronisation)
+void SIM_Reconstructor::fit_all(bool defer)
 {
   TimerScope ts(this);
   cudaEvent_t a;
@@ -1196,11 +1198,16 @@ void SIM_Reconstructor::fit_all()
   stage_begin("fit", &a, &l0);
   if (fit_without_search()) {
     fit_on_device();
-  } else if (!device_search_possible() || !fit_search_on_device()) {
-    for (int d = 0; d < ndirs_; ++d) fit_direction(d);
-    check_launch(upload_amps(), "fit results");
+  } else if (!device_search_possible() || !fit_search_on_device(defer)) {
+    fit_on_host();
   }
   stage_end("fit", a, l0);
+}
+
+void SIM_Reconstructor::fit_on_host()
+{
+  for (int d = 0; d < ndirs_; ++d) fit_direction(d);
+  check_launch(upload_amps(), "fit results");
 }
 
 // The k0 search runs on the device unless a host decision is part of it:
@@ -1220,11 +1227,11 @@ bool SIM_Reconstructor::device_search_possible() const
 // (overlaps at the guess, cross-correlation peak, parabola refinement), the
 // overlaps rebuilt at the refined k0, the cluster search of fitk0andmodamps,
 // then the other orders' amplitudes at the fitted k0; the amplitudes are
-// finished like the no-search branch's.  One synchronisation at the end
-// brings the fitted k0 to the host (the filter's set-up needs it).  Returns
-// false, having changed nothing the host search depends on, when a climb
-// left the device's line cache; the host search then runs instead.
-bool SIM_Reconstructor::fit_search_on_device()
+// finished like the no-search branch's, and the last kernel leaves the fit in
+// mapped host memory.  Deferred, nothing waits: the fused filter takes the
+// pattern vectors from the device fit results.  Otherwise returns
+// finish_search().
+bool SIM_Reconstructor::fit_search_on_device(bool defer)
 {
   ReconParams& p = opt.p;
   const ImageParams& ip = opt.ip;
@@ -1296,28 +1303,49 @@ bool SIM_Reconstructor::fit_search_on_device()
     run_overlaps(oa);
     check_launch(launch_modamp_batch(ma, stream_, &launches_), "modamp");
   }
-  check_launch(launch_fit_finish(d_fitslots_, fit_finish_args(), d_fit_, stream_, &launches_), "fit results");
-  // the fitted k0s and the search's counters through mapped host memory
-  double* base = dh_pinned_ + 320;
-  check_launch(launch_copy_out(d_kst_, base, (size_t)ndirs_ * 6, d_sinfo_, base + 32, 2, stream_, &launches_),
-               "fit results");
-  check(cudaStreamSynchronize(stream_), "k0 search");
-  const float* kst = (const float*)(h_pinned_ + 320);
-  const int* info = (const int*)(h_pinned_ + 352);
+  FitFinishArgs ff = fit_finish_args();
+  ff.kdev = d_kst_ + 2;
+  ff.host = (FitHost*)(dh_pinned_ + kFitHostAt);
+  ff.info = d_sinfo_;
+  check_launch(launch_fit_finish(d_fitslots_, ff, d_fit_, stream_, &launches_), "fit results");
   // the count of builds takes a searched volume's twice, as it always has
   fit_counts_[0] += 2 * ndirs_ + (long long)rest.size();
-  fit_counts_[1] += reductions + info[0];
+  fit_counts_[1] += reductions;
   fit_counts_[2] += ndirs_;
   cur_o1_ = cur_o2_ = -1;
   cache_.clear();
-  if (info[1] != 0) return false;  // a climb left the line cache: the host search runs
-  for (int d = 0; d < ndirs_; ++d) {
-    k0_[d] = float2v{kst[6 * d + 4], kst[6 * d + 5]};
-    if (ip.curTimeIdx == 0) k0_time0_[d] = k0_[d];
-  }
   p.recalcarrays = 1;  // fit_direction's setting, kept for callers that read it
-  amps_on_device_only_ = true;
+  search_pending_ = true;
+  if (defer) return true;
+  check(cudaStreamSynchronize(stream_), "k0 search");
+  return finish_search();
+}
+
+// The host's part of a device search, after a synchronisation.  Returns false,
+// having changed nothing the host search depends on, when a climb left the
+// device's line cache: the host search has to run instead.
+bool SIM_Reconstructor::finish_search()
+{
+  search_pending_ = false;
+  const FitHost* f = (const FitHost*)(h_pinned_ + kFitHostAt);
+  fit_counts_[1] += f->info[0];
+  if (f->info[1] != 0) return false;
+  for (int d = 0; d < ndirs_; ++d) {
+    k0_[d] = float2v{f->k0[d].x, f->k0[d].y};
+    if (opt.ip.curTimeIdx == 0) k0_time0_[d] = k0_[d];
+    for (int o = 0; o < norders_; ++o) amp_[d][o] = float2v{f->amp[d * norders_ + o].x, f->amp[d * norders_ + o].y};
+  }
+  amps_on_device_only_ = false;
   return true;
+}
+
+// filterbands' lateral cutoff (gpuFunctionsImpl.cu:1241-1243), float arithmetic
+float SIM_Reconstructor::filter_rdistcutoff() const
+{
+  const float dxy = opt.ip.dxy;
+  float rdistcutoff = (opt.p.na * 2 / (opt.ip.wave[0] / 1000.0));
+  if (rdistcutoff > 1. / (2. * dxy)) rdistcutoff = 1. / (2. * dxy);
+  return rdistcutoff;
 }
 
 FitFinishArgs SIM_Reconstructor::fit_finish_args() const
@@ -1334,6 +1362,8 @@ FitFinishArgs SIM_Reconstructor::fit_finish_args() const
     fa.noisevar[i] = noisevar_[i];
     fa.rnv[i] = 1.f / noisevar_[i];
   }
+  for (int d = 0; d < ndirs_; ++d) fa.k0[d] = make_float2(k0_[d].x, k0_[d].y);
+  fa.rdistcutoff = filter_rdistcutoff();
   return fa;
 }
 
@@ -1474,16 +1504,14 @@ void SIM_Reconstructor::prepare_asm_tables()
   asm_tables_valid_ = true;
 }
 
-void SIM_Reconstructor::filter_and_assemble()
+// The arguments of the filter and the assembly.  What depends on the fitted k0
+// is the host's; the fused filter takes it from the device fit results instead.
+void SIM_Reconstructor::filter_args(FilterArgs& fa, AssembleArgs& aa) const
 {
-  TimerScope ts(this);
   const ReconParams& p = opt.p;
   const ImageParams& ip = opt.ip;
-  cudaEvent_t ev;
-  long long l0;
-  stage_begin("filter", &ev, &l0);
   // filterbands scalars (gpuFunctionsImpl.cu:1222-1298), float arithmetic
-  FilterArgs fa{};
+  fa = FilterArgs{};
   fa.ndirs = ndirs_;
   fa.norders = norders_;
   fa.nx = nx_;
@@ -1493,15 +1521,9 @@ void SIM_Reconstructor::filter_and_assemble()
   float dkz = ip.dz > 0 ? (1 / (nz_ * ip.dz)) : p.dkzotf;
   float kzscale = dkz / p.dkzotf;
   float k0mag = sqrt(k0_[0].x * k0_[0].x + k0_[0].y * k0_[0].y);
-  float lambdaem = (ip.wave[0] / p.nimm) / 1000.0;
-  float lambdaexc = 0.88 * lambdaem;
-  float alpha = asinf(p.na / p.nimm);
-  float rdistcutoff = (p.na * 2 / (ip.wave[0] / 1000.0));
-  if (rdistcutoff > 1. / (2. * dxy)) rdistcutoff = 1. / (2. * dxy);
+  const float rdistcutoff = filter_rdistcutoff();
   int zdc[kMaxOrders] = {0};
   filter_zdc(zdc);
-  (void)alpha;
-  (void)lambdaexc;
   float apocutoff = rdistcutoff + k0mag * (norders_ - 1);
   float zapocutoff = p.bBessel ? zdc[0] : (norders_ > 1 ? zdc[1] : 0);
   fa.dkx = 1. / (nx_ * dxy);
@@ -1528,9 +1550,8 @@ void SIM_Reconstructor::filter_and_assemble()
   fa.otf.dkrotf = p.dkrotf;
   fa.otf.kzscale = kzscale;
   for (int o = 0; o < norders_; ++o) fa.otf.otf[o] = d_otf_ + (size_t)o * p.nxotf * p.nzotf;
-  const bool one_otf = !p.bOneOTFperAngle || ndirs_otf_ == 1;
 
-  AssembleArgs aa{};
+  aa = AssembleArgs{};
   aa.bands = d_spec_;
   aa.ndirs = ndirs_;
   aa.norders = norders_;
@@ -1549,10 +1570,28 @@ void SIM_Reconstructor::filter_and_assemble()
   aa.S = d_S_;
   aa.out = d_out_;
   aa.tables = d_asmtab_;
+}
+
+// whether the filter runs inside the assembly's band load
+bool SIM_Reconstructor::filter_fused(const FilterArgs& fa, const AssembleArgs& aa) const
+{
+  return filter_fusion_ && assemble_filter_fusable(aa, fa, one_otf());
+}
+
+void SIM_Reconstructor::filter_and_assemble()
+{
+  TimerScope ts(this);
+  const ReconParams& p = opt.p;
+  cudaEvent_t ev;
+  long long l0;
+  stage_begin("filter", &ev, &l0);
+  FilterArgs fa{};
+  AssembleArgs aa{};
+  filter_args(fa, aa);
   if (!asm_tables_current(aa)) throw std::runtime_error("assembly tables not prepared for this geometry");
   // the filter runs inside the assembly's band load where it can; else as
   // its own in-place pass per direction (filterbands_kernel1 x 2 + kernel3)
-  const bool fused = filter_fusion_ && assemble_filter_fusable(aa, fa, one_otf);
+  const bool fused = filter_fused(fa, aa);
   if (!fused)
     for (int d = 0; d < ndirs_; ++d) {
       const int dir_ = p.bOneOTFperAngle ? d : 0;
@@ -1565,11 +1604,10 @@ void SIM_Reconstructor::filter_and_assemble()
   stage_end("filter", ev, l0);
 
   stage_begin("assemble", &ev, &l0);
-  K0List k0l{};
-  for (int d = 0; d < ndirs_; ++d) k0l.k[d] = make_float2(k0_[d].x, k0_[d].y);
   float fact = p.explodefact / 0.5;
-  check_launch(launch_ramp_tables(k0l, aa, dxy / p.zoomfact, fact, d_ex_, d_ey_, stream_, &launches_), "ramp");
-  if (fused) check_launch(launch_assemble_filtered(aa, fa, one_otf, stream_, &launches_), "filter + assemble");
+  check_launch(launch_ramp_tables(d_fit_, aa, opt.ip.dxy / p.zoomfact, fact, d_ex_, d_ey_, stream_, &launches_),
+               "ramp");
+  if (fused) check_launch(launch_assemble_filtered(aa, fa, one_otf(), stream_, &launches_), "filter + assemble");
   else check_launch(launch_assemble(aa, stream_, &launches_), "assemble");
   stage_end("assemble", ev, l0);
 }
@@ -1585,11 +1623,22 @@ int SIM_Reconstructor::process_one_volume(bool sync)
     return last_result_;
   }
   last_result_ = 1;
+  search_pending_ = false;
   separate();
-  fit_all();
+  // with the fused filter nothing up to the result needs the fit on the host
+  // (and the bands stay as they are): one synchronisation at the end
+  FilterArgs fa{};
+  AssembleArgs aa{};
+  filter_args(fa, aa);
+  fit_all(sync && filter_fused(fa, aa));
   prepare_asm_tables();  // after the fit: in Bessel mode the in-band planes depend on k0
   filter_and_assemble();
   if (sync) check(cudaStreamSynchronize(stream_), "processOneVolume");
+  if (search_pending_ && !finish_search()) {
+    fit_on_host();
+    filter_and_assemble();
+    check(cudaStreamSynchronize(stream_), "processOneVolume");
+  }
   have_raw_ = false;  // the bands are consumed (filtered in place)
   return 1;
 }

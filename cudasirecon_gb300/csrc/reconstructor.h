@@ -99,12 +99,18 @@ class SIM_Reconstructor {
   void stage_raw(const void* raw, bool u16);
   void ingest();
   void separate();
-  void fit_all();
+  void fit_all(bool defer = false);
+  void fit_on_host();
   void fit_direction(int d);
   bool fit_without_search() const;
   void fit_on_device();
   bool device_search_possible() const;
-  bool fit_search_on_device();
+  bool fit_search_on_device(bool defer);
+  bool finish_search();
+  float filter_rdistcutoff() const;
+  void filter_args(simrecon::FilterArgs& fa, simrecon::AssembleArgs& aa) const;
+  bool filter_fused(const simrecon::FilterArgs& fa, const simrecon::AssembleArgs& aa) const;
+  bool one_otf() const { return !opt.p.bOneOTFperAngle || ndirs_otf_ == 1; }
   simrecon::FitFinishArgs fit_finish_args() const;
   int upload_amps();
   void sync_amps() const;
@@ -252,6 +258,8 @@ class SIM_Reconstructor {
   bool raw_staged_ = false;  // d_raw_ holds a stack staged by setRaw/setFile
   bool have_raw_ = false;
   bool rescaled_ = false;
+  bool search_pending_ = false;  // a device search's results are not on the host yet
+  static constexpr int kFitHostAt = 320;  // FitHost in h_pinned_, in doubles
   // overlap state for the candidate evaluator
   int cur_o1_ = -1, cur_o2_ = -1;
   double sumx_ = 0, sumy_ = 0;
