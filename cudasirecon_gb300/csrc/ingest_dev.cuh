@@ -12,6 +12,34 @@ __device__ __forceinline__ int raw_section(int d, int p, int z, int nz, int ndir
   return fastSI ? (z * ndirs * nph + d * nph + p) : (d * nz * nph + z * nph + p);
 }
 
+// What the CTAs of blockIdx.y transform: a raw section and the plane of spec it
+// goes to.  The whole stack is taken in plane order (the y pass follows in the
+// reverse of it), a part of it in section order.
+struct IngestPlane {
+  int section, plane;  // plane id = (d*nph + p)*nz + z
+};
+__device__ __forceinline__ IngestPlane ingest_plane(const IngestArgs& a)
+{
+  int d, p, z;
+  if (a.nsec == 0) {
+    const int pl = blockIdx.y, dp = pl / a.nz;
+    z = pl - dp * a.nz;
+    d = dp / a.nphases;
+    p = dp - d * a.nphases;
+    return IngestPlane{raw_section(d, p, z, a.nz, a.ndirs, a.nphases, a.fastSI), pl};
+  }
+  const int s = a.sec0 + blockIdx.y, q = s / a.nphases;
+  p = s - q * a.nphases;
+  if (a.fastSI) {
+    z = q / a.ndirs;
+    d = q - z * a.ndirs;
+  } else {
+    d = q / a.nz;
+    z = q - d * a.nz;
+  }
+  return IngestPlane{s, (d * a.nphases + p) * a.nz + z};
+}
+
 template <typename T>
 __device__ __forceinline__ float flat(const T* __restrict__ plane, const IngestArgs& a, int y, int x)
 {

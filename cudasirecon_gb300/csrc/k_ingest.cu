@@ -57,12 +57,10 @@ __global__ void __launch_bounds__(kThreads) k_ingest_x(IngestArgs a, FFTPlan pla
   extern __shared__ float2 sm[];
   __shared__ float diffr[2 * 256];
   const int nx = a.nx, ny = a.ny, nxh = nx / 2 + 1;
-  const int pl = blockIdx.y;  // plane id = (d*nph + p)*nz + z
-  const int z = pl % a.nz;
-  const int dp = pl / a.nz;
-  const int p = dp % a.nphases, d = dp / a.nphases;
+  const IngestPlane ip = ingest_plane(a);
+  const int pl = ip.plane;
   const int y0 = blockIdx.x * 2 * nl;
-  const T* plane = (const T*)a.raw + (size_t)raw_section(d, p, z, a.nz, a.ndirs, a.nphases, a.fastSI) * nx * ny;
+  const T* plane = (const T*)a.raw + (size_t)ip.section * nx * ny;
   float* smr = (float*)sm;  // row r at x -> smr[2*((r>>1)*ldl + x) + (r&1)]
   const int napo = a.napodize;
   const int nrows = 2 * nl;
@@ -191,16 +189,14 @@ __global__ void __launch_bounds__(kIngestWarps * 32, 3) k_ingest_xw(IngestArgs a
   static_assert(XB >= N, "exchange buffer too small for the split");
   extern __shared__ __align__(16) unsigned char ig_dyn[];
   const int ny = a.ny, nxh = N / 2 + 1;
-  const int pl = blockIdx.y;  // plane id = (d*nph + p)*nz + z
-  const int z = pl % a.nz;
-  const int dp = pl / a.nz;
-  const int ph = dp % a.nphases, d = dp / a.nphases;
+  const IngestPlane ip = ingest_plane(a);
+  const int pl = ip.plane;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane / P, p = lane - g * P;
   const int gi = warp * G + g;
   float2* xb = (float2*)ig_dyn + gi * XB;
   unsigned char* rg = ig_dyn + (size_t)kIngestWarps * G * XB * sizeof(float2) + (size_t)gi * 2 * RB;
-  const T* plane = (const T*)a.raw + (size_t)raw_section(d, ph, z, a.nz, a.ndirs, a.nphases, a.fastSI) * N * ny;
+  const T* plane = (const T*)a.raw + (size_t)ip.section * N * ny;
   const int pairs = (ny + 1) / 2;
   const int lbase = (blockIdx.x * kIngestWarps + warp) * G * kIngestPairs + g;  // pair of turn it: lbase + G*it
   const int napo = a.napodize;
@@ -424,12 +420,12 @@ __global__ void __launch_bounds__(kThreads) k_separate_z1(float2* spec, const fl
 
 static size_t fft_smem(int n, int lines, int elems) { return fft_stage_smem(n, lines, elems, kThreads); }
 
-int launch_ingest(const IngestArgs& a, cudaStream_t s, long long* launches)
+int launch_ingest_x(const IngestArgs& a, cudaStream_t s, long long* launches)
 {
-  FFTPlan px, py;
-  if (!get_fft_plan(a.nx, &px) || !get_fft_plan(a.ny, &py)) return -1;
+  FFTPlan px;
+  if (!get_fft_plan(a.nx, &px)) return -1;
   const int nxh = a.nx / 2 + 1;
-  const int nplanes = a.ndirs * a.nphases * a.nz;
+  const int nplanes = a.nsec ? a.nsec : a.ndirs * a.nphases * a.nz;
   const int ldl = a.nx + 1;
   int nl = std::max(1, std::min(kMaxElems / a.nx, 256));
   nl = std::min(nl, (a.ny + 1) / 2);
@@ -453,14 +449,9 @@ int launch_ingest(const IngestArgs& a, cudaStream_t s, long long* launches)
       k_ingest_xw<float, N><<<gw, kIngestWarps * 32, bytes, s>>>(a, px.twr);
     }
   };
-  TfPlan tx, ty;
+  TfPlan tx;
   const bool wx = a.nx == 512 || a.nx == 1024 || a.nx == 256;  // warp kernels
   const TfKernels* kx = !wx && fft_two_factor(kSiteIngestX, a.nx) ? tf_kernels(a.nx, &tx) : nullptr;
-  // 1024 rows keep their compiled kernel: 1.72 against 1.93 ms per 1024^2 x 64
-  // volume (256 rows: 0.046 two-factor against 0.057 ms per 256^2 x 32)
-  const TfKernels* ky = a.ny == 512 || a.ny == 256 || (a.ny != 1024 && fft_two_factor(kSiteIngestY, a.ny))
-                            ? tf_kernels(a.ny, &ty)
-                            : nullptr;
   if (a.nx == 512) go_w.template operator()<512>();
   else if (a.nx == 1024) go_w.template operator()<1024>();
   else if (a.nx == 256) go_w.template operator()<256>();
@@ -488,25 +479,43 @@ int launch_ingest(const IngestArgs& a, cudaStream_t s, long long* launches)
     }
   });
   if (kt) kt->end("k_ingest_x", s, (double)nplanes * a.nx * a.ny * (a.raw_is_u16 ? 2 : 4) + specb);
+  if (launches) *launches += 1;
+  return (int)cudaGetLastError();
+}
+
+int launch_ingest_y(const IngestArgs& a, int plane0, int nplanes, cudaStream_t s, long long* launches)
+{
+  FFTPlan py;
+  if (!get_fft_plan(a.ny, &py)) return -1;
+  const int nxh = a.nx / 2 + 1;
+  const double specb = (double)nplanes * a.ny * nxh * sizeof(float2);
+  float2* spec = a.spec + (size_t)plane0 * a.ny * nxh;
+  TfPlan ty;
+  // 1024 rows keep their compiled kernel: 1.72 against 1.93 ms per 1024^2 x 64
+  // volume (256 rows: 0.046 two-factor against 0.057 ms per 256^2 x 32)
+  const TfKernels* ky = a.ny == 512 || a.ny == 256 || (a.ny != 1024 && fft_two_factor(kSiteIngestY, a.ny))
+                            ? tf_kernels(a.ny, &ty)
+                            : nullptr;
   int W = std::max(1, std::min(32, kMaxElems / a.ny));
   size_t smy = fft_smem(a.ny, W, a.ny * (W + 1));
   dim3 gy((nxh + W - 1) / W, nplanes);
+  KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
   if (a.ny == 1024) {
     const size_t bytes = ColFft<1024, colfft_r1(1024), 8>::kSmemElems * sizeof(float2);
     allow_dynamic_smem((const void*)k_fft_cols_4s<1024>, bytes);
-    k_fft_cols_4s<1024><<<dim3((nxh + 7) / 8, nplanes), kThreads, bytes, s>>>(a.spec, nxh, py.tw);
+    k_fft_cols_4s<1024><<<dim3((nxh + 7) / 8, nplanes), kThreads, bytes, s>>>(spec, nxh, py.tw);
   } else if (ky) {
-    const int rc = ky->fft_cols(a.spec, nxh, nplanes, ty, s);
+    const int rc = ky->fft_cols(spec, nxh, nplanes, ty, s);
     if (rc != 0) return rc;
   } else {
     dispatch_fft_len(kSiteIngestY, a.ny, [&]<int NF>() {
       allow_dynamic_smem((const void*)k_fft_cols<-1, NF>, smy);
-      k_fft_cols<-1, NF><<<gy, kThreads, smy, s>>>(a.spec, a.ny, nxh, py, W);
+      k_fft_cols<-1, NF><<<gy, kThreads, smy, s>>>(spec, a.ny, nxh, py, W);
     });
   }
   if (kt) kt->end("k_fft_y", s, 2 * specb);
-  if (launches) *launches += 2;
+  if (launches) *launches += 1;
   return (int)cudaGetLastError();
 }
 
@@ -582,42 +591,55 @@ __global__ void __launch_bounds__(kThreads) k_separate4(float2* spec, const floa
 }
 
 namespace {
+// One CTA per row.  The position in the raw row is formed as a float pair (the
+// section's offset in double, once per CTA): four double additions an element
+// and the 64-bit divisions of a flat index were the kernel's time (300 x 192,
+// 200 sections: 188 us, 57 us here).
 template <typename T>
-__global__ void k_precondition(const __grid_constant__ PrecondArgs a)
+__global__ void __launch_bounds__(128) k_precondition(const __grid_constant__ PrecondArgs a)
 {
-  const size_t plane = (size_t)a.ny * a.nx, n = (size_t)a.nimg * plane;
-  const T* raw = (const T*)a.raw;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int s = (int)(i / plane);
-    const size_t r = i - (size_t)s * plane;
-    const int y = (int)(r / a.nx), xo = (int)(r - (size_t)y * a.nx);
-    const T* sec = raw + (size_t)s * a.ny * a.nx_raw;
-    const float bgx = a.bgx ? a.bgx[s] : 0.f;
-    // load_and_flatfield of raw pixel (yy, k)
-    auto flat = [&](int yy, int k) {
-      const size_t q = (size_t)yy * a.nx_raw + k;
-      const float bg = a.bg ? a.bg[q] : a.bgconst;
-      const float sl = a.slope ? a.slope[q] : 1.0f;
-      return (((float)sec[q] - bg) - bgx) * sl * a.inscale;
-    };
+  __shared__ float2 off;  // xin = (xo - nx/2 + shift) + off
+  const int sl = blockIdx.x / a.ny, y = blockIdx.x - sl * a.ny, s = a.sec0 + sl;
+  const T* sec = (const T*)a.raw + (size_t)s * a.ny * a.nx_raw;
+  float* out = a.out + ((size_t)s * a.ny + y) * a.nx;
+  const float bgx = a.bgx ? a.bgx[s] : 0.f;
+  const bool deskew = a.deskew_factor != 0.f;
+  if (deskew && threadIdx.x == 0) {
+    // z of this raw section (loadImageData's order, cudaSirecon.cpp:1374-1382)
+    const int z = a.fastSI ? s / (a.ndirs * a.nphases) : (s / a.nphases) % a.nz;
+    const double c = a.nx_raw / 2. - (double)a.deskew_factor * (z - a.nz / 2.);
+    off.x = (float)c;
+    off.y = (float)(c - (double)off.x);
+  }
+  __syncthreads();
+  // load_and_flatfield of raw pixel (yy, k)
+  auto flat = [&](int yy, int k) {
+    const size_t q = (size_t)yy * a.nx_raw + k;
+    const float bg = a.bg ? a.bg[q] : a.bgconst;
+    const float sl = a.slope ? a.slope[q] : 1.0f;
+    return (((float)sec[q] - bg) - bgx) * sl * a.inscale;
+  };
+  const float2 o = deskew ? off : make_float2(0.f, 0.f);
+#pragma unroll 4
+  for (int xo = threadIdx.x; xo < a.nx; xo += 128) {
     float v = 0.f;
-    if (a.deskew_factor == 0.f) {
+    if (!deskew) {
       if (xo < a.nx_raw) v = flat(y, xo);
     } else {
-      // z of this raw section (loadImageData's order, cudaSirecon.cpp:1374-1382)
-      const int z = a.fastSI ? s / (a.ndirs * a.nphases) : (s / a.nphases) % a.nz;
-      const float xin = (float)((double)xo - a.nx / 2. + a.extra_shift - (double)a.deskew_factor * (z - a.nz / 2.) +
-                                a.nx_raw / 2.);
+      const float p = (float)(2 * (xo + a.extra_shift) - a.nx) * 0.5f;  // exact
+      const float t = __fadd_rn(p, o.x), b = __fsub_rn(t, p);
+      const float e = __fadd_rn(__fsub_rn(p, __fsub_rn(t, b)), __fsub_rn(o.x, b));
+      const float xin = __fadd_rn(t, __fadd_rn(e, o.y));
       if (xin >= 0 && xin < a.nx_raw) {
         const int i0 = (int)floorf(xin);
-        const float off = xin - floorf(xin);
+        const float w = xin - floorf(xin);
         // the reference reads the next pixel of the section buffer: the next
         // row's first one at the end of a row (zero past the last row)
         const float a1 = i0 + 1 < a.nx_raw ? flat(y, i0 + 1) : (y + 1 < a.ny ? flat(y + 1, 0) : 0.f);
-        v = __fadd_rn(__fmul_rn(1.f - off, flat(y, i0)), __fmul_rn(off, a1));
+        v = __fadd_rn(__fmul_rn(1.f - w, flat(y, i0)), __fmul_rn(w, a1));
       }
     }
-    a.out[i] = v;
+    out[xo] = v;
   }
 }
 }  // namespace
@@ -625,11 +647,11 @@ __global__ void k_precondition(const __grid_constant__ PrecondArgs a)
 int launch_precondition(const PrecondArgs& a, cudaStream_t s, long long* launches)
 {
   const size_t n = (size_t)a.nimg * a.ny * a.nx;
-  const unsigned nb = (unsigned)std::min<size_t>((n + kThreads - 1) / kThreads, 152 * 16);
+  const unsigned nb = (unsigned)a.nimg * a.ny;
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
-  if (a.raw_is_u16) k_precondition<uint16_t><<<nb, kThreads, 0, s>>>(a);
-  else k_precondition<float><<<nb, kThreads, 0, s>>>(a);
+  if (a.raw_is_u16) k_precondition<uint16_t><<<nb, 128, 0, s>>>(a);
+  else k_precondition<float><<<nb, 128, 0, s>>>(a);
   if (kt) kt->end("k_precondition", s, (double)a.nimg * a.ny * a.nx_raw * (a.raw_is_u16 ? 2 : 4) + 4.0 * n);
   if (launches) *launches += 1;
   return (int)cudaGetLastError();

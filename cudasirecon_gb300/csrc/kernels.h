@@ -64,8 +64,8 @@ struct IngestArgs {
   int napodize;
   const float* apofact;  // device [napodize]
   float2* spec;          // [ndirs*nphases*nz][ny][nx/2+1]
+  int sec0, nsec;        // the x pass takes raw sections sec0 .. sec0 + nsec - 1; nsec = 0: every plane
 };
-// flat-field + apodize + 2D R2C FFT of every raw plane into spec
 // Allow `func` to be launched with `bytes` of dynamic shared memory.  The
 // limit is per kernel and device and is only ever raised: host threads that
 // launch the same kernel with different sizes (handles of different shapes
@@ -73,7 +73,10 @@ struct IngestArgs {
 // launch.
 void allow_dynamic_smem(const void* func, size_t bytes);
 
-int launch_ingest(const IngestArgs& a, cudaStream_t s, long long* launches);
+// flat-field + apodize + x half of the 2D R2C FFT of raw planes into spec
+int launch_ingest_x(const IngestArgs& a, cudaStream_t s, long long* launches);
+// the y half, in place, of planes plane0 .. plane0 + nplanes - 1
+int launch_ingest_y(const IngestArgs& a, int plane0, int nplanes, cudaStream_t s, long long* launches);
 
 // The load steps before the transforms when the raw planes are not taken as
 // they are: load_and_flatfield (cudaSirecon.cpp:1715-1731) with a per-section
@@ -84,7 +87,8 @@ int launch_ingest(const IngestArgs& a, cudaStream_t s, long long* launches);
 struct PrecondArgs {
   const void* raw;  // [nimg][ny][nx_raw] uint16 or float
   int raw_is_u16;
-  int nx_raw, ny, nx, nz, ndirs, nphases, fastSI, nimg;
+  int nx_raw, ny, nx, nz, ndirs, nphases, fastSI;
+  int sec0, nimg;      // raw sections sec0 .. sec0 + nimg - 1
   const float* bg;     // [ny][nx_raw] or null (then bgconst)
   const float* slope;  // [ny][nx_raw] or null (then 1)
   float bgconst;

@@ -573,6 +573,7 @@ SIM_Reconstructor::~SIM_Reconstructor()
     for (cudaEvent_t e : {ev_raw_ready_[b], ev_raw_free_[b], ev_out_ready_[b], ev_out_free_[b]})
       if (e) cudaEventDestroy(e);
   if (h2d_stream_) cudaStreamDestroy(h2d_stream_);
+  if (ev_part_) cudaEventDestroy(ev_part_);
   if (d2h_stream_) cudaStreamDestroy(d2h_stream_);
   if (d_raw_alt_) cudaFree(d_raw_alt_);
   if (d_out_extra_) cudaFree(d_out_extra_);
@@ -676,15 +677,50 @@ void SIM_Reconstructor::reset_profile()
 // -------------------------------------------------------------- ingestion
 void SIM_Reconstructor::stage_raw(const void* raw, bool u16)
 {
-  const size_t n = (size_t)nimg_ * nx_raw_ * ny_;
+  const size_t sec = (size_t)nx_raw_ * ny_ * (u16 ? 2 : 4);
   raw_u16_ = u16;
-  check(cudaMemcpyAsync(d_raw_, raw, n * (u16 ? 2 : 4), cudaMemcpyHostToDevice, stream_), "raw upload");
   have_raw_ = true;
   raw_staged_ = true;
-  ingest();
+  // Large stacks go up in parts of 4 MB or more and each part's x transforms
+  // run while the next is copied; the y transforms of a direction follow its
+  // last part.  (fastSI sections interleave the directions: one y pass.)
+  constexpr size_t kPart = (size_t)4 << 20;
+  const int group = opt.p.bFastSIM ? nimg_ : nz_ * nph_;  // consecutive sections of one y pass
+  const int part = (int)std::max<size_t>(1, (kPart + sec - 1) / sec);
+  if (profiling_ || nimg_ != ndirs_ * nph_ * nz_ || (size_t)nimg_ * sec < 2 * kPart) {
+    check(cudaMemcpyAsync(d_raw_, raw, (size_t)nimg_ * sec, cudaMemcpyHostToDevice, stream_), "raw upload");
+    ingest();
+  } else {
+    ensure_copy_stream();
+    rescaled_ = false;
+    // the copies may not pass work still reading d_raw_
+    check(cudaEventRecord(ev_part_, stream_), "raw upload");
+    check(cudaStreamWaitEvent(h2d_stream_, ev_part_, 0), "raw upload");
+    for (int s0 = 0; s0 < nimg_;) {
+      const int end = std::min(nimg_, s0 / group * group + group);
+      int n = std::min(part, end - s0);
+      if (end - s0 - n < part / 2) n = end - s0;
+      check(cudaMemcpyAsync((char*)d_raw_ + s0 * sec, (const char*)raw + s0 * sec, n * sec, cudaMemcpyHostToDevice,
+                            h2d_stream_),
+            "raw upload");
+      check(cudaEventRecord(ev_part_, h2d_stream_), "raw upload");
+      check(cudaStreamWaitEvent(stream_, ev_part_, 0), "raw upload");
+      const IngestArgs ia = ingest_args(s0, n);
+      check_launch(launch_ingest_x(ia, stream_, &launches_), "ingest");
+      s0 += n;
+      if (s0 == end) check_launch(launch_ingest_y(ia, end - group, group, stream_, &launches_), "ingest");
+    }
+  }
   // setRaw copies the caller's stack (interface.cpp:19-25): return once the
   // upload and the ingest kernels are done with it
   check(cudaStreamSynchronize(stream_), "ingest");
+}
+
+void SIM_Reconstructor::ensure_copy_stream()
+{
+  if (h2d_stream_) return;
+  check(cudaStreamCreateWithFlags(&h2d_stream_, cudaStreamNonBlocking), "copy stream");
+  check(cudaEventCreateWithFlags(&ev_part_, cudaEventDisableTiming), "copy event");
 }
 
 void SIM_Reconstructor::ingest()
@@ -693,6 +729,17 @@ void SIM_Reconstructor::ingest()
   cudaEvent_t a;
   long long l0;
   stage_begin("ingest", &a, &l0);
+  const IngestArgs ia = ingest_args(0, 0);
+  check_launch(launch_ingest_x(ia, stream_, &launches_), "ingest");
+  check_launch(launch_ingest_y(ia, 0, ndirs_ * nph_ * nz_, stream_, &launches_), "ingest");
+  stage_end("ingest", a, l0);
+  rescaled_ = false;
+}
+
+// The ingest's arguments for raw sections sec0 .. sec0 + nsec - 1 (nsec = 0:
+// all), after queueing their preconditioning where the planes need it
+IngestArgs SIM_Reconstructor::ingest_args(int sec0, int nsec)
+{
   IngestArgs ia{};
   ia.raw = d_raw_;
   ia.raw_is_u16 = raw_u16_;
@@ -724,7 +771,8 @@ void SIM_Reconstructor::ingest()
     pa.ndirs = ndirs_;
     pa.nphases = nph_;
     pa.fastSI = opt.p.bFastSIM;
-    pa.nimg = nimg_;
+    pa.sec0 = sec0;
+    pa.nimg = nsec ? nsec : nimg_;
     pa.bg = d_bgslope_;
     pa.slope = d_bgslope_ ? d_bgslope_ + (size_t)nx_raw_ * ny_ : nullptr;
     pa.bgconst = opt.p.constbkgd;
@@ -741,9 +789,9 @@ void SIM_Reconstructor::ingest()
     ia.bgconst = 0.f;
     ia.inscale = 1.f;
   }
-  check_launch(launch_ingest(ia, stream_, &launches_), "ingest");
-  stage_end("ingest", a, l0);
-  rescaled_ = false;
+  ia.sec0 = sec0;
+  ia.nsec = nsec;
+  return ia;
 }
 
 void SIM_Reconstructor::set_raw_float(const float* raw, int nx, int ny, int nz)
@@ -1793,7 +1841,7 @@ void SIM_Reconstructor::process_series(const void* const* raws, bool u16, float*
     check(cudaMalloc((void**)&d_out_extra_, out_bytes), "series output buffer");
     series_bytes_ = (size_t)nimg_ * nx_raw_ * ny_ * sizeof(float) + out_bytes;
     d_out_alt_ = d_out_extra_;
-    check(cudaStreamCreateWithFlags(&h2d_stream_, cudaStreamNonBlocking), "series stream");
+    ensure_copy_stream();
     check(cudaStreamCreateWithFlags(&d2h_stream_, cudaStreamNonBlocking), "series stream");
     for (int b = 0; b < 2; ++b)
       for (cudaEvent_t* e : {&ev_raw_ready_[b], &ev_raw_free_[b], &ev_out_ready_[b], &ev_out_free_[b]})

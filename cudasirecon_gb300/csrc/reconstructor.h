@@ -98,6 +98,8 @@ class SIM_Reconstructor {
   bool load_corr(std::string* err);
   void stage_raw(const void* raw, bool u16);
   void ingest();
+  simrecon::IngestArgs ingest_args(int sec0, int nsec);
+  void ensure_copy_stream();
   void separate();
   void fit_all(bool defer = false);
   void fit_on_host();
@@ -229,6 +231,7 @@ class SIM_Reconstructor {
   float* d_out_alt_ = nullptr;   // the output buffer not holding the last result
   float* d_out_extra_ = nullptr;  // the allocation behind the second output buffer
   cudaStream_t h2d_stream_ = nullptr, d2h_stream_ = nullptr;
+  cudaEvent_t ev_part_ = nullptr;
   cudaEvent_t ev_raw_ready_[2] = {nullptr, nullptr}, ev_raw_free_[2] = {nullptr, nullptr};
   cudaEvent_t ev_out_ready_[2] = {nullptr, nullptr}, ev_out_free_[2] = {nullptr, nullptr};
   // small page-locked host buffer for results of the fit, mapped into the

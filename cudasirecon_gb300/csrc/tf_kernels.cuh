@@ -145,12 +145,10 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
   constexpr int N = G::N, nxh = N / 2 + 1;
   extern __shared__ __align__(16) float2 sm[];
   const int ny = a.ny;
-  const int pl = blockIdx.y;  // plane id = (d*nph + p)*nz + z
-  const int z = pl % a.nz;
-  const int dp = pl / a.nz;
-  const int p = dp % a.nphases, d = dp / a.nphases;
+  const IngestPlane ip = ingest_plane(a);
+  const int pl = ip.plane;
   const int y0 = blockIdx.x * 2 * G::W;
-  const T* plane = (const T*)a.raw + (size_t)raw_section(d, p, z, a.nz, a.ndirs, a.nphases, a.fastSI) * N * ny;
+  const T* plane = (const T*)a.raw + (size_t)ip.section * N * ny;
   float* smr = (float*)sm;  // row r at x -> smr[2*((r>>1)*N + x) + (r&1)]
   const int napo = a.napodize;
   const bool plainbg = !a.bg && !a.slope;
@@ -596,7 +594,7 @@ struct TfEntry {
   static int ingest_x(const IngestArgs& a, const TfPlan& pl, cudaStream_t s)
   {
     using G = TfRow<R1, R2>;
-    const dim3 g((a.ny + 2 * G::W - 1) / (2 * G::W), a.ndirs * a.nphases * a.nz);
+    const dim3 g((a.ny + 2 * G::W - 1) / (2 * G::W), a.nsec ? a.nsec : a.ndirs * a.nphases * a.nz);
     if (a.raw_is_u16) {
       allow_dynamic_smem((const void*)k_tf_ingest<uint16_t, R1, R2>, G::kSmem);
       k_tf_ingest<uint16_t, R1, R2><<<g, G::kThreads, G::kSmem, s>>>(a, pl.tw);
