@@ -4,10 +4,12 @@
 //   k_mo_section    per section: camera-pixel fix, border background
 //                   (radialft.cpp:228-237, 487-503), edge apodisation (695-720)
 //   k_mo_argmax_*   bead centre: peak of the phase average + parabolas (507-614)
-//   k_mo_separate   background subtraction (299-305) and band separation
-//                   (440-485) into full-complex band volumes
-//   k_mo_fft_*      3D forward FFT per band (339-348); y and z only over the
-//                   kx >= 0 half the OTF keeps
+//   k_tf_mo_rows    background subtraction (299-305), band separation (440-485)
+//                   and the x transform (339-348) into half spectra; then
+//                   k_tf_cols and k_z_forward.  For other lengths:
+//   k_mo_separate   the separation into full-complex band volumes
+//   k_mo_fft_*      3D forward FFT per band; y and z only over the kx >= 0
+//                   half the OTF keeps
 //   k_mo_shift_comp shift of the bead to the origin (846-874) and bead-size
 //                   compensation (784-841, 1155-1167), fused
 //   k_mo_radial     radial average per (band, kz) over a precomputed table of
@@ -31,6 +33,8 @@
 #include "kernels.h"
 #include "makeotf.h"
 #include "reg_fft.cuh"
+#include "tf_kernels.h"
+#include "z_fft.cuh"
 #include "sim_common.cuh"
 
 namespace simrecon {
@@ -316,6 +320,7 @@ __global__ void __launch_bounds__(kMoThreads) k_mo_fft_cols(float2* data, int n,
 // ------------------------------------------------- shift + bead compensation
 struct ShiftCompArgs {
   int nx, ny, nz, nph, norders, compensate;
+  int pitch;                 // elements per row of a band: nx, or nx/2 + 1
   float dkx, dky, dkz;       // beadsize_compensate's float sampling
   float k0x[kMoMaxPhases];   // per order
   float k0y[kMoMaxPhases];
@@ -397,7 +402,7 @@ __global__ void __launch_bounds__(kMoThreads) k_mo_shift_comp(float2* bands, con
   const float dphiz = (float)(2.0 * M_PI * (double)zc / a.nz);
   const float dphiy = (float)(2.0 * M_PI * (double)yc / a.ny);
   const float dphix = (float)(2.0 * M_PI * (double)xc / a.nx);
-  const size_t vol = (size_t)a.nz * a.ny * a.nx;
+  const size_t vol = (size_t)a.nz * a.ny * a.pitch;
   const int b0 = order == 0 ? 0 : 2 * order - 1, b1 = order == 0 ? 0 : min(2 * order, a.nph - 1);
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nh; t += (size_t)gridDim.x * blockDim.x) {
     int x = (int)(t % nxh);
@@ -418,7 +423,7 @@ __global__ void __launch_bounds__(kMoThreads) k_mo_shift_comp(float2* bands, con
       ratio = sphere_ratio(a, rho);
     }
     for (int b = b0; b <= b1; ++b) {
-      float2* e = bands + b * vol + ((size_t)z * a.ny + y) * a.nx + x;
+      float2* e = bands + b * vol + ((size_t)z * a.ny + y) * a.pitch + x;
       const float2 v = *e;
       float2 w = make_float2(__fsub_rn(__fmul_rn(v.x, c), __fmul_rn(v.y, s)),
                              __fadd_rn(__fmul_rn(v.x, s), __fmul_rn(v.y, c)));
@@ -439,13 +444,13 @@ __global__ void __launch_bounds__(kMoThreads) k_mo_shift_comp(float2* bands, con
 // for each: 66 us at 128^2 x 64 x 5, 26 us here).
 __global__ void __launch_bounds__(128) k_mo_radial(const float2* __restrict__ bands, const int* __restrict__ bin_start,
                                                    const int* __restrict__ bin_pix, int nbins, int nx, int ny, int nz,
-                                                   float2* avg)
+                                                   int pitch, float2* avg)
 {
   const int bin = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int kz = blockIdx.y, b = blockIdx.z;
   if (bin >= nbins) return;
   const int nxh = nx / 2 + 1;
-  const float2* plane = bands + ((size_t)b * nz + kz) * ny * nx;
+  const float2* plane = bands + ((size_t)b * nz + kz) * ny * pitch;
   const int s0 = bin_start[bin], s1 = bin_start[bin + 1];
   float re = 0.f, im = 0.f;
   for (int i0 = s0; i0 < s1; i0 += 32) {
@@ -454,7 +459,7 @@ __global__ void __launch_bounds__(128) k_mo_radial(const float2* __restrict__ ba
     if (lane < n) {
       const int p = bin_pix[i0 + lane];
       const int y = p / nxh, x = p - y * nxh;
-      v = plane[(size_t)y * nx + x];
+      v = plane[(size_t)y * pitch + x];
     }
     if (n == 32) {
 #pragma unroll
@@ -776,6 +781,14 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
   if (!get_fft_plan(nx, &px) || !get_fft_plan(ny, &py) || (nz > 1 && !get_fft_plan(nz, &pz)))
     return mo_fail(err, "PSF dimensions must factor into 2, 3, 5 and 7");
 
+  // Lengths with factor pairs and a z length of the list: half spectra
+  // throughout (separation and transforms 63 us at 128^2 x 64 x 5); any other
+  // by full rows in shared-memory stages (136 us there).
+  TfPlan tx, ty;
+  const TfKernels* kx = fft_two_factor(kSiteMakeOtf, nx) ? tf_kernels(nx, &tx) : nullptr;
+  const TfKernels* ky = fft_two_factor(kSiteMakeOtf, ny) ? tf_kernels(ny, &ty) : nullptr;
+  const bool tf = kx && kx->mo_rows && ky && (nz == 1 || z_length_ok(nz));
+  const int pitch = tf ? nxh : nx;
   // host-side constants with the reference's float arithmetic
   ApoFact fact;
   for (int l = 0; l < kNapodize; ++l)
@@ -825,6 +838,7 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
   }
   ShiftCompArgs sc{};
   sc.nx = nx, sc.ny = ny, sc.nz = nz, sc.nph = nph, sc.norders = norders, sc.compensate = o.compensate;
+  sc.pitch = pitch;
   sc.dkx = (float)(1. / (nx * o.dr));
   sc.dky = (float)(1. / (ny * o.dr));
   sc.dkz = (float)(1. / (nz * o.dz));
@@ -875,7 +889,7 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
                            {(void**)&d_center, 4 * sizeof(float)},
                            {(void**)&d_bval, nparts * sizeof(float)},
                            {(void**)&d_bidx, nparts * sizeof(long long)},
-                           {(void**)&d_bands, (size_t)nph * nvox * sizeof(float2)},
+                           {(void**)&d_bands, (size_t)nph * nz * ny * pitch * sizeof(float2)},
                            {(void**)&d_avg, (size_t)nph * nbins * nz * sizeof(float2)},
                            {(void**)&d_bstart, (nbins + 1) * sizeof(int)},
                            {(void**)&d_bpix, std::max<size_t>(1, bin_pix.size()) * sizeof(int)},
@@ -904,36 +918,58 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
                                            fact);
   k_mo_argmax_partial<<<nparts, kMoThreads, 0, s>>>(d_psf, nx, ny, nz, nph, d_bval, d_bidx);
   k_mo_center<<<1, kMoThreads, 0, s>>>(d_psf, nx, ny, nz, nph, d_bval, d_bidx, nparts, d_center);
-  k_mo_separate<<<4 * 152, kMoThreads, 0, s>>>(d_psf, d_bg, nx, ny, nz, nph, sepm, d_bands);
-  // 3D forward FFT of every band: x rows, then y and z over kx <= nx/2
-  {
-    const int rows = nph * nz * ny;
-    int nl = std::max(1, std::min(rows, kFftElems / nx));
-    size_t smr = fft_stage_smem(nx, nl, nl * (nx + 1), kMoThreads);
-    dispatch_fft_len(kSiteMakeOtf, nx, [&]<int NF>() {
-      set_smem(k_mo_fft_rows<NF>, smr);
-      k_mo_fft_rows<NF><<<(rows + nl - 1) / nl, kMoThreads, smr, s>>>(d_bands, nx, rows, px, nl);
-    });
-    int Wy = std::max(1, std::min(32, kFftElems / ny));
-    size_t smy = fft_stage_smem(ny, Wy, ny * (Wy + 1), kMoThreads);
-    dispatch_fft_len(kSiteMakeOtf, ny, [&]<int NF>() {
-      set_smem(k_mo_fft_cols<NF>, smy);
-      k_mo_fft_cols<NF><<<dim3((nxh + Wy - 1) / Wy, nph * nz), kMoThreads, smy, s>>>(d_bands, ny, (size_t)nx, nxh,
-                                                                                     nxy, py, Wy, 0);
-    });
-    if (nz > 1) {
-      int Wz = std::max(1, std::min(32, kFftElems / nz));
-      size_t smz = fft_stage_smem(nz, Wz, nz * (Wz + 1), kMoThreads);
-      dispatch_fft_len(kSiteMakeOtf, nz, [&]<int NF>() {
-        set_smem(k_mo_fft_cols<NF>, smz);
-        k_mo_fft_cols<NF><<<dim3((nxh + Wz - 1) / Wz, ny, nph), kMoThreads, smz, s>>>(d_bands, nz, nxy, nxh,
-                                                                                     (size_t)nx, pz, Wz, nvox);
+  if (tf) {
+    // separation inside the x transform, half spectra [band][z][ky][kx <= nx/2]
+    MoRowsArgs ra{};
+    ra.psf = d_psf;
+    ra.bg = d_bg;
+    ra.ny = ny;
+    ra.nz = nz;
+    ra.nph = nph;
+    std::copy(sepm.m, sepm.m + nph * nph, ra.m);
+    ra.bands = d_bands;
+    int rc = kx->mo_rows(ra, tx, s);
+    if (rc == 0) rc = ky->fft_cols(d_bands, nxh, nph * nz, ty, s);
+    if (rc == 0 && nz > 1) rc = launch_z_forward(d_bands, nz, nph, (size_t)ny * nxh, pz.tw, s);
+    if (rc != 0) {
+      cudaStreamSynchronize(s);
+      cudaEventDestroy(ev0);
+      cudaEventDestroy(ev1);
+      cudaFree(arena);
+      return mo_fail(err, "makeotf transforms could not be launched");
+    }
+  } else {
+    k_mo_separate<<<4 * 152, kMoThreads, 0, s>>>(d_psf, d_bg, nx, ny, nz, nph, sepm, d_bands);
+    // 3D forward FFT of every band: x rows, then y and z over kx <= nx/2
+    {
+      const int rows = nph * nz * ny;
+      int nl = std::max(1, std::min(rows, kFftElems / nx));
+      size_t smr = fft_stage_smem(nx, nl, nl * (nx + 1), kMoThreads);
+      dispatch_fft_len(kSiteMakeOtf, nx, [&]<int NF>() {
+        set_smem(k_mo_fft_rows<NF>, smr);
+        k_mo_fft_rows<NF><<<(rows + nl - 1) / nl, kMoThreads, smr, s>>>(d_bands, nx, rows, px, nl);
       });
+      int Wy = std::max(1, std::min(32, kFftElems / ny));
+      size_t smy = fft_stage_smem(ny, Wy, ny * (Wy + 1), kMoThreads);
+      dispatch_fft_len(kSiteMakeOtf, ny, [&]<int NF>() {
+        set_smem(k_mo_fft_cols<NF>, smy);
+        k_mo_fft_cols<NF><<<dim3((nxh + Wy - 1) / Wy, nph * nz), kMoThreads, smy, s>>>(d_bands, ny, (size_t)nx, nxh,
+                                                                                       nxy, py, Wy, 0);
+      });
+      if (nz > 1) {
+        int Wz = std::max(1, std::min(32, kFftElems / nz));
+        size_t smz = fft_stage_smem(nz, Wz, nz * (Wz + 1), kMoThreads);
+        dispatch_fft_len(kSiteMakeOtf, nz, [&]<int NF>() {
+          set_smem(k_mo_fft_cols<NF>, smz);
+          k_mo_fft_cols<NF><<<dim3((nxh + Wz - 1) / Wz, ny, nph), kMoThreads, smz, s>>>(d_bands, nz, nxy, nxh,
+                                                                                       (size_t)nx, pz, Wz, nvox);
+        });
+      }
     }
   }
   k_mo_shift_comp<<<dim3(8 * 152, nph / 2 + 1), kMoThreads, 0, s>>>(d_bands, d_center, sc);
   k_mo_radial<<<dim3((nbins + 3) / 4, nz, nph), 128, 0, s>>>(d_bands, d_bstart, d_bpix, nbins, nx, ny, nz,
-                                                                 d_avg);
+                                                                 pitch, d_avg);
   k_mo_finish<<<1, 1024, 0, s>>>(d_avg, fa, d_out, d_scal);
   cudaEventRecord(ev1, s);
   e = cudaGetLastError();

@@ -232,6 +232,55 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
   }
 }
 
+// makeotf: two rows of one band as a complex line, the band separated from the
+// phases' rows as they are loaded (k_mo_separate's operations; the phases come
+// from L2 for all bands but the first), half spectra out.  Bound by the loads
+// of nph sections per band: 128^2 x 64 x 5 42 us, where the separation into
+// full complex rows and their transform took 18 + 43 us and left twice the
+// bytes to the y and z transforms.
+template <int R1, int R2>
+__global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
+    k_tf_mo_rows(const __grid_constant__ MoRowsArgs a, const float2* __restrict__ tw)
+{
+  using G = TfRow<R1, R2>;
+  constexpr int N = G::N, nxh = N / 2 + 1;
+  extern __shared__ __align__(16) float2 sm[];
+  const int z = blockIdx.y, b = blockIdx.z, y0 = blockIdx.x * 2 * G::W;
+  const size_t nxy = (size_t)a.ny * N;
+  const float* psf = a.psf + (size_t)z * a.nph * nxy;
+  float* smr = (float*)sm;  // row r at x -> smr[2*((r>>1)*N + x) + (r&1)]
+  for (int t = threadIdx.x; t < 2 * G::W * N; t += G::kThreads) {
+    const int r = t / N, x = t - r * N, y = y0 + r;
+    float acc = 0.f;
+    if (y < a.ny)
+      for (int j = 0; j < a.nph; ++j) {
+        const float v = __fsub_rn(__ldg(psf + j * nxy + (size_t)y * N + x), __ldg(a.bg + z * a.nph + j));
+        acc = a.nph == 1 ? v : __fadd_rn(acc, __fmul_rn(v, a.m[b * a.nph + j]));
+      }
+    smr[2 * ((r >> 1) * N + x) + (r & 1)] = acc;
+  }
+  __syncthreads();
+  float2 u[R2];
+  tf_row_lines<R1, R2, -1>(sm, tw, u);
+  __syncthreads();  // the exchange is taken: the lines go back in place
+  {
+    const int l = threadIdx.x / R1, k1 = threadIdx.x - l * R1;
+    if (l < G::W) {
+#pragma unroll
+      for (int k2 = 0; k2 < R2; ++k2) sm[l * N + k1 + R1 * k2] = u[k2];
+    }
+  }
+  __syncthreads();
+  float2* dst = a.bands + ((size_t)b * a.nz + z) * a.ny * nxh;
+  for (int t = threadIdx.x; t < G::W * nxh; t += G::kThreads) {
+    const int l = t / nxh, k = t - l * nxh;
+    const float2 zk = sm[l * N + k], zn = sm[l * N + (k == 0 ? 0 : N - k)];
+    const int y = y0 + 2 * l;
+    if (y < a.ny) dst[(size_t)y * nxh + k] = make_float2(0.5f * (zk.x + zn.x), 0.5f * (zk.y - zn.y));
+    if (y + 1 < a.ny) dst[(size_t)(y + 1) * nxh + k] = make_float2(0.5f * (zk.y + zn.y), -0.5f * (zk.x - zn.x));
+  }
+}
+
 // ----------------------------------------------------------------- overlaps
 // radial table of one kz: order slot o at [o * (nxotf + 1)], entry i the OTF
 // interpolated to kz at radial bins i and i + 1 (flat indices clamped to the
@@ -604,14 +653,21 @@ struct TfEntry {
     }
     return (int)cudaGetLastError();
   }
+  static int mo_rows(const MoRowsArgs& a, const TfPlan& pl, cudaStream_t s)
+  {
+    using G = TfRow<R1, R2>;
+    allow_dynamic_smem((const void*)k_tf_mo_rows<R1, R2>, G::kSmem);
+    k_tf_mo_rows<R1, R2><<<dim3((a.ny + 2 * G::W - 1) / (2 * G::W), a.nz, a.nph), G::kThreads, G::kSmem, s>>>(a, pl.tw);
+    return (int)cudaGetLastError();
+  }
   static constexpr bool even = R1 * R2 % 2 == 0;
   template <bool E>
   static constexpr TfKernels make()
   {
     if constexpr (E)
-      return {R1, R2, asm_x, ovl_x, ovl_y, TfOvlY<R1, R2>::W, fft_cols, fft_rows_conj, ingest_x};
+      return {R1, R2, asm_x, ovl_x, ovl_y, TfOvlY<R1, R2>::W, fft_cols, fft_rows_conj, ingest_x, mo_rows};
     else
-      return {R1, R2, nullptr, ovl_x, ovl_y, TfOvlY<R1, R2>::W, fft_cols, fft_rows_conj, nullptr};
+      return {R1, R2, nullptr, ovl_x, ovl_y, TfOvlY<R1, R2>::W, fft_cols, fft_rows_conj, nullptr, nullptr};
   }
   static constexpr TfKernels kernels() { return make<even>(); }
 };

@@ -16,6 +16,15 @@ struct AsmX2Launch {
   bool real;
 };
 
+// makeotf's band separation and x half of the transform of every band
+struct MoRowsArgs {
+  const float* psf;  // [nz * nph][ny][n], phase fastest
+  const float* bg;   // [nz * nph]
+  int ny, nz, nph;
+  float m[kMaxPhases * kMaxPhases];  // band = sum over phases of m[band * nph + phase] * section
+  float2* bands;     // [nph][nz][ny][n/2+1]
+};
+
 // Every function returns a CUDA error code (0: launched).
 struct TfKernels {
   int r1, r2;
@@ -33,6 +42,7 @@ struct TfKernels {
   int (*fft_rows_conj)(const float2* in, float2* out, int nrows, const TfPlan& pl, cudaStream_t s);
   // flat field, edge blends and the x half of the 2D transform of every raw plane
   int (*ingest_x)(const IngestArgs& a, const TfPlan& pl, cudaStream_t s);
+  int (*mo_rows)(const MoRowsArgs& a, const TfPlan& pl, cudaStream_t s);
 };
 // the kernels of length n and its plan; null where n has no factor pair
 const TfKernels* tf_kernels(int n, TfPlan* plan);

@@ -31,4 +31,7 @@ int launch_separate_z(float2* spec, const float* scale, const float* sepmat, siz
 int launch_asm_zn(const float2* S, float* out, int X, int Y, int Z, unsigned long long active, const float2* tw,
                   int split, cudaStream_t s);
 
+// forward z transform of nbands volumes [nz][plane], in place (z_length_ok(nz))
+int launch_z_forward(float2* data, int nz, int nbands, size_t plane, const float2* tw, cudaStream_t s);
+
 }  // namespace simrecon
