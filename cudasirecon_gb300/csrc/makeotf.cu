@@ -15,10 +15,10 @@
 //   k_mo_radial     radial average per (band, kz) over a precomputed table of
 //                   the pixels of each kr bin (876-921): float sums in the
 //                   reference's pixel order (deterministic)
-//   k_mo_finish     one CTA: Hermitian symmetry (923-934), modify (1169-1186),
-//                   cleanup (938-999), fixorigin (1188-1224), rescale
-//                   (1226-1242), combine_reim (746-782), conj (411-415) and the
-//                   output layout of outputdata (1073-1099)
+//   k_mo_finish_*   Hermitian symmetry (923-934), modify (1169-1186), cleanup
+//                   (938-999), fixorigin (1188-1224), rescale (1226-1242),
+//                   combine_reim (746-782), conj (411-415) and the output
+//                   layout of outputdata (1073-1099)
 // The float32 steps whose rounding decides something downstream (apodisation,
 // the phase average and its argmax, the parabola fits, the separation, the
 // shift phases and the bin index) use explicitly rounded operations so they
@@ -44,7 +44,6 @@ namespace {
 constexpr int kMoThreads = 256;
 constexpr int kNapodize = 10;
 constexpr int kBorder = 20;
-constexpr int kMoMaxPhases = 9;
 
 struct ApoFact {
   float f[kNapodize];
@@ -74,24 +73,22 @@ __global__ void __launch_bounds__(kMoThreads) k_mo_section(float* psf, float* bg
     // kept; the FP64 adder has a sixtyfourth of the FP32 rate here)
     float hi = 0.f, lo = 0.f;
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int y = threadIdx.x >> 5; y < ny; y += nw) {
-      const bool full = y < kBorder || y > ny - kBorder;
-      const float* row = sec + (size_t)y * nx;
+    for (int y0 = threadIdx.x >> 5; y0 < ny; y0 += 4 * nw)  // four rows' loads in flight
       for (int x0 = lane; x0 < nx; x0 += 128) {
-        float v[4];
+        float v[16];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int x = x0 + 32 * q;
-          v[q] = x < nx && (full || x < kBorder || x > nx - kBorder) ? row[x] : 0.f;
+        for (int q = 0; q < 16; ++q) {
+          const int x = x0 + 32 * (q & 3), y = y0 + (q >> 2) * nw;
+          const bool in = y < ny && x < nx && (y < kBorder || y > ny - kBorder || x < kBorder || x > nx - kBorder);
+          v[q] = in ? sec[(size_t)y * nx + x] : 0.f;
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < 16; ++q) {
           const float h = __fadd_rn(hi, v[q]), w = __fsub_rn(h, hi);
           lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(h, w)), __fsub_rn(v[q], w)));
           hi = h;
         }
       }
-    }
     double s = (double)hi + (double)lo;
     s = block_sum_d(s, red);
     if (threadIdx.x == 0) s_bg = (float)(s / border_count);
@@ -123,11 +120,18 @@ __global__ void __launch_bounds__(kMoThreads) k_mo_section(float* psf, float* bg
 }
 
 // ------------------------------------------------------------------- centre
-// phase average of one voxel (float32, phases summed in order, then / nph)
+// phase average of one voxel (float32, phases summed in order, then / nph);
+// the loads do not wait for the additions
 __device__ __forceinline__ float mo_avg(const float* __restrict__ psf, int nph, size_t nxy, int z, size_t rem)
 {
+  const float* p0 = psf + (size_t)z * nph * nxy + rem;
+  float v[kMoMaxPhases];
+#pragma unroll
+  for (int p = 0; p < kMoMaxPhases; ++p) v[p] = p < nph ? p0[p * nxy] : 0.f;
   float s = 0.f;
-  for (int p = 0; p < nph; ++p) s = __fadd_rn(s, psf[((size_t)z * nph + p) * nxy + rem]);
+#pragma unroll
+  for (int p = 0; p < kMoMaxPhases; ++p)
+    if (p < nph) s = __fadd_rn(s, v[p]);
   return __fdiv_rn(s, (float)nph);
 }
 
@@ -165,28 +169,30 @@ __device__ __forceinline__ void mo_block_argmax(float& bv, long long& bi, float*
     }
 }
 
+// blockIdx.y: the plane.  Bound by memory; with a 64-bit division per voxel and
+// each phase's load behind the last addition 22 us at 128^2 x 64 x 5, 11 here.
 // Only values > 0 count (the reference starts from maxval = 0 with a strict
 // comparison), so the initial state is (0, none).
 __global__ void __launch_bounds__(kMoThreads) k_mo_argmax_partial(const float* __restrict__ psf, int nx, int ny,
-                                                                  int nz, int nph, float* bval, long long* bidx)
+                                                                  int nph, float* bval, long long* bidx)
 {
   __shared__ float sv[32];
   __shared__ long long si[32];
-  const size_t nxy = (size_t)nx * ny, nv = nxy * nz;
+  const int nxy = nx * ny, z = blockIdx.y;
   float bv = 0.f;
   long long bi = -1;
-  for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
-    int z = (int)(v / nxy);
-    float a = mo_avg(psf, nph, nxy, z, v - (size_t)z * nxy);
+#pragma unroll 2
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nxy; v += gridDim.x * blockDim.x) {
+    const float a = mo_avg(psf, nph, nxy, z, v);
     if (a > bv) {
       bv = a;
-      bi = (long long)v;
+      bi = (long long)z * nxy + v;
     }
   }
   mo_block_argmax(bv, bi, sv, si);
   if (threadIdx.x == 0) {
-    bval[blockIdx.x] = bv;
-    bidx[blockIdx.x] = bi;
+    bval[z * gridDim.x + blockIdx.x] = bv;
+    bidx[z * gridDim.x + blockIdx.x] = bi;
   }
 }
 
@@ -217,32 +223,41 @@ __global__ void k_mo_center(const float* __restrict__ psf, int nx, int ny, int n
   long long bi = -1;
   for (int i = threadIdx.x; i < nparts; i += blockDim.x) mo_better(bv, bi, bval[i], bidx[i]);
   mo_block_argmax(bv, bi, sv, si);
-  if (threadIdx.x == 0) {
-    const int nxe = (nx % 2) ? nx + 1 : nx + 2;
-    int maxk = 0, maxi = 0, maxj = 0;
-    float maxval = 0.f;
-    if (bi >= 0) {
-      size_t nxy = (size_t)nx * ny;
-      maxk = (int)(bi / nxy);
-      size_t rem = bi - (size_t)maxk * nxy;
-      maxi = (int)(rem / nx);
-      maxj = (int)(rem - (size_t)maxi * nx);
-      maxval = bv;
+  if (threadIdx.x >= 32) return;
+  // lanes 0..5: the peak's neighbours below and above in z, y and x
+  bi = __shfl_sync(0xffffffffu, bi, 0);
+  bv = __shfl_sync(0xffffffffu, bv, 0);
+  const int nxe = (nx % 2) ? nx + 1 : nx + 2;
+  int at[3] = {0, 0, 0};
+  const int n[3] = {nz, ny, nxe};
+  if (bi >= 0) {
+    const size_t nxy = (size_t)nx * ny;
+    at[0] = (int)(bi / nxy);
+    const size_t rem = bi - (size_t)at[0] * nxy;
+    at[1] = (int)(rem / nx);
+    at[2] = (int)(rem - (size_t)at[1] * nx);
+  }
+  const float maxval = bi >= 0 ? bv : 0.f;
+  const int lane = threadIdx.x;
+  float side = 0.f;
+  if (lane < 6) {
+    int w[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      w[k] = at[k];
+      if (lane >> 1 == k) w[k] += lane & 1 ? (at[k] + 1 >= n[k] ? 1 - n[k] : 1) : (at[k] < 1 ? n[k] - 1 : -1);
     }
-    int im = maxi - 1 < 0 ? maxi - 1 + ny : maxi - 1, ip = maxi + 1 >= ny ? maxi + 1 - ny : maxi + 1;
-    int jm = maxj - 1 < 0 ? maxj - 1 + nxe : maxj - 1, jp = maxj + 1 >= nxe ? maxj + 1 - nxe : maxj + 1;
-    int km = maxk - 1 < 0 ? maxk - 1 + nz : maxk - 1, kp = maxk + 1 >= nz ? maxk + 1 - nz : maxk + 1;
-    float zc = (float)maxk;
-    if (nz > 1)
-      zc = __fadd_rn((float)maxk, mo_fitparabola(mo_avg_at(psf, nx, ny, nph, km, maxi, maxj), maxval,
-                                                 mo_avg_at(psf, nx, ny, nph, kp, maxi, maxj)));
-    float yc = __fadd_rn((float)maxi, mo_fitparabola(mo_avg_at(psf, nx, ny, nph, maxk, im, maxj), maxval,
-                                                     mo_avg_at(psf, nx, ny, nph, maxk, ip, maxj)));
-    float xc = __fadd_rn((float)maxj, mo_fitparabola(mo_avg_at(psf, nx, ny, nph, maxk, maxi, jm), maxval,
-                                                     mo_avg_at(psf, nx, ny, nph, maxk, maxi, jp)));
-    center[0] = xc;
-    center[1] = yc;
-    center[2] = zc;
+    side = mo_avg_at(psf, nx, ny, nph, w[0], w[1], w[2]);
+  }
+  const float up = __shfl_down_sync(0xffffffffu, side, 1);
+  // lane 2k: the centre along axis k and the shift's phase per frequency
+  // (radialft.cpp:853-855: 2*M_PI*c/n in double, stored as float)
+  if (lane < 6 && !(lane & 1)) {
+    const int k = lane >> 1, peak = k == 0 ? at[0] : k == 1 ? at[1] : at[2];
+    float c = (float)peak;
+    if (k > 0 || nz > 1) c = __fadd_rn(c, mo_fitparabola(side, maxval, up));
+    center[2 - k] = c;
+    center[5 - k] = (float)(2.0 * M_PI * (double)c / (k == 0 ? nz : k == 1 ? ny : nx));
   }
 }
 
@@ -390,18 +405,15 @@ __device__ __forceinline__ float sphere_ratio(const ShiftCompArgs& a, float rho)
 }
 
 // blockIdx.y: the order; its one or two bands share the shift's rotation and
-// the compensation.  Bound by HBM and the series' issue: 128^2 x 64 x 5 with
-// the closed form in double for every band 370 us, 73 us here (cold caches).
+// the compensation.  Bound by memory and the series' issue: 128^2 x 64 x 5 with
+// the closed form in double for every band 370 us, with only the phases per
+// frequency divided in double by every thread 73 us, 34 us here (cold caches).
 __global__ void __launch_bounds__(kMoThreads) k_mo_shift_comp(float2* bands, const float* center, ShiftCompArgs a)
 {
   const int nxh = a.nx / 2 + 1;
   const int order = blockIdx.y;
   const size_t nh = (size_t)a.nz * a.ny * nxh;
-  const float xc = center[0], yc = center[1], zc = center[2];
-  // radialft.cpp:853-855: 2*M_PI*c/n in double, stored as float
-  const float dphiz = (float)(2.0 * M_PI * (double)zc / a.nz);
-  const float dphiy = (float)(2.0 * M_PI * (double)yc / a.ny);
-  const float dphix = (float)(2.0 * M_PI * (double)xc / a.nx);
+  const float dphix = center[3], dphiy = center[4], dphiz = center[5];
   const size_t vol = (size_t)a.nz * a.ny * a.pitch;
   const int b0 = order == 0 ? 0 : 2 * order - 1, b1 = order == 0 ? 0 : min(2 * order, a.nph - 1);
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < nh; t += (size_t)gridDim.x * blockDim.x) {
@@ -494,15 +506,16 @@ struct FinishArgs {
 
 __device__ __forceinline__ float2 c_mulf(float2 a, float f) { return make_float2(__fmul_rn(a.x, f), __fmul_rn(a.y, f)); }
 
-__global__ void __launch_bounds__(1024) k_mo_finish(float2* avg, FinishArgs a, float* out, float* scal)
+// One CTA per band: symmetry, modify, cleanup and the origin (band 0), in place
+__global__ void __launch_bounds__(1024) k_mo_finish_band(float2* bands, FinishArgs a)
 {
-  __shared__ double red[32];
-  __shared__ float s_scale;
   __shared__ double s_sums[64];
-  const int nz = a.nz, nb = a.nbins;
-  // Hermitian symmetry along kz per (band, bin), a thread per (row, kz pair)
+  const int nz = a.nz, nb = a.nbins, p = blockIdx.x, order = (p + 1) / 2;
+  float2* avg = bands + (size_t)p * nb * nz;
+  // Hermitian symmetry along kz per bin, a thread per (bin, kz pair)
   const int half = nz / 2;
-  for (int t = threadIdx.x; t < a.nph * nb * (half + 1); t += blockDim.x) {
+#pragma unroll 4
+  for (int t = threadIdx.x; t < nb * (half + 1); t += blockDim.x) {
     const int row = t / (half + 1), kz = t - row * (half + 1);
     float2* r = avg + (size_t)row * nz;
     if (kz == 0) {
@@ -515,144 +528,142 @@ __global__ void __launch_bounds__(1024) k_mo_finish(float2* avg, FinishArgs a, f
     r[nz - kz] = make_float2(v.x, -v.y);
   }
   __syncthreads();
-  if (threadIdx.x == 0) s_scale = 1.f;
-  for (int p = 0; p < a.nph; ++p) {
-    const int order = (p + 1) / 2;
-    float2* o = avg + (size_t)p * nb * nz;
+  // modify (radialft.cpp:1169-1186)
+  if (a.ifixz) {
+    for (int kz = threadIdx.x; kz < nz; kz += blockDim.x)
+      if (kz != 0 || order > 0) avg[kz] = avg[nz + kz];
     __syncthreads();
-    // modify (radialft.cpp:1169-1186)
-    if (a.ifixz)
-      for (int kz = threadIdx.x; kz < nz; kz += blockDim.x)
-        if (kz != 0 || order > 0) o[kz] = o[nz + kz];
-    __syncthreads();
-    if (a.ifixr)
-      for (int kx = a.ifixr + threadIdx.x; kx < nb; kx += blockDim.x) {
-        float2 u = o[(size_t)kx * nz + 1], w = o[(size_t)kx * nz + nz - 1];
-        o[(size_t)kx * nz] = make_float2(__fdiv_rn(__fadd_rn(u.x, w.x), 2.f), __fdiv_rn(__fadd_rn(u.y, w.y), 2.f));
-      }
-    __syncthreads();
-    // cleanup (radialft.cpp:938-999, single objective)
-    if (!a.bessel && a.cleanup)
-      for (int ix = threadIdx.x; ix < nb; ix += blockDim.x) {
-        float2* row = o + (size_t)ix * nz;
-        float kr = __fmul_rn((float)ix, a.cl_dkr);
-        if (kr <= a.cl_krmax) {
-          float beta = asinf(__fdiv_rn(__fsub_rn(a.cl_na, __fmul_rn(kr, a.cl_lamda)), a.cl_nimm));
-          float kzedge = __fmul_rn(__fdiv_rn(a.cl_nimm, a.cl_lamda), __fsub_rn(cosf(beta), a.cl_cosalpha));
-          float q = __fdiv_rn(kzedge, a.cl_dkz);
-          if (order == 0) {
-            int kzstart = (int)rintf(__fadd_rn(q, 1.f));
-            int kzend = nz - kzstart;
-            for (int iz = max(kzstart, 0); iz <= kzend && iz < nz; ++iz) row[iz] = make_float2(0.f, 0.f);
-          } else if (order == 1) {
-            int jotf = (int)rint((double)q + 0.999);
-            int kzend = a.leavekz[0] - jotf;
-            for (int iz = 0; iz <= kzend && iz < nz; ++iz) {
-              row[iz] = make_float2(0.f, 0.f);
-              if (iz != 0) row[nz - iz] = make_float2(0.f, 0.f);
-            }
-            for (int iz = max(a.leavekz[1] + jotf + 1, 0); iz < nz / 2 + 1; ++iz) {
-              row[iz] = make_float2(0.f, 0.f);
-              row[(nz - iz) % nz] = make_float2(0.f, 0.f);
-            }
-          } else {
-            int jotf = (int)rint((double)q + 0.999);
-            for (int iz = max(a.leavekz[2] + jotf, 0); iz < nz / 2 + 1; ++iz) {
-              row[iz] = make_float2(0.f, 0.f);
-              row[(nz - iz) % nz] = make_float2(0.f, 0.f);
-            }
-          }
-        } else {
-          for (int iz = 0; iz < nz; ++iz) row[iz] = make_float2(0.f, 0.f);
-        }
-      }
-    __syncthreads();
-    // fixorigin on band 0 (radialft.cpp:1188-1224)
-    if (p == 0 && a.fix_kx1 > 0) {
-      // a warp per kr: the lanes' double sums, then across the warp
-      const int lane = threadIdx.x & 31;
-      for (int i = threadIdx.x >> 5; i <= a.fix_kx2; i += blockDim.x >> 5) {
-        double s = 0.0;
-        for (int j = lane; j < (i == 0 ? 1 : nz); j += 32) s += o[(size_t)i * nz + j].x;
-        for (int q = 16; q > 0; q >>= 1) s += __shfl_down_sync(0xffffffffu, s, q);
-        if (lane == 0) s_sums[i] = s;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        const float meani = (float)(0.5 * (a.fix_kx1 + a.fix_kx2));
-        const int numvals = a.fix_kx2 - a.fix_kx1 + 1;
-        double totsum = 0, ysum = 0, sqsum = 0;
-        for (int i = a.fix_kx1; i <= a.fix_kx2; ++i) {
-          float d = __fsub_rn((float)i, meani);
-          totsum += s_sums[i];
-          ysum += s_sums[i] * (double)d;
-          sqsum += (double)__fmul_rn(d, d);
-        }
-        const float slope = (float)(ysum / sqsum);
-        const float av = (float)(totsum / numvals);
-        for (int i = 0; i < a.fix_kx1; ++i) {
-          float lineval = __fadd_rn(av, __fmul_rn(__fsub_rn((float)i, meani), slope));
-          float2 v = o[(size_t)i * nz];
-          v.x = (float)((double)v.x - (s_sums[i] - (double)lineval));
-          o[(size_t)i * nz] = v;
-        }
-      }
-      __syncthreads();
-    }
-    // rescale (radialft.cpp:1226-1242): factor from band 0 (or each band with -rescale)
-    if (threadIdx.x == 0 && (order == 0 || a.rescale)) s_scale = __fdiv_rn(1.f, o[0].x);
-    __syncthreads();
-    const float sc = s_scale;
-    for (int i = threadIdx.x; i < nb * nz; i += blockDim.x) o[i] = c_mulf(o[i], sc);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) *scal = s_scale;
-  // combine_reim (radialft.cpp:746-782)
-  if (!a.five_bands && a.nph > 1) {
-    for (int ord = 1; ord < a.norders; ++ord) {
-      float2* re_b = avg + (size_t)(2 * ord - 1) * nb * nz;
-      float2* im_b = avg + (size_t)(2 * ord) * nb * nz;
-      const int n = (a.nx / 2 + 1) * nz;
-      double sr = 0.0, si = 0.0;
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        sr += (double)hypotf(re_b[i].x, re_b[i].y);
-        si += (double)hypotf(im_b[i].x, im_b[i].y);
+  if (a.ifixr) {
+    for (int kx = a.ifixr + threadIdx.x; kx < nb; kx += blockDim.x) {
+      float2* row = avg + (size_t)kx * nz;
+      const float2 u = row[1], w = row[nz - 1];
+      row[0] = make_float2(__fdiv_rn(__fadd_rn(u.x, w.x), 2.f), __fdiv_rn(__fadd_rn(u.y, w.y), 2.f));
+    }
+    __syncthreads();
+  }
+  // cleanup (radialft.cpp:938-999, single objective): a warp per row
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const float2 zero = make_float2(0.f, 0.f);
+  if (!a.bessel && a.cleanup) {
+    for (int ix = warp; ix < nb; ix += nw) {
+      float2* row = avg + (size_t)ix * nz;
+      const float kr = __fmul_rn((float)ix, a.cl_dkr);
+      if (!(kr <= a.cl_krmax)) {
+        for (int iz = lane; iz < nz; iz += 32) row[iz] = zero;
+        continue;
       }
-      sr = block_sum_d(sr, red);
-      __syncthreads();
-      si = block_sum_d(si, red);
-      __shared__ float s_c, s_s;
-      if (threadIdx.x == 0) {
-        double phi = atan(si / sr);
-        const size_t q = (size_t)(a.nx / 4) * nz;
-        float r0 = re_b[q].x, i0 = im_b[q].x;
-        if (r0 < 0 && i0 > 0) phi += M_PI;
-        else if (r0 < 0 && i0 < 0) phi = M_PI - phi;
-        else if (r0 > 0 && i0 > 0) phi = -phi;
-        if (ord == 1 && a.pishift) phi = M_PI - phi;
-        s_c = (float)cos(phi);
-        s_s = (float)sin(-phi);
+      const float beta = asinf(__fdiv_rn(__fsub_rn(a.cl_na, __fmul_rn(kr, a.cl_lamda)), a.cl_nimm));
+      const float kzedge = __fmul_rn(__fdiv_rn(a.cl_nimm, a.cl_lamda), __fsub_rn(cosf(beta), a.cl_cosalpha));
+      const float q = __fdiv_rn(kzedge, a.cl_dkz);
+      if (order == 0) {
+        const int kzstart = (int)rintf(__fadd_rn(q, 1.f)), kzend = nz - kzstart;
+        for (int iz = max(kzstart, 0) + lane; iz <= kzend && iz < nz; iz += 32) row[iz] = zero;
+        continue;
       }
-      __syncthreads();
-      const float c = s_c, s = s_s;
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        float2 u = c_mulf(re_b[i], c), w = c_mulf(im_b[i], s);
-        re_b[i] = make_float2(__fadd_rn(u.x, w.x), __fadd_rn(u.y, w.y));
-        im_b[i] = make_float2(0.f, 0.f);
+      const int jotf = (int)rint((double)q + 0.999);
+      if (order == 1)
+        for (int iz = lane; iz <= a.leavekz[0] - jotf && iz < nz; iz += 32) {
+          row[iz] = zero;
+          if (iz != 0) row[nz - iz] = zero;
+        }
+      for (int iz = max(order == 1 ? a.leavekz[1] + jotf + 1 : a.leavekz[2] + jotf, 0) + lane; iz < nz / 2 + 1;
+           iz += 32) {
+        row[iz] = zero;
+        row[(nz - iz) % nz] = zero;
       }
-      __syncthreads();
+    }
+    __syncthreads();
+  }
+  // fixorigin on band 0 (radialft.cpp:1188-1224)
+  if (p == 0 && a.fix_kx1 > 0) {
+    // a warp per kr: the lanes' double sums, then across the warp
+    for (int i = warp; i <= a.fix_kx2; i += nw) {
+      double s = 0.0;
+      for (int j = lane; j < (i == 0 ? 1 : nz); j += 32) s += avg[(size_t)i * nz + j].x;
+      for (int q = 16; q > 0; q >>= 1) s += __shfl_down_sync(0xffffffffu, s, q);
+      if (lane == 0) s_sums[i] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const float meani = (float)(0.5 * (a.fix_kx1 + a.fix_kx2));
+      const int numvals = a.fix_kx2 - a.fix_kx1 + 1;
+      double totsum = 0, ysum = 0, sqsum = 0;
+      for (int i = a.fix_kx1; i <= a.fix_kx2; ++i) {
+        float d = __fsub_rn((float)i, meani);
+        totsum += s_sums[i];
+        ysum += s_sums[i] * (double)d;
+        sqsum += (double)__fmul_rn(d, d);
+      }
+      const float slope = (float)(ysum / sqsum);
+      const float av = (float)(totsum / numvals);
+      for (int i = 0; i < a.fix_kx1; ++i) {
+        float lineval = __fadd_rn(av, __fmul_rn(__fsub_rn((float)i, meani), slope));
+        float2 v = avg[(size_t)i * nz];
+        v.x = (float)((double)v.x - (s_sums[i] - (double)lineval));
+        avg[(size_t)i * nz] = v;
+      }
     }
   }
-  __syncthreads();
+}
+
+// One CTA per band of the output: rescale (radialft.cpp:1226-1242) by band 0
+// (or each band by itself with -rescale), combine_reim (746-782), conj
+// (411-415) and the layout of outputdata (1073-1099).  The two kernels are
+// chains of small passes over a few thousand values, bound by latency: a CTA
+// per band and order takes 12 + 16 us at 65 x 64 x 5 where one CTA for
+// everything took 55.
+__global__ void __launch_bounds__(1024) k_mo_finish(const float2* __restrict__ avg, FinishArgs a, float* out,
+                                                    float* scal)
+{
+  __shared__ double red[32];
+  __shared__ float s_c, s_s;
+  const int nb = a.nbins, nz = a.nz, n = nb * nz, ob = blockIdx.x;
+  const bool combine = !a.five_bands && a.nph > 1 && ob > 0;
+  const int src = combine ? 2 * ob - 1 : ob;
+  const float2* re_b = avg + (size_t)src * n;
+  const float2* im_b = re_b + n;
+  const float sc = __fdiv_rn(1.f, a.rescale ? re_b[0].x : avg[0].x);
+  const float sc2 = combine && a.rescale ? __fdiv_rn(1.f, im_b[0].x) : sc;
+  if (ob == 0 && threadIdx.x == 0) *scal = __fdiv_rn(1.f, a.rescale ? avg[(size_t)(a.nph - 1) * n].x : avg[0].x);
+  float c = 1.f, s = 0.f;
+  if (combine) {
+    double sr = 0.0, si = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const float2 u = c_mulf(re_b[i], sc), w = c_mulf(im_b[i], sc2);
+      sr += (double)hypotf(u.x, u.y);
+      si += (double)hypotf(w.x, w.y);
+    }
+    sr = block_sum_d(sr, red);
+    __syncthreads();
+    si = block_sum_d(si, red);
+    if (threadIdx.x == 0) {
+      double phi = atan(si / sr);
+      const size_t q = (size_t)(a.nx / 4) * nz;
+      const float r0 = c_mulf(re_b[q], sc).x, i0 = c_mulf(im_b[q], sc2).x;
+      if (r0 < 0 && i0 > 0) phi += M_PI;
+      else if (r0 < 0 && i0 < 0) phi = M_PI - phi;
+      else if (r0 > 0 && i0 > 0) phi = -phi;
+      if (ob == 1 && a.pishift) phi = M_PI - phi;
+      s_c = (float)cos(phi);
+      s_s = (float)sin(-phi);
+    }
+    __syncthreads();
+    c = s_c;
+    s = s_s;
+  }
   // output bands: all with -5bands, else 0 and the combined 2*o-1
-  const int nout = a.five_bands ? a.nph : a.norders;
-  for (int t = threadIdx.x; t < nout * nb * nz; t += blockDim.x) {
-    int ob = t / (nb * nz), r = t - ob * (nb * nz);
-    int src = (a.five_bands || ob == 0) ? ob : 2 * ob - 1;
-    float2 v = avg[(size_t)src * nb * nz + r];
+  float2* dst = (float2*)out + (size_t)ob * n;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    float2 v = c_mulf(re_b[i], sc);
+    if (combine) {
+      const float2 u = c_mulf(v, c), w = c_mulf(c_mulf(im_b[i], sc2), s);
+      v = make_float2(__fadd_rn(u.x, w.x), __fadd_rn(u.y, w.y));
+    }
     if (a.conj) v.y = -v.y;
-    out[2 * (size_t)t] = v.x;
-    out[2 * (size_t)t + 1] = v.y;
+    dst[i] = v;
   }
 }
 
@@ -782,7 +793,7 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
     return mo_fail(err, "PSF dimensions must factor into 2, 3, 5 and 7");
 
   // Lengths with factor pairs and a z length of the list: half spectra
-  // throughout (separation and transforms 63 us at 128^2 x 64 x 5); any other
+  // throughout (separation and transforms 57 us at 128^2 x 64 x 5); any other
   // by full rows in shared-memory stages (136 us there).
   TfPlan tx, ty;
   const TfKernels* kx = fft_two_factor(kSiteMakeOtf, nx) ? tf_kernels(nx, &tx) : nullptr;
@@ -873,7 +884,7 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
 
   // device buffers
   const size_t nxy = (size_t)nx * ny, nvox = nxy * nz;
-  const int nparts = 2 * 152;
+  const int chunks = std::max(1, std::min((nx * ny + kMoThreads - 1) / kMoThreads, 8 * 152 / nz)), nparts = chunks * nz;
   const int nout = o.five_bands ? nph : norders;
   struct Buf {
     void** p;
@@ -886,7 +897,7 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
   int *d_bstart = nullptr, *d_bpix = nullptr;
   std::vector<Buf> bufs = {{(void**)&d_psf, (size_t)nsec * nxy * sizeof(float)},
                            {(void**)&d_bg, (size_t)nsec * sizeof(float)},
-                           {(void**)&d_center, 4 * sizeof(float)},
+                           {(void**)&d_center, 6 * sizeof(float)},
                            {(void**)&d_bval, nparts * sizeof(float)},
                            {(void**)&d_bidx, nparts * sizeof(long long)},
                            {(void**)&d_bands, (size_t)nph * nz * ny * pitch * sizeof(float2)},
@@ -916,7 +927,7 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
 
   k_mo_section<<<nsec, kMoThreads, 0, s>>>(d_psf, d_bg, nx, ny, o.background >= 0, o.background, border_count,
                                            fact);
-  k_mo_argmax_partial<<<nparts, kMoThreads, 0, s>>>(d_psf, nx, ny, nz, nph, d_bval, d_bidx);
+  k_mo_argmax_partial<<<dim3(chunks, nz), kMoThreads, 0, s>>>(d_psf, nx, ny, nph, d_bval, d_bidx);
   k_mo_center<<<1, kMoThreads, 0, s>>>(d_psf, nx, ny, nz, nph, d_bval, d_bidx, nparts, d_center);
   if (tf) {
     // separation inside the x transform, half spectra [band][z][ky][kx <= nx/2]
@@ -970,7 +981,8 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
   k_mo_shift_comp<<<dim3(8 * 152, nph / 2 + 1), kMoThreads, 0, s>>>(d_bands, d_center, sc);
   k_mo_radial<<<dim3((nbins + 3) / 4, nz, nph), 128, 0, s>>>(d_bands, d_bstart, d_bpix, nbins, nx, ny, nz,
                                                                  pitch, d_avg);
-  k_mo_finish<<<1, 1024, 0, s>>>(d_avg, fa, d_out, d_scal);
+  k_mo_finish_band<<<nph, 1024, 0, s>>>(d_avg, fa);
+  k_mo_finish<<<nout, 1024, 0, s>>>(d_avg, fa, d_out, d_scal);
   cudaEventRecord(ev1, s);
   e = cudaGetLastError();
   std::vector<float> center(4, 0.f);

@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
 // makeotf: two rows of one band as a complex line, the band separated from the
 // phases' rows as they are loaded (k_mo_separate's operations; the phases come
 // from L2 for all bands but the first), half spectra out.  Bound by the loads
-// of nph sections per band: 128^2 x 64 x 5 42 us, where the separation into
+// of nph sections per band: 128^2 x 64 x 5 35 us, where the separation into
 // full complex rows and their transform took 18 + 43 us and left twice the
 // bytes to the y and z transforms.
 template <int R1, int R2>
@@ -249,14 +249,21 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
   const size_t nxy = (size_t)a.ny * N;
   const float* psf = a.psf + (size_t)z * a.nph * nxy;
   float* smr = (float*)sm;  // row r at x -> smr[2*((r>>1)*N + x) + (r&1)]
+#pragma unroll 4
   for (int t = threadIdx.x; t < 2 * G::W * N; t += G::kThreads) {
     const int r = t / N, x = t - r * N, y = y0 + r;
     float acc = 0.f;
-    if (y < a.ny)
-      for (int j = 0; j < a.nph; ++j) {
-        const float v = __fsub_rn(__ldg(psf + j * nxy + (size_t)y * N + x), __ldg(a.bg + z * a.nph + j));
-        acc = a.nph == 1 ? v : __fadd_rn(acc, __fmul_rn(v, a.m[b * a.nph + j]));
-      }
+    if (y < a.ny) {
+      float v[kMoMaxPhases];
+#pragma unroll
+      for (int j = 0; j < kMoMaxPhases; ++j) v[j] = j < a.nph ? __ldg(psf + j * nxy + (size_t)y * N + x) : 0.f;
+#pragma unroll
+      for (int j = 0; j < kMoMaxPhases; ++j)
+        if (j < a.nph) {
+          v[j] = __fsub_rn(v[j], __ldg(a.bg + z * a.nph + j));
+          acc = a.nph == 1 ? v[j] : __fadd_rn(acc, __fmul_rn(v[j], a.m[b * a.nph + j]));
+        }
+    }
     smr[2 * ((r >> 1) * N + x) + (r & 1)] = acc;
   }
   __syncthreads();

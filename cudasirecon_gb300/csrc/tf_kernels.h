@@ -16,12 +16,13 @@ struct AsmX2Launch {
   bool real;
 };
 
+constexpr int kMoMaxPhases = 9;
 // makeotf's band separation and x half of the transform of every band
 struct MoRowsArgs {
   const float* psf;  // [nz * nph][ny][n], phase fastest
   const float* bg;   // [nz * nph]
   int ny, nz, nph;
-  float m[kMaxPhases * kMaxPhases];  // band = sum over phases of m[band * nph + phase] * section
+  float m[kMoMaxPhases * kMoMaxPhases];  // band = sum over phases of m[band * nph + phase] * section
   float2* bands;     // [nph][nz][ny][n/2+1]
 };
 
