@@ -74,7 +74,7 @@ struct __align__(16) SearchCtl {
   int pad;
   float pos[kSB];            // the batch's positions along its line
   int j[kSB];                // their line steps
-  float2 kc[kSB];            // candidate vectors k1 * fitorder2
+  float4 khl[kSB];           // candidate vectors k1 * fitorder2 * dxy as float pairs: x hi, lo, y hi, lo
   double red[kSCmax][kSB][2];  // every CTA's partial XStarY (leader only)
   double res[kSB][2];        // the batch's XStarY (leader only)
 };
@@ -90,7 +90,7 @@ struct ClimbResult {
 // angle, 944-985 for the magnitude), replayed from the line's cached values;
 // x1 / amp1 carry over from the previous line as in the reference (declared
 // once, not reset between the two searches).
-__device__ ClimbResult run_climb(const SearchLine& L, float x1, float amp1)
+__device__ __forceinline__ ClimbResult run_climb(const SearchLine& L, float x1, float amp1)
 {
   ClimbResult r{0, 0, 0.f, x1, amp1};
   auto has = [&](int j) { return j >= -kSL && j <= kSL && L.have[j + kSL]; };
@@ -146,7 +146,6 @@ struct Controller {
   float k0mag, k0angle, delta_angle, delta_mag;
   float afit, mfit;    // fitted angle, magnitude
   float x1, amp1;      // carried between the lines
-  float sx;            // sum |X|^2 as float
   float angle_px;      // pixels of the overlaps' spectrum per step of angle, of magnitude
   float mag_px;
 };
@@ -163,7 +162,7 @@ __device__ __forceinline__ int line_start(float px_per_step)
 
 // position of step j from its neighbour towards the start (float-accumulated
 // like the reference's angle += deltaangle)
-__device__ void set_pos(SearchLine& L, int j, float base, float delta)
+__device__ __forceinline__ void set_pos(SearchLine& L, int j, float base, float delta)
 {
   if (j == 0) L.pos[kSL] = base;
   else if (j > 0) L.pos[j + kSL] = __fadd_rn(L.pos[j - 1 + kSL], delta);
@@ -172,7 +171,7 @@ __device__ void set_pos(SearchLine& L, int j, float base, float delta)
 
 // queue steps j, j+s, ... (or the start batch) of the current line; the
 // candidate vectors are formed by the leader's threads in parallel
-__device__ void request_line(const Controller& c, SearchLine& L, SearchCtl& ctl, int j)
+__device__ __forceinline__ void request_line(const Controller& c, SearchLine& L, SearchCtl& ctl, int j)
 {
   const bool ang = c.phase == kPhaseAngle;
   const float base = ang ? c.k0angle : c.k0mag;
@@ -185,11 +184,20 @@ __device__ void request_line(const Controller& c, SearchLine& L, SearchCtl& ctl,
     ctl.j[n] = jj;
     ++n;
   };
-  if (j == 0 || j == 1) {
+  if (j == 0) {  // a new line: nothing is evaluated yet
     const int n0 = line_start(ang ? c.angle_px : c.mag_px);
-    add(0);
-    for (int i = 1; i <= n0; ++i) add(i);
-    for (int i = 1; i <= n0; ++i) add(-i);
+    float up = base, dn = base;
+    L.pos[kSL] = ctl.pos[0] = base;
+    ctl.j[0] = 0;
+    for (int i = 1; i <= n0; ++i) {
+      up = __fadd_rn(up, delta);
+      dn = __fsub_rn(dn, delta);
+      L.pos[kSL + i] = ctl.pos[i] = up;
+      L.pos[kSL - i] = ctl.pos[n0 + i] = dn;
+      ctl.j[i] = i;
+      ctl.j[n0 + i] = -i;
+    }
+    n = 2 * n0 + 1;
   } else {
     const int s = j > 0 ? 1 : -1;
     for (int i = 0; i < kSLineK; ++i) add(j + s * i);
@@ -199,10 +207,10 @@ __device__ void request_line(const Controller& c, SearchLine& L, SearchCtl& ctl,
   ctl.nbatch = n;
 }
 
-// Consume the finished batch, advance the search, queue the next batch (or
-// none).  Runs on one thread; lines[0] is the angle line, lines[1] the
+// Advance the search over the finished batch (its values are in the line),
+// queue the next batch (or none).  Runs on one thread; lines[0] is the angle line, lines[1] the
 // magnitude line.
-__device__ void control(Controller& c, SearchLine* lines, SearchCtl& ctl, const K0SearchArgs& a, int dir)
+__device__ __forceinline__ void control(Controller& c, SearchLine* lines, SearchCtl& ctl, const K0SearchArgs& a, int dir)
 {
   const int nb = ctl.nbatch;
   if (c.phase == kPhaseFinal && nb > 0) {
@@ -216,15 +224,6 @@ __device__ void control(Controller& c, SearchLine* lines, SearchCtl& ctl, const 
     c.phase = kPhaseDone;
     ctl.nbatch = 0;
     return;
-  }
-  if (nb > 0) {
-    SearchLine& L = lines[c.phase == kPhaseAngle ? 0 : 1];
-    for (int i = 0; i < nb; ++i) {
-      const float mx = __fdiv_rn(__double2float_rn(ctl.res[i][0]), c.sx);
-      const float my = __fdiv_rn(__double2float_rn(ctl.res[i][1]), c.sx);
-      L.val[ctl.j[i] + kSL] = __fadd_rn(__fmul_rn(mx, mx), __fmul_rn(my, my));
-      L.have[ctl.j[i] + kSL] = 1;
-    }
   }
   ctl.nbatch = 0;
   while (c.phase == kPhaseAngle || c.phase == kPhaseMag) {
@@ -273,113 +272,154 @@ __device__ __forceinline__ float2 phase_factor(int x, int n, float hi, float lo)
 }
 
 // XStarY partial sums of CC candidates over this CTA's tile: per row the x
-// sum with the x phase factors, times the row's y factor; two rows per pass
-// share the x factors.  acc: per-thread sums.
+// sum with the x phase factors, times the row's y factor; kRows rows per pass
+// share the x factors (with two, their shared-memory reads took as long as the
+// FMAs), and the next loads of P are in flight meanwhile.  acc: per-thread sums.
+constexpr int kRows = 4;
+__device__ __forceinline__ unsigned long long pack2(float x, float y)
+{
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v)
+{
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
 template <int CC>
 __device__ __forceinline__ void tile_sums(const float2* __restrict__ pmap, int nx, const float2* ex, const float2* ey,
-                                          int tw, int th, int x0, int y0, int warp, int lane, float2 (&acc)[CC])
+                                          int tw, int th, int tp, int warp, int lane, float2 (&acc)[CC])
 {
 #pragma unroll
   for (int k = 0; k < CC; ++k) acc[k] = make_float2(0.f, 0.f);
-  const int y1 = y0 + th, x1 = x0 + tw;
-  for (int y = y0 + 2 * warp; y < y1; y += 2 * kSW) {
-    const bool two = y + 1 < y1;
-    float2 r0[CC], r1[CC];
+  // rows and columns past the tile repeat its last: their x factors are zero
+  // and their rows' sums are not taken
+  auto load = [&](int y, int x, float2 (&p)[kRows]) {
+    const float2* col = pmap + min(x, tw - 1);
 #pragma unroll
-    for (int k = 0; k < CC; ++k) r0[k] = r1[k] = make_float2(0.f, 0.f);
-    for (int x = x0 + lane; x < x1; x += 32) {
-      const float2 p0 = __ldg(pmap + (size_t)y * nx + x);
-      const float2 p1 = two ? __ldg(pmap + (size_t)(y + 1) * nx + x) : make_float2(0.f, 0.f);
+    for (int r = 0; r < kRows; ++r) p[r] = __ldg(col + min(y + r, th - 1) * nx);
+  };
+  float2 p[kRows];
+  load(kRows * warp, lane, p);
+  for (int y = kRows * warp; y < th; y += kRows * kSW) {
+    unsigned long long r[kRows][CC];  // (re, im): both parts of a product's sum in one paired FMA
+#pragma unroll
+    for (int q = 0; q < kRows; ++q)
+#pragma unroll
+      for (int k = 0; k < CC; ++k) r[q][k] = 0;
+    for (int x = 0; x < tw; x += 32) {
+      unsigned long long a[kRows], b[kRows];
+#pragma unroll
+      for (int q = 0; q < kRows; ++q) {
+        a[q] = pack2(p[q].x, p[q].x);
+        b[q] = pack2(-p[q].y, p[q].y);
+      }
+      if (x + 32 < tw) load(y, x + 32 + lane, p);
+      else load(y + kRows * kSW, lane, p);
+      const float2* el = ex + x + lane;
 #pragma unroll
       for (int k = 0; k < CC; ++k) {
-        const float2 e = ex[k * tw + (x - x0)];
-        r0[k].x = fmaf(p0.x, e.x, fmaf(-p0.y, e.y, r0[k].x));
-        r0[k].y = fmaf(p0.x, e.y, fmaf(p0.y, e.x, r0[k].y));
-        r1[k].x = fmaf(p1.x, e.x, fmaf(-p1.y, e.y, r1[k].x));
-        r1[k].y = fmaf(p1.x, e.y, fmaf(p1.y, e.x, r1[k].y));
+        const float2 e = el[k * tp];
+        const unsigned long long f = pack2(e.x, e.y), g = pack2(e.y, e.x);
+#pragma unroll
+        for (int q = 0; q < kRows; ++q) r[q][k] = fma2(a[q], f, fma2(b[q], g, r[q][k]));
       }
     }
 #pragma unroll
-    for (int k = 0; k < CC; ++k) {
-      const float2 e0 = ey[k * th + (y - y0)];
-      acc[k].x += r0[k].x * e0.x - r0[k].y * e0.y;
-      acc[k].y += r0[k].x * e0.y + r0[k].y * e0.x;
-      if (two) {
-        const float2 e1 = ey[k * th + (y + 1 - y0)];
-        acc[k].x += r1[k].x * e1.x - r1[k].y * e1.y;
-        acc[k].y += r1[k].x * e1.y + r1[k].y * e1.x;
+    for (int q = 0; q < kRows; ++q)
+      if (y + q < th) {
+#pragma unroll
+        for (int k = 0; k < CC; ++k) {
+          const float2 e = ey[k * th + y + q], v = unpack2(r[q][k]);
+          acc[k].x += v.x * e.x - v.y * e.y;
+          acc[k].y += v.x * e.y + v.y * e.x;
+        }
       }
-    }
   }
 }
 
+// (s, e) + (t, f), the rounding error of the sum kept
+__device__ __forceinline__ void pair_add(float& s, float& e, float t, float f)
+{
+  const float u = __fadd_rn(s, t), b = __fsub_rn(u, s);
+  e = __fadd_rn(__fadd_rn(e, f), __fadd_rn(__fsub_rn(s, __fsub_rn(u, b)), __fsub_rn(t, b)));
+  s = u;
+}
+
 // The CTA's sums of CC candidates into the leader's partial-sum table at
-// candidate c0: the threads' float sums transposed through shared memory, each
-// thread adding 2 CC values' share of kSeg neighbours as a float pair (the
-// rounding error of every addition kept, 48 bits; the FP64 adder runs at a
-// sixtyfourth of the FP32 rate here, and shuffling doubles through the warps
-// took 20 us a batch), the segments' totals in double.
+// candidate c0: the threads' float sums transposed through shared memory, a
+// warp per value, its lanes' shares and the lanes added as float pairs (48
+// bits; the FP64 adder runs at a sixtyfourth of the FP32 rate here, and chains
+// of it were the longest part of a batch on a small map).
 template <int CC>
-__device__ __forceinline__ void tile_reduce(const float2 (&acc)[CC], float* sacc, double* sseg, SearchCtl* lead,
-                                            int rank, int c0, int tid)
+__device__ __forceinline__ void tile_reduce(const float2 (&acc)[CC], float* sacc, SearchCtl* lead, int rank, int c0,
+                                            int n, int tid)
 {
   constexpr int V = 2 * CC, kPitch = V + 1;
-  constexpr int kSegs = kST / (V <= 8 ? 8 : V <= 16 ? 16 : 32), kSeg = kST / kSegs;  // V segment threads or more
+  static_assert(V <= kSW, "a warp per value");
+  __syncthreads();  // the last pass has read its sums
 #pragma unroll
   for (int k = 0; k < CC; ++k) {
     sacc[tid * kPitch + 2 * k] = acc[k].x;
     sacc[tid * kPitch + 2 * k + 1] = acc[k].y;
   }
   __syncthreads();
-  const int v = tid % (kST / kSegs), seg = tid / (kST / kSegs);
-  if (v < V) {
-    float s = 0.f, e = 0.f;
-    for (int i = 0; i < kSeg; ++i) {
-      const float x = sacc[(seg * kSeg + i) * kPitch + v];
-      const float t = __fadd_rn(s, x), bb = __fsub_rn(t, s);
-      e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(x, bb)));
-      s = t;
-    }
-    sseg[seg * V + v] = (double)s + (double)e;
+  const int v = tid >> 5, lane = tid & 31;
+  if (v >= 2 * n) return;
+  float x[kSW];
+#pragma unroll
+  for (int i = 0; i < kSW; ++i) x[i] = sacc[(i * 32 + lane) * kPitch + v];
+  float s = x[0], e = 0.f, t = x[1], f = 0.f;
+#pragma unroll
+  for (int i = 2; i < kSW; i += 2) {
+    pair_add(s, e, x[i], 0.f);
+    pair_add(t, f, x[i + 1], 0.f);
   }
-  __syncthreads();
-  if (tid < V) {
-    double t = 0.0;
-    for (int g = 0; g < kSegs; ++g) t += sseg[g * V + tid];
-    lead->red[rank][c0 + (tid >> 1)][tid & 1] = t;
-  }
+  pair_add(s, e, t, f);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    pair_add(s, e, __shfl_xor_sync(0xffffffffu, s, o), __shfl_xor_sync(0xffffffffu, e, o));
+  if (lane == 0) lead->red[rank][c0 + (v >> 1)][v & 1] = (double)s + (double)e;
 }
 
 template <int CC>
 __device__ void chunk(const float2* __restrict__ pmap, int nx, const float2* ex, const float2* ey, int tw, int th,
-                      int x0, int y0, float* sacc, double* sseg, SearchCtl* lead, int rank, int c0)
+                      int tp, float* sacc, SearchCtl* lead, int rank, int c0, int n)
 {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float2 acc[CC];
-  tile_sums<CC>(pmap, nx, ex, ey, tw, th, x0, y0, warp, lane, acc);
-  tile_reduce<CC>(acc, sacc, sseg, lead, rank, c0, tid);
+  tile_sums<CC>(pmap, nx, ex, ey, tw, th, tp, warp, lane, acc);
+  tile_reduce<CC>(acc, sacc, lead, rank, c0, n, tid);
 }
 
-// C: the most candidates one pass holds (phase tables in shared memory);
-// SC: CTAs per cluster.
-// Bound by latency: per batch two cluster barriers, the phase tables, one pass
-// of FMAs over P and the reduction.  Whole search of three directions, with 25
-// candidates a first batch, doubles shuffled through the warps and 8 CTAs,
-// and now: 128^2 131 -> 39 us, 512^2 215 -> 63, 1024 x 960 433 -> 132 us.
+// C: candidates of one pass; SC: CTAs per cluster; ntab candidates' phase
+// tables at a time.
+// Bound by latency on small maps (three batches, each two cluster barriers, the
+// control thread, the phase tables and the reduction), by the issue of the sums
+// on large ones: a pass of 8 candidates over 256 x 240 of P takes 39k cycles,
+// half of them issuing.  Search of three directions with 25 candidates a first
+// batch, doubles shuffled through the warps and 8 CTAs; with passes of up to 16
+// candidates over two rows, their tables and segment sums in double each; and
+// now: 128^2 131, 41, 33 us; 512^2 215, 63, 50; 1024 x 960 433, 127, 91 us.
 template <int C, int SC>
-__global__ void __launch_bounds__(kST, 1) k_k0_search(const __grid_constant__ K0SearchArgs a)
+__global__ void __launch_bounds__(kST, 1) k_k0_search(const __grid_constant__ K0SearchArgs a, int ntab)
 {
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned rank = cluster.block_rank();
   const int dir = blockIdx.x / SC;  // one cluster per direction
-  const float2* __restrict__ pmap = a.pmap[dir];
   __shared__ SearchCtl ctl;
   __shared__ SearchLine lines[2];
-  __shared__ double sseg[kST / 8 * 8];
-  __shared__ float2 kloc[kSB];
-  __shared__ float2 khl[kSB][2];  // k dxy of each candidate and axis as hi + lo floats
+  __shared__ float4 khl[kSB];
   __shared__ int nloc;
-  extern __shared__ float2 tab[];  // phase tables, then the reduction's transposed sums
+  extern __shared__ float2 tab[];  // phase tables [ntab][tp], [ntab][th], then the reduction's transposed sums
   SearchCtl* lead = cluster.map_shared_rank(&ctl, 0);
   const int tid = threadIdx.x;
   const int nx = a.nx, ny = a.ny;
@@ -388,91 +428,102 @@ __global__ void __launch_bounds__(kST, 1) k_k0_search(const __grid_constant__ K0
   const int tx = rank % TX, ty = rank / TX;
   const int x0 = tx * nx / TX, x1 = (tx + 1) * nx / TX;
   const int y0 = ty * ny / 4, y1 = (ty + 1) * ny / 4;
-  const int tw = x1 - x0, th = y1 - y0;
-  float* sacc = (float*)(tab + (size_t)C * ((nx + TX - 1) / TX + (ny + 3) / 4));
+  const int tw = x1 - x0, th = y1 - y0, tp = (tw + 31) & ~31;
+  float* sacc = (float*)(tab + (size_t)ntab * (((nx + TX - 1) / TX + 31 & ~31) + (ny + 3) / 4));
+  const float2* __restrict__ pmap = a.pmap[dir] + (size_t)y0 * nx + x0;
 
-  Controller c{};
+  __shared__ Controller held;  // the control thread's, between the batches
+  float sx = 1.f;  // sum |X|^2
   if (rank == 0) {
+    sx = __double2float_rn(a.sumxy[dir][0]);
     for (int i = tid; i < 2 * kSL + 1; i += kST) lines[0].have[i] = lines[1].have[i] = 0;
     if (tid == 0) {
+      Controller c{};
       const float2 k0 = *a.k0find[dir];
       c.phase = kPhaseAngle;
       c.k0mag = __fsqrt_rn(__fadd_rn(__fmul_rn(k0.x, k0.x), __fmul_rn(k0.y, k0.y)));
       c.k0angle = atan2f(k0.y, k0.x);
       c.delta_angle = a.delta_angle;
       c.delta_mag = a.delta_mag;
-      c.sx = __double2float_rn(a.sumxy[dir][0]);
       // the overlaps beat at k0 * fitorder2; one pixel is 1 / (n dxy)
       const float ext = (float)max(nx, ny) * a.dxy * (float)a.fitorder2;
       c.angle_px = c.k0mag * a.delta_angle * ext;
       c.mag_px = a.delta_mag * ext;
       ctl.nbatch = 0;
+      held = c;
     }
   }
   const float fac = (float)a.fitorder2;
   int it = 0;
   for (; it < kSMaxBatches; ++it) {
     if (rank == 0) {
-      __syncthreads();  // the previous batch's sums are in ctl.res; the line caches are clear
+      __syncthreads();  // the line has the previous batch's values; the line caches are clear
       if (tid == 0) {
+        Controller c = held;
         control(c, lines, ctl, a, dir);
         c.ncand += ctl.nbatch;
+        held = c;
       }
       __syncthreads();
-      // the candidate vectors (getmodamp: k1 = mag (cosf, sinf)(angle), times fitorder2 - fitorder1)
+      // the candidate vectors (getmodamp: k1 = mag (cosf, sinf)(angle), times
+      // fitorder2 - fitorder1) and, once for all CTAs, their double products
+      // with the pixel size (FP64 is slow on this GPU)
       if (tid < ctl.nbatch) {
         const float2 k1 = ctl.vary_angle ? polar_rn(ctl.fixed, ctl.pos[tid]) : polar_rn(ctl.pos[tid], ctl.fixed);
-        ctl.kc[tid] = make_float2(__fmul_rn(k1.x, fac), __fmul_rn(k1.y, fac));
+        const double kx = (double)__fmul_rn(k1.x, fac) * (double)a.dxy;
+        const double ky = (double)__fmul_rn(k1.y, fac) * (double)a.dxy;
+        const float hx = (float)kx, hy = (float)ky;
+        ctl.khl[tid] = make_float4(hx, (float)(kx - (double)hx), hy, (float)(ky - (double)hy));
       }
     }
     cluster.sync();  // the batch (or the end) is visible to every CTA
     if (tid == 0) nloc = lead->nbatch;
-    if (tid < kSB) kloc[tid] = lead->kc[tid];
+    if (tid < kSB) khl[tid] = lead->khl[tid];
     __syncthreads();
     const int nb = nloc;
     if (nb == 0) break;
-    if (tid < 2 * kSB) khl[tid >> 1][tid & 1] = make_float2(0.f, 0.f);  // padding of the last pass
-    __syncthreads();
-    if (tid < 2 * nb) {  // the double products once per candidate and axis (FP64 is slow on this GPU)
-      const float2 kk = kloc[tid >> 1];
-      const double kd = (double)((tid & 1) ? kk.y : kk.x) * (double)a.dxy;
-      const float hi = (float)kd;
-      khl[tid >> 1][tid & 1] = make_float2(hi, (float)(kd - (double)hi));
-    }
-    __syncthreads();
-    for (int c0 = 0; c0 < nb;) {
-      // the smallest compiled pass that takes what is left (padded with zero
-      // vectors, whose sums nothing reads)
-      const int rem = nb - c0;
-      const int cc = rem == 1 ? 1 : rem <= 4 ? 4 : rem <= 8 || C < 12 ? (C < 8 ? 4 : 8) : rem <= 12 || C < 16 ? 12 : 16;
-      float2* ex = tab;                    // [cc][tw]
-      float2* ey = tab + (size_t)cc * tw;  // [cc][th]
-      for (int e = tid; e < cc * (tw + th); e += kST) {
-        const int k = e / (tw + th), r = e - k * (tw + th);
-        const bool isx = r < tw;
-        const float2 hl = khl[c0 + k][isx ? 0 : 1];
-        if (isx) ex[k * tw + r] = phase_factor(x0 + r, nx, hl.x, hl.y);
-        else ey[k * th + (r - tw)] = phase_factor(y0 + (r - tw), ny, hl.x, hl.y);
+    for (int g0 = 0; g0 < nb; g0 += ntab) {
+      const int ng = min(ntab, nb - g0);
+      const int np = ng == 1 ? 1 : (ng + C - 1) / C * C;  // whole passes: the padding's sums are not kept
+      float2* ex = tab;                    // [np][tp]
+      float2* ey = tab + (size_t)np * tp;  // [np][th]
+      if (g0 > 0) __syncthreads();         // the tables are read
+      for (int e = tid; e < np * (tp + th); e += kST) {
+        const int k = e / (tp + th), r = e - k * (tp + th);
+        const float4 kk = khl[min(g0 + k, nb - 1)];
+        if (r >= tp) ey[k * th + (r - tp)] = phase_factor(y0 + (r - tp), ny, kk.z, kk.w);
+        else ex[k * tp + r] = r < tw ? phase_factor(x0 + r, nx, kk.x, kk.y) : make_float2(0.f, 0.f);
       }
       __syncthreads();
-      if (C >= 16 && cc == 16) chunk<C >= 16 ? 16 : 1>(pmap, nx, ex, ey, tw, th, x0, y0, sacc, sseg, lead, rank, c0);
-      else if (C >= 12 && cc == 12) chunk<C >= 12 ? 12 : 1>(pmap, nx, ex, ey, tw, th, x0, y0, sacc, sseg, lead, rank, c0);
-      else if (C >= 8 && cc == 8) chunk<C >= 8 ? 8 : 1>(pmap, nx, ex, ey, tw, th, x0, y0, sacc, sseg, lead, rank, c0);
-      else if (cc == 4) chunk<4>(pmap, nx, ex, ey, tw, th, x0, y0, sacc, sseg, lead, rank, c0);
-      else chunk<1>(pmap, nx, ex, ey, tw, th, x0, y0, sacc, sseg, lead, rank, c0);
-      __syncthreads();  // tables and sums are reused by the next pass
-      c0 += cc;
+      for (int c0 = 0; c0 < ng; c0 += C) {
+        const int n = min(C, ng - c0);
+        if (n > 1) chunk<C>(pmap, nx, ex + c0 * tp, ey + c0 * th, tw, th, tp, sacc, lead, rank, g0 + c0, n);
+        else chunk<1>(pmap, nx, ex + c0 * tp, ey + c0 * th, tw, th, tp, sacc, lead, rank, g0 + c0, n);
+      }
     }
     cluster.sync();  // every CTA's partial sums are in the leader
-    if (rank == 0 && tid < 2 * nb) {
-      double s = 0.0;
-      for (int r = 0; r < SC; ++r) s += ctl.red[r][tid >> 1][tid & 1];
-      ctl.res[tid >> 1][tid & 1] = s;
+    if (rank == 0 && tid < 2 * kSB) {
+      double v[SC];
+#pragma unroll
+      for (int r = 0; r < SC; ++r) v[r] = tid < 2 * nb ? ctl.red[r][tid >> 1][tid & 1] : 0.0;
+#pragma unroll
+      for (int h = SC / 2; h > 0; h >>= 1)
+#pragma unroll
+        for (int r = 0; r < h; ++r) v[r] += v[r + h];
+      if (tid < 2 * nb) ctl.res[tid >> 1][tid & 1] = v[0];
+      const float m = __fdiv_rn(__double2float_rn(v[0]), sx);
+      const float my = __shfl_down_sync(0xffffffffu, m, 1);
+      if (tid < 2 * nb && !(tid & 1)) {  // the step's |modamp|^2 (the final evaluation's place is not read)
+        SearchLine& L = lines[ctl.vary_angle ? 0 : 1];
+        L.val[ctl.j[tid >> 1] + kSL] = __fadd_rn(__fmul_rn(m, m), __fmul_rn(my, my));
+        L.have[ctl.j[tid >> 1] + kSL] = 1;
+      }
     }
   }
   // no CTA leaves while another may still read the leader's shared memory
   cluster.sync();
   if (rank == 0 && tid == 0) {
+    Controller c = held;
     if (c.phase != kPhaseDone && c.status == 0) c.status = 2;  // batch limit reached
     atomicAdd(a.info, c.ncand);
     if (c.status) atomicOr(a.info + 1, c.status);
@@ -486,19 +537,20 @@ __global__ void __launch_bounds__(kST, 1) k_k0_search(const __grid_constant__ K0
 // size, so only where the device can hold such a cluster
 static int search_ctas(int nx, int ny) { return (long long)nx * ny >= kSearchWide ? 16 : 8; }
 
-// dynamic shared memory of a search with C candidates per pass
-static size_t search_smem(int nx, int ny, int C, int sc)
+// Dynamic shared memory: ntab candidates' phase tables (x in whole warps) and a
+// pass's sums
+static size_t search_smem(int nx, int ny, int C, int ntab, int sc)
 {
-  const size_t tw = ((size_t)nx + sc / 4 - 1) / (sc / 4), th = ((size_t)ny + 3) / 4;
-  return C * (tw + th) * sizeof(float2) + (size_t)kST * (2 * C + 1) * sizeof(float);
+  const size_t tp = (((size_t)nx + sc / 4 - 1) / (sc / 4) + 31) / 32 * 32, th = ((size_t)ny + 3) / 4;
+  return ntab * (tp + th) * sizeof(float2) + (size_t)kST * (2 * C + 1) * sizeof(float);
 }
 
-// candidates per pass: the phase tables of a tile and the transposed sums
-// within 160 KB of shared memory
-static int search_chunk(int nx, int ny, int sc)
+// Candidates whose phase tables are built together, all of a batch where 164 KB
+// hold them; 0: not even four fit
+static int search_tables(int nx, int ny, int sc)
 {
-  for (int c : {16, 12, 8, 4})
-    if (search_smem(nx, ny, c, sc) <= 160 * 1024) return c;
+  for (int n : {32, 24, 16, 8, 4})
+    if (search_smem(nx, ny, n > 4 ? 8 : 4, n, sc) <= 164 * 1024) return n;
   return 0;
 }
 
@@ -508,14 +560,15 @@ static int search_chunk(int nx, int ny, int sc)
 // tile.
 bool k0_search_supported(int nx, int ny)
 {
-  return nx >= 64 && ny >= 8 && (long long)nx * ny <= 1024LL * 1024 && search_chunk(nx, ny, 8) > 0;
+  return nx >= 64 && ny >= 8 && (long long)nx * ny <= 1024LL * 1024 && search_tables(nx, ny, 8) > 0 &&
+         4 * (((size_t)nx + 1) / 2 + ((size_t)ny + 3) / 4) * sizeof(float2) + kST * 9 * sizeof(float) <= 160 * 1024;
 }
 
 int launch_k0_search(const K0SearchArgs& a, cudaStream_t s, long long* launches)
 {
   if (a.nx < 64 || a.ny < 8 || a.ndirs < 1 || a.ndirs > kMaxDirs) return -1;
-  auto go = [&](auto kern, int C, int sc) -> int {
-    const size_t smem = search_smem(a.nx, a.ny, C, sc);
+  auto go = [&](auto kern, int C, int ntab, int sc) -> int {
+    const size_t smem = search_smem(a.nx, a.ny, C, ntab, sc);
     // raised only (under a lock): handles of other shapes launch concurrently
     allow_dynamic_smem((const void*)kern, smem);
     cudaLaunchConfig_t cfg{};
@@ -540,18 +593,14 @@ int launch_k0_search(const K0SearchArgs& a, cudaStream_t s, long long* launches)
         return -2;
       }
     }
-    return (int)cudaLaunchKernelEx(&cfg, kern, a);
+    return (int)cudaLaunchKernelEx(&cfg, kern, a, ntab);
   };
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
   auto by_chunk = [&]<int SC>() {
-    switch (search_chunk(a.nx, a.ny, SC)) {
-      case 16: return go(k_k0_search<16, SC>, 16, SC);
-      case 12: return go(k_k0_search<12, SC>, 12, SC);
-      case 8: return go(k_k0_search<8, SC>, 8, SC);
-      case 4: return go(k_k0_search<4, SC>, 4, SC);
-      default: return -1;
-    }
+    const int ntab = search_tables(a.nx, a.ny, SC);
+    if (ntab >= 8) return go(k_k0_search<8, SC>, 8, ntab, SC);
+    return ntab == 4 ? go(k_k0_search<4, SC>, 4, 4, SC) : -1;
   };
   int rc = -2;
   if (search_ctas(a.nx, a.ny) == 16) rc = by_chunk.template operator()<16>();
