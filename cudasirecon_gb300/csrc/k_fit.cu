@@ -142,65 +142,6 @@ __global__ void __launch_bounds__(kThreads) k_ovl_build_x(const __grid_constant_
   }
 }
 
-// Warp-level variant for the row lengths with a register configuration:
-// each warp owns 32/P consecutive overlap lines (line = 2 * row + ov), builds
-// their elements into a warp-private buffer, and each group of P lanes runs
-// its line's inverse x FFT in registers and stores it (no CTA barrier).
-template <int N>
-struct OvlLanes {
-  static constexpr int P = N == 1024 ? 32 : (N == 512 || N == 256 ? 16 : 0);
-};
-constexpr int kOvlWarps = 4;
-
-// Five CTAs per SM (at most 96 registers, no spills): the kernel is bound by
-// its resident warps (per 512^2 x 48 volume: 0.64 ms with three CTAs, 0.55
-// with four, 0.51 with five, 0.54 with six and spills)
-template <int N>
-__global__ void __launch_bounds__(kOvlWarps * 32, 5) k_ovl_build_xw(const __grid_constant__ OverlapArgs a, const float2* __restrict__ twr)
-{
-  constexpr int P = OvlLanes<N>::P, E = N / P, G = 32 / P;
-  constexpr int XB = (P + 1) * E + 1;
-  constexpr int LB = N > XB ? N : XB;  // line buffer, reused as the exchange buffer
-  __shared__ float2 lines[kOvlWarps][G][LB];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane / P, p = lane - g * P;
-  const int ny = a.ny, nzb = 2 * a.zdc + 1;
-  const int nlines = 2 * nzb * ny;
-  const int l0 = (blockIdx.x * kOvlWarps + warp) * G;
-  // build the warp's G lines (all 32 lanes, consecutive j); the kz part of
-  // the OTF lookups is the same along a line
-  const float rdk = 1.f / a.otf.dkrotf;
-  const OvlItem& it = a.item[blockIdx.z];
-  const float2 ks = ovl_shift(it);
-#pragma unroll
-  for (int gl = 0; gl < G; ++gl) {
-    const int L = l0 + gl;
-    if (L >= nlines) {
-      for (int j = lane; j < N; j += 32) lines[warp][gl][j] = make_float2(0.f, 0.f);
-      continue;
-    }
-    const int row = L >> 1, ov = L & 1;
-    const int zb = row / ny, i = row - zb * ny;
-    const OtfKz kzi = otf_kz(a.otf, zb - a.zdc);
-    for (int j = lane; j < N; j += 32) lines[warp][gl][j] = ovl_value(a, it, ks, ov, zb, i, j, kzi, rdk);
-  }
-  __syncwarp();
-  float2 v[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) v[e] = lines[warp][g][p + P * e];
-  __syncwarp();  // every lane has its values before the buffer becomes the exchange
-  reg_line<N, P, +1>(v, p, lines[warp][g], twr, true);
-  const int L = l0 + g;
-  if (L < nlines) {
-    const int row = L >> 1, ov = L & 1;
-    float2* dst = it.ovl + (size_t)ov * nzb * ny * N + (size_t)row * N;
-#pragma unroll
-    for (int m = 0; m < E / P; ++m)
-#pragma unroll
-      for (int k2 = 0; k2 < P; ++k2) dst[p + P * m + E * k2] = v[m * P + k2];
-  }
-}
-
 template <int NF>
 __global__ void __launch_bounds__(kThreads) k_ovl_y_accum(const __grid_constant__ OverlapArgs a, FFTPlan plan, int W, int planes_per_group,
                                                           int xoff)
@@ -260,8 +201,7 @@ __global__ void __launch_bounds__(kThreads) k_ovl_y_accum(const __grid_constant_
   }
 }
 
-// Four-step variant (col_fft.cuh layout) of k_ovl_y_accum for ny in
-// {256, 512}: per kz plane of the group, stage 1 transforms the 8 columns of
+// Four-step variant (col_fft.cuh layout) of k_ovl_y_accum for 512 rows: per kz plane of the group, stage 1 transforms the 8 columns of
 // both overlaps (half of the threads each, rows loaded straight from HBM),
 // stage 2 gives each thread one (column, k1) of both, and conj(X)Y, |X|^2,
 // |Y|^2 accumulate in registers over the planes.
@@ -293,13 +233,20 @@ __global__ void __launch_bounds__(kThreads, 2) k_ovl_y4(const __grid_constant__ 
   float2 acc[R2];
 #pragma unroll
   for (int k2 = 0; k2 < R2; ++k2) acc[k2] = make_float2(0.f, 0.f);
-  double sx = 0.0, sy = 0.0;
+  float sx = 0.f, ex = 0.f, sy = 0.f, ey = 0.f;  // float pairs: the FP64 adder has a sixtyfourth of the FP32 rate
+  unsigned live = 0;                             // the thread's rows with elements
+  if (c1 < nc) {
+    const float2 ks = ovl_shift(im);
+#pragma unroll
+    for (int e = 0; e < R1; ++e) live |= (ovl_row_dead(a, ks, ov1, j1 + R2 * e) ? 0u : 1u) << e;
+  }
   for (int zb = zb0; zb < zb1; ++zb) {
+    if (ovl_plane_dead(a, zb)) continue;
     {
       const float2* src = im.ovl + (size_t)ov1 * vol + (size_t)zb * ny * nx + c0 + c1;
       float2 v[R1];
 #pragma unroll
-      for (int e = 0; e < R1; ++e) v[e] = c1 < nc ? src[(size_t)(j1 + R2 * e) * nx] : make_float2(0.f, 0.f);
+      for (int e = 0; e < R1; ++e) v[e] = live >> e & 1 ? src[(size_t)(j1 + R2 * e) * nx] : make_float2(0.f, 0.f);
       reg_dft<R1, +1>(v);
 #pragma unroll
       for (int kk = 1; kk < R1; ++kk) {
@@ -330,8 +277,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_ovl_y4(const __grid_constant__ 
         py += cmag2(Y[k2]);
       }
       if (c2 < nc) {  // columns past nx are zero padding, not data
-        sx += (double)px;
-        sy += (double)py;
+        pair_sum(sx, ex, px);
+        pair_sum(sy, ey, py);
       }
     }
     __syncthreads();
@@ -341,8 +288,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_ovl_y4(const __grid_constant__ 
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2) dst[(size_t)(k1 + R1 * k2) * nx] = acc[k2];
   }
-  double tx = block_sum_d(sx, red);
-  double ty = block_sum_d(sy, red);
+  double tx = block_sum_d((double)sx + (double)ex, red);
+  double ty = block_sum_d((double)sy + (double)ey, red);
   if (threadIdx.x == 0) {
     int cta = blockIdx.y * gridDim.x + blockIdx.x;
     im.sums[2 * cta] = tx;
@@ -696,13 +643,21 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   if (!get_fft_plan(a.nx, &px) || !get_fft_plan(a.ny, &py)) return -1;
   const int nzb = 2 * a.zdc + 1, ni = a.nitems;
   if (ni < 1 || ni > kMaxOvlItems) return -1;
-  // 1024 rows: 1.25 ms a 1024^2 x 64 pair with the Stockham stages, 0.26 with
-  // the two-factor kernel
+  // Rows of 256, 512 and 1024 (whose register kernels these replaced: a line per
+  // half or whole warp, 0.131, 0.400 and 3.01 ms per 256^2 x 32, 512^2 x 48 and
+  // 1024^2 x 64 volume against 0.112, 0.353 and 2.17) take the two-factor kernel
+  // whatever the plan file says, as they took the register ones.
+  const bool reg_row = a.nx == 256 || a.nx == 512 || a.nx == 1024;
   TfPlan tx, ty;
   const TfKernels* kx =
-      a.otf.nxotf <= kOvlTabMax && fft_two_factor(kSiteOvlX, a.nx) ? tf_kernels(a.nx, &tx) : nullptr;
-  const TfKernels* ky = fft_two_factor(kSiteOvlY, a.ny) ? tf_kernels(a.ny, &ty) : nullptr;
+      a.otf.nxotf <= kOvlTabMax && (reg_row || fft_two_factor(kSiteOvlX, a.nx)) ? tf_kernels(a.nx, &tx) : nullptr;
+  // 512 rows keep the compiled column kernel (0.209 against 0.270 ms per
+  // 512^2 x 48 volume); 256 rows are as fast either way (0.078, 0.076), 1024
+  // took the Stockham stages (1.25 a pair of 1024^2 x 64 against 0.26)
+  const TfKernels* ky = a.ny == 256 || (a.ny != 512 && fft_two_factor(kSiteOvlY, a.ny)) ? tf_kernels(a.ny, &ty) : nullptr;
   // 1) build + x inverse FFT
+  // the Stockham y stage reads every row
+  a.skip_rows = !a.all_rows && (a.ny == 512 || ky);
   const int ldl = a.nx + 1;
   int rows = std::max(1, kMaxElems / (2 * a.nx));
   rows = std::min(rows, nzb * a.ny);
@@ -713,16 +668,7 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   const double ovlb = 2.0 * ni * nzb * a.ny * a.nx * sizeof(float2);
   const double bandplanes = (double)ni * nzb * a.ny * (a.nx / 2 + 1) * sizeof(float2);
   if (kt) kt->begin(s);
-  auto launch_w = [&]<int N>() {
-    constexpr int G = 32 / OvlLanes<N>::P;
-    const int nlines = 2 * nzb * a.ny;
-    const int per_cta = kOvlWarps * G;
-    k_ovl_build_xw<N><<<dim3((nlines + per_cta - 1) / per_cta, 1, ni), kOvlWarps * 32, 0, s>>>(a, px.twr);
-  };
-  if (a.nx == 512) launch_w.template operator()<512>();
-  else if (a.nx == 1024) launch_w.template operator()<1024>();
-  else if (a.nx == 256) launch_w.template operator()<256>();
-  else if (kx) {
+  if (kx) {
     const int rc = kx->ovl_x(a, tx, s);
     if (rc != 0) return rc;
   } else
@@ -742,7 +688,7 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   const size_t fsm = fft_stage_smem(a.ny, 2 * W, tile, threads);
   const int xoff = (int)(fsm / sizeof(float2));
   size_t sm2 = fsm + (size_t)a.ny * W * sizeof(float2);
-  if (a.ny == 512 || a.ny == 256) {
+  if (a.ny == 512) {
     // 8 columns per CTA; plane groups so that the grid covers the GPU
     tiles = (a.nx + 7) / 8;
     groups = std::max(1, std::min(nzb, (4 * 152 + ni * tiles - 1) / (ni * tiles)));
@@ -761,7 +707,6 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
     k_ovl_y4<N, R1><<<dim3(tiles, groups, ni), kThreads, bytes, s>>>(a, py.tw, ppg);
   };
   if (a.ny == 512) go4.template operator()<512, 32>();
-  else if (a.ny == 256) go4.template operator()<256, 16>();
   else if (ky) {
     const int rc = ky->ovl_y(a, ty, ppg, groups, s);
     if (rc != 0) return rc;

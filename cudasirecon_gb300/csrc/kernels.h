@@ -142,6 +142,8 @@ struct OverlapArgs {
   float r2_le, r2_lt, m_le, m_f;
   int zdc;              // planes -zdc..zdc are built
   int nokz0;
+  int all_rows;         // every row of ovl is needed (the debug dump)
+  int skip_rows;        // rows without support are neither stored nor read (set by launch_overlaps)
   OTFView otf;          // geometry of the OTF tables (the pointers are the items')
 };
 int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches);
@@ -154,6 +156,22 @@ __device__ __forceinline__ float2 ovl_shift(const OvlItem& it)
   if (it.kdev == nullptr) return make_float2(it.kx, it.ky);
   const float2 k = *it.kdev;
   return make_float2(__fmul_rn(k.x, it.kfac), __fmul_rn(k.y, it.kfac));
+}
+// Row i of overlap ov has no element: the row, or the partner's (overlap 0 at
+// k - shift, overlap 1 at k + shift), lies outside the support circle.
+// Separately rounded and with a margin, so that the kernels that leave such
+// rows out and those that do not read them agree, whatever they contract.
+__device__ __forceinline__ bool ovl_row_dead(const OverlapArgs& a, float2 ks, int ov, int i)
+{
+  const float y1 = __fmul_rn((float)(i > a.ny / 2 ? i - a.ny : i), a.dky);
+  const float y2 = ov == 0 ? __fsub_rn(y1, ks.y) : __fadd_rn(y1, ks.y);
+  const float cut = __fmul_rn(a.r2_le, 1.00001f);
+  return a.skip_rows && (__fmul_rn(y1, y1) > cut || __fmul_rn(y2, y2) > cut);
+}
+// plane zb has no element
+__device__ __forceinline__ bool ovl_plane_dead(const OverlapArgs& a, int zb)
+{
+  return a.skip_rows && a.nokz0 && zb == a.zdc;
 }
 #endif
 

@@ -870,6 +870,7 @@ OverlapArgs SIM_Reconstructor::overlap_args(int o2, float k0x, float k0y) const
   a.order0_2_factor = order0_2_factor;
   a.zdc = p.bBessel ? overlap_zdc_bessel(o2, k0x, k0y) : zdc_ovl_;
   a.nokz0 = effective_nokz0(opt);
+  a.all_rows = p.bSaveOverlaps;
   a.otf.nzotf = p.nzotf;
   a.otf.nxotf = p.nxotf;
   a.otf.dkrotf = p.dkrotf;

@@ -124,6 +124,14 @@ __device__ __forceinline__ float2 otf_lookup_rr(const float2* __restrict__ otf, 
 
 __device__ __forceinline__ float cmag2(float2 a) { return a.x * a.x + a.y * a.y; }
 
+// x onto the float pair (s, e): the rounding error of every addition is kept
+__device__ __forceinline__ void pair_sum(float& s, float& e, float x)
+{
+  const float h = __fadd_rn(s, x), w = __fsub_rn(h, s);
+  e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(h, w)), __fsub_rn(x, w)));
+  s = h;
+}
+
 // Block-wide sum of a double (all threads must call).  Result valid in thread 0.
 __device__ __forceinline__ double block_sum_d(double v, double* scratch /* >= 32 */)
 {

@@ -364,8 +364,9 @@ __device__ __forceinline__ float2 ovl_element(const OverlapArgs& a, const OvlIte
 
 // W lines (line = 2 * row + overlap) of one kz plane per CTA.  Bound by the
 // elements' issue and latency; per kz plane the two radial OTF tables replace
-// 16 scattered loads and the kz interpolation of every element.  Nine builds
-// of 640 x 384 x 30: 1.40 -> 0.48 ms (2.2 TB/s of the overlap rows).
+// 16 scattered loads and the kz interpolation of every element; rows outside
+// the support are left out.  Nine builds of 640 x 384 x 30: 1.40 ms by the
+// Stockham stages, 0.37 with every row, 0.33 now.
 template <int R1, int R2>
 __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
     k_tf_ovl_x(const __grid_constant__ OverlapArgs a, const float2* __restrict__ tw)
@@ -381,6 +382,9 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
   const OvlItem& it = a.item[blockIdx.z];
   const float2 ks = ovl_shift(it);
   const bool empty = z0 == 0 && a.nokz0;
+  // lines without an element are left out
+  auto dead = [&](int l) { return ovl_plane_dead(a, zb) || ovl_row_dead(a, ks, (L0 + l) & 1, (L0 + l) >> 1); };
+  if (!__syncthreads_or(threadIdx.x < nl && !dead(threadIdx.x))) return;
   if (!empty) ovl_build_tab(a, it, otf_kz(a.otf, z0), tab);
   __syncthreads();
   for (int t = threadIdx.x; t < G::W * N; t += G::kThreads) {
@@ -393,7 +397,7 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
   float2 u[R2];
   tf_row_lines<R1, R2, +1>(sm, tw, u);
   const int l = threadIdx.x / R1, k1 = threadIdx.x - l * R1;
-  if (l < nl) {
+  if (l < nl && !dead(l)) {
     const int L = L0 + l;
     float2* dst = it.ovl + ((size_t)(L & 1) * nzb + zb) * ny * N + (size_t)(L >> 1) * N + k1;
 #pragma unroll
@@ -405,8 +409,9 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
 // fastest, overlap, j or k1).  In the second stage the threads of a column's
 // two overlaps sit W lanes apart; they exchange half of their values by
 // shuffles, so each sums conj(X) Y of every other k2 in registers over the
-// planes and neither holds both overlaps.  Nine pairs of 1024^2 x 64: 11.2 ->
-// 2.34 ms (2.1 TB/s of the overlap rows), of 640 x 384 x 30 1.29 -> 0.37 ms.
+// planes and neither holds both overlaps.  Nine pairs of 1024^2 x 64: 11.2 ms
+// by the Stockham stages, 2.2 reading every row and with FP64 sums, 1.92 now
+// (2.5 TB/s of the overlap rows); of 640 x 384 x 30 1.29, 0.30, 0.26 ms.
 template <int R1, int R2>
 struct TfOvlY {
   static constexpr int N = R1 * R2;
@@ -439,13 +444,20 @@ __global__ void __launch_bounds__(TfOvlY<R1, R2>::kThreads, TfOvlY<R1, R2>::kCta
   float2 acc[G::kHalf];
 #pragma unroll
   for (int i = 0; i < G::kHalf; ++i) acc[i] = make_float2(0.f, 0.f);
-  double sq = 0.0;
+  float sq = 0.f, sqe = 0.f;  // a float pair: the FP64 adder has a sixtyfourth of the FP32 rate
+  unsigned live = 0;          // the thread's rows with elements
+  if (in && q < R2) {
+    const float2 ks = ovl_shift(it);
+#pragma unroll
+    for (int e = 0; e < R1; ++e) live |= (ovl_row_dead(a, ks, ov, q + R2 * e) ? 0u : 1u) << e;
+  }
   for (int zb = zb0; zb < zb1; ++zb) {
+    if (ovl_plane_dead(a, zb)) continue;
     if (q < R2) {
       const float2* src = src0 + (size_t)zb * N * nx;
       float2 v[R1];
 #pragma unroll
-      for (int e = 0; e < R1; ++e) v[e] = in ? src[(size_t)(q + R2 * e) * nx] : make_float2(0.f, 0.f);
+      for (int e = 0; e < R1; ++e) v[e] = live >> e & 1 ? src[(size_t)(q + R2 * e) * nx] : make_float2(0.f, 0.f);
       reg_dft<R1, +1>(v);
       tf_twiddle<R1, +1>(v, tw, R2, q);
 #pragma unroll
@@ -460,7 +472,7 @@ __global__ void __launch_bounds__(TfOvlY<R1, R2>::kThreads, TfOvlY<R1, R2>::kCta
     float ps = 0.f;
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2) ps += cmag2(u[k2]);
-    sq += (double)ps;
+    pair_sum(sq, sqe, ps);
 #pragma unroll
     for (int i = 0; i < G::kHalf; ++i) {
       // overlap 0's thread keeps k2 = 2 i, overlap 1's keeps 2 i + 1
@@ -480,8 +492,9 @@ __global__ void __launch_bounds__(TfOvlY<R1, R2>::kThreads, TfOvlY<R1, R2>::kCta
     for (int i = 0; i < G::kHalf; ++i)
       if (2 * i + ov < R2) dst[(size_t)(q + R1 * (2 * i + ov)) * nx] = acc[i];
   }
-  const double tx = block_sum_d(ov ? 0.0 : sq, red);
-  const double ty = block_sum_d(ov ? sq : 0.0, red);
+  const double st = (double)sq + (double)sqe;
+  const double tx = block_sum_d(ov ? 0.0 : st, red);
+  const double ty = block_sum_d(ov ? st : 0.0, red);
   if (threadIdx.x == 0) {
     const int cta = blockIdx.y * gridDim.x + blockIdx.x;
     it.sums[2 * cta] = tx;
