@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const S
   __shared__ FilterTerms terms;
   const Slot sl = slots[blockIdx.y];
   const int nx = a.nx, ny = a.ny, nz = a.nz, nxh = nx / 2 + 1;
-  const int c0 = blockIdx.x * W;
+  const int c0 = a.tx0 + blockIdx.x * W;
   const size_t plane = (size_t)ny * nxh;
   const int order = sl.order;
   const int d0 = sl.dir < 0 ? 0 : sl.dir;
@@ -380,6 +380,11 @@ __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const S
   const float2* bi = order == 0 ? nullptr : a.bands + ((size_t)d0 * a.nphases + 2 * order) * nz * plane;
   const size_t dstride = (size_t)a.nphases * nz * plane;  // next direction's band 0
   const int ylo = ny / 2 - 1;                              // ky in [-ylo, ny/2]
+  if (c0 < a.cx0 || c0 >= a.cx1) {  // no data: zeros for the x pass
+    for (int t = threadIdx.x; t < Y * W; t += blockDim.x)
+      if (c0 + t % W < nx) a.T[((size_t)blockIdx.y * Y + t / W) * nx + c0 + t % W] = make_float2(0.f, 0.f);
+    return;
+  }
   build_filter_tab(fa, fa.norders, sl.kz, tab);
   build_filter_terms(fa, fk, d0, order, sl.kz, c0 - (nx / 2 - 1), min(W, nx - c0), terms);
   FilterSlot fsl{br, bi, plane, dstride, nx, ny, nz, order, d0, sl.kz};
@@ -479,7 +484,7 @@ __global__ void __launch_bounds__(kXwWarps * 32, 2) k_asm_xw(AssembleArgs a, con
   auto prefetch = [&](int si) {
     if (act && si < ns) {
       const float2* trow = a.T + ((size_t)(s0 + si) * Y + yr) * nx;
-      for (int q = p; q < nx / 2; q += P) {
+      for (int q = a.tx0 / 2 + p; q < a.tx1 / 2; q += P) {
         const unsigned dst = (unsigned)__cvta_generic_to_shared(&rg[si & 1][2 * q]);
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(trow + 2 * q) : "memory");
       }
@@ -489,6 +494,8 @@ __global__ void __launch_bounds__(kXwWarps * 32, 2) k_asm_xw(AssembleArgs a, con
   float2 acc[E];
 #pragma unroll
   for (int i = 0; i < E; ++i) acc[i] = make_float2(0.f, 0.f);
+  for (int q = p; q < nx; q += P)  // the columns that are not stored stay zero in both entries
+    if (q < a.tx0 || q >= a.tx1) rg[0][q] = rg[1][q] = make_float2(0.f, 0.f);
   prefetch(0);
   for (int si = 0; si < ns; ++si) {  // same trip count for every lane of the warp
     const Slot sl = slots[s0 + si];
@@ -897,6 +904,25 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
   const bool xw = a.X == 2 * a.nx && (a.X == 1024 || a.X == 512 || a.X == 256);
   const bool x_real = a.Z == 1 && np_out == 1 && (xw || use_x2(a));
   if (a.X > kAccPerThread * kThreads && !use_x2(a)) return -3;
+  // With the filter in the load, columns beyond the lateral support
+  // (filtered_rows' sqrtf(kx^2 + ky^2) > rdistcutoff, whatever ky) are zero, an
+  // eighth of them at 1.42 NA, 528 nm and 80 nm pixels: no filter and no
+  // transform.  k_asm_xw does not read them either; in k_asm_x2 a test per
+  // load cost more than the loads (0.50 against 0.46 ms per 640 x 384 x 30), so
+  // for it and the Stockham stages they are stored as zeros.
+  AssembleArgs ac = a;
+  ac.cx0 = 0;
+  ac.cx1 = nx;
+  if (filt) {
+    auto dead = [&](int c) { return std::fabs((float)(c - (nx / 2 - 1)) * filt->dkx) > filt->rdistcutoff; };
+    int lo = 0, hi = nx;
+    while (lo < hi - 1 && dead(lo)) ++lo;
+    while (hi > lo + 1 && dead(hi - 1)) --hi;
+    ac.cx0 = lo & ~7;
+    ac.cx1 = std::min(nx, (hi + 7) & ~7);
+  }
+  ac.tx0 = xw ? ac.cx0 : 0;
+  ac.tx1 = xw ? ac.cx1 : nx;
   // process whole planes in groups whose slots fit in T
   size_t np = p0.size();
   size_t pi = 0;
@@ -909,7 +935,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
     int nsl = p0[pj - 1] + pn[pj - 1] - first;
     // T holds slots [first, first + nsl); shift the slot pointer so that
     // blockIdx.y indexes T from 0
-    AssembleArgs ay = a;
+    const AssembleArgs& ay = ac;
     KernelTimer* kt = kernel_timer();
     if (kt) kt->begin(s);
     if (use_y2(a)) {
@@ -921,7 +947,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
       auto go = [&]<int YN>() {
         const size_t bytes = ColFft<YN, colfft_r1(YN), 8>::kSmemElems * sizeof(float2) + tabb;
         allow_dynamic_smem((const void*)k_asm_y4f<YN>, bytes);
-        k_asm_y4f<YN><<<dim3((nx + 7) / 8, nsl), kThreads, bytes, s>>>(ay, d_slots + first, py.tw, *filt, fk);
+        k_asm_y4f<YN><<<dim3((ac.tx1 - ac.tx0 + 7) / 8, nsl), kThreads, bytes, s>>>(ay, d_slots + first, py.tw, *filt, fk);
       };
       if (a.Y == 1024) go.template operator()<1024>();
       else if (a.Y == 512) go.template operator()<512>();
@@ -948,7 +974,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
       kt->end(filt ? "k_asm_y_filter" : "k_asm_y", s, rd + (double)nsl * per_slot * sizeof(float2));
     }
     // k_asm_x reads T[(slot - first)]: pass a shifted T base
-    AssembleArgs ax = a;
+    AssembleArgs ax = ac;
     ax.T = a.T - (size_t)first * per_slot;
     if (kt) kt->begin(s);
     auto launch_xw = [&]<int XN>() {

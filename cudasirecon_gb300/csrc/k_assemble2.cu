@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(kThreads, MR <= 16 ? 4 : 3) k_asm_y2(AssembleA
   extern __shared__ __align__(16) float2 sm[];
   const Slot sl = slots[blockIdx.y];
   const int nx = a.nx, ny = a.ny, nz = a.nz, nxh = nx / 2 + 1;
-  const int W = 1 << lw, c0 = blockIdx.x << lw;
+  const int W = 1 << lw, c0 = a.tx0 + (blockIdx.x << lw);
   const int R1 = pl.r1, R2 = pl.r2;
   const int ld = (R2 | 1) << lw;  // k1 pitch of the exchange: odd multiple of W, conflict-free reads
   const size_t plane = (size_t)ny * nxh;
@@ -55,6 +55,13 @@ __global__ void __launch_bounds__(kThreads, MR <= 16 ? 4 : 3) k_asm_y2(AssembleA
   // the row-major values, then the exchange of both parities over them
   float4* tab = (float4*)(sm + ((2 * R1 * ld + 1) & ~1));  // [2][no][nxotf]
   if constexpr (FILT) {
+    if (c0 < a.cx0 || c0 >= a.cx1) {  // no data: zeros for the x pass
+      for (int t = threadIdx.x; t < a.Y << lw; t += kThreads) {
+        const int c = c0 + (t & (W - 1));
+        if (c < nx) a.T[((size_t)blockIdx.y * a.Y + (t >> lw)) * nx + c] = make_float2(0.f, 0.f);
+      }
+      return;
+    }
     __shared__ FilterTerms terms;
     build_filter_tab(fa, no, sl.kz, tab);
     build_filter_terms(fa, fk, d0, order, sl.kz, c0 - (nx / 2 - 1), min(W, nx - c0), terms);
@@ -175,7 +182,7 @@ int launch_asm_y2(const AssembleArgs& a, const void* d_slots, int nslots, const 
   const size_t elems = (2 * pl.r1 * ld + 1) & ~(size_t)1;
   const size_t tabb = filt ? 2 * (size_t)filt->norders * filt->otf.nxotf * sizeof(float4) : 0;
   const size_t bytes = elems * sizeof(float2) + tabb;
-  const dim3 g((a.nx + (1 << lw) - 1) >> lw, nslots);
+  const dim3 g((a.tx1 - a.tx0 + (1 << lw) - 1) >> lw, nslots);
   const Slot* slots = (const Slot*)d_slots;
   auto go = [&]<bool FILT>() {
     const FilterArgs fa = filt ? *filt : FilterArgs{};

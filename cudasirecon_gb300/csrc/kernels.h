@@ -325,6 +325,9 @@ struct AssembleArgs {
   const float2* ey;     // [ndirs*norders][Y]
   float2* T;            // scratch: [maxslots][Y][nx]
   size_t tcap;          // capacity of T in complex elements
+  // set by the launch: columns of T with data (cx0 a multiple of 8, cx1 one or
+  // nx; the others are zero) and the columns of T that are stored and read
+  int cx0, cx1, tx0, tx1;
   float2* S;            // [Z][Y][X]
   float* out;           // [Z][Y][X]
   void* tables;         // device slot tables (assemble_tables_bytes), uploaded by assemble_tables_upload
