@@ -355,7 +355,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_asm_y4(AssembleArgs a, const Sl
 // filter (for kz and, for order 0, -kz) follow the transform buffer.
 // Three CTAs per SM (at most 80 registers): the filter phase needs the warps
 // more than the transform stages need registers (1.61 -> 1.31 ms per
-// 512^2 x 48 volume against two CTAs per SM).
+// 512^2 x 48 volume against two CTAs per SM).  Bound by the filter's issue and
+// its instruction fetch: 0.99 ms there with pairs of pixels, per-CTA term lists
+// and the columns beyond the support left out.
 template <int Y>
 __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const Slot* __restrict__ slots,
                                                      const float2* __restrict__ tw,
@@ -782,7 +784,7 @@ int launch_filter(const FilterArgs& a, cudaStream_t s, long long* launches)
 namespace {
 // Doubled grids take the half-length transforms of k_assemble2.cu, except
 // where a compiled doubled-length kernel is the faster one: per 512^2 x 48
-// volume the y pass takes 1.31 ms (k_asm_y4f) against 1.45, the x pass
+// volume the y pass took 1.31 ms (k_asm_y4f; now 0.99) against 1.45, the x pass
 // 0.56 ms (k_asm_xw) against 0.87; per 256^2 x 32 volume 0.254 / 0.256 and
 // 0.096 / 0.102 ms
 bool use_y2(const AssembleArgs& a) { return !colfft_r1(a.Y) && asm_y2_supported(a); }

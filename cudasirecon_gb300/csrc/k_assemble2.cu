@@ -30,9 +30,9 @@ constexpr int kThreads = 256;
 // fit in the CTA, else 4 (a 32-byte sector of a row of T).
 // Bound by the filter's issue slots and latency.  Filter + y transform per
 // volume, before (k_filter and the Stockham stages) and now: 1024^2 x 64
-// 25.3 -> 7.5 ms, 640 x 384 x 30 2.87 -> 0.89 ms, 1024 x 960 0.293 -> 0.080 ms.
+// 25.3 -> 6.2 ms, 640 x 384 x 30 2.87 -> 0.67 ms, 1024 x 960 0.293 -> 0.077 ms.
 // At 256/512/1024 output rows the compiled k_asm_y4f stays: 1.31 against
-// 1.45 ms per 512^2 x 48 volume.
+// 1.45 ms per 512^2 x 48 volume (0.99 now).
 template <bool FILT, int MR>
 __global__ void __launch_bounds__(kThreads, MR <= 16 ? 4 : 3) k_asm_y2(AssembleArgs a, const Slot* __restrict__ slots,
                                                                     TfPlan pl, int lw,

@@ -12,14 +12,18 @@
 // accumulated straight into a 2D map P(x, y).  Every candidate k0 of the
 // search is then a 2D weighted sum over P.
 //
-//   k_ovl_build_x   build both overlaps (OTF-weighted band values) row by
-//                   row and inverse-FFT along x
-//   k_ovl_y_accum   inverse FFT along y, accumulate conj(X)Y, |X|^2, |Y|^2
-//                   over a group of kz planes
+//   k_tf_ovl_x      build both overlaps (OTF-weighted band values) row by
+//                   row and inverse-FFT along x (tf_kernels.cuh; lengths
+//                   without a factor pair: k_ovl_build_x)
+//   k_tf_ovl_y,     inverse FFT along y, accumulate conj(X)Y, |X|^2, |Y|^2
+//   k_ovl_y4        over a group of kz planes (512 rows: k_ovl_y4; lengths
+//                   without a factor pair: k_ovl_y_accum)
 //   k_p_reduce      sum the plane-group partial maps, finish |X|^2, |Y|^2
-//   k_fft_rows/cols cross-correlation FFT of conj(P)
+//   k_tf_rows_conj, cross-correlation FFT of conj(P) (else k_fft_rows/cols2)
+//   k_tf_cols
 //   k_argmax_*      intensity peak with its neighbours
-//   k_modamp_*      sum_xy P e^{i phi_c} for a batch of candidates
+//   k_modamp_*      sum_xy P e^{i phi_c} for a batch of candidates, k_modamp1_*
+//                   for one candidate of each pair
 #include <algorithm>
 
 #include "col_fft.cuh"

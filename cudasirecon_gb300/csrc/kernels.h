@@ -342,9 +342,10 @@ int assemble_tables_upload(const AssembleArgs& a);
 int launch_assemble(const AssembleArgs& a, cudaStream_t s, long long* launches);
 // Filter and assembly in one pass: the Wiener filter of every direction
 // applied in the assembly's band load (the bands are left unfiltered in
-// memory).  Available for 3 directions, 2 or 3 orders, one OTF for all
-// directions, zoomed y lengths 256/512/1024 and OTF lookups that stay inside
-// the table; returns -10 (nothing launched) otherwise.
+// memory).  Available for one OTF for all directions, equal order-0 noise
+// factors, zoomed y lengths 256/512/1024 or twice a length with a factor pair,
+// and OTF lookups that stay inside the table; returns -10 (nothing launched)
+// otherwise.
 bool assemble_filter_fusable(const AssembleArgs& a, const FilterArgs& f, bool one_otf);
 int launch_assemble_filtered(const AssembleArgs& a, const FilterArgs& f, bool one_otf, cudaStream_t s,
                              long long* launches);

@@ -136,7 +136,8 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
 // flat field and both edge blends in shared memory, the transform, the split
 // of the two real spectra (the steps of k_ingest_x).  Latency-bound, the
 // shared-memory passes in line: 640 x 384 x 30 0.685 -> 0.464 ms against the
-// Stockham stages, 300 x 192 x 40 (one direction) 0.083 -> 0.046 ms.
+// Stockham stages (0.400 with paired additions), 300 x 192 x 40 (one
+// direction) 0.083 -> 0.044 ms.
 template <typename T, int R1, int R2>
 __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
     k_tf_ingest(const __grid_constant__ IngestArgs a, const float2* __restrict__ tw)
@@ -509,7 +510,7 @@ __global__ void __launch_bounds__(TfOvlY<R1, R2>::kThreads, TfOvlY<R1, R2>::kCta
 // compiled sizes at run time spilled 2 to 4 KB a thread and took minutes to
 // build).
 // Per volume, against the Stockham stages on the doubled length: 1024^2 x 64
-// 22.5 -> 3.2 ms, 640 x 384 x 30 2.61 -> 0.51 ms, 1024 x 960 0.243 -> 0.050 ms.
+// 22.5 -> 2.9 ms, 640 x 384 x 30 2.61 -> 0.46 ms, 1024 x 960 0.243 -> 0.043 ms.
 //
 // Geometry of a factor pair: W output rows per CTA of at most 128 threads
 template <int R1, int R2>
