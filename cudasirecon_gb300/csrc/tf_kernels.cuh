@@ -366,8 +366,10 @@ __device__ __forceinline__ float2 ovl_element(const OverlapArgs& a, const OvlIte
 // W lines (line = 2 * row + overlap) of one kz plane per CTA.  Bound by the
 // elements' issue and latency; per kz plane the two radial OTF tables replace
 // 16 scattered loads and the kz interpolation of every element; rows outside
-// the support are left out.  Nine builds of 640 x 384 x 30: 1.40 ms by the
-// Stockham stages, 0.37 with every row, 0.33 now.
+// the support are left out, and a line at a time leaves its row's arithmetic to
+// the uniform registers.  Nine builds of 640 x 384 x 30: 1.40 ms by the
+// Stockham stages, 0.37 with every row, 0.33 with a line per few threads, 0.31
+// now; of 1024^2 x 64 2.16 and 1.98.
 template <int R1, int R2>
 __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
     k_tf_ovl_x(const __grid_constant__ OverlapArgs a, const float2* __restrict__ tw)
@@ -388,11 +390,24 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
   if (!__syncthreads_or(threadIdx.x < nl && !dead(threadIdx.x))) return;
   if (!empty) ovl_build_tab(a, it, otf_kz(a.otf, z0), tab);
   __syncthreads();
-  for (int t = threadIdx.x; t < G::W * N; t += G::kThreads) {
-    const int l = t / N, j = t - l * N;
-    float2 v = make_float2(0.f, 0.f);
-    if (!empty && l < nl) v = ovl_element(a, it, ks, (L0 + l) & 1, z0, (L0 + l) >> 1, j, tab, rdk);
-    sm[t] = v;
+  // a line at a time, whose row is the same for the whole CTA, unless that
+  // leaves more than a seventh of the threads' turns idle
+  constexpr int kTurns = (N + G::kThreads - 1) / G::kThreads * G::kThreads;
+  if constexpr (7 * (kTurns - N) <= N) {
+    for (int l = 0; l < G::W; ++l) {
+      const bool live = !empty && l < nl && !dead(l);
+      const int ov = (L0 + l) & 1, i = (L0 + l) >> 1;
+#pragma unroll 2
+      for (int j = threadIdx.x; j < N; j += G::kThreads)
+        sm[l * N + j] = live ? ovl_element(a, it, ks, ov, z0, i, j, tab, rdk) : make_float2(0.f, 0.f);
+    }
+  } else {
+    for (int t = threadIdx.x; t < G::W * N; t += G::kThreads) {
+      const int l = t / N, j = t - l * N;
+      float2 v = make_float2(0.f, 0.f);
+      if (!empty && l < nl) v = ovl_element(a, it, ks, (L0 + l) & 1, z0, (L0 + l) >> 1, j, tab, rdk);
+      sm[t] = v;
+    }
   }
   __syncthreads();
   float2 u[R2];
