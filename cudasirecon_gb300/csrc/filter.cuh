@@ -62,7 +62,8 @@ inline FilterK make_filter_k(const FilterArgs& a)
   return k;
 }
 
-// Every looked-up radius is <= rdistcutoff, so the table is never left when
+// Every looked-up radius is <= rdistcutoff (filter_rows and sum_terms hold the
+// pixels outside at the edge), so the table is never left when
 // floor(rdistcutoff / dkrotf) + 3 <= nxotf (+ 3: a cross term's interpolation
 // radius comes from an approximate square root and may pass rdistcutoff by
 // an ulp) and no kz index, |kz| <= nz/2, leaves it along kz; otherwise the
@@ -71,6 +72,38 @@ inline bool filter_needs_clamp(const FilterArgs& a, const FilterK& k)
 {
   return !(std::floor(a.rdistcutoff * k.rdkrotf) + 3 <= a.otf.nxotf) ||
          !(a.nz == 1 || (a.nz / 2) * (double)a.otf.kzscale + 1.0 < a.otf.nzotf);
+}
+
+// Two pixels of column kx on the data rows r0 and r0 + 1, as a thread of the
+// fused assembly filters them: rows in transform order, row r at ky = r or
+// r - ny; row ny/2 holds the pixel ky = -ny/2 for the filter (both passes of
+// the reference index rows as y in [-ny/2, ny/2 - 1]).
+struct FilterRows {
+  int ky[2];
+  float yf[2], rd[2];  // rd: the radius at which the pixel's own OTF is looked up
+  bool in[2];          // a row of the image, inside the support
+};
+__host__ __device__ __forceinline__ FilterRows filter_rows(float dky, float cutoff, int ny, float x1f, int r0)
+{
+  FilterRows p;
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+  for (int i = 0; i < 2; ++i) {
+    const int r = r0 + i;
+    p.ky[i] = r <= ny / 2 ? r : r - ny;
+    const int kyf = p.ky[i] == ny / 2 ? -(ny / 2) : p.ky[i];
+    p.yf[i] = kyf * dky;
+    const float rd = sqrtf(x1f * x1f + p.yf[i] * p.yf[i]);
+    const bool inside = rd <= cutoff;
+    p.in[i] = r < ny && inside;
+    // A pixel outside goes through the filter with its neighbour and is dropped
+    // there.  It can lie dky beyond the support, more bins than
+    // filter_needs_clamp leaves where the image is short against the OTF, so
+    // its lookup stays at the edge.
+    p.rd[i] = inside ? rd : cutoff;
+  }
+  return p;
 }
 
 // the switches fixed at compile time on the table path
@@ -425,9 +458,7 @@ __device__ __forceinline__ void filter_scale_pair(const FilterArgs& a, const Fil
 }
 
 // Filtered values of column kx on the data rows r0 and r0 + 1 (r0 + 1 may be
-// past the end): rows in transform order, row r at ky = r or r - ny.  A row
-// ny/2 holds the pixel ky = -ny/2 for the filter (both passes of the reference
-// index rows as y in [-ny/2, ny/2 - 1]).
+// past the end), filter_rows' pixels
 __device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const FilterK& fk, const FilterSlot& f,
                                               const FilterTerms& terms, const float4* tab, int kx, int r0, float2& v0,
                                               float2& v1)
@@ -435,22 +466,17 @@ __device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const Filter
   v0 = v1 = make_float2(0.f, 0.f);
   const int nd = fa.ndirs, no = fa.norders;
   const int nxh = f.nx / 2 + 1;
-  int ky[2];
-  size_t ind[2];
-  float yf[2], rd[2];
-  bool in[2];
   const float x1f = kx * fa.dkx;
   const bool conj = kx < 0;
   int z = conj ? -f.kz : f.kz;
   if (z < 0) z += f.nz;
+  const FilterRows p = filter_rows(fa.dky, fa.rdistcutoff, f.ny, x1f, r0);
+  const int(&ky)[2] = p.ky;
+  const float(&yf)[2] = p.yf, (&rd)[2] = p.rd;
+  const bool(&in)[2] = p.in;
+  size_t ind[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const int r = r0 + i;
-    ky[i] = r <= f.ny / 2 ? r : r - f.ny;
-    const int kyf = ky[i] == f.ny / 2 ? -(f.ny / 2) : ky[i];
-    yf[i] = kyf * fa.dky;
-    rd[i] = sqrtf(x1f * x1f + yf[i] * yf[i]);
-    in[i] = r < f.ny && rd[i] <= fa.rdistcutoff;
     int y = conj ? -ky[i] : ky[i];
     if (y < 0) y += f.ny;
     ind[i] = (size_t)z * f.plane + (size_t)y * nxh + (conj ? -kx : kx);
