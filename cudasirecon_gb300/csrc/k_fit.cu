@@ -651,10 +651,15 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   // half or whole warp, 0.131, 0.400 and 3.01 ms per 256^2 x 32, 512^2 x 48 and
   // 1024^2 x 64 volume against 0.112, 0.353 and 2.17) take the two-factor kernel
   // whatever the plan file says, as they took the register ones.
+  // Its radial tables need every kz index inside the OTF (otf_kz's wrapped one
+  // is negative where |kz| exceeds the OTF's extent, a PSF step of more than
+  // 1 / (axial cutoff)); k_ovl_build_x's lookups clamp at both ends.
   const bool reg_row = a.nx == 256 || a.nx == 512 || a.nx == 1024;
+  const bool kz_inside = a.zdc * a.otf.kzscale <= a.otf.nzotf;
   TfPlan tx, ty;
-  const TfKernels* kx =
-      a.otf.nxotf <= kOvlTabMax && (reg_row || fft_two_factor(kSiteOvlX, a.nx)) ? tf_kernels(a.nx, &tx) : nullptr;
+  const TfKernels* kx = kz_inside && a.otf.nxotf <= kOvlTabMax && (reg_row || fft_two_factor(kSiteOvlX, a.nx))
+                            ? tf_kernels(a.nx, &tx)
+                            : nullptr;
   // 512 rows keep the compiled column kernel (0.209 against 0.270 ms per
   // 512^2 x 48 volume); 256 rows are as fast either way (0.078, 0.076), 1024
   // took the Stockham stages (1.25 a pair of 1024^2 x 64 against 0.26)

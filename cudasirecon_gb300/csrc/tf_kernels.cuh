@@ -292,7 +292,8 @@ __global__ void __launch_bounds__(TfRow<R1, R2>::kThreads)
 // ----------------------------------------------------------------- overlaps
 // radial table of one kz: order slot o at [o * (nxotf + 1)], entry i the OTF
 // interpolated to kz at radial bins i and i + 1 (flat indices clamped to the
-// table like otf_lookup_rr's; entry nxotf stands for every bin past the end)
+// table's end like otf_lookup_rr's; entry nxotf stands for every bin past the
+// end).  The kz index is not negative (launch_overlaps).
 __device__ __forceinline__ void ovl_build_tab(const OverlapArgs& a, const OvlItem& it, const OtfKz& kz, float4* tab)
 {
   const int nxo = a.otf.nxotf, nzo = a.otf.nzotf, last = nxo * nzo - 1;
