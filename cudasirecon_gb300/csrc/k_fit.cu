@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_ovl_y4(const __grid_constant__ 
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2) dst[(size_t)(k1 + R1 * k2) * nx] = acc[k2];
   }
-  double tx = block_sum_d((double)sx + (double)ex, red);
-  double ty = block_sum_d((double)sy + (double)ey, red);
+  double tx = block_sum_d(pair_value(sx, ex), red);
+  double ty = block_sum_d(pair_value(sy, ey), red);
   if (threadIdx.x == 0) {
     int cta = blockIdx.y * gridDim.x + blockIdx.x;
     im.sums[2 * cta] = tx;

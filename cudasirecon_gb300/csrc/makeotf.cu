@@ -90,6 +90,12 @@ __global__ void __launch_bounds__(kMoThreads) k_mo_section(float* psf, float* bg
         }
       }
     double s = (double)hi + (double)lo;
+    if (!isfinite(hi)) {  // past the float range: the thread's pixels once more in double
+      s = 0.0;
+      for (int y = threadIdx.x >> 5; y < ny; y += nw)
+        for (int x = lane; x < nx; x += 32)
+          if (y < kBorder || y > ny - kBorder || x < kBorder || x > nx - kBorder) s += (double)sec[(size_t)y * nx + x];
+    }
     s = block_sum_d(s, red);
     if (threadIdx.x == 0) s_bg = (float)(s / border_count);
   }

@@ -132,6 +132,13 @@ __device__ __forceinline__ void pair_sum(float& s, float& e, float x)
   s = h;
 }
 
+// The pair's value.  Past an overflow, or a term that is not finite, the error
+// term is inf - inf: s alone is then the sum.
+__device__ __forceinline__ double pair_value(float s, float e)
+{
+  return isfinite(s) ? (double)s + (double)e : (double)s;
+}
+
 // Block-wide sum of a double (all threads must call).  Result valid in thread 0.
 __device__ __forceinline__ double block_sum_d(double v, double* scratch /* >= 32 */)
 {

@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(TfOvlY<R1, R2>::kThreads, TfOvlY<R1, R2>::kCta
     for (int i = 0; i < G::kHalf; ++i)
       if (2 * i + ov < R2) dst[(size_t)(q + R1 * (2 * i + ov)) * nx] = acc[i];
   }
-  const double st = (double)sq + (double)sqe;
+  const double st = pair_value(sq, sqe);
   const double tx = block_sum_d(ov ? 0.0 : st, red);
   const double ty = block_sum_d(ov ? st : 0.0, red);
   if (threadIdx.x == 0) {
