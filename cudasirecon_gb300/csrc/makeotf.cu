@@ -385,7 +385,7 @@ __device__ __forceinline__ float2 pair_mul(float2 a, float bh, float bl)
 __device__ __forceinline__ float sphere_ratio(const ShiftCompArgs& a, float rho)
 {
   const float2 x = pair_mul(make_float2(rho, 0.f), a.c_hi, a.c_lo);
-  if (x.x <= 1.f) {
+  if (fabsf(x.x) <= 1.f) {
     constexpr SphereCoef co;
     const float2 u = pair_mul(x, x.x, x.y);
     float2 s = make_float2(co.hi[kSphereTerms - 1], co.lo[kSphereTerms - 1]);

@@ -1,6 +1,7 @@
 """GPU: sums kept as float pairs at the end of the float range.  An infinite
-sum stays infinite (an amplitude over it is then 0, not NaN), and a sum past
-the range whose mean is inside stays a number."""
+sum stays infinite (an amplitude over it is then 0, not NaN), a sum past the
+range whose mean is inside stays a number, and the bead's form factor takes
+the sign of the diameter as it always did."""
 import json
 import os
 import subprocess
@@ -67,3 +68,11 @@ def test_makeotf_background_past_the_float_range():
     d = got - want
     assert np.linalg.norm(d) <= 1e-5 * np.linalg.norm(want)
     assert np.abs(d).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("diam", [0.1, 1.5])
+def test_bead_diameter_sign(diam):
+    psf = syn.bead_psf_stack(64, 72, 8, syn.Optics(), nphases=5, peak_photons=5e4, seed=3)
+    args = ["-angle", "0.2388", "-ls", "0.21", "-xyres", "0.08", "-zres", "0.125", "-na", "1.42", "-nimm", "1.515",
+            "-wavelength", "528", "-nphases", "5", "-beaddiam"]
+    assert np.array_equal(sr.make_otf(psf, args + [str(diam)]), sr.make_otf(psf, args + [str(-diam)]))
