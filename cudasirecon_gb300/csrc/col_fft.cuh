@@ -19,8 +19,6 @@
 
 namespace simrecon {
 
-#ifdef __CUDACC__
-
 template <int N, int R1, int W>
 struct ColFft {
   static constexpr int R2 = N / R1;
@@ -29,6 +27,8 @@ struct ColFft {
   static_assert(N % R1 == 0, "R1 must divide N");
   static_assert(W == 8, "the bank-conflict-free layout assumes 8 columns per CTA");
 };
+
+#ifdef __CUDACC__
 
 // Stage 1 for every (c, j) item of the CTA; load(row, c) -> float2 (0 outside
 // the data).  tw: table of N twiddles exp(-2 pi i k / N).  Ends with a CTA

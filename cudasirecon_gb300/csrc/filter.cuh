@@ -106,6 +106,28 @@ __host__ __device__ __forceinline__ FilterRows filter_rows(float dky, float cuto
   return p;
 }
 
+// The terms of the Wiener denominator that a CTA's pixels can meet, in shared
+// memory: p = (-shift y twice, |amp|^2 / noisevar twice), aligned pairs for the
+// paired instructions; q = (shift x, first entry of the order's radial table).
+// Three runs: side orders whose suppressed centre no column of the CTA reaches
+// (up to nplain), the other side orders (up to nside), order 0 (up to n).  A
+// term whose support no column reaches is left out.
+struct FilterTerms {
+  float4 p[kMaxDirs * (2 * kMaxOrders - 1)];
+  float2 q[kMaxDirs * (2 * kMaxOrders - 1)];
+  int nplain, nside, n;
+};
+
+// Shared memory of the radial tables, [2][norders][nxotf].  Entries are the
+// values alone: with the step to the next bin beside each (one 16-byte load a
+// lookup) the tables took twice the space and twice the building, the fused
+// kernels lost a CTA per SM from 66 bins on, and 512^2 x 48 took 1.23 ms at 129
+// bins and 2.51 at 513, against 1.02 and 1.41 (0.98 either way at 65).
+inline size_t filter_tab_bytes(int norders, int nxotf) { return 2 * (size_t)norders * nxotf * sizeof(float2); }
+// The fused kernels' tables at most: with the transform buffer of 1024 rows two
+// CTAs stay resident on an SM (three up to 129 bins and three orders)
+constexpr size_t kFusedTabMax = 32 * 1024;
+
 // the switches fixed at compile time on the table path
 inline int filter_flags(const FilterArgs& a)
 {
@@ -129,21 +151,21 @@ __device__ __forceinline__ float dev_suppress(float x)
 // plane's radial table (TAB; its entries are the kz interpolation of the
 // bilinear lookup, so the result is the same interpolation), else the
 // bilinear lookup itself.
-// A table entry is (t[ir], t[ir + 1] - t[ir]): one 16-byte load and two FMAs.
 // The bin is the integer nearest to krindex - 1/2, taken from the mantissa of
 // a sum with 1.5 * 2^23 (additions on the FP32 pipe; float-to-int and back
 // are quarter-rate): a krindex on a bin boundary may give the bin below with
 // ar = 1, the same value.  krindex < nxotf, far below 2^22.
 template <bool CLAMP, bool TAB>
-__device__ __forceinline__ float2 filter_otf(const FilterArgs& a, const float4* tabz, int o, float krindex,
+__device__ __forceinline__ float2 filter_otf(const FilterArgs& a, const float2* tabz, int o, float krindex,
                                              const OtfKz& kzi)
 {
   if (TAB) {
     const float m = (krindex - 0.5f) + 12582912.f;
     const int ir = __float_as_int(m) - 0x4B400000;
     const float ar = krindex - (m - 12582912.f);
-    const float4 t = tabz[o * a.otf.nxotf + ir];
-    return make_float2(fmaf(ar, t.z, t.x), fmaf(ar, t.w, t.y));
+    const float2* t = tabz + o * a.otf.nxotf + ir;
+    const float2 t0 = t[0], t1 = t[1];
+    return make_float2(fmaf(ar, t1.x - t0.x, t0.x), fmaf(ar, t1.y - t0.y, t0.y));
   }
   return otf_lookup_rr<CLAMP>(a.otf.otf[o], a.otf, krindex, kzi);
 }
@@ -155,7 +177,7 @@ __device__ __forceinline__ float2 filter_otf(const FilterArgs& a, const float4* 
 template <int ND, int NO, bool CLAMP, bool TAB, int FL>
 __device__ __forceinline__ float2 filter_scale(const FilterArgs& a, const FilterK& k, const float* termw,
                                                float ampmag2, int dir, int order, int z0, float rdist1, float x1f,
-                                               float y1f, const float4* tabz)
+                                               float y1f, const float2* tabz)
 {
   const bool suppress = FL >= 0 ? (FL & 1) != 0 : a.suppress != 0;
   const bool dampen0 = FL >= 0 ? (FL & 2) != 0 : a.dampen0 != 0;
@@ -266,13 +288,14 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
 __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
 // |OTF|^2 of order slot T at two radial indices (filter_otf's table lookup)
-__device__ __forceinline__ float2 otf_mag2_pair(const float4* T, float2 kri)
+__device__ __forceinline__ float2 otf_mag2_pair(const float2* T, float2 kri)
 {
   const float2 m = add2(add2(kri, dup2(-0.5f)), dup2(12582912.f));
   const float2 ar = fma2(add2(m, dup2(-12582912.f)), dup2(-1.f), kri);
-  const float4 t0 = T[__float_as_int(m.x) - 0x4B400000], t1 = T[__float_as_int(m.y) - 0x4B400000];
-  const float2 v0 = fma2(dup2(ar.x), make_float2(t0.z, t0.w), make_float2(t0.x, t0.y));
-  const float2 v1 = fma2(dup2(ar.y), make_float2(t1.z, t1.w), make_float2(t1.x, t1.y));
+  const float2 *t0 = T + (__float_as_int(m.x) - 0x4B400000), *t1 = T + (__float_as_int(m.y) - 0x4B400000);
+  const float2 a0 = t0[0], b0 = t0[1], a1 = t1[0], b1 = t1[1];
+  const float2 v0 = fma2(dup2(ar.x), csub(b0, a0), a0);
+  const float2 v1 = fma2(dup2(ar.y), csub(b1, a1), a1);
   return make_float2(fmaf(v0.x, v0.x, v0.y * v0.y), fmaf(v1.x, v1.x, v1.y * v1.y));
 }
 
@@ -284,18 +307,6 @@ __device__ __forceinline__ float2 sqrt_pair(float2 x)
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
   return r;
 }
-
-// The terms of the Wiener denominator that a CTA's pixels can meet, in shared
-// memory: p = (-shift y twice, |amp|^2 / noisevar twice), aligned pairs for the
-// paired instructions; q = (shift x, first entry of the order's radial table).
-// Three runs: side orders whose suppressed centre no column of the CTA reaches
-// (up to nplain), the other side orders (up to nside), order 0 (up to n).  A
-// term whose support no column reaches is left out.
-struct FilterTerms {
-  float4 p[kMaxDirs * (2 * kMaxOrders - 1)];
-  float2 q[kMaxDirs * (2 * kMaxOrders - 1)];
-  int nplain, nside, n;
-};
 
 // built by the CTA's first warp; a barrier must follow.  kx0: the CTA's first
 // column, ncol of them.
@@ -347,7 +358,7 @@ __device__ __forceinline__ void build_filter_terms(const FilterArgs& a, const Fi
 enum : int { kTermPlain = 0, kTermSuppressed = 1, kTermOrder0 = 2 };
 template <int KIND>
 __device__ __forceinline__ float2 sum_terms(const FilterArgs& a, const FilterK& k, const FilterTerms& terms, int i0,
-                                            int i1, float xabs, float2 yabs, float zf3, const float4* tabz, float2 sum)
+                                            int i1, float xabs, float2 yabs, float zf3, const float2* tabz, float2 sum)
 {
 #pragma unroll 1
   for (int i = i0; i < i1; ++i) {
@@ -409,7 +420,7 @@ __device__ __forceinline__ void load_fit(const FilterArgs& a, FilterSlot& f)
 // the columns' reach.
 __device__ __forceinline__ void filter_scale_pair(const FilterArgs& a, const FilterK& k, const FilterTerms& terms,
                                                   const FilterSlot& f, int z0, float2 rdist1, float x1f, float2 y1f,
-                                                  const float4* tabz, float2& s0, float2& s1)
+                                                  const float2* tabz, float2& s0, float2& s1)
 {
   const int order = f.order, i1 = f.dir * a.norders + order;
   const float ampmag2 = f.ampmag2;
@@ -460,7 +471,7 @@ __device__ __forceinline__ void filter_scale_pair(const FilterArgs& a, const Fil
 // Filtered values of column kx on the data rows r0 and r0 + 1 (r0 + 1 may be
 // past the end), filter_rows' pixels
 __device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const FilterK& fk, const FilterSlot& f,
-                                              const FilterTerms& terms, const float4* tab, int kx, int r0, float2& v0,
+                                              const FilterTerms& terms, const float2* tab, int kx, int r0, float2& v0,
                                               float2& v1)
 {
   v0 = v1 = make_float2(0.f, 0.f);
@@ -487,7 +498,7 @@ __device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const Filter
     const float xs = conj ? -x1f : x1f;
     const float2 ys = make_float2(conj ? (float)(-ky[0]) * fa.dky : yf[0], conj ? (float)(-ky[1]) * fa.dky : yf[1]);
     const int zs = conj ? -f.kz : f.kz;
-    const float4* tz = tab + (conj ? no * fa.otf.nxotf : 0);
+    const float2* tz = tab + (conj ? no * fa.otf.nxotf : 0);
     // one denominator for every direction (fk.order0_shared): direction d's own
     // term and the (d, 0) term its sum skips are the same OTF value
     float2 b0 = in[0] ? f.br[ind[0]] : make_float2(0.f, 0.f), b1 = in[1] ? f.br[ind[1]] : make_float2(0.f, 0.f);
@@ -523,20 +534,16 @@ __device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const Filter
 }
 
 // The radial tables of plane zp: each order's OTF interpolated to kz = zp
-// (pass 0) and to the conjugate pass's kz = -zp (pass 1) along kr, with the
-// step to the next bin: [2][no][nxotf]
-__device__ __forceinline__ void build_filter_tab(const FilterArgs& a, int no, int zp, float4* tab)
+// (pass 0) and to the conjugate pass's kz = -zp (pass 1) along kr:
+// [2][no][nxotf]
+__device__ __forceinline__ void build_filter_tab(const FilterArgs& a, int no, int zp, float2* tab)
 {
   const int nxo = a.otf.nxotf, nzo = a.otf.nzotf;
   for (int t = threadIdx.x; t < 2 * no * nxo; t += blockDim.x) {
     const int pass = t / (no * nxo), r = t - pass * no * nxo, o = r / nxo, ir = r - o * nxo;
     const OtfKz kz = otf_kz(a.otf, pass ? -zp : zp);
-    auto at = [&](int i) {
-      const float2 va = __ldg(a.otf.otf[o] + i * nzo + kz.iz), vb = __ldg(a.otf.otf[o] + i * nzo + kz.izp);
-      return make_float2(va.x * (1 - kz.az) + vb.x * kz.az, va.y * (1 - kz.az) + vb.y * kz.az);
-    };
-    const float2 t0 = at(ir), t1 = at(ir + 1 < nxo ? ir + 1 : ir);
-    tab[t] = make_float4(t0.x, t0.y, t1.x - t0.x, t1.y - t0.y);
+    const float2 va = __ldg(a.otf.otf[o] + ir * nzo + kz.iz), vb = __ldg(a.otf.otf[o] + ir * nzo + kz.izp);
+    tab[t] = make_float2(va.x * (1 - kz.az) + vb.x * kz.az, va.y * (1 - kz.az) + vb.y * kz.az);
   }
 }
 

@@ -59,7 +59,7 @@ __device__ __forceinline__ void apply_side(float2& re, float2& im, float2 scale,
 template <int ND, int NO, bool CLAMP, bool TAB, int FL = -1>
 __global__ void __launch_bounds__(kThreads) k_filter(const __grid_constant__ FilterArgs a, const __grid_constant__ FilterK k)
 {
-  extern __shared__ float4 tab[];
+  extern __shared__ float2 tab[];
   const int nx = a.nx, ny = a.ny, nz = a.nz, nxh = nx / 2 + 1;
   const int order = blockIdx.z, iz = blockIdx.y;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const S
   static_assert(R2 * W <= kThreads, "one stage-1 item per thread");
   static_assert(Y * W <= CF::kSmemElems, "phase A fits the transform buffer");
   extern __shared__ __align__(16) float2 sm[];
-  float4* tab = (float4*)(sm + CF::kSmemElems);  // [2][norders][nxotf]
+  float2* tab = sm + CF::kSmemElems;  // [2][norders][nxotf]
   __shared__ FilterTerms terms;
   const Slot sl = slots[blockIdx.y];
   const int nx = a.nx, ny = a.ny, nz = a.nz, nxh = nx / 2 + 1;
@@ -739,16 +739,13 @@ int launch_filter(const FilterArgs& a, cudaStream_t s, long long* launches)
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
   // per-plane radial tables when the lookups stay inside the table and the
-  // tables fit in 96 KB of shared memory
-  const size_t tabb = 2 * (size_t)no * a.otf.nxotf * sizeof(float4);
-  const bool tab = !clamp && tabb <= 96 * 1024;
+  // tables fit in 48 KB of shared memory
+  const size_t tabb = filter_tab_bytes(no, a.otf.nxotf);
+  const bool tab = !clamp && tabb <= 48 * 1024;
   // the table path with the three switches fixed at compile time
   const int fl = filter_flags(a);
   auto tab_path = [&]<int NO>() {
-    auto go = [&]<int FL>() {
-      allow_dynamic_smem((const void*)k_filter<3, NO, false, true, FL>, tabb);
-      k_filter<3, NO, false, true, FL><<<g, kThreads, tabb, s>>>(a, k);
-    };
+    auto go = [&]<int FL>() { k_filter<3, NO, false, true, FL><<<g, kThreads, tabb, s>>>(a, k); };
     switch (fl) {
       case 0: go.template operator()<0>(); break;
       case 1: go.template operator()<1>(); break;
@@ -843,8 +840,6 @@ int assemble_tables_upload(const AssembleArgs& a)
 }
 
 namespace {
-constexpr size_t kFusedTabMax = 32 * 1024;  // OTF tables of the fused kernel (two CTAs per SM stay resident)
-
 int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s, long long* launches);
 }  // namespace
 
@@ -856,7 +851,7 @@ bool assemble_filter_fusable(const AssembleArgs& a, const FilterArgs& f, bool on
   const FilterK k = make_filter_k(f);
   if (!k.order0_shared) return false;
   if (filter_needs_clamp(f, k)) return false;
-  return 2 * (size_t)f.norders * f.otf.nxotf * sizeof(float2) <= kFusedTabMax;
+  return filter_tab_bytes(f.norders, f.otf.nxotf) <= kFusedTabMax;
 }
 
 int launch_assemble_filtered(const AssembleArgs& a, const FilterArgs& f, bool one_otf, cudaStream_t s,
@@ -945,7 +940,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
       if (rc != 0) return rc;
     } else if (filt) {
       const FilterK fk = make_filter_k(*filt);
-      const size_t tabb = 2 * (size_t)filt->norders * filt->otf.nxotf * sizeof(float4);
+      const size_t tabb = filter_tab_bytes(filt->norders, filt->otf.nxotf);
       auto go = [&]<int YN>() {
         const size_t bytes = ColFft<YN, colfft_r1(YN), 8>::kSmemElems * sizeof(float2) + tabb;
         allow_dynamic_smem((const void*)k_asm_y4f<YN>, bytes);

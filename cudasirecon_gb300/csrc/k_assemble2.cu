@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kThreads, MR <= 16 ? 4 : 3) k_asm_y2(AssembleA
   const size_t dstride = (size_t)a.nphases * nz * plane;  // next direction's band 0
   const int no = a.norders;
   // the row-major values, then the exchange of both parities over them
-  float4* tab = (float4*)(sm + ((2 * R1 * ld + 1) & ~1));  // [2][no][nxotf]
+  float2* tab = sm + 2 * R1 * ld;  // [2][no][nxotf]
   if constexpr (FILT) {
     if (c0 < a.cx0 || c0 >= a.cx1) {  // no data: zeros for the x pass
       for (int t = threadIdx.x; t < a.Y << lw; t += kThreads) {
@@ -179,8 +179,8 @@ int launch_asm_y2(const AssembleArgs& a, const void* d_slots, int nslots, const 
   if (!get_tf_plan(a.ny, &pl)) return -1;
   const int lw = 2 * pl.r2 * 8 <= kThreads ? 3 : 2;
   const size_t ld = (size_t)(pl.r2 | 1) << lw;
-  const size_t elems = (2 * pl.r1 * ld + 1) & ~(size_t)1;
-  const size_t tabb = filt ? 2 * (size_t)filt->norders * filt->otf.nxotf * sizeof(float4) : 0;
+  const size_t elems = 2 * pl.r1 * ld;
+  const size_t tabb = filt ? filter_tab_bytes(filt->norders, filt->otf.nxotf) : 0;
   const size_t bytes = elems * sizeof(float2) + tabb;
   const dim3 g((a.tx1 - a.tx0 + (1 << lw) - 1) >> lw, nslots);
   const Slot* slots = (const Slot*)d_slots;

@@ -50,4 +50,25 @@ int main()
 def test_pair_lookups_stay_in_the_table(tmp_path):
     pairs, outside, worst = (int(v) for v in host_probe.run(PROBE, tmp_path).split())
     assert pairs > 100000 and outside > 1000
-    assert worst <= 0  # the last entry is nxotf - 1
+    assert worst < 0  # a lookup reads its entry and the next; the last is nxotf - 1
+
+
+SHARED = r"""
+#include <cstdio>
+#include "col_fft.cuh"
+#include "filter.cuh"
+using namespace simrecon;
+int main()
+{
+  const size_t fixed = ColFft<1024, 32, 8>::kSmemElems * sizeof(float2) + sizeof(FilterTerms);
+  const size_t sm = 228 * 1024, reserved = 1024;  // of an SM; per CTA
+  for (int nxotf : {65, 129}) std::printf("%zu ", sm / (fixed + filter_tab_bytes(3, nxotf) + reserved));
+  std::printf("%zu\n", sm / (fixed + kFusedTabMax + reserved));
+}
+"""
+
+
+def test_fused_filter_keeps_its_ctas(tmp_path):
+    """1024 output rows, three orders: three CTAs per SM with the OTFs of 128-
+    and 256-pixel PSFs, two with the largest tables that are taken."""
+    assert [int(v) for v in host_probe.run(SHARED, tmp_path).split()] == [3, 3, 2]
