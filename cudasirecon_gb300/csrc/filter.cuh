@@ -128,6 +128,16 @@ inline size_t filter_tab_bytes(int norders, int nxotf) { return 2 * (size_t)nord
 // CTAs stay resident on an SM (three up to 129 bins and three orders)
 constexpr size_t kFusedTabMax = 32 * 1024;
 
+// |x| of a term's distance at column x1f, (x1f + kxo) - sx, less what rounding
+// or a fused product can move it: a term is left out of a CTA's list, or taken
+// for an unsuppressed one, only where no rounding of the per-pixel test can
+// disagree.
+__host__ __device__ __forceinline__ float filter_x_least(float x1f, float kxo, float sx)
+{
+  const float slack = 1e-6f * (fabsf(x1f) + fabsf(kxo) + fabsf(sx));  // 16 units of the largest sum
+  return fmaxf(fabsf(x1f + kxo - sx) - slack, 0.f);
+}
+
 // the switches fixed at compile time on the table path
 inline int filter_flags(const FilterArgs& a)
 {
@@ -336,7 +346,7 @@ __device__ __forceinline__ void build_filter_terms(const FilterArgs& a, const Fi
         for (int c = 0; c < ncol; ++c) {
           float x1f = (kx0 + c) * a.dkx;
           if (order == 0) x1f = fabsf(x1f);  // order 0 is filtered at the stored element's own pixel
-          const float x2 = x1f + kxo - sx;
+          const float x2 = filter_x_least(x1f, kxo, sx);
           reach = reach || x2 * x2 < k.r2_in;
           supp = supp || (a.suppress && x2 * x2 <= k.r2_supp);
         }

@@ -72,3 +72,47 @@ def test_fused_filter_keeps_its_ctas(tmp_path):
     """1024 output rows, three orders: three CTAs per SM with the OTFs of 128-
     and 256-pixel PSFs, two with the largest tables that are taken."""
     assert [int(v) for v in host_probe.run(SHARED, tmp_path).split()] == [3, 3, 2]
+
+
+TERMS = r"""
+#include <cmath>
+#include <cstdio>
+#include <random>
+#include "filter.cuh"
+using namespace simrecon;
+int main()
+{
+  std::mt19937 g(7);
+  auto u = [&](float a, float b) { return a + (b - a) * (float)(g() / 4294967296.0); };
+  long long near = 0, missed = 0, kept = 0, far = 0;
+  for (int t = 0; t < 400000; ++t) {
+    const int n = 64 << (g() % 6), kx = (int)(g() % n) - n / 2;
+    const float dkx = 1.f / (n * u(0.04f, 0.12f)), kxo = u(-10.f, 10.f);
+    // a column whose distance is the bound, to a few units in the last place
+    const float r = g() % 2 ? u(3.f, 7.f) : 10 * dkx;
+    float sx = (float)((double)kx * dkx + kxo + (g() % 2 ? r : -r));
+    for (int i = (int)(g() % 7); i > 0; --i) sx = std::nextafter(sx, g() % 2 ? 1e9f : -1e9f);
+    const float r2 = r * r;
+    // the distance as a compiler may form it: separate, or the product fused
+    const float x1f = kx * dkx;
+    const float d[2] = {x1f + kxo - sx, std::fma((float)kx, dkx, kxo) - sx};
+    const float least = filter_x_least(x1f, kxo, sx);
+    for (float x : d) {
+      const bool in = x * x <= r2 || std::fma(x, x, 0.f) < r2;
+      near += in;
+      missed += in && !(least * least <= r2);
+    }
+    const float away = 1.001f * r;  // well outside: the term is not kept
+    const float sf = x1f + kxo + away;
+    const float lf = filter_x_least(x1f, kxo, sf);
+    if (r > 3.f) ++far, kept += lf * lf <= r2;
+  }
+  std::printf("%lld %lld %lld %lld\n", near, missed, far, kept);
+}
+"""
+
+
+def test_terms_are_left_out_only_out_of_reach(tmp_path):
+    near, missed, far, kept = (int(v) for v in host_probe.run(TERMS, tmp_path).split())
+    assert near > 100000 and far > 100000
+    assert missed == 0 and kept == 0
