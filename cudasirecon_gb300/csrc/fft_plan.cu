@@ -241,6 +241,14 @@ int chosen_path(int site, int n)
 }
 }  // namespace
 
+bool fft_plan_open(FftSite site, int n)
+{
+  if (!reg_fft_lanes(n)) return true;
+  if (t_seen) t_seen->insert({(int)site, n});
+  const int c = chosen_path(site, n);
+  return c < 0 || c == kPathTwoFactor;
+}
+
 bool reg_fft_site_enabled(FftSite site, int n)
 {
   if (t_seen) t_seen->insert({(int)site, n});
@@ -251,11 +259,7 @@ bool reg_fft_site_enabled(FftSite site, int n)
 bool fft_two_factor(FftSite site, int n)
 {
   int r1, r2;
-  if (!tf_factor(n, &r1, &r2)) return false;
-  if (!reg_fft_lanes(n)) return true;
-  if (t_seen) t_seen->insert({(int)site, n});
-  const int c = chosen_path(site, n);
-  return c < 0 || c == kPathTwoFactor;
+  return tf_factor(n, &r1, &r2) && fft_plan_open(site, n);
 }
 
 void fft_site_force(int site, int path) { t_force_site = site, t_force_path = path; }

@@ -27,6 +27,7 @@
 #include "filter.cuh"
 #include "kernels.h"
 #include "reg_fft.cuh"
+#include "tf_fft.cuh"
 #include "z_fft.cuh"
 
 namespace simrecon {
@@ -778,18 +779,18 @@ int launch_filter(const FilterArgs& a, cudaStream_t s, long long* launches)
   return (int)cudaGetLastError();
 }
 
-namespace {
 // Doubled grids take the half-length transforms of k_assemble2.cu, except
 // where a compiled doubled-length kernel is the faster one: per 512^2 x 48
-// volume the y pass took 1.31 ms (k_asm_y4f; now 0.99) against 1.45, the x pass
+// volume the y pass took 1.31 ms (k_asm_y4f; now 0.98) against 1.45, the x pass
 // 0.56 ms (k_asm_xw) against 0.87; per 256^2 x 32 volume 0.254 / 0.256 and
-// 0.096 / 0.102 ms
-bool use_y2(const AssembleArgs& a) { return !colfft_r1(a.Y) && asm_y2_supported(a); }
-bool use_x2(const AssembleArgs& a)
+// 0.096 / 0.102 ms.  A plan that names another path for the doubled length is
+// followed.
+void assemble_choose(AssembleArgs& a)
 {
-  return !(a.X == 2 * a.nx && (a.X == 1024 || a.X == 512 || a.X == 256)) && asm_x2_supported(a);
+  a.y2 = !colfft_r1(a.Y) && asm_y2_supported(a) && fft_plan_open(kSiteAsmY, a.Y);
+  a.x2 = !(a.X == 2 * a.nx && (a.X == 1024 || a.X == 512 || a.X == 256)) && asm_x2_supported(a) &&
+         fft_plan_open(kSiteAsmX, a.X);
 }
-}  // namespace
 
 int launch_ramp_tables(const FitDev* fit, const AssembleArgs& a, float dxyz, float fact, float2* ex, float2* ey,
                        cudaStream_t s, long long* launches)
@@ -797,7 +798,7 @@ int launch_ramp_tables(const FitDev* fit, const AssembleArgs& a, float dxyz, flo
   const int ndirs = a.ndirs, norders = a.norders, X = a.X, Y = a.Y;
   if (ndirs < 1 || ndirs > kMaxDirs) return -1;
   int n = ndirs * norders * (X + Y);
-  k_ramp<<<std::min(1024, (n + 255) / 256), 256, 0, s>>>(fit, ndirs, norders, X, Y, dxyz, fact, ex, ey, use_x2(a));
+  k_ramp<<<std::min(1024, (n + 255) / 256), 256, 0, s>>>(fit, ndirs, norders, X, Y, dxyz, fact, ex, ey, a.x2);
   if (launches) *launches += 1;
   return (int)cudaGetLastError();
 }
@@ -847,7 +848,7 @@ bool assemble_filter_fusable(const AssembleArgs& a, const FilterArgs& f, bool on
 {
   if (!one_otf || f.bessel || a.ndirs != f.ndirs || a.norders != f.norders) return false;
   if (a.nx != f.nx || a.ny != f.ny || a.nz != f.nz) return false;
-  if (!use_y2(a) && !colfft_r1(a.Y)) return false;
+  if (!a.y2 && !colfft_r1(a.Y)) return false;
   const FilterK k = make_filter_k(f);
   if (!k.order0_shared) return false;
   if (filter_needs_clamp(f, k)) return false;
@@ -899,8 +900,8 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
 
   // one output plane and an x pass that writes real parts: no z pass
   const bool xw = a.X == 2 * a.nx && (a.X == 1024 || a.X == 512 || a.X == 256);
-  const bool x_real = a.Z == 1 && np_out == 1 && (xw || use_x2(a));
-  if (a.X > kAccPerThread * kThreads && !use_x2(a)) return -3;
+  const bool x_real = a.Z == 1 && np_out == 1 && (xw || a.x2);
+  if (a.X > kAccPerThread * kThreads && !a.x2) return -3;
   // With the filter in the load, columns beyond the lateral support
   // (filtered_rows' sqrtf(kx^2 + ky^2) > rdistcutoff, whatever ky) are zero, an
   // eighth of them at 1.42 NA, 528 nm and 80 nm pixels: no filter and no
@@ -935,7 +936,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
     const AssembleArgs& ay = ac;
     KernelTimer* kt = kernel_timer();
     if (kt) kt->begin(s);
-    if (use_y2(a)) {
+    if (a.y2) {
       const int rc = launch_asm_y2(ay, d_slots + first, nsl, filt, s);
       if (rc != 0) return rc;
     } else if (filt) {
@@ -983,7 +984,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
                      s>>>(ax, d_p0 + pi, d_pn + pi, d_slots, d_pz + pi, px.twr, x_real);
     };
     // the warp kernel's prefetch ring holds X/2 = nx columns (zoom factor 2)
-    if (use_x2(a)) {
+    if (a.x2) {
       const int rc = launch_asm_x2(ax, d_slots, d_p0 + pi, d_pn + pi, d_pz + pi, (int)(pj - pi), x_real, s);
       if (rc != 0) return rc;
     } else if (a.X == 1024 && a.nx == 512) launch_xw.template operator()<1024>();
@@ -1007,7 +1008,7 @@ int assemble_impl(const AssembleArgs& a, const FilterArgs* filt, cudaStream_t s,
   }
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
-  const int split = use_x2(a);
+  const int split = a.x2;
   const int zr1 = a.Z % 16 == 0 ? a.Z / 16 : 0;
   if (a.Z == 1 && !split && ((size_t)a.X * a.Y) % 2 == 0) {
     const size_t npairs = (size_t)a.X * a.Y / 2;

@@ -320,6 +320,9 @@ struct AssembleArgs {
   const float2* bands;  // all directions [ndirs][nph][nz][ny][nxh]
   int ndirs, norders, nphases, nx, ny, nz;
   int X, Y, Z;          // zoomed output grid
+  // the x (y) pass takes the doubled-grid kernels (assemble_choose): decided once
+  // a volume, as the columns of ex and S, and the filter's place, depend on it
+  int x2, y2;
   int zdc[kMaxOrders];  // in-band planes of each order after filtering
   const float2* ex;     // [ndirs*norders][X] phase-ramp factors along x
   const float2* ey;     // [ndirs*norders][Y]
@@ -339,6 +342,8 @@ size_t assemble_tables_bytes(const AssembleArgs& a);
 // Writes the tables of `a` into a.tables (synchronous copy; call outside the
 // timed/captured work, again whenever zdc changes).
 int assemble_tables_upload(const AssembleArgs& a);
+// sets a.x2 and a.y2 from the geometry and the FFT plan
+void assemble_choose(AssembleArgs& a);
 int launch_assemble(const AssembleArgs& a, cudaStream_t s, long long* launches);
 // Filter and assembly in one pass: the Wiener filter of every direction
 // applied in the assembly's band load (the bands are left unfiltered in

@@ -804,7 +804,8 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
   TfPlan tx, ty;
   const TfKernels* kx = fft_two_factor(kSiteMakeOtf, nx) ? tf_kernels(nx, &tx) : nullptr;
   const TfKernels* ky = fft_two_factor(kSiteMakeOtf, ny) ? tf_kernels(ny, &ty) : nullptr;
-  const bool tf = kx && kx->mo_rows && ky && (nz == 1 || z_length_ok(nz));
+  const bool zn = nz == 1 || (z_length_ok(nz) && fft_plan_open(kSiteMakeOtf, nz));
+  const bool tf = kx && kx->mo_rows && ky && zn;
   const int pitch = tf ? nxh : nx;
   // host-side constants with the reference's float arithmetic
   ApoFact fact;

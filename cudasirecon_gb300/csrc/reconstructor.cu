@@ -1553,6 +1553,20 @@ void SIM_Reconstructor::prepare_asm_tables()
   asm_tables_valid_ = true;
 }
 
+// The assembly's kernels of one volume (another thread may record a plan in
+// the middle of it)
+void SIM_Reconstructor::choose_assembly()
+{
+  AssembleArgs a{};
+  a.nx = nx_;
+  a.ny = ny_;
+  a.X = X_;
+  a.Y = Y_;
+  assemble_choose(a);
+  asm_x2_ = a.x2;
+  asm_y2_ = a.y2;
+}
+
 // The arguments of the filter and the assembly.  What depends on the fitted k0
 // is the host's; the fused filter takes it from the device fit results instead.
 void SIM_Reconstructor::filter_args(FilterArgs& fa, AssembleArgs& aa) const
@@ -1616,6 +1630,8 @@ void SIM_Reconstructor::filter_args(FilterArgs& fa, AssembleArgs& aa) const
   aa.ey = d_ey_;
   aa.T = d_T_;
   aa.tcap = tcap_;
+  aa.x2 = asm_x2_;
+  aa.y2 = asm_y2_;
   aa.S = d_S_;
   aa.out = d_out_;
   aa.tables = d_asmtab_;
@@ -1676,6 +1692,7 @@ int SIM_Reconstructor::process_one_volume(bool sync)
   separate();
   // with the fused filter nothing up to the result needs the fit on the host
   // (and the bands stay as they are): one synchronisation at the end
+  choose_assembly();
   FilterArgs fa{};
   AssembleArgs aa{};
   filter_args(fa, aa);
@@ -1782,6 +1799,7 @@ bool SIM_Reconstructor::capture_volume(int b, void* raw, float* out, int t, cuda
     g.exec = nullptr;
   }
   prepare_asm_tables();  // synchronous upload, outside the capture
+  choose_assembly();
   d_raw_ = raw;
   d_out_ = out;
   const long long l0 = launches_;
@@ -2160,11 +2178,13 @@ static const char* site_kernel(int site)
   }
 }
 
-// the sites that have a two-factor kernel next to the other two paths
+// the sites that have a two-factor kernel next to the other two paths (the
+// assembly's lengths are the doubled grid's)
 static bool fft_two_factor_site(int site, int n)
 {
   int r1, r2;
-  return site != kSiteSeparateZ && site != kSiteAsmY && site != kSiteAsmX && site != kSiteAsmZ && tf_factor(n, &r1, &r2);
+  if (site == kSiteSeparateZ || site == kSiteAsmZ) return false;
+  return (site == kSiteAsmY || site == kSiteAsmX) ? n % 4 == 0 && tf_factor(n / 2, &r1, &r2) : tf_factor(n, &r1, &r2);
 }
 
 // Measure, for every (FFT site, length) a volume of this handle queries and
@@ -2203,12 +2223,20 @@ std::string SIM_Reconstructor::tune_fft(int reps)
           profile_json();
           profiling_ = false;
           fft_site_unforce();
-          auto it = kprof_.find(kname);
-          if (it != kprof_.end()) best[path] = std::min(best[path], it->second.ms);
+          // (y assembly: the filter runs inside the two-factor kernel, else before)
+          std::vector<const char*> kernels = {kname};
+          if (site == kSiteAsmY) kernels.insert(kernels.end(), {"k_asm_y_filter", "k_filter"});
+          double ms = 0;
+          for (const char* k : kernels) {
+            auto it = kprof_.find(k);
+            if (it != kprof_.end()) ms += it->second.ms;
+          }
+          if (ms > 0) best[path] = std::min(best[path], ms);
         }
       int path = kPathStockham;
       for (int q = 0; q < kNumFftPaths; ++q)
         if (best[q] <= best[path]) path = q;
+      if (best[path] >= 1e30) continue;  // the site's kernel did not run
       double other = 1e30;
       for (int q = 0; q < kNumFftPaths; ++q)
         if (q != path) other = std::min(other, best[q]);

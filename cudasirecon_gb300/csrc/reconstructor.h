@@ -110,6 +110,7 @@ class SIM_Reconstructor {
   bool fit_search_on_device(bool defer);
   bool finish_search();
   float filter_rdistcutoff() const;
+  void choose_assembly();
   void filter_args(simrecon::FilterArgs& fa, simrecon::AssembleArgs& aa) const;
   bool filter_fused(const simrecon::FilterArgs& fa, const simrecon::AssembleArgs& aa) const;
   bool one_otf() const { return !opt.p.bOneOTFperAngle || ndirs_otf_ == 1; }
@@ -261,6 +262,7 @@ class SIM_Reconstructor {
   bool raw_staged_ = false;  // d_raw_ holds a stack staged by setRaw/setFile
   bool have_raw_ = false;
   bool rescaled_ = false;
+  int asm_x2_ = 0, asm_y2_ = 0;  // choose_assembly's, for the volume at hand
   bool search_pending_ = false;  // a device search's results are not on the host yet
   static constexpr int kFitHostAt = 320;  // FitHost in h_pinned_, in doubles
   // overlap state for the candidate evaluator

@@ -35,8 +35,11 @@ bool tf_factor(int n, int* r1, int* r2);
 // plan with device twiddles, cached per (device, n); false where n has no pair
 bool get_tf_plan(int n, TfPlan* plan);
 
-// whether `site` takes its two-factor kernel for length n: n has a pair, and
-// neither a force, the environment nor the plan cache names another path
+// neither a force, the environment nor the plan cache names the register path
+// or the Stockham stages for length n at `site`
+bool fft_plan_open(FftSite site, int n);
+// whether `site` takes its two-factor kernel for length n: n has a pair and the
+// plan leaves it
 bool fft_two_factor(FftSite site, int n);
 
 constexpr int kTfSizes[] = {8, 9, 10, 12, 14, 15, 16, 18, 20, 21, 24, 25, 27, 28, 30, 32};
