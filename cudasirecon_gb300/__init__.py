@@ -79,6 +79,8 @@ def load_library(path: str | None = None) -> C.CDLL:
     lib.SRX_fitCounts.argtypes = [vp, C.POINTER(C.c_longlong)]
     lib.SRX_tuneFFT.restype = ip
     lib.SRX_tuneFFT.argtypes = [vp, ip, C.c_char_p, ip]
+    lib.SRX_fftPath.restype = ip
+    lib.SRX_fftPath.argtypes = [ip, ip, C.c_char_p, ip]
     lib.SRX_fftPlanChoice.restype = ip
     lib.SRX_fftPlanChoice.argtypes = [ip, ip, C.c_char_p, ip]
     lib.SRX_setFilterFusion.restype = None
@@ -447,14 +449,29 @@ FFT_SITES = {"ingest_x": 0, "ingest_y": 1, "separate_z": 2, "overlap_x": 3, "ove
              "crosscorr_cols": 6, "assemble_y": 7, "assemble_x": 8, "assemble_z": 9, "makeotf": 10}
 
 
+FFT_PATHS = ("stockham", "register", "two-factor", "compiled")
+
+
+def fft_path(site: str, n: int):
+    """(path, source): the path that the FFT call site runs length n by."""
+    lib = load_library()
+    buf = C.create_string_buffer(64)
+    r = lib.SRX_fftPath(FFT_SITES[site], int(n), buf, len(buf))
+    if r < 0:
+        raise SIReconError("unknown FFT site")
+    return FFT_PATHS[r], buf.value.decode()
+
+
 def fft_plan_choice(site: str, n: int):
-    """(register path?, source) the FFT call site uses for length n."""
+    """(register path?, source): the plan's choice between the register path
+    and the others for length n at the FFT call site.  What the site runs is
+    fft_path's answer: most sites have two-factor or compiled kernels besides."""
     lib = load_library()
     buf = C.create_string_buffer(64)
     r = lib.SRX_fftPlanChoice(FFT_SITES[site], int(n), buf, len(buf))
     if r < 0:
         raise SIReconError("unknown FFT site")
-    return bool(r), buf.value.decode()
+    return r == 1, buf.value.decode()
 
 
 def fft_selftest(x: np.ndarray, inverse: bool = False, columns: bool = False) -> np.ndarray:

@@ -13,6 +13,7 @@
 #include "makeotf.h"
 #include "reconstructor.h"
 #include "server.h"
+#include "tf_fft.cuh"
 
 namespace simrecon {
 int makeotf_main(int argc, const char* const* argv, std::string* err);
@@ -225,6 +226,16 @@ int SRX_fftPlanChoice(int site, int n, char* source, int maxlen)
     source[maxlen - 1] = '\0';
   }
   return r;
+}
+
+int SRX_fftPath(int site, int n, char* source, int maxlen)
+{
+  if (site < 0 || site >= simrecon::kSiteSelfTest || n < 1) return -1;
+  if (source && maxlen > 0) {
+    std::strncpy(source, simrecon::fft_path_source(site, n), (size_t)maxlen - 1);
+    source[maxlen - 1] = '\0';
+  }
+  return simrecon::fft_path((simrecon::FftSite)site, n);
 }
 
 int SRX_lastProcessResult(SIM_Reconstructor* sr) { return need(sr) ? sr->last_process_result() : -1; }

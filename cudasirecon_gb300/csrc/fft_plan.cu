@@ -19,6 +19,7 @@
 #include "kernels.h"
 #include "reg_fft.cuh"
 #include "tf_fft.cuh"
+#include "z_fft.cuh"
 
 namespace simrecon {
 
@@ -101,7 +102,7 @@ namespace {
 const char* const kSiteNames[kNumFftSites] = {"ingest_x", "ingest_y", "separate_z", "overlap_x", "overlap_y",
                                               "crosscorr_rows", "crosscorr_cols", "assemble_y", "assemble_x",
                                               "assemble_z", "makeotf", "selftest"};
-const char* const kPathNames[kNumFftPaths] = {"stockham", "register", "two-factor"};
+const char* const kPathNames[] = {"stockham", "register", "two-factor", "compiled"};
 thread_local int t_force_site = -1, t_force_path = 0;
 thread_local std::set<std::pair<int, int>>* t_seen = nullptr;
 
@@ -256,16 +257,74 @@ bool reg_fft_site_enabled(FftSite site, int n)
   return c >= 0 ? c == kPathRegister : builtin_choice(site, n);
 }
 
-bool fft_two_factor(FftSite site, int n)
+namespace {
+// a kernel compiled for the length, taken whatever the plan says
+bool compiled_at(int site, int n)
+{
+  const bool pow2 = n == 256 || n == 512 || n == 1024;
+  switch (site) {
+    case kSiteIngestX: return pow2;       // k_ingest_xw
+    case kSiteIngestY: return n == 1024;  // k_fft_cols_4s
+    case kSiteOvlY: return n == 512;      // k_ovl_y4
+    case kSiteAsmY:                       // k_asm_y4f, k_asm_y4
+    case kSiteAsmX: return pow2;          // k_asm_xw
+    case kSiteAsmZ: return z_length_ok(n) || n == 80 || n == 96 || n == 128;  // k_asm_zr, k_asm_z2; k_asm_z4
+    case kSiteSeparateZ:                  // k_separate_zn; k_separate4
+      return (z_length_ok(n) && !reg_fft_lanes(n)) || n == 32 || n == 48 || n == 64 || n == 80 || n == 96 || n == 128;
+    default: return false;
+  }
+}
+// a two-factor kernel; *fixed: taken whatever the plan says, in the place of
+// the compiled kernels that these lengths had
+bool two_factor_at(int site, int n, bool* fixed)
 {
   int r1, r2;
-  return tf_factor(n, &r1, &r2) && fft_plan_open(site, n);
+  *fixed = false;
+  switch (site) {
+    case kSiteIngestX: return n % 2 == 0 && tf_factor(n, &r1, &r2);
+    case kSiteIngestY: *fixed = n == 256 || n == 512; break;
+    case kSiteOvlX: *fixed = n == 256 || n == 512 || n == 1024; break;
+    case kSiteOvlY: *fixed = n == 256; break;
+    case kSiteCorrRows:
+    case kSiteCorrCols:
+    case kSiteMakeOtf: break;
+    case kSiteAsmY:
+    case kSiteAsmX: return n % 4 == 0 && tf_factor(n / 2, &r1, &r2);
+    default: return false;
+  }
+  return tf_factor(n, &r1, &r2);
+}
+}  // namespace
+
+bool fft_two_factor_choice(FftSite site, int n)
+{
+  bool fixed;
+  return !compiled_at(site, n) && two_factor_at(site, n, &fixed) && !fixed;
+}
+
+int fft_path(FftSite site, int n)
+{
+  bool fixed;
+  if (compiled_at(site, n)) return kPathCompiled;
+  if (two_factor_at(site, n, &fixed) && (fixed || fft_plan_open(site, n))) return kPathTwoFactor;
+  return reg_fft_lanes(n) && reg_fft_site_enabled(site, n) ? kPathRegister : kPathStockham;
+}
+
+// where fft_path's answer comes from: the plan's source only where a plan has a
+// say
+const char* fft_path_source(int site, int n)
+{
+  bool fixed;
+  if (compiled_at(site, n) || !reg_fft_lanes(n) || (two_factor_at(site, n, &fixed) && fixed)) return "built-in";
+  const char* src = "";
+  fft_plan_choice(site, n, &src);
+  return src;
 }
 
 void fft_site_force(int site, int path) { t_force_site = site, t_force_path = path; }
 void fft_site_unforce() { t_force_site = -1; }
 void fft_sites_track(std::set<std::pair<int, int>>* seen) { t_seen = seen; }
-const char* fft_path_name(int path) { return path >= 0 && path < kNumFftPaths ? kPathNames[path] : "?"; }
+const char* fft_path_name(int path) { return path >= 0 && path <= kPathCompiled ? kPathNames[path] : "?"; }
 const char* fft_site_name(int site) { return site >= 0 && site < kNumFftSites ? kSiteNames[site] : "?"; }
 
 bool fft_plan_record(int site, int n, int path, double ms, double ms_other, std::string* err)
@@ -276,8 +335,10 @@ bool fft_plan_record(int site, int n, int path, double ms, double ms_other, std:
   return save_tuned(err);
 }
 
-// 1 register path, 0 Stockham stages; *source: "forced", "environment",
-// "tuned", "built-in" or "stockham-only" (no register path for n)
+// The plan's choice: 1 register path, 0 Stockham stages, 2 (forced or recorded)
+// two-factor kernel; *source: "forced", "environment", "tuned", "built-in" (which
+// of the first two, where the site has no other kernel for n) or
+// "stockham-only" (no register path for n)
 int fft_plan_choice(int site, int n, const char** source)
 {
   const char* src = "built-in";
@@ -288,7 +349,7 @@ int fft_plan_choice(int site, int n, const char** source)
     r = 0;
   } else if (t_force_site == site) {
     src = "forced";
-    r = t_force_path == kPathRegister;
+    r = t_force_path;
   } else if (std::getenv("SIMRECON_FFT_REGISTER_SITES")) {
     src = "environment";
     r = reg_fft_site_enabled((FftSite)site, n);
@@ -298,7 +359,7 @@ int fft_plan_choice(int site, int n, const char** source)
     auto it = g_tuned.table.find({device_name(), site, n});
     if (it != g_tuned.table.end()) {
       src = "tuned";
-      r = it->second.first == kPathRegister;
+      r = it->second.first;
     } else {
       r = builtin_choice((FftSite)site, n);
     }

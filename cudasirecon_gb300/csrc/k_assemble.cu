@@ -787,9 +787,8 @@ int launch_filter(const FilterArgs& a, cudaStream_t s, long long* launches)
 // followed.
 void assemble_choose(AssembleArgs& a)
 {
-  a.y2 = !colfft_r1(a.Y) && asm_y2_supported(a) && fft_plan_open(kSiteAsmY, a.Y);
-  a.x2 = !(a.X == 2 * a.nx && (a.X == 1024 || a.X == 512 || a.X == 256)) && asm_x2_supported(a) &&
-         fft_plan_open(kSiteAsmX, a.X);
+  a.y2 = asm_y2_supported(a) && fft_path(kSiteAsmY, a.Y) == kPathTwoFactor;
+  a.x2 = asm_x2_supported(a) && fft_path(kSiteAsmX, a.X) == kPathTwoFactor;
 }
 
 int launch_ramp_tables(const FitDev* fit, const AssembleArgs& a, float dxyz, float fact, float2* ex, float2* ey,

@@ -654,19 +654,19 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   // Its radial tables need every kz index inside the OTF (otf_kz's wrapped one
   // is negative where |kz| exceeds the OTF's extent, a PSF step of more than
   // 1 / (axial cutoff)); k_ovl_build_x's lookups clamp at both ends.
-  const bool reg_row = a.nx == 256 || a.nx == 512 || a.nx == 1024;
   const bool kz_inside = a.zdc * a.otf.kzscale <= a.otf.nzotf;
   TfPlan tx, ty;
-  const TfKernels* kx = kz_inside && a.otf.nxotf <= kOvlTabMax && (reg_row || fft_two_factor(kSiteOvlX, a.nx))
+  const TfKernels* kx = kz_inside && a.otf.nxotf <= kOvlTabMax && fft_path(kSiteOvlX, a.nx) == kPathTwoFactor
                             ? tf_kernels(a.nx, &tx)
                             : nullptr;
   // 512 rows keep the compiled column kernel (0.209 against 0.270 ms per
   // 512^2 x 48 volume); 256 rows are as fast either way (0.078, 0.076), 1024
   // took the Stockham stages (1.25 a pair of 1024^2 x 64 against 0.26)
-  const TfKernels* ky = a.ny == 256 || (a.ny != 512 && fft_two_factor(kSiteOvlY, a.ny)) ? tf_kernels(a.ny, &ty) : nullptr;
+  const int ypath = fft_path(kSiteOvlY, a.ny);
+  const TfKernels* ky = ypath == kPathTwoFactor ? tf_kernels(a.ny, &ty) : nullptr;
   // 1) build + x inverse FFT
   // the Stockham y stage reads every row
-  a.skip_rows = !a.all_rows && (a.ny == 512 || ky);
+  a.skip_rows = !a.all_rows && (ypath == kPathCompiled || ky);
   const int ldl = a.nx + 1;
   int rows = std::max(1, kMaxElems / (2 * a.nx));
   rows = std::min(rows, nzb * a.ny);
@@ -697,7 +697,7 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
   const size_t fsm = fft_stage_smem(a.ny, 2 * W, tile, threads);
   const int xoff = (int)(fsm / sizeof(float2));
   size_t sm2 = fsm + (size_t)a.ny * W * sizeof(float2);
-  if (a.ny == 512) {
+  if (ypath == kPathCompiled) {
     // 8 columns per CTA; plane groups so that the grid covers the GPU
     tiles = (a.nx + 7) / 8;
     groups = std::max(1, std::min(nzb, (4 * 152 + ni * tiles - 1) / (ni * tiles)));
@@ -715,7 +715,7 @@ int launch_overlaps(OverlapArgs& a, cudaStream_t s, long long* launches)
     allow_dynamic_smem((const void*)k_ovl_y4<N, R1>, bytes);
     k_ovl_y4<N, R1><<<dim3(tiles, groups, ni), kThreads, bytes, s>>>(a, py.tw, ppg);
   };
-  if (a.ny == 512) go4.template operator()<512, 32>();
+  if (ypath == kPathCompiled) go4.template operator()<512, 32>();
   else if (ky) {
     const int rc = ky->ovl_y(a, ty, ppg, groups, s);
     if (rc != 0) return rc;
@@ -744,8 +744,8 @@ int launch_crosscorr_peak(const float2* pmap, int n, float2* cc, int nx, int ny,
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
   TfPlan tx, ty;
-  const TfKernels* kx = fft_two_factor(kSiteCorrRows, nx) ? tf_kernels(nx, &tx) : nullptr;
-  const TfKernels* ky = fft_two_factor(kSiteCorrCols, ny) ? tf_kernels(ny, &ty) : nullptr;
+  const TfKernels* kx = fft_path(kSiteCorrRows, nx) == kPathTwoFactor ? tf_kernels(nx, &tx) : nullptr;
+  const TfKernels* ky = fft_path(kSiteCorrCols, ny) == kPathTwoFactor ? tf_kernels(ny, &ty) : nullptr;
   if (kx) {
     const int rc = kx->fft_rows_conj(pmap, cc, rows, tx, s);
     if (rc != 0) return rc;

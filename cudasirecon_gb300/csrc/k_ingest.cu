@@ -450,12 +450,13 @@ int launch_ingest_x(const IngestArgs& a, cudaStream_t s, long long* launches)
     }
   };
   TfPlan tx;
-  const bool wx = a.nx == 512 || a.nx == 1024 || a.nx == 256;  // warp kernels
-  const TfKernels* kx = !wx && fft_two_factor(kSiteIngestX, a.nx) ? tf_kernels(a.nx, &tx) : nullptr;
-  if (a.nx == 512) go_w.template operator()<512>();
-  else if (a.nx == 1024) go_w.template operator()<1024>();
-  else if (a.nx == 256) go_w.template operator()<256>();
-  else if (kx && kx->ingest_x) {
+  const int path = fft_path(kSiteIngestX, a.nx);
+  const TfKernels* kx = path == kPathTwoFactor ? tf_kernels(a.nx, &tx) : nullptr;
+  if (path == kPathCompiled) {
+    if (a.nx == 512) go_w.template operator()<512>();
+    else if (a.nx == 1024) go_w.template operator()<1024>();
+    else go_w.template operator()<256>();
+  } else if (kx && kx->ingest_x) {
     const int rc = kx->ingest_x(a, tx, s);
     if (rc != 0) return rc;
   } else
@@ -493,15 +494,14 @@ int launch_ingest_y(const IngestArgs& a, int plane0, int nplanes, cudaStream_t s
   TfPlan ty;
   // 1024 rows keep their compiled kernel: 1.72 against 1.93 ms per 1024^2 x 64
   // volume (256 rows: 0.046 two-factor against 0.057 ms per 256^2 x 32)
-  const TfKernels* ky = a.ny == 512 || a.ny == 256 || (a.ny != 1024 && fft_two_factor(kSiteIngestY, a.ny))
-                            ? tf_kernels(a.ny, &ty)
-                            : nullptr;
+  const int path = fft_path(kSiteIngestY, a.ny);
+  const TfKernels* ky = path == kPathTwoFactor ? tf_kernels(a.ny, &ty) : nullptr;
   int W = std::max(1, std::min(32, kMaxElems / a.ny));
   size_t smy = fft_smem(a.ny, W, a.ny * (W + 1));
   dim3 gy((nxh + W - 1) / W, nplanes);
   KernelTimer* kt = kernel_timer();
   if (kt) kt->begin(s);
-  if (a.ny == 1024) {
+  if (path == kPathCompiled) {
     const size_t bytes = ColFft<1024, colfft_r1(1024), 8>::kSmemElems * sizeof(float2);
     allow_dynamic_smem((const void*)k_fft_cols_4s<1024>, bytes);
     k_fft_cols_4s<1024><<<dim3((nxh + 7) / 8, nplanes), kThreads, bytes, s>>>(spec, nxh, py.tw);
@@ -700,6 +700,7 @@ int launch_separate(float2* spec, const float* scale, const float* sepmat, int n
       default: go.template operator()<8>(); break;
     }
   } else if (z_length_ok(nz) && !reg_fft_lanes(nz) && (nphases == 3 || nphases == 5)) {
+    // (3 phases: a length with a register path keeps the path that the plan names)
     const int rc = launch_separate_z(spec, scale, sepmat, (size_t)ny * nxh, nz, ndirs, nphases, pz.tw, s);
     if (rc != 0) return rc;
   } else {

@@ -40,7 +40,9 @@ bool fft_radix_plan(int n, int* radix, int* nstages);
 // or where a site has them the two-factor kernels).  The tuner forces a choice on the calling thread, tracks which
 // (site, length) pairs a run queries, and records measured choices in the
 // on-disk plan cache that every process reads.
-enum : int { kPathStockham = 0, kPathRegister = 1, kPathTwoFactor = 2, kNumFftPaths = 3 };
+// kPathCompiled: a kernel compiled for the length, taken whatever the plan says
+// (never recorded).
+enum : int { kPathStockham = 0, kPathRegister = 1, kPathTwoFactor = 2, kNumFftPaths = 3, kPathCompiled = 3 };
 const char* fft_path_name(int path);
 void fft_site_force(int site, int path);
 void fft_site_unforce();
@@ -48,6 +50,7 @@ void fft_sites_track(std::set<std::pair<int, int>>* seen);  // nullptr stops tra
 const char* fft_site_name(int site);
 bool fft_plan_record(int site, int n, int path, double ms, double ms_other, std::string* err);
 int fft_plan_choice(int site, int n, const char** source);
+const char* fft_path_source(int site, int n);
 std::string fft_plan_cache_path();
 
 // -------------------------------------------------------------------- ingest
@@ -83,7 +86,7 @@ int launch_ingest_y(const IngestArgs& a, int plane0, int nplanes, cudaStream_t s
 // extra background, then deskewOneSection (1733-1760): a shift along x that
 // grows with z (linear interpolation), or, without deskew, the first nx
 // columns.  out = [nimg][ny][nx] float in raw section order, ready for
-// launch_ingest with no background, unit slope and unit scale.
+// launch_ingest_x with no background, unit slope and unit scale.
 struct PrecondArgs {
   const void* raw;  // [nimg][ny][nx_raw] uint16 or float
   int raw_is_u16;

@@ -802,8 +802,8 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
   // throughout (separation and transforms 57 us at 128^2 x 64 x 5); any other
   // by full rows in shared-memory stages (136 us there).
   TfPlan tx, ty;
-  const TfKernels* kx = fft_two_factor(kSiteMakeOtf, nx) ? tf_kernels(nx, &tx) : nullptr;
-  const TfKernels* ky = fft_two_factor(kSiteMakeOtf, ny) ? tf_kernels(ny, &ty) : nullptr;
+  const TfKernels* kx = fft_path(kSiteMakeOtf, nx) == kPathTwoFactor ? tf_kernels(nx, &tx) : nullptr;
+  const TfKernels* ky = fft_path(kSiteMakeOtf, ny) == kPathTwoFactor ? tf_kernels(ny, &ty) : nullptr;
   const bool zn = nz == 1 || (z_length_ok(nz) && fft_plan_open(kSiteMakeOtf, nz));
   const bool tf = kx && kx->mo_rows && ky && zn;
   const int pitch = tf ? nxh : nx;

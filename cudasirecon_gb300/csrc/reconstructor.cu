@@ -2178,15 +2178,6 @@ static const char* site_kernel(int site)
   }
 }
 
-// the sites that have a two-factor kernel next to the other two paths (the
-// assembly's lengths are the doubled grid's)
-static bool fft_two_factor_site(int site, int n)
-{
-  int r1, r2;
-  if (site == kSiteSeparateZ || site == kSiteAsmZ) return false;
-  return (site == kSiteAsmY || site == kSiteAsmX) ? n % 4 == 0 && tf_factor(n / 2, &r1, &r2) : tf_factor(n, &r1, &r2);
-}
-
 // Measure, for every (FFT site, length) a volume of this handle queries and
 // the register path supports, the site's kernel time with the register path
 // and with the Stockham stages, on the staged raw stack (each run restarts
@@ -2215,7 +2206,7 @@ std::string SIM_Reconstructor::tune_fft(int reps)
       std::fill(best, best + kNumFftPaths, 1e30);
       for (int rep = 0; rep < std::max(1, reps); ++rep)
         for (int path = 0; path < kNumFftPaths; ++path) {
-          if (path == kPathTwoFactor && !fft_two_factor_site(site, n)) continue;
+          if (path == kPathTwoFactor && !fft_two_factor_choice((FftSite)site, n)) continue;
           fft_site_force(site, path);
           profiling_ = true;
           reset_profile();

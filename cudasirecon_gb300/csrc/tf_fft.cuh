@@ -35,15 +35,17 @@ bool tf_factor(int n, int* r1, int* r2);
 // plan with device twiddles, cached per (device, n); false where n has no pair
 bool get_tf_plan(int n, TfPlan* plan);
 
+// The path that `site` runs length n by: what the launchers take and what
+// SRX_fftPath reports.  The lengths of the assembly's x and y sites are those of
+// the doubled grid, the z separation's those of 5-phase stacks.
+int fft_path(FftSite site, int n);
 // neither a force, the environment nor the plan cache names the register path
 // or the Stockham stages for length n at `site`
 bool fft_plan_open(FftSite site, int n);
-// whether `site` takes its two-factor kernel for length n: n has a pair and the
-// plan leaves it
-bool fft_two_factor(FftSite site, int n);
+// whether `site` has a two-factor kernel for length n that a plan may choose
+bool fft_two_factor_choice(FftSite site, int n);
 
 constexpr int kTfSizes[] = {8, 9, 10, 12, 14, 15, 16, 18, 20, 21, 24, 25, 27, 28, 30, 32};
-constexpr int kTfMax = 32;
 // kernel class of a plan: the largest DFT it needs
 inline int tf_class(const TfPlan& p) { return p.r1 <= 16 ? 16 : 32; }
 

@@ -212,19 +212,35 @@ void SRX_fitCounts(SIM_Reconstructor* sr, long long* out3);
 /* No counterpart in the reference.  FFT plan autotuning.  The library's FFT
  * call sites (site ids: 0 ingest x, 1 ingest y, 2 separation z, 3 overlap x,
  * 4 overlap y, 5/6 cross-correlation rows/columns, 7/8/9 assembly y/x/z,
- * 10 makeotf) run a length either with the register path (lengths 32, 48,
- * 64, 96, 128, 256, 512, 1024) or with the shared-memory Stockham stages.
+ * 10 makeotf) have up to four ways to run a length:
+ *   0 the shared-memory Stockham stages (any length),
+ *   1 the register path (lengths 32, 48, 64, 96, 128, 256, 512, 1024),
+ *   2 the two-factor kernels (lengths 64 to 1024 that are a product of two of
+ *     the compiled DFT sizes; at the assembly's y and x sites, whose lengths are
+ *     those of the doubled grid, twice such a length),
+ *   3 a kernel compiled for the length (256, 512, 1024 at some sites, short z).
+ * 3 is taken wherever it exists, and at the overlap rows of 256, 512 and 1024,
+ * overlap columns of 256 and ingest columns of 256 and 512 2 always is.  For the
+ * other lengths of the register path a plan decides between 0, 1 and 2, and
+ * without one 2 is taken where it exists.
  * SRX_tuneFFT runs the handle's staged raw stack (SR_setRaw first) once per
- * choice and repeat for every site and length its volume uses, times the
- * site's kernel with CUDA events, and records the faster choice in the plan
+ * choice and repeat for every such site and length its volume uses, times the
+ * site's kernel with CUDA events, and records the fastest choice in the plan
  * cache file (SIMRECON_FFT_PLAN_CACHE, else ~/.cache/cudasirecon_gb300/
  * fft_plans.tsv; one line per GPU model, site and length) that every process
- * then uses.  It leaves the handle's fit state as after processing that stack
- * at time point 0.  Returns the length of the JSON report written to json
- * (truncated to maxlen), or -1 (SR_getLastError).
- * SRX_fftPlanChoice: 1 register path, 0 Stockham, -1 bad site, with the
- * choice's source ("tuned", "built-in", "environment", "stockham-only"). */
+ * then uses.  A recorded line stays in force until the length is tuned again,
+ * also when the library has since gained a faster path.  It leaves the handle's
+ * fit state as after processing that stack at time point 0.  Returns the length
+ * of the JSON report written to json (truncated to maxlen), or -1
+ * (SR_getLastError).
+ * SRX_fftPath: which of the four runs length n at `site` (z separation: of a
+ * 5-phase stack), -1 bad site; source: "tuned", "environment" or "built-in".
+ * SRX_fftPlanChoice: the plan's choice alone, with its source: 0, 1 or 2 if
+ * "tuned", 0 or 1 if "environment"; "built-in" is the default between 0 and 1
+ * for a site that has neither 2 nor 3 for the length, "stockham-only" a length
+ * without register path; -1 bad site. */
 int SRX_tuneFFT(SIM_Reconstructor* sr, int reps, char* json, int maxlen);
+int SRX_fftPath(int site, int n, char* source, int maxlen);
 int SRX_fftPlanChoice(int site, int n, char* source, int maxlen);
 
 /* No counterpart in the reference.  What the last SR_processOneVolume
