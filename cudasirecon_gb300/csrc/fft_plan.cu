@@ -384,6 +384,8 @@ void allow_dynamic_smem(const void* func, size_t bytes)
   }
 }
 
+cudaError_t default_stream_wait() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 bool fft_length_ok(int n)
 {
   std::vector<int> r;
@@ -419,7 +421,8 @@ bool get_fft_plan(int n, FFTPlan* plan)
   }
   float2* d = nullptr;
   if (cudaMalloc(&d, sizeof(float2) * 2 * n) != cudaSuccess) return false;
-  if (cudaMemcpy(d, tw.data(), sizeof(float2) * 2 * n, cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (cudaMemcpy(d, tw.data(), sizeof(float2) * 2 * n, cudaMemcpyHostToDevice) != cudaSuccess ||
+      default_stream_wait() != cudaSuccess) {
     cudaFree(d);
     return false;
   }
@@ -469,7 +472,8 @@ bool get_tf_plan(int n, TfPlan* plan)
       }
   float2* d = nullptr;
   if (cudaMalloc(&d, sizeof(float2) * tw.size()) != cudaSuccess) return false;
-  if (cudaMemcpy(d, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (cudaMemcpy(d, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+      default_stream_wait() != cudaSuccess) {
     cudaFree(d);
     return false;
   }

@@ -836,6 +836,7 @@ int assemble_tables_upload(const AssembleArgs& a)
   put(d.pn, t.pn.data(), t.pn.size() * sizeof(int));
   put(d.pz, t.pzo.data(), t.pzo.size() * sizeof(int));
   put(d.zact, t.zact.data(), t.zact.size());
+  if (e == cudaSuccess) e = default_stream_wait();
   return (int)e;
 }
 

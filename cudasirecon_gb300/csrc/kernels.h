@@ -76,6 +76,11 @@ struct IngestArgs {
 // launch.
 void allow_dynamic_smem(const void* func, size_t bytes);
 
+// Waits for the copies and fills made through the default stream.  cudaMemcpy
+// from pageable memory may return before its last bytes are on the device, and
+// cudaMemset always may; the handles' streams do not wait for the default one.
+cudaError_t default_stream_wait();
+
 // flat-field + apodize + x half of the 2D R2C FFT of raw planes into spec
 int launch_ingest_x(const IngestArgs& a, cudaStream_t s, long long* launches);
 // the y half, in place, of planes plane0 .. plane0 + nplanes - 1

@@ -553,6 +553,7 @@ bool SIM_Reconstructor::setup(int nx, int ny, int nimages, int nwaves, const Sta
   check(cudaMemset(d_fitslots_, 0, (size_t)kMaxDirs * kMaxOrders * 4 * sizeof(double)), "memset");
   if (precondition_) check(cudaMemset(d_bgx_, 0, (size_t)nimg_ * sizeof(float)), "memset");
   if (p.bBgInExtHdr) ensure_precondition_buffers();
+  check(default_stream_wait(), "upload");
   check_launch(upload_amps(), "fit init");
   check(cudaStreamSynchronize(stream_), "fit init");
   if (p.bUsecorr && !load_corr(err)) return false;
@@ -1756,6 +1757,7 @@ bool SIM_Reconstructor::load_corr(std::string* err)
   if (!d_bgslope_) check(cudaMalloc((void**)&d_bgslope_, 2 * n * sizeof(float)), "calibration buffer");
   check(cudaMemcpy(d_bgslope_, bg.data(), n * sizeof(float), cudaMemcpyHostToDevice), "calibration upload");
   check(cudaMemcpy(d_bgslope_ + n, sl.data(), n * sizeof(float), cudaMemcpyHostToDevice), "calibration upload");
+  check(default_stream_wait(), "calibration upload");
   return true;
 }
 
@@ -1986,6 +1988,7 @@ void SIM_Reconstructor::ensure_precondition_buffers()
   d_pre_ = pre_own_;
   d_bgx_ = pre_own_ + npre;
   check(cudaMemset(d_bgx_, 0, (size_t)nimg_ * sizeof(float)), "memset");
+  check(default_stream_wait(), "memset");
   series_bytes_ += npre * sizeof(float) + (size_t)nimg_ * sizeof(float);
 }
 
@@ -2294,6 +2297,7 @@ void SIM_Reconstructor::set_file(int it, int iw)
       }
       check(cudaMemcpy(d_bgx_, bgx_host_.data(), (size_t)nimg_ * sizeof(float), cudaMemcpyHostToDevice),
             "section backgrounds");
+      check(default_stream_wait(), "section backgrounds");
     }
     stage_raw(all.data(), false);
   }
