@@ -1358,8 +1358,6 @@ bool SIM_Reconstructor::fit_search_on_device(bool defer)
   ff.host = (FitHost*)(dh_pinned_ + kFitHostAt);
   ff.info = d_sinfo_;
   check_launch(launch_fit_finish(d_fitslots_, ff, d_fit_, stream_, &launches_), "fit results");
-  // the count of builds takes a searched volume's twice, as it always has
-  fit_counts_[0] += 2 * ndirs_ + (long long)rest.size();
   fit_counts_[1] += reductions;
   fit_counts_[2] += ndirs_;
   cur_o1_ = cur_o2_ = -1;
