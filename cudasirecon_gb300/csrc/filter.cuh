@@ -80,8 +80,18 @@ inline bool filter_needs_clamp(const FilterArgs& a, const FilterK& k)
 // the reference index rows as y in [-ny/2, ny/2 - 1]).
 struct FilterRows {
   int ky[2];
-  float yf[2], rd[2];  // rd: the radius at which the pixel's own OTF is looked up
-  bool in[2];          // a row of the image, inside the support
+  float yf[2], rd[2];
+  bool in[2];  // a row of the image, inside the support
+  // The radii at which the pixels' own OTF is looked up.  A pixel outside goes
+  // through the filter with its neighbour and is dropped there; it can lie dky
+  // beyond the support, more bins than filter_needs_clamp leaves where the image
+  // is short against the OTF, so its lookup stays at the edge.  (Formed where it
+  // is used: held in rd, the pass of 640 x 384 x 30 took 0.670 instead of
+  // 0.641 ms.)
+  __host__ __device__ __forceinline__ float2 own(float cutoff) const
+  {
+    return make_float2(fminf(rd[0], cutoff), fminf(rd[1], cutoff));
+  }
 };
 __host__ __device__ __forceinline__ FilterRows filter_rows(float dky, float cutoff, int ny, float x1f, int r0)
 {
@@ -94,14 +104,8 @@ __host__ __device__ __forceinline__ FilterRows filter_rows(float dky, float cuto
     p.ky[i] = r <= ny / 2 ? r : r - ny;
     const int kyf = p.ky[i] == ny / 2 ? -(ny / 2) : p.ky[i];
     p.yf[i] = kyf * dky;
-    const float rd = sqrtf(x1f * x1f + p.yf[i] * p.yf[i]);
-    const bool inside = rd <= cutoff;
-    p.in[i] = r < ny && inside;
-    // A pixel outside goes through the filter with its neighbour and is dropped
-    // there.  It can lie dky beyond the support, more bins than
-    // filter_needs_clamp leaves where the image is short against the OTF, so
-    // its lookup stays at the edge.
-    p.rd[i] = inside ? rd : cutoff;
+    p.rd[i] = sqrtf(x1f * x1f + p.yf[i] * p.yf[i]);
+    p.in[i] = r < ny && p.rd[i] <= cutoff;
   }
   return p;
 }
@@ -122,7 +126,9 @@ struct FilterTerms {
 // values alone: with the step to the next bin beside each (one 16-byte load a
 // lookup) the tables took twice the space and twice the building, the fused
 // kernels lost a CTA per SM from 66 bins on, and 512^2 x 48 took 1.23 ms at 129
-// bins and 2.51 at 513, against 1.02 and 1.41 (0.98 either way at 65).
+// bins and 2.51 at 513, against 1.02 and 1.41.  At 65 bins the wider entries cost
+// or gained little: 0.98 either way there, 1024^2 x 8 0.76 against 0.78 with
+// values, 640 x 384 x 30 0.66 against 0.64.
 inline size_t filter_tab_bytes(int norders, int nxotf) { return 2 * (size_t)norders * nxotf * sizeof(float2); }
 // The fused kernels' tables at most: with the transform buffer of 1024 rows two
 // CTAs stay resident on an SM (three up to 129 bins and three orders)
@@ -493,7 +499,7 @@ __device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const Filter
   if (z < 0) z += f.nz;
   const FilterRows p = filter_rows(fa.dky, fa.rdistcutoff, f.ny, x1f, r0);
   const int(&ky)[2] = p.ky;
-  const float(&yf)[2] = p.yf, (&rd)[2] = p.rd;
+  const float(&yf)[2] = p.yf;
   const bool(&in)[2] = p.in;
   size_t ind[2];
 #pragma unroll
@@ -517,7 +523,7 @@ __device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const Filter
       if (in[1]) b1 = cadd(b1, f.br[d * f.dstride + ind[1]]);
     }
     float2 s0, s1;
-    filter_scale_pair(fa, fk, terms, f, zs, make_float2(rd[0], rd[1]), xs, ys, tz, s0, s1);
+    filter_scale_pair(fa, fk, terms, f, zs, p.own(fa.rdistcutoff), xs, ys, tz, s0, s1);
     v0 = cmul(b0, s0);
     v1 = cmul(b1, s1);
     if (conj) {
@@ -529,7 +535,7 @@ __device__ __forceinline__ void filtered_rows(const FilterArgs& fa, const Filter
     float2 re0 = in[0] ? f.br[ind[0]] : zero, im0 = in[0] ? f.bi[ind[0]] : zero;
     float2 re1 = in[1] ? f.br[ind[1]] : zero, im1 = in[1] ? f.bi[ind[1]] : zero;
     float2 s0, s1;
-    filter_scale_pair(fa, fk, terms, f, f.kz, make_float2(rd[0], rd[1]), x1f, make_float2(yf[0], yf[1]), tab, s0, s1);
+    filter_scale_pair(fa, fk, terms, f, f.kz, p.own(fa.rdistcutoff), x1f, make_float2(yf[0], yf[1]), tab, s0, s1);
     if (conj) {
       re0.y = -re0.y;
       im0.y = -im0.y;

@@ -387,15 +387,9 @@ __device__ __forceinline__ void tile_reduce(const float2 (&acc)[CC], float* sacc
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
     pair_add(s, e, __shfl_xor_sync(0xffffffffu, s, o), __shfl_xor_sync(0xffffffffu, e, o));
-  double total = (double)s + (double)e;
-  if (!isfinite(s)) {  // (every lane's) past the float range: once more in double
-    total = 0.0;
-#pragma unroll
-    for (int i = 0; i < kSW; ++i) total += (double)x[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-  }
-  if (lane == 0) lead->red[rank][c0 + (v >> 1)][v & 1] = total;
+  // (a sum past the float range that a double would hold does not get here: the
+  // correlation's peak, whose square is a float, is infinite long before)
+  if (lane == 0) lead->red[rank][c0 + (v >> 1)][v & 1] = pair_value(s, e);
 }
 
 template <int CC>

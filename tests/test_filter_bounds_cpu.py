@@ -36,10 +36,9 @@ int main()
             const FilterRows p = filter_rows(a.dky, a.rdistcutoff, ny, kx * a.dkx, r);
             if (!p.in[0] && !p.in[1]) continue;  // neither is looked up
             ++pairs;
-            for (int i = 0; i < 2; ++i) {
-              outside += !p.in[i];
-              worst = std::max(worst, (int)std::floor(p.rd[i] * k.rdkrotf) - (nxotf - 1));
-            }
+            outside += !p.in[0] + !p.in[1];
+            const float2 own = p.own(a.rdistcutoff);
+            for (float r : {own.x, own.y}) worst = std::max(worst, (int)std::floor(r * k.rdkrotf) - (nxotf - 1));
           }
       }
   std::printf("%lld %lld %d\n", pairs, outside, worst);
