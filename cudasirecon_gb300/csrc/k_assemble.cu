@@ -15,9 +15,11 @@
 // exp(i phi_{d,o}(x, y))) with w = 1 for order 0 and 2 otherwise.  The ramp
 // does not depend on z, so the z transform commutes with the sum:
 //     out = Re( IFFTz( S ) ),  S = sum_{d,o} w ramp_{d,o} * IFFTxy(band_{d,o})
-// k_asm_y (pruned, zero-padded y IFFT of every in-band kz plane),
-// k_asm_x (zero-padded x IFFT, ramp, weighted sum over all (d, o) into S)
-// and k_asm_z (one z IFFT of S, real part) write the zoomed output once.
+// A y pass (pruned, zero-padded IFFT of every in-band kz plane, the filter in
+// its load: k_asm_y4f, k_asm_y2), an x pass (IFFT, ramp, weighted sum over all
+// (d, o) into S: k_asm_xw, k_asm_x2) and a z pass (one IFFT of S, real part:
+// k_asm_zn.cu, k_asm_z4) write the zoomed output once.  k_asm_y, k_asm_y4, k_asm_x
+// and k_asm_z are those passes for the grids and plans that the others leave.
 #include <algorithm>
 #include <cmath>
 #include <vector>

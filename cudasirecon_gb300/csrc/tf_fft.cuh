@@ -1,5 +1,6 @@
-// Two-factor transforms of run-time length n = R1 * R2 for the lengths that
-// have no compiled transform of their own.
+// Two-factor transforms of the lengths n = R1 * R2 with both factors among 16
+// compiled DFT sizes: most lengths from 64 to 1024, and 256, 512 and 1024 where
+// their own kernels were slower.
 //
 //   X[k1 + R1 k2] = sum_j W_n^(j k1) W_R2^(j k2) sum_e x[j + R2 e] W_R1^(e k1)
 //
@@ -10,10 +11,11 @@
 // One shared-memory round trip and two barriers per tile, where the Stockham
 // stages make one per radix and two more to fill and empty the tile.
 //
-// R1 and R2 are chosen at run time from a fixed set of compiled DFT sizes
-// (tf_switch: a branch that the whole CTA takes alike), so one kernel serves
-// every length; registers are those of the largest size it may take, hence
-// the two kernel classes MR = 16 and 32.
+// The kernels are compiled per pair (tf_kernels.cuh, instantiated in
+// k_tf_0.cu .. k_tf_7.cu).  k_asm_y2 alone chooses R1 and R2 at run time
+// (tf_switch: a branch that the whole CTA takes alike), as its filter is most of
+// its code; its registers are those of the largest size it may take, hence its
+// two classes MR = 16 and 32.
 //
 // Half-shifted form: the outputs of a transform zero-padded to twice its
 // length fall into two of length n, the even ones of x and the odd ones of
@@ -46,7 +48,7 @@ bool fft_plan_open(FftSite site, int n);
 bool fft_two_factor_choice(FftSite site, int n);
 
 constexpr int kTfSizes[] = {8, 9, 10, 12, 14, 15, 16, 18, 20, 21, 24, 25, 27, 28, 30, 32};
-// kernel class of a plan: the largest DFT it needs
+// k_asm_y2's class of a plan: the largest DFT it needs
 inline int tf_class(const TfPlan& p) { return p.r1 <= 16 ? 16 : 32; }
 
 #ifdef __CUDACC__

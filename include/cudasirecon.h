@@ -250,9 +250,11 @@ int SRX_fftPlanChoice(int site, int n, char* source, int maxlen);
 int SRX_lastProcessResult(SIM_Reconstructor* sr);
 
 /* Wiener filter placement (default on): inside the band load of the
- * assembly's y transform where supported (3 directions, one OTF, zoomed y
- * 256/512/1024), else -- or with on = 0 -- as its own in-place pass over the
- * bands, as the reference's filterbands does.  Both give the same volume
+ * assembly's y transform where supported (one OTF for all directions, not in
+ * Bessel mode, zoomed y 256/512/1024 or twice a length with a two-factor plan,
+ * an OTF that the support stays inside of, of at most 682 radial bins with three
+ * orders), else -- or with on = 0 -- as its own in-place pass over the bands, as
+ * the reference's filterbands does.  Both give the same volume
  * within float rounding.  After SR_processOneVolume the band contents
  * (SRX_getBand) are unspecified. */
 void SRX_setFilterFusion(SIM_Reconstructor* sr, int on);
