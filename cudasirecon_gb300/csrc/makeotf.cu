@@ -512,28 +512,11 @@ struct FinishArgs {
 
 __device__ __forceinline__ float2 c_mulf(float2 a, float f) { return make_float2(__fmul_rn(a.x, f), __fmul_rn(a.y, f)); }
 
-// One CTA per band: symmetry, modify, cleanup and the origin (band 0), in place
-__global__ void __launch_bounds__(1024) k_mo_finish_band(float2* bands, FinishArgs a)
+// One band's part of it
+__device__ __forceinline__ void finish_band(float2* bands, const FinishArgs& a, int p, double* s_sums)
 {
-  __shared__ double s_sums[64];
-  const int nz = a.nz, nb = a.nbins, p = blockIdx.x, order = (p + 1) / 2;
+  const int nz = a.nz, nb = a.nbins, order = (p + 1) / 2;
   float2* avg = bands + (size_t)p * nb * nz;
-  // Hermitian symmetry along kz per bin, a thread per (bin, kz pair)
-  const int half = nz / 2;
-#pragma unroll 4
-  for (int t = threadIdx.x; t < nb * (half + 1); t += blockDim.x) {
-    const int row = t / (half + 1), kz = t - row * (half + 1);
-    float2* r = avg + (size_t)row * nz;
-    if (kz == 0) {
-      r[0].y = 0.f;
-      continue;
-    }
-    float2 u = r[kz], w = r[nz - kz];
-    float2 v = make_float2(__fdiv_rn(__fadd_rn(u.x, w.x), 2.f), __fdiv_rn(__fsub_rn(u.y, w.y), 2.f));
-    r[kz] = v;
-    r[nz - kz] = make_float2(v.x, -v.y);
-  }
-  __syncthreads();
   // modify (radialft.cpp:1169-1186)
   if (a.ifixz) {
     for (int kz = threadIdx.x; kz < nz; kz += blockDim.x)
@@ -541,10 +524,20 @@ __global__ void __launch_bounds__(1024) k_mo_finish_band(float2* bands, FinishAr
     __syncthreads();
   }
   if (a.ifixr) {
-    for (int kx = a.ifixr + threadIdx.x; kx < nb; kx += blockDim.x) {
+    // With one plane the next element along kz is the next bin's, and the last
+    // bin's is the next band's first (after the last band: zero): a bin is
+    // replaced only when the bin before has read it.
+    for (int k0 = a.ifixr; k0 < nb; k0 += blockDim.x) {
+      const int kx = k0 + threadIdx.x;
       float2* row = avg + (size_t)kx * nz;
-      const float2 u = row[1], w = row[nz - 1];
-      row[0] = make_float2(__fdiv_rn(__fadd_rn(u.x, w.x), 2.f), __fdiv_rn(__fadd_rn(u.y, w.y), 2.f));
+      float2 u = make_float2(0.f, 0.f), w = u;
+      if (kx < nb) {
+        if (nz > 1 || kx < nb - 1 || p < a.nph - 1) u = row[1];
+        w = row[nz - 1];
+      }
+      __syncthreads();
+      if (kx < nb)
+        row[0] = make_float2(__fdiv_rn(__fadd_rn(u.x, w.x), 2.f), __fdiv_rn(__fadd_rn(u.y, w.y), 2.f));
     }
     __syncthreads();
   }
@@ -610,6 +603,37 @@ __global__ void __launch_bounds__(1024) k_mo_finish_band(float2* bands, FinishAr
         avg[(size_t)i * nz] = v;
       }
     }
+  }
+}
+
+// Symmetry, modify, cleanup and the origin (band 0), in place: one CTA per band,
+// or one for all of them in turn (one plane with -ifixkr: finish_band)
+__global__ void __launch_bounds__(1024) k_mo_finish_band(float2* bands, FinishArgs a)
+{
+  __shared__ double s_sums[64];
+  const int nz = a.nz, nb = a.nbins;
+  // Hermitian symmetry along kz per bin, a thread per (bin, kz pair)
+  const int half = nz / 2;
+  for (int p = blockIdx.x; p < a.nph; p += gridDim.x) {
+    float2* avg = bands + (size_t)p * nb * nz;
+#pragma unroll 4
+    for (int t = threadIdx.x; t < nb * (half + 1); t += blockDim.x) {
+      const int row = t / (half + 1), kz = t - row * (half + 1);
+      float2* r = avg + (size_t)row * nz;
+      if (kz == 0) {
+        r[0].y = 0.f;
+        continue;
+      }
+      float2 u = r[kz], w = r[nz - kz];
+      float2 v = make_float2(__fdiv_rn(__fadd_rn(u.x, w.x), 2.f), __fdiv_rn(__fsub_rn(u.y, w.y), 2.f));
+      r[kz] = v;
+      r[nz - kz] = make_float2(v.x, -v.y);
+    }
+  }
+  __syncthreads();
+  for (int p = blockIdx.x; p < a.nph; p += gridDim.x) {
+    finish_band(bands, a, p, s_sums);
+    __syncthreads();
   }
 }
 
@@ -988,7 +1012,7 @@ bool makeotf_run(const float* psf, int nx, int ny, int nsec, const MakeOtfOption
   k_mo_shift_comp<<<dim3(8 * 152, nph / 2 + 1), kMoThreads, 0, s>>>(d_bands, d_center, sc);
   k_mo_radial<<<dim3((nbins + 3) / 4, nz, nph), 128, 0, s>>>(d_bands, d_bstart, d_bpix, nbins, nx, ny, nz,
                                                                  pitch, d_avg);
-  k_mo_finish_band<<<nph, 1024, 0, s>>>(d_avg, fa);
+  k_mo_finish_band<<<nz == 1 && o.ifixr ? 1 : nph, 1024, 0, s>>>(d_avg, fa);
   k_mo_finish<<<nout, 1024, 0, s>>>(d_avg, fa, d_out, d_scal);
   cudaEventRecord(ev1, s);
   e = cudaGetLastError();
