@@ -207,7 +207,7 @@ def ncu_limiter(kernel):
         return None
     if not e or "issue_active_pct" not in e:
         return None
-    return {k: e[k] for k in ("issue_active_pct", "dram_throughput_pct", "sm_throughput_pct", "full_capture") if k in e}
+    return {k: e[k] for k in ("issue_active_pct", "dram_throughput_pct", "full_capture", "capture_workload") if k in e}
 
 
 def ncu_limiter_name(kernel):

@@ -358,9 +358,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_asm_y4(AssembleArgs a, const Sl
 // filter (for kz and, for order 0, -kz) follow the transform buffer.
 // Three CTAs per SM (at most 80 registers): the filter phase needs the warps
 // more than the transform stages need registers (1.61 -> 1.31 ms per
-// 512^2 x 48 volume against two CTAs per SM).  Bound by the filter's issue and
-// its instruction fetch: 0.99 ms there with pairs of pixels, per-CTA term lists
-// and the columns beyond the support left out.
+// 512^2 x 48 volume against two CTAs per SM).  Bound by issue (62 % of the slots,
+// the ALU pipe before the FMA pipe) and latency: 0.98 ms there with pairs of
+// pixels, per-CTA term lists and the columns beyond the support left out.
 template <int Y>
 __global__ void __launch_bounds__(kThreads, 3) k_asm_y4f(AssembleArgs a, const Slot* __restrict__ slots,
                                                      const float2* __restrict__ tw,

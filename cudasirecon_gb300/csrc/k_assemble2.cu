@@ -28,11 +28,13 @@ constexpr int kThreads = 256;
 // both parities' stage-1 results then overwrite them, so the tile costs the
 // same shared memory as a doubled column would.  W is 8 where 2 R2 W threads
 // fit in the CTA, else 4 (a 32-byte sector of a row of T).
-// Bound by the filter's issue slots and latency.  Filter + y transform per
-// volume, before (k_filter and the Stockham stages) and now: 1024^2 x 64
-// 25.3 -> 6.2 ms, 640 x 384 x 30 2.87 -> 0.67 ms, 1024 x 960 0.293 -> 0.077 ms.
+// Bound by the filter's issue slots and latency (the register bounds of the two
+// classes spill 52 and 196 bytes a thread around the transforms).  Filter + y
+// transform per volume, before (k_filter and the Stockham stages) and now:
+// 640 x 384 x 30 2.87 -> 0.64 ms, 1024 x 960 0.293 -> 0.080 ms, 1024^2 x 64 25.3 ->
+// 6.2 ms (with tables of values and steps; 2 % more since).
 // At 256/512/1024 output rows the compiled k_asm_y4f stays: 1.31 against
-// 1.45 ms per 512^2 x 48 volume (0.99 now).
+// 1.45 ms per 512^2 x 48 volume (0.98 now).
 template <bool FILT, int MR>
 __global__ void __launch_bounds__(kThreads, MR <= 16 ? 4 : 3) k_asm_y2(AssembleArgs a, const Slot* __restrict__ slots,
                                                                     TfPlan pl, int lw,

@@ -411,6 +411,7 @@ __device__ void chunk(const float2* __restrict__ pmap, int nx, const float2* ex,
 // batch, doubles shuffled through the warps and 8 CTAs; with passes of up to 16
 // candidates over two rows, their tables and segment sums in double each; and
 // now: 128^2 131, 41, 33 us; 512^2 215, 63, 50; 1024 x 960 433, 127, 91 us.
+// (128 registers a thread; passes of 8 spill 28 and 40 bytes at 16 and 8 CTAs.)
 template <int C, int SC>
 __global__ void __launch_bounds__(kST, 1) k_k0_search(const __grid_constant__ K0SearchArgs a, int ntab)
 {
