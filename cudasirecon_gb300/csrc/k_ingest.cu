@@ -700,7 +700,9 @@ int launch_separate(float2* spec, const float* scale, const float* sepmat, int n
       default: go.template operator()<8>(); break;
     }
   } else if (z_length_ok(nz) && !reg_fft_lanes(nz) && (nphases == 3 || nphases == 5)) {
-    // (3 phases: a length with a register path keeps the path that the plan names)
+    // (3 phases: a length with a register path keeps the staged kernel and the
+    // path that the plan names: 32, 48 and 64 sections of 256^2 0.119, 0.154 and
+    // 0.210 ms; k_separate_zn would take 0.032, 0.053 and 0.072)
     const int rc = launch_separate_z(spec, scale, sepmat, (size_t)ny * nxh, nz, ndirs, nphases, pz.tw, s);
     if (rc != 0) return rc;
   } else {
